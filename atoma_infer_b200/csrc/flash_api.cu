@@ -6,14 +6,13 @@
 #include "atoma_flash.h"
 #include "common.cuh"
 #include "mha_params.h"
+#include "workspace_pool.h"
 
 #include <cstdarg>
 #include <atomic>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <string>
-#include <tuple>
 #include <vector>
 
 namespace atoma {
@@ -155,58 +154,44 @@ const DeviceInfo &current_device_info() {
     return di;
 }
 
-void *get_workspace(cudaStream_t stream, size_t bytes, int tag) {
-    struct Buf {
-        void *ptr = nullptr;
-        size_t size = 0;
-    };
-    static std::mutex mu;
-    static std::map<std::tuple<int, int, cudaStream_t>, Buf> bufs;   // (device, tag, stream handle): exact, no hashing
+namespace {
+// report: set the call's status where there is no block.
+void *workspace(cudaStream_t stream, size_t bytes, int tag, bool report) {
+    static WorkspacePool pool;
     int dev = 0;
     cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lock(mu);
-    Buf &b = bufs[std::make_tuple(dev, tag, stream)];
-    if (b.size >= bytes) return b.ptr;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(stream, &cap);
-    if (cap != cudaStreamCaptureStatusNone) {
-        set_status(kErrUnsupported,
-                   "workspace of %zu bytes must be allocated before stream capture: run the op once "
-                   "eagerly on this stream first",
-                   bytes);
-        return nullptr;
-    }
-    if (b.ptr) {
-        // Never free a block that has been handed out: a CUDA graph captured earlier on this stream has
-        // the old pointer baked into its kernel nodes and may be replayed after this call.  The old
-        // block is retired (kept alive until process exit); workspaces grow rarely and only to the
-        // largest shape seen.
-        static std::vector<void *> retired;
-        retired.push_back(b.ptr);
-        b.ptr = nullptr;
-        b.size = 0;
-    }
-    const size_t want = (bytes + (1u << 20) - 1) & ~static_cast<size_t>((1u << 20) - 1);
-    cudaError_t e = cudaMalloc(&b.ptr, want);
-    if (e != cudaSuccess) {
-        set_status(static_cast<int>(e), "workspace cudaMalloc(%zu): %s", want, cudaGetErrorString(e));
-        b.ptr = nullptr;
-        return nullptr;
-    }
-    // Zero-initialised once; users keep it clean (decode arrival counters are self-resetting).
-    cudaMemsetAsync(b.ptr, 0, want, stream);
-    b.size = want;
-    return b.ptr;
-}
-
-void *try_workspace(cudaStream_t stream, size_t bytes, int tag) {
-    void *p = get_workspace(stream, bytes, tag);
-    if (!p) {
-        clear_status();
-        cudaGetLastError();
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaSuccess;
+    size_t asked = bytes;
+    void *p = pool.get(WorkspacePool::Key(dev, tag, stream), bytes, !capturing, [&](size_t size) -> void * {
+        void *block = nullptr;
+        asked = size;
+        e = cudaMalloc(&block, size);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        // Zero-initialised once; users keep it clean (decode arrival counters are self-resetting).
+        cudaMemsetAsync(block, 0, size, stream);
+        return block;
+    });
+    if (!p && report) {
+        if (capturing)
+            set_status(kErrUnsupported,
+                       "workspace of %zu bytes must be allocated before stream capture: run the op once "
+                       "eagerly on this stream first",
+                       bytes);
+        else
+            set_status(static_cast<int>(e), "workspace cudaMalloc(%zu): %s", asked, cudaGetErrorString(e));
     }
     return p;
 }
+}  // namespace
+
+void *get_workspace(cudaStream_t stream, size_t bytes, int tag) { return workspace(stream, bytes, tag, true); }
+void *try_workspace(cudaStream_t stream, size_t bytes, int tag) { return workspace(stream, bytes, tag, false); }
 
 EncodeTiledFn get_encode_tiled() {
     static EncodeTiledFn fn = nullptr;
