@@ -280,7 +280,7 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent
             const bool whole = first == it - (prefix[b + 1] - prefix[b]);
             const int slot = b + cta;   // CTAs and sequences both ascend: no two runs share a slot
             if (part == 0) {
-                alpha_s[h] = l > 0.f ? 1.f / l : 0.f;
+                alpha_s[h] = l == 0.f ? 0.f : 1.f / l;
                 if (!whole && h < H) {
                     partial_ml[(static_cast<int64_t>(slot) * NH + h) * 2] = m_ref;
                     partial_ml[(static_cast<int64_t>(slot) * NH + h) * 2 + 1] = l;
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(NH * 8) latent_decode_merge_kernel(const atoma
     float *out = a.out + (static_cast<int64_t>(a.query_start[b]) * H + h0) * R + col;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-        if (h0 + i < H) out[i * R] = den[i] > 0.f ? num[i] / den[i] : 0.f;
+        if (h0 + i < H) out[i * R] = den[i] == 0.f ? 0.f : num[i] / den[i];   // a NaN sum stays one
 }
 
 size_t ld_smem(int nh, int64_t R, int64_t B) {

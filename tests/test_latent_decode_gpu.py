@@ -60,6 +60,31 @@ def test_against_float64(H, R, out_cols, bs, window, sink, lens):
     assert _lib.lib().atoma_latent_decode_timeouts() == 0
 
 
+@pytest.mark.parametrize("lens", [(4096,), (200,) * 3, (65, 64, 3000)])
+@pytest.mark.parametrize("where", ["query", "cached row"])
+def test_nan_stays_nan(lens, where):
+    """One NaN in a query, or in one cached row: every sum of that head (of all heads) is NaN whether one CTA served the sequence or several whose
+    runs were merged, and the other sequences' are not."""
+    H, R, bs = 8, 192, 16
+    each = [-(-n // bs) for n in lens]
+    table, at = torch.zeros((len(lens), max(each)), dtype=torch.int32), 0
+    for b, n in enumerate(each):
+        table[b, :n] = torch.arange(at, at + n)
+        at += n
+    cache = randn_t((at * bs, R), 1, torch.bfloat16, DEV)
+    q = randn_t((len(lens), H, R), 2, torch.float32, DEV, scale=R ** -0.5)
+    hit, i32 = len(lens) - 1, lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    if where == "query":
+        q[hit, 3, 100] = float("nan")
+    else:
+        cache[int(table[hit, 1]) * bs + 5] = float("nan")
+    out = ops.latent_attention_paged(q.reshape(len(lens), -1), cache, torch.tensor([n - 1 for n in lens], device=DEV), i32(list(range(len(lens)))), table.to(DEV), None, H, R,
+                                     bs, 0, 0.3, 1, query_start=i32(list(range(len(lens) + 1))), max_seq_len=max(lens), out_cols=128)[:, :, :128]
+    want = torch.zeros((len(lens), H), dtype=torch.bool, device=DEV)
+    want[hit, slice(3, 4) if where == "query" else slice(None)] = True
+    assert torch.equal(out.isnan().all(2), want) and torch.equal(out.isnan().any(2), want)
+
+
 @pytest.mark.parametrize("T,H,n,R,row,gated", [(1, 3, 32, 64, 64, False), (33, 2, 64, 192, 256, True), (64, 5, 128, 512, 576, True), (65, 2, 32, 128, 128, False)])
 def test_values_of_a_few_tokens(T, H, n, R, row, gated):
     """Operands rounded to bfloat16 (2^-8 of the input), float32 sums, one rounding of the result; 65 tokens take the general path."""
