@@ -311,8 +311,8 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent
     } else if (warp == 4) {
         // ============================ loads ============================
         // A copy moves eight neighbouring rows: one run of bytes in memory, R / 64 swizzled groups of 1 KiB in shared memory (cp.async, a 16-byte
-        // piece each, kept only some 30 KB of an SM's loads in flight: 2.9 us a tile).  What lies behind a sequence's end is zero: the group that
-        // holds the end goes by plain loads.
+        // piece each, kept only some 30 KB of an SM's loads in flight: 2.9 us a tile).  What lies before a window or behind a sequence's end is zero: the
+        // groups that hold them go by plain loads.
         const __nv_bfloat16 *cache = static_cast<const __nv_bfloat16 *>(a.latent_cache);
         const int bs = static_cast<int>(a.block_size), group_bytes = kLdGroup * R * 2;
         int it = 0;
@@ -337,20 +337,22 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent
                     break;
                 }
                 unsigned char *dst = ring + st * stage_bytes;
-                const int whole = min(kLdKeys, k_hi - j0) / kLdGroup;   // groups inside the sequence
-                for (int g = whole; g < kLdKeys / kLdGroup; ++g) {
+                // Groups [cut, whole) lie inside the keys that are seen.  The others go by plain loads, with zeros for what is not seen: a hidden row's
+                // weight is 0, which does not make a sum of a row that holds an infinity or NaN.
+                const int cut = j0 < k_lo ? 1 : 0, whole = max(cut, min(kLdKeys, k_hi - j0) / kLdGroup);
+                for (int g = cut ? 0 : whole; g < kLdKeys / kLdGroup; g = g == 0 && cut ? whole : g + 1) {
                     const int64_t first = __shfl_sync(0xffffffffu, row, g);
                     for (int i = lane; i < kLdGroup * pieces; i += 32) {
-                        const int r = i / pieces, c = i - r * pieces;
+                        const int r = i / pieces, c = i - r * pieces, key = j0 + g * kLdGroup + r;
                         uint4 v = make_uint4(0, 0, 0, 0);
-                        if (j0 + g * kLdGroup + r < k_hi) v = *reinterpret_cast<const uint4 *>(cache + (first + r) * R + c * 8);
+                        if (key >= k_lo && key < k_hi) v = *reinterpret_cast<const uint4 *>(cache + (first + r) * R + c * 8);
                         *reinterpret_cast<uint4 *>(dst + g * group_bytes + (c >> 3) * 1024 + r * 128 + (((c & 7) ^ r) << 4)) = v;
                     }
                 }
                 fence_proxy_async();   // generic-proxy writes -> visible to the tensor core's async reads
                 __syncwarp();
-                if (elect_one_sync()) mbar_arrive_expect_tx(&full[st], whole * group_bytes);
-                for (int g = 0; g < whole; ++g) {
+                if (elect_one_sync()) mbar_arrive_expect_tx(&full[st], (whole - cut) * group_bytes);
+                for (int g = cut; g < whole; ++g) {
                     const int first = __shfl_sync(0xffffffffu, row, g);
                     if (elect_one_sync()) tma_load_3d(dst + g * group_bytes, &map, &full[st], 0, first, 0);
                     __syncwarp();
