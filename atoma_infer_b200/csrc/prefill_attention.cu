@@ -90,27 +90,28 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
-// 2^x of a pair on the FMA pipe: x = n + f, n the nearest integer (the sum with 1.5 * 2^23 holds it in its low bits), 2^f by a degree-4
-// polynomial, the least-maximum fit over [-1/2, 1/2] by reweighted least squares (2.6e-6 off; P is rounded to 16 bits, 4.9e-4 at the
-// least), n added to the exponent.  Below 2^-126 it
-// stops at a subnormal, which the row sum takes as zero; NaN stays beyond every finite sum (the row's output is NaN, as with ex2).
+// 2^x of a pair on the FMA pipe: x = n + f, n the nearest integer (the sum with 1.5 * 2^23 holds it in its low bits), 2^f by a degree-6
+// polynomial with constant term 1, the least-maximum fit over [-1/2, 1/2] by reweighted least squares, times 2^n: 7.4e-8 off at most, 2.6e-8 in the mean
+// square (ex2.approx 1.45e-7 and 5.8e-8, measured over [-126, 8]; degree 5 1.65e-7 and 6.6e-8).  As with ex2.approx.ftz what is below
+// 2^-126 is 0 (n = -127 gives the factor 0), and NaN stays NaN.
 __device__ __forceinline__ void exp2_poly2(uint64_t x2, float &p0, float &p1) {
     float x0, x1;
     upk2(x2, x0, x1);
-    asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(x0));   // -126
-    asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(x1));
+    asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(x0));   // -127
+    asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(x1));
     x2 = pk2(x0, x1);
     const uint64_t big = pk2(12582912.f, 12582912.f), minus_big = pk2(-12582912.f, -12582912.f), minus = pk2(-1.f, -1.f);
     const uint64_t t = add2(x2, big), f = fma2(add2(t, minus_big), minus, x2);
-    uint64_t y = fma2(f, pk2(0.009570102207362652f, 0.009570102207362652f), pk2(0.05591786280274391f, 0.05591786280274391f));
-    y = fma2(y, f, pk2(0.240247443318367f, 0.240247443318367f));
-    y = fma2(y, f, pk2(0.6931217908859253f, 0.6931217908859253f));
-    y = fma2(y, f, pk2(0.9999992847442627f, 0.9999992847442627f));
-    float t0, t1, y0, y1;
+    uint64_t y = fma2(f, pk2(0.00015353361959569156f, 0.00015353361959569156f), pk2(0.0013398875016719103f, 0.0013398875016719103f));
+    y = fma2(y, f, pk2(0.00961843691766262f, 0.00961843691766262f));
+    y = fma2(y, f, pk2(0.055503327399492264f, 0.055503327399492264f));
+    y = fma2(y, f, pk2(0.24022646248340607f, 0.24022646248340607f));
+    y = fma2(y, f, pk2(0.6931471824645996f, 0.6931471824645996f));
+    y = fma2(y, f, pk2(1.f, 1.f));
+    float t0, t1;
     upk2(t, t0, t1);
-    upk2(y, y0, y1);
-    p0 = __uint_as_float(__float_as_uint(y0) + (__float_as_uint(t0) << 23));
-    p1 = __uint_as_float(__float_as_uint(y1) + (__float_as_uint(t1) << 23));
+    const uint64_t scale = pk2(__uint_as_float((__float_as_uint(t0) << 23) + 0x3f800000u), __uint_as_float((__float_as_uint(t1) << 23) + 0x3f800000u));
+    upk2(mul2_ftz(y, scale), p0, p1);
 }
 // P = 2^(s sc - m) of 32 scores as packed 16-bit pairs, and their sum.  MIX: every fourth pair leaves the special-function unit for the FMA
 // pipe (the unit's 16 results a cycle and SM are what bounds the softmax of heads of 64 and 128); tiles with masked scores take the

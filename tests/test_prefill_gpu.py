@@ -120,6 +120,23 @@ def test_prefill_tc_lse():
         np.testing.assert_allclose(got[:, s:s + n], want_lse[b, :, :n], rtol=2e-4, atol=2e-4)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("column", range(8))
+def test_prefill_tc_nan_stays_nan(D, column):
+    """One key of NaN, at every place of the eight columns that the softmax treats alike: the rows that see it, in masked tiles and in whole ones, are
+    NaN with the log-sum-exp of a row without a sum (+inf), the rows before it are what they are without it."""
+    T, at = 600, 64 + column
+    cu = u32([0, T])
+    q, k, v = randn_t((T, 2, D), 1, torch.bfloat16, DEV), randn_t((T, 1, D), 2, torch.bfloat16, DEV), randn_t((T, 1, D), 3, torch.bfloat16, DEV)
+    plain = ops.flash_attn_varlen(q, k, v, cu, cu, T, T, D ** -0.5, True)
+    k[at] = float("nan")
+    out, lse = ops.flash_attn_varlen(q, k, v, cu, cu, T, T, D ** -0.5, True, with_lse=True)
+    assert ops.last_mha_path() == "prefill_tc"
+    assert bool(out[at:].isnan().all()) and torch.equal(out[:at], plain[:at])
+    lse = lse.view(2, T)
+    assert bool(torch.isposinf(lse[:, at:]).all()) and bool(lse[:, :at].isfinite().all())
+
+
 @pytest.mark.skipif(not RefLib.available(), reason="oracle/_ref not built")
 def test_prefill_tc_matches_reference_kernels_at_2k():
     ref = RefLib()
