@@ -6,9 +6,9 @@
 //   2. the talk matrix: mixed[h, pair] = sum_g talk[h, g] a[g, pair], a product of its own over the heads,
 //   3. values: a warp applies its two heads' mixed weights (bfloat16, as before).
 // What bounded the mix on CUDA cores was shared memory (32 float32 weights read per pair and head; 4000 warp instructions per tile and
-// warp), so it runs on the tensor cores too, at float32's precision: weights (scaled by 2^15) and talk (scaled to 2^8 per row) are each
-// split into two float16 pieces of 11 bits, and hi hi + hi lo + lo hi is summed in float32 (what is dropped is 2^-22 of a term, or
-// 2^-40 of the talk entry where the weight itself is below 2^-18).  mma.sync and not tcgen05: the three products per tile are 16 rows or one head-square deep.
+// warp), so it runs on the tensor cores too, at float32's precision: weights and talk are each split into three bfloat16 pieces of 8 bits, which
+// hold all of a float32's 24 and its whole range, and the six products of pieces down to 2^-16 of a term are summed in float32 (what is dropped is
+// 2^-25 of a term).  mma.sync and not tcgen05: the products per tile are 16 rows or one head-square deep.
 // One CTA holds all heads (64 accumulator registers per thread for two heads), so there is no cluster exchange, and the keys of a long row of
 // tiles are cut into segments, whose float32 sums simply add (no softmax): 128 row blocks of one prompt over 74 CTA pairs left the SMs idle half of
 // the time.  Keys of the next tile are copied under the mix, values under the scores.
@@ -25,8 +25,7 @@ namespace {
 
 using namespace hybrid;
 
-constexpr int kStRows = 16, kStKeys = 32, kStMaxSegs = 8;
-constexpr float kStWeightScale = 32768.f;
+constexpr int kStRows = 16, kStKeys = 32, kStMaxSegs = 8, kStPieces = 3;
 
 __device__ __forceinline__ float st_weight(float dot, float scale, float softcap, float inv_cap, float slope, float dist, float head_bias) {
     float s = dot * scale;
@@ -37,18 +36,20 @@ __device__ __forceinline__ float st_weight(float dot, float scale, float softcap
 
 template <int HT>   // heads = 16 HT
 struct StLayout {
-    static constexpr int H = 16 * HT, kPair = 2 * H + 16, kRow = kStKeys * kPair + 16;   // bytes of a pair's weights, of a query row's
-    static constexpr int kWeights = kStRows * kRow;                                       // one of the two pieces
+    static constexpr int H = 16 * HT, kPair = 4 * H + 32, kRow = kStKeys * kPair + 16;   // bytes of a pair's float32 weights, of a query row's
     static constexpr int kMixRow = 2 * kStKeys + 16, kMixHead = kStRows * kMixRow + 16;
-    static constexpr int kTalkRow = 2 * H + 16;
-    static constexpr int w_off = 0, m_off = 2 * kWeights, t_off = m_off + H * kMixHead, s_off = t_off + 2 * H * kTalkRow, kv_off = s_off + H * 4;
+    static constexpr int kTalkRow = 2 * H + 16, kTalk = H * kTalkRow;                    // one piece of the talk matrix
+    static constexpr int w_off = 0, m_off = kStRows * kRow, t_off = m_off + H * kMixHead, kv_off = t_off + kStPieces * kTalk;
     __host__ __device__ static size_t total(int G, int D, int DV) { return kv_off + static_cast<size_t>(G) * kStKeys * (D + 8 + DV + 8) * 2; }
 };
 
-__device__ __forceinline__ void st_split(float a, float b, uint32_t &hi, uint32_t &lo) {
-    const __half ah = __float2half_rn(a), bh = __float2half_rn(b);
-    hi = pack2<__half>(__half2float(ah), __half2float(bh));
-    lo = pack2<__half>(a - __half2float(ah), b - __half2float(bh));
+// a float32's three bfloat16 pieces, the largest first
+__device__ __forceinline__ void st_split(float x, float (&piece)[kStPieces]) {
+#pragma unroll
+    for (int i = 0; i < kStPieces; ++i) {
+        piece[i] = __bfloat162float(__float2bfloat16_rn(x));
+        x -= piece[i];
+    }
 }
 
 template <int HT>
@@ -68,8 +69,7 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
     const int all_end = p0 + rows, j_begin = seg * seg_keys, j_end = min(all_end, j_begin + seg_keys);
     if (j_begin >= all_end) return;
     const int32_t *bt = a.block_tables + static_cast<int64_t>(b) * a.max_blocks;
-    unsigned char *wh = sm + L::w_off, *wl = wh + L::kWeights, *mix = sm + L::m_off, *th = sm + L::t_off, *tl = th + H * L::kTalkRow;
-    float *unscale = reinterpret_cast<float *>(sm + L::s_off);
+    unsigned char *weights = sm + L::w_off, *mix = sm + L::m_off, *talk = sm + L::t_off;
     __nv_bfloat16 *Ks = reinterpret_cast<__nv_bfloat16 *>(sm + L::kv_off), *Vs = Ks + G * kStKeys * (D + 8);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t4 = lane & 3, rq = lane >> 2;
     const __nv_bfloat16 *kc = static_cast<const __nv_bfloat16 *>(a.k_cache), *vc = static_cast<const __nv_bfloat16 *>(a.v_cache);
@@ -95,21 +95,13 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
         cp_async_commit();
     };
     stage(kc, Ks, D, j_begin);
-    // ---- the talk matrix in two pieces, a row scaled so that its largest entry is 2^7 .. 2^8 ----
-    for (int h = warp; h < H; h += NW) {
-        float mx = 0.f;
-        const float t = lane < H ? a.talk[h * H + lane] : 0.f;
-        mx = fabsf(t);
+    // ---- the talk matrix in three pieces ----
+    for (int i = tid; i < H * H; i += NT) {
+        float piece[kStPieces];
+        st_split(a.talk[i], piece);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const int e = mx > 0.f ? ilogbf(mx) : 0;
-        const float up = ldexpf(1.f, 7 - e);
-        if (lane < H) {
-            const __half hi = __float2half_rn(t * up);
-            *reinterpret_cast<__half *>(th + h * L::kTalkRow + lane * 2) = hi;
-            *reinterpret_cast<__half *>(tl + h * L::kTalkRow + lane * 2) = __float2half_rn(t * up - __half2float(hi));
-        }
-        if (lane == 0) unscale[h] = ldexpf(1.f, e - 7 - 15);
+        for (int k = 0; k < kStPieces; ++k)
+            *reinterpret_cast<__nv_bfloat16 *>(talk + k * L::kTalk + i / H * L::kTalkRow + i % H * 2) = __float2bfloat16_rn(piece[k]);
     }
     // ---- this warp's heads: query fragments, constants ----
     const int h0 = 2 * warp, rep = H / G;
@@ -139,7 +131,7 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
         cp_async_wait_all();
         __syncthreads();   // the keys are there; everyone is done with the last tile's values and mixed weights
         stage(vc, Vs, DV, j0);
-        // ---- 1. scores and weights of two heads; both heads' pieces of a pair go out in one word ----
+        // ---- 1. scores and weights of two heads; both heads' weights of a pair go out together ----
         float w0[4][4];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
@@ -163,69 +155,48 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int row = rq + (e >> 1) * 8, key = nt * 8 + 2 * t4 + (e & 1), dist = p0 + row - (j0 + key);
-                    const float w = row < rows && dist >= 0 ? st_weight(s[nt][e], a.scale, a.softcap, inv_cap, slope[x], static_cast<float>(dist), hb[x]) * kStWeightScale : 0.f;
-                    if (x == 0) {
-                        w0[nt][e] = w;
-                    } else {
-                        uint32_t hi, lo;
-                        st_split(w0[nt][e], w, hi, lo);
-                        const int at = row * L::kRow + key * L::kPair + h0 * 2;
-                        *reinterpret_cast<uint32_t *>(wh + at) = hi;
-                        *reinterpret_cast<uint32_t *>(wl + at) = lo;
-                    }
+                    const float w = row < rows && dist >= 0 ? st_weight(s[nt][e], a.scale, a.softcap, inv_cap, slope[x], static_cast<float>(dist), hb[x]) : 0.f;
+                    if (x == 0) w0[nt][e] = w;
+                    else *reinterpret_cast<float2 *>(weights + row * L::kRow + key * L::kPair + h0 * 4) = make_float2(w0[nt][e], w);
                 }
         }
         __syncthreads();   // all heads' weights are there, and the keys are done with
         if (j0 + kStKeys < j_end) stage(kc, Ks, D, j0 + kStKeys);
         else cp_async_commit();   // an empty group: the values' is always the one before the last
         // ---- 2. the heads talk: a warp takes whole query rows ----
-        {
-            uint32_t ah[HT][HT][4], al[HT][HT][4];
+#pragma unroll 1
+        for (int mt = 0; mt < HT; ++mt) {
+            uint32_t ta[kStPieces][HT][4];
 #pragma unroll
-            for (int mt = 0; mt < HT; ++mt)
+            for (int k = 0; k < kStPieces; ++k)
 #pragma unroll
-                for (int kk = 0; kk < HT; ++kk) {
-                    const int at = (mt * 16 + (lane & 15)) * L::kTalkRow + (kk * 16 + (lane >> 4) * 8) * 2;
-                    ldmatrix_x4(ah[mt][kk], smem_u32(th + at));
-                    ldmatrix_x4(al[mt][kk], smem_u32(tl + at));
-                }
+                for (int kk = 0; kk < HT; ++kk)
+                    ldmatrix_x4(ta[k][kk], smem_u32(talk + k * L::kTalk + (mt * 16 + (lane & 15)) * L::kTalkRow + (kk * 16 + (lane >> 4) * 8) * 2));
             for (int row = warp; row < kStRows; row += NW)
 #pragma unroll
-                for (int n2 = 0; n2 < 2; ++n2) {   // 16 keys
-                    uint32_t bh[2][2 * HT], bl[2][2 * HT];
-                    if constexpr (HT == 2) {
+                for (int nt = 0; nt < kStKeys / 8; ++nt) {
+                    uint32_t wb[kStPieces][HT][2];
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            const int at = row * L::kRow + ((2 * n2 + i) * 8 + (lane & 7)) * L::kPair + (lane >> 3) * 16;
-                            ldmatrix_x4(bh[i], smem_u32(wh + at));
-                            ldmatrix_x4(bl[i], smem_u32(wl + at));
+                    for (int kk = 0; kk < HT; ++kk)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float2 w = *reinterpret_cast<const float2 *>(weights + row * L::kRow + (nt * 8 + rq) * L::kPair + (kk * 16 + 8 * e + 2 * t4) * 4);
+                            float px[kStPieces], py[kStPieces];
+                            st_split(w.x, px);
+                            st_split(w.y, py);
+#pragma unroll
+                            for (int k = 0; k < kStPieces; ++k) wb[k][kk][e] = pack2<__nv_bfloat16>(px[k], py[k]);
                         }
-                    } else {
-                        uint32_t r[4];
-                        const int at = row * L::kRow + (n2 * 16 + (lane >> 4) * 8 + (lane & 7)) * L::kPair + ((lane >> 3) & 1) * 16;
-                        ldmatrix_x4(r, smem_u32(wh + at));
-                        bh[0][0] = r[0], bh[0][1] = r[1], bh[1][0] = r[2], bh[1][1] = r[3];
-                        ldmatrix_x4(r, smem_u32(wl + at));
-                        bl[0][0] = r[0], bl[0][1] = r[1], bl[1][0] = r[2], bl[1][1] = r[3];
-                    }
+                    float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int mt = 0; mt < HT; ++mt)
+                    for (int order = kStPieces - 1; order >= 0; --order)   // the smallest products first
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            float c[4] = {0.f, 0.f, 0.f, 0.f};
+                        for (int k = 0; k <= order; ++k)
 #pragma unroll
-                            for (int kk = 0; kk < HT; ++kk) {
-                                Mma16816<__half>::run(c, al[mt][kk], bh[i][2 * kk], bh[i][2 * kk + 1]);
-                                Mma16816<__half>::run(c, ah[mt][kk], bl[i][2 * kk], bl[i][2 * kk + 1]);
-                            }
-#pragma unroll
-                            for (int kk = 0; kk < HT; ++kk) Mma16816<__half>::run(c, ah[mt][kk], bh[i][2 * kk], bh[i][2 * kk + 1]);
-                            const int h = mt * 16 + rq;
-                            const float u0 = unscale[h], u1 = unscale[h + 8];
-                            unsigned char *m = mix + h * L::kMixHead + row * L::kMixRow + ((2 * n2 + i) * 8 + 2 * t4) * 2;
-                            *reinterpret_cast<uint32_t *>(m) = pack2<__nv_bfloat16>(c[0] * u0, c[1] * u0);
-                            *reinterpret_cast<uint32_t *>(m + 8 * L::kMixHead) = pack2<__nv_bfloat16>(c[2] * u1, c[3] * u1);
-                        }
+                            for (int kk = 0; kk < HT; ++kk) Mma16816<__nv_bfloat16>::run(c, ta[k][kk], wb[order - k][kk][0], wb[order - k][kk][1]);
+                    unsigned char *m = mix + (mt * 16 + rq) * L::kMixHead + row * L::kMixRow + (nt * 8 + 2 * t4) * 2;
+                    *reinterpret_cast<uint32_t *>(m) = pack2<__nv_bfloat16>(c[0], c[1]);
+                    *reinterpret_cast<uint32_t *>(m + 8 * L::kMixHead) = pack2<__nv_bfloat16>(c[2], c[3]);
                 }
         }
         asm volatile("cp.async.wait_group 1;" ::: "memory");   // the values

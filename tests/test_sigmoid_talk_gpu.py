@@ -1,4 +1,4 @@
-"""Sigmoid attention with talking heads over prompt portions (the talk matrix as a split float16 product, keys in segments) against float64.
+"""Sigmoid attention with talking heads over prompt portions (the talk matrix as a product of split pieces, keys in segments) against float64.
 
 Bound per output entry: a score is a float32 sum of bfloat16 products, a weight and the mix are within 1e-5 of sum_g |talk| a_g; the mixed weight is
 rounded to bfloat16 (8 bits: 2^-8 of it at most) before it meets the value, the result once more."""
@@ -20,6 +20,31 @@ F64 = torch.float64
     (16, 16, 64, 16, 16, ((0, 700),), 8.0, True, 0.0),                          # a prompt whose later rows take two segments
 ])
 def test_against_float64(H, G, D, V, bs, seqs, cap, slopes, bias):
+    def edit(talk):
+        talk[1] *= 1e-4                  # rows of other sizes
+        talk[2] *= 300.0
+        talk[3] = 0.0
+
+    _compare(H, G, D, V, bs, seqs, cap, slopes, bias, edit, 1e-9)
+
+
+@pytest.mark.parametrize("H", [16, 32])
+def test_small_weights_keep_their_bits(H):
+    """Heads whose weights are near e^-40 everywhere: the mix is float32's, whatever the weights' size."""
+    _compare(H, 4, 64, 64, 16, ((0, 40), (700, 20)), 8.0, False, -40.0, lambda talk: None, 0.0)
+
+
+@pytest.mark.parametrize("H", [16, 32])
+def test_small_talk_rows(H):
+    """Rows of the talk matrix far below and far above one, down to float32's smallest normal values (their outputs may be flushed to zero: 1e-36)."""
+    def edit(talk):
+        for h, scale in enumerate([1e-10, 1e-25, 2.0 ** -110, 2.0 ** -121, 2.0 ** -125, 1e10, 1e20, 1e30]):
+            talk[h] *= scale
+
+    _compare(H, 4, 64, 64, 16, ((0, 40), (700, 20)), 8.0, True, -1.0, edit, 1e-36)
+
+
+def _compare(H, G, D, V, bs, seqs, cap, slopes, bias, edit, floor):
     g = torch.Generator().manual_seed(2)
     each = [-(-(c + n) // bs) for c, n in seqs]
     pool = torch.randperm(sum(each), generator=g).to(torch.int32)
@@ -33,9 +58,7 @@ def test_against_float64(H, G, D, V, bs, seqs, cap, slopes, bias):
     sl = torch.tensor([2.0 ** (-8.0 * (h + 1) / H) for h in range(H)], device=DEV) if slopes else None
     hb = randn_t((H,), 4, torch.float32, DEV, scale=0.5) + bias
     talk = torch.eye(H, device=DEV) + randn_t((H, H), 5, torch.float32, DEV, scale=0.3)
-    talk[1] *= 1e-4                  # rows of other sizes: the pieces are scaled per row
-    talk[2] *= 300.0
-    talk[3] = 0.0
+    edit(talk)
     pos = torch.cat([torch.arange(c, c + n) for c, n in seqs]).to(DEV)
     tseq = torch.arange(len(seqs), dtype=torch.int32).repeat_interleave(torch.tensor([n for _, n in seqs])).to(DEV)
     out = ops.sigmoid_attention_paged(q, kc, vc, pos, tseq, table.to(DEV), sl, hb, talk, H, G, D, V, bs, D ** -0.5, cap, max(n for _, n in seqs)).double()
@@ -56,7 +79,7 @@ def test_against_float64(H, G, D, V, bs, seqs, cap, slopes, bias):
         flat = lambda x: x.transpose(0, 1).reshape(n, H * V)
         want, bound = flat(torch.bmm(mixed, v)), flat(torch.bmm(slack, v.abs()))
         diff = (out[t0:t0 + n] - want).abs()
-        excess = diff - (bound + 2.0 ** -8 * want.abs() + 1e-9)
+        excess = diff - (bound + 2.0 ** -8 * want.abs() + floor)
         assert bool((excess <= 0).all()), f"sequence {b}: worst excess {float(excess.max()):.3e}"
         t0 += n
 
