@@ -332,6 +332,16 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // ---- packed float32 pairs: one issue slot for two operations ----
 __device__ __forceinline__ uint64_t pk2(float lo, float hi) {
     uint64_t r;
+// n / (1 + e) for e >= 0 (inf and NaN included), 1 ulp: the reciprocal unit's estimate, one step of Newton's iteration, one product.  For
+// epilogues that divide per element, where the compiler's division takes three times the instructions and a branch.  Where e passes 2^126
+// it divides by 2^126 (the quotient is below n times the smallest normal number either way).
+__device__ __forceinline__ float over_one_plus(float n, float e) {
+    float d = 1.f + e, r;
+    d = d > 8.507059e37f ? 8.507059e37f : d;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return n * fmaf(r, fmaf(-d, r, 1.f), r);
+}
+
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
     return r;
 }

@@ -601,7 +601,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                             const T *ge = reinterpret_cast<const T *>(&gv[c * 4 + i]);
 #pragma unroll
                             for (int e = 0; e < 8; ++e)
-                                ov[8 * i + e] = __float_as_uint(__fdividef(__uint_as_float(ov[8 * i + e]), 1.f + __expf(-static_cast<float>(ge[e]))));
+                                ov[8 * i + e] = __float_as_uint(over_one_plus(__uint_as_float(ov[8 * i + e]), expf(-static_cast<float>(ge[e]))));
                         }
                     }
 #pragma unroll

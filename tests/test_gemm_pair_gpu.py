@@ -79,6 +79,22 @@ def test_gated_activations(dtype, T, F, K, act):
     assert _lib.lib().atoma_gemm_pair_timeouts() == 0
 
 
+@pytest.mark.parametrize("dtype", [BF, torch.float16])
+def test_activation_is_float32(dtype):
+    """Rows of x with one entry make both products exact, so a result differs from the rounded float64 one only where float32's error reaches over the
+    middle of two neighbours: with four operations of half to one unit (2^-24; 1.1e-7 of the value in the mean) and neighbours 2^-8 to 2^-7 (2^-11 to 2^-10) of the
+    value apart, in the share 2 x 1.1e-7 x 2^7.5 of the entries."""
+    T, F, K = 192, 32768, 64
+    x = torch.zeros((T, K), dtype=dtype, device=DEV)
+    x[torch.arange(T), torch.arange(T) % K] = torch.tensor([0.5, 1.0, 2.0], dtype=dtype, device=DEV).repeat_interleave(K)
+    w = randn_t((2 * F, K), 12, dtype, DEV, scale=2.0)
+    got = ops.gate_up_silu(x, w)
+    z = x.double() @ w.double().T
+    want = (z[:, :F] / (1 + torch.exp(-z[:, :F])) * z[:, F:]).to(dtype)
+    share = (got != want).double().mean().item()
+    assert share < 2.2e-7 * 2.0 ** (7.5 if dtype == BF else 10.5), share
+
+
 @pytest.mark.parametrize("scale_input", [False, True])
 @pytest.mark.parametrize("T,E,top,W,F", [
     (1, 3, 2, 64, 64),         # two chunks of one row
