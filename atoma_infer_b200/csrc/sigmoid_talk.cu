@@ -9,10 +9,13 @@
 // warp), so it runs on the tensor cores too, at float32's precision: weights and talk are each split into three bfloat16 pieces of 8 bits, which
 // hold all of a float32's 24 and its whole range, and the six products of pieces down to 2^-16 of a term are summed in float32 (what is dropped is
 // 2^-25 of a term).  mma.sync and not tcgen05: the products per tile are 16 rows or one head-square deep.
-// One CTA holds all heads (64 accumulator registers per thread for two heads), so there is no cluster exchange, and the keys of a long row of
-// tiles are cut into segments, whose float32 sums simply add (no softmax): 128 row blocks of one prompt over 74 CTA pairs left the SMs idle half of
-// the time.  Keys of the next tile are copied under the mix, values under the scores.
-// 2048 tokens, 32 heads of 64 on 8: 1218 us on the CUDA-core mix (hybrid_attention.cu), 492 here.
+// One CTA holds all heads (64 accumulator registers per thread for two heads), so there is no cluster exchange, and the keys are cut into segments,
+// whose float32 sums simply add (no softmax): 128 row blocks of one prompt over 74 CTA pairs left the SMs idle half of the time.  A
+// segment is 512 keys from a multiple of 512 on whatever the step looks like, so a position's sums depend on its keys alone.  A CTA takes one
+// segment, or, in steps whose row blocks fill the SMs without, all of its rows' segments one after the other; the sums between take at most 256 MiB
+// (kStScratch), and longer steps go in runs of tokens.  Keys of the next tile are copied under the mix, values under the scores.
+// 2048 tokens, 32 heads of 64 on 8: 1218 us on the CUDA-core mix (hybrid_attention.cu), 506 here; 8000 tokens before 17 new ones 3308 and 250.  A prompt of one to
+// sixteen row blocks and few keys is slower than there (64 tokens: 31 and 38 us): all heads wait for each other in one CTA.
 #include "common.cuh"
 #include "hybrid_common.cuh"
 
@@ -25,7 +28,8 @@ namespace {
 
 using namespace hybrid;
 
-constexpr int kStRows = 16, kStKeys = 32, kStMaxSegs = 8, kStPieces = 3;
+constexpr int kStRows = 16, kStKeys = 32, kStSegKeys = 512, kStPieces = 3;
+constexpr int64_t kStScratch = 256ll << 20;
 
 __device__ __forceinline__ float st_weight(float dot, float scale, float softcap, float inv_cap, float slope, float dist, float head_bias) {
     float s = dot * scale;
@@ -52,8 +56,11 @@ __device__ __forceinline__ void st_split(float x, float (&piece)[kStPieces]) {
     }
 }
 
+// Row blocks of every sequence that start on the step's tokens lo .. hi - 1.  slots: segments that have a place of their own in `partial` for every token
+// (blockIdx.z: which segment this CTA takes; sigmoid_talk_sum_kernel adds them), or 1: this CTA takes them all and keeps the running sum there.  Both add the
+// segments in order, so they give the same bits.  No scratch: one chain over all keys.
 template <int HT>
-__global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_sigmoid_attn_args a, int seg_keys, int segs, float *__restrict__ partial) {
+__global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_sigmoid_attn_args a, int lo, int hi, int slots, float *__restrict__ partial) {
     using L = StLayout<HT>;
     constexpr int H = L::H, NW = 8 * HT, NT = 256 * HT;
     extern __shared__ __align__(16) unsigned char sm[];
@@ -62,11 +69,12 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
     const int G = static_cast<int>(a.G), D = static_cast<int>(a.dim), DV = static_cast<int>(a.vdim), bs = static_cast<int>(a.block_size);
     const int b = blockIdx.y, seg = blockIdx.z;
     const int t_begin = a.query_start[b], n_q = a.query_start[b + 1] - t_begin;
-    const int r0 = static_cast<int>(gridDim.x - 1 - blockIdx.x) * kStRows;   // the rows with the most keys first
-    if (r0 >= n_q) return;
-    const int rows = min(kStRows, n_q - r0), tok0 = t_begin + r0;
+    const int first = max(0, lo - t_begin + kStRows - 1) / kStRows, last = (min(n_q, hi - t_begin) + kStRows - 1) / kStRows - 1;   // this run's row blocks
+    const int blk = last - static_cast<int>(blockIdx.x);   // the rows with the most keys first
+    if (n_q <= 0 || blk < first) return;
+    const int r0 = blk * kStRows, rows = min(kStRows, n_q - r0), tok0 = t_begin + r0;
     const int ctx = static_cast<int>(a.positions[t_begin]), p0 = ctx + r0, total = ctx + n_q;
-    const int all_end = p0 + rows, j_begin = seg * seg_keys, j_end = min(all_end, j_begin + seg_keys);
+    const int all_end = p0 + rows, j_begin = seg * kStSegKeys, j_end = seg == slots - 1 ? all_end : min(all_end, j_begin + kStSegKeys);
     if (j_begin >= all_end) return;
     const int32_t *bt = a.block_tables + static_cast<int64_t>(b) * a.max_blocks;
     unsigned char *weights = sm + L::w_off, *mix = sm + L::m_off, *talk = sm + L::t_off;
@@ -126,6 +134,27 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[x][i][0] = o[x][i][1] = o[x][i][2] = o[x][i][3] = 0.f;
     const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
+    // the sums of a segment, out of the accumulators: into its place, onto the running sum, or, where no other segment follows or precedes, out
+    bool more = false;   // a running sum waits in this token's place
+    auto put = [&](bool last) {
+        const bool out = last && (slots == 1 || all_end <= kStSegKeys);
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt) {
+                if (nt * 8 >= DV) continue;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int row = rq + 8 * e, col = (h0 + x) * DV + nt * 8 + 2 * t4;
+                    if (row >= rows) continue;
+                    float2 s = make_float2(o[x][nt][2 * e], o[x][nt][2 * e + 1]);
+                    float2 *place = reinterpret_cast<float2 *>(partial + (static_cast<int64_t>(tok0 + row - lo) * slots + seg) * H * DV + col);
+                    if (more) s = make_float2(place->x + s.x, place->y + s.y);
+                    if (out) *reinterpret_cast<uint32_t *>(static_cast<__nv_bfloat16 *>(a.out) + static_cast<int64_t>(tok0 + row) * H * DV + col) = pack2<__nv_bfloat16>(s.x, s.y);
+                    else *place = s;
+                }
+            }
+    };
 
     for (int j0 = j_begin; j0 < j_end; j0 += kStKeys) {
         cp_async_wait_all();
@@ -163,42 +192,48 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
         __syncthreads();   // all heads' weights are there, and the keys are done with
         if (j0 + kStKeys < j_end) stage(kc, Ks, D, j0 + kStKeys);
         else cp_async_commit();   // an empty group: the values' is always the one before the last
-        // ---- 2. the heads talk: a warp takes whole query rows ----
+        // ---- 2. the heads talk: a warp takes whole query rows, eight (32 heads: registers) or sixteen keys at a time ----
+        constexpr int kN = HT == 2 ? 1 : 2;
+        for (int row = warp; row < kStRows; row += NW)
 #pragma unroll 1
-        for (int mt = 0; mt < HT; ++mt) {
-            uint32_t ta[kStPieces][HT][4];
+            for (int n2 = 0; n2 < kStKeys / 8; n2 += kN) {
+                uint32_t wb[kN][kStPieces][HT][2];
 #pragma unroll
-            for (int k = 0; k < kStPieces; ++k)
-#pragma unroll
-                for (int kk = 0; kk < HT; ++kk)
-                    ldmatrix_x4(ta[k][kk], smem_u32(talk + k * L::kTalk + (mt * 16 + (lane & 15)) * L::kTalkRow + (kk * 16 + (lane >> 4) * 8) * 2));
-            for (int row = warp; row < kStRows; row += NW)
-#pragma unroll
-                for (int nt = 0; nt < kStKeys / 8; ++nt) {
-                    uint32_t wb[kStPieces][HT][2];
+                for (int i = 0; i < kN; ++i)
 #pragma unroll
                     for (int kk = 0; kk < HT; ++kk)
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
-                            const float2 w = *reinterpret_cast<const float2 *>(weights + row * L::kRow + (nt * 8 + rq) * L::kPair + (kk * 16 + 8 * e + 2 * t4) * 4);
+                            const float2 w = *reinterpret_cast<const float2 *>(weights + row * L::kRow + ((n2 + i) * 8 + rq) * L::kPair + (kk * 16 + 8 * e + 2 * t4) * 4);
                             float px[kStPieces], py[kStPieces];
                             st_split(w.x, px);
                             st_split(w.y, py);
 #pragma unroll
-                            for (int k = 0; k < kStPieces; ++k) wb[k][kk][e] = pack2<__nv_bfloat16>(px[k], py[k]);
+                            for (int k = 0; k < kStPieces; ++k) wb[i][k][kk][e] = pack2<__nv_bfloat16>(px[k], py[k]);
                         }
-                    float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int order = kStPieces - 1; order >= 0; --order)   // the smallest products first
+                for (int mt = 0; mt < HT; ++mt) {
+                    uint32_t ta[kStPieces][HT][4];
 #pragma unroll
-                        for (int k = 0; k <= order; ++k)
+                    for (int k = 0; k < kStPieces; ++k)
 #pragma unroll
-                            for (int kk = 0; kk < HT; ++kk) Mma16816<__nv_bfloat16>::run(c, ta[k][kk], wb[order - k][kk][0], wb[order - k][kk][1]);
-                    unsigned char *m = mix + (mt * 16 + rq) * L::kMixHead + row * L::kMixRow + (nt * 8 + 2 * t4) * 2;
-                    *reinterpret_cast<uint32_t *>(m) = pack2<__nv_bfloat16>(c[0], c[1]);
-                    *reinterpret_cast<uint32_t *>(m + 8 * L::kMixHead) = pack2<__nv_bfloat16>(c[2], c[3]);
+                        for (int kk = 0; kk < HT; ++kk)
+                            ldmatrix_x4(ta[k][kk], smem_u32(talk + k * L::kTalk + (mt * 16 + (lane & 15)) * L::kTalkRow + (kk * 16 + (lane >> 4) * 8) * 2));
+#pragma unroll
+                    for (int i = 0; i < kN; ++i) {
+                        float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                        for (int order = kStPieces - 1; order >= 0; --order)   // the smallest products first
+#pragma unroll
+                            for (int k = 0; k <= order; ++k)
+#pragma unroll
+                                for (int kk = 0; kk < HT; ++kk) Mma16816<__nv_bfloat16>::run(c, ta[k][kk], wb[i][order - k][kk][0], wb[i][order - k][kk][1]);
+                        unsigned char *m = mix + (mt * 16 + rq) * L::kMixHead + row * L::kMixRow + ((n2 + i) * 8 + 2 * t4) * 2;
+                        *reinterpret_cast<uint32_t *>(m) = pack2<__nv_bfloat16>(c[0], c[1]);
+                        *reinterpret_cast<uint32_t *>(m + 8 * L::kMixHead) = pack2<__nv_bfloat16>(c[2], c[3]);
+                    }
                 }
-        }
+            }
         asm volatile("cp.async.wait_group 1;" ::: "memory");   // the values
         __syncthreads();
         // ---- 3. values ----
@@ -219,38 +254,29 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
                     }
             }
         }
+        if (slots == 1 && partial && j0 + kStKeys < j_end && (j0 + kStKeys) % kStSegKeys == 0) {   // a segment ends here
+            put(false);
+            more = true;
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[x][i][0] = o[x][i][1] = o[x][i][2] = o[x][i][3] = 0.f;
+        }
     }
     cp_async_wait_all();
-    const bool whole = all_end <= seg_keys;
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            if (nt * 8 >= DV) continue;
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int row = rq + 8 * e, col = (h0 + x) * DV + nt * 8 + 2 * t4;
-                if (row >= rows) continue;
-                if (whole)
-                    *reinterpret_cast<uint32_t *>(static_cast<__nv_bfloat16 *>(a.out) + static_cast<int64_t>(tok0 + row) * H * DV + col) =
-                        pack2<__nv_bfloat16>(o[x][nt][2 * e], o[x][nt][2 * e + 1]);
-                else
-                    *reinterpret_cast<float2 *>(partial + (static_cast<int64_t>(tok0 + row) * segs + seg) * H * DV + col) =
-                        make_float2(o[x][nt][2 * e], o[x][nt][2 * e + 1]);
-            }
-        }
+    put(true);
 }
 
 // A token's segments, in order; tokens of one segment are out already.
-__global__ void __launch_bounds__(256) sigmoid_talk_sum_kernel(const atoma_sigmoid_attn_args a, const float *__restrict__ partial, int seg_keys, int segs) {
+__global__ void __launch_bounds__(256) sigmoid_talk_sum_kernel(const atoma_sigmoid_attn_args a, const float *__restrict__ partial, int lo, int hi, int segs) {
     pdl_launch_dependents();
     pdl_wait();
-    const int64_t t = blockIdx.x;
+    const int64_t t = lo + static_cast<int64_t>(blockIdx.x);
     const int b = a.token_seq[t], t_begin = a.query_start[b], n_q = a.query_start[b + 1] - t_begin;
     const int r0 = static_cast<int>(t - t_begin) / kStRows * kStRows, end = static_cast<int>(a.positions[t_begin]) + min(r0 + kStRows, n_q);
-    const int n = (end + seg_keys - 1) / seg_keys, row = static_cast<int>(a.H * a.vdim);
-    if (n < 2) return;
-    const float *p = partial + t * segs * row;
+    const int n = min(segs, (end + kStSegKeys - 1) / kStSegKeys), row = static_cast<int>(a.H * a.vdim);
+    if (n < 2 || t_begin + r0 < lo || t_begin + r0 >= hi) return;
+    const float *p = partial + (t - lo) * segs * row;
     for (int i = threadIdx.x * 4; i < row; i += 1024) {
         float4 s = *reinterpret_cast<const float4 *>(p + i);
         for (int k = 1; k < n; ++k) {
@@ -274,30 +300,38 @@ bool hyb_sigmoid_talk_ok(const atoma_sigmoid_attn_args &a) {
 }
 
 bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
-    const int64_t blocks = (a.max_query_len + kStRows - 1) / kStRows, longest = a.max_seq_len > 0 ? a.max_seq_len : 0;
-    // Segments of 512 keys (16 tiles) even out the rows of a few prompts over the SMs; at most eight, so that their sums stay small.  With four row
-    // blocks per SM and more, or an unknown length, whole rows do.
-    int seg_keys = 1 << 30, segs = 1;
-    if (longest > 512 && (a.T + kStRows - 1) / kStRows < 4ll * current_device_info().sm_count) {
-        seg_keys = static_cast<int>(std::max<int64_t>(512, ((longest + kStMaxSegs - 1) / kStMaxSegs + kStKeys - 1) / kStKeys * kStKeys));
-        segs = static_cast<int>((longest + seg_keys - 1) / seg_keys);
-    }
+    const int64_t longest = a.max_seq_len > 0 ? a.max_seq_len : a.max_blocks * a.block_size;
+    const int64_t segs = std::min<int64_t>(65535, (longest + kStSegKeys - 1) / kStSegKeys), blocks = (a.T + kStRows - 1) / kStRows;
+    const int64_t place = a.H * a.vdim * 4;   // bytes of a token's sums
+    int64_t slots = 1, run = a.T;
     float *partial = nullptr;
     if (segs > 1) {
-        partial = static_cast<float *>(try_workspace(stream, static_cast<size_t>(a.T) * segs * a.H * a.vdim * 4, kWorkspaceHybridAttn));
-        if (!partial) seg_keys = 1 << 30, segs = 1;   // whole rows need none
+        // a segment per CTA unless the row blocks are four per SM and more, or two and the segments' sums do not fit at once
+        auto fits = [&](int64_t n) { return std::max<int64_t>(kStRows, kStScratch / (n * place) / kStRows * kStRows); };
+        const int64_t sms = current_device_info().sm_count;
+        slots = blocks >= 4 * sms || (blocks >= 2 * sms && fits(segs) < a.T) ? 1 : segs;
+        run = std::min(a.T, fits(slots));
+        partial = static_cast<float *>(try_workspace(stream, static_cast<size_t>((run + kStRows) * slots * place), kWorkspaceHybridAttn));   // a run's last row block may end behind it
+        if (!partial) slots = 1, run = a.T;   // no scratch: one chain needs none
     }
     const int G = static_cast<int>(a.G), D = static_cast<int>(a.dim), DV = static_cast<int>(a.vdim);
     auto kernel = a.H == 16 ? sigmoid_talk_kernel<1> : sigmoid_talk_kernel<2>;
     const size_t smem = a.H == 16 ? StLayout<1>::total(G, D, DV) : StLayout<2>::total(G, D, DV);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-    if (e == cudaSuccess)
-        e = launch_ex(kernel, dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(a.B), static_cast<unsigned>(segs)), dim3(16 * static_cast<unsigned>(a.H)), smem, stream,
-                      a, seg_keys, segs, partial);
-    if (!hybrid::launched(e, "sigmoid_talk_kernel")) return false;
-    if (segs == 1) return true;
-    return hybrid::launched(launch_ex(sigmoid_talk_sum_kernel, dim3(static_cast<unsigned>(a.T)), dim3(256), 0, stream, a, static_cast<const float *>(partial), seg_keys, segs),
-                            "sigmoid_talk_sum_kernel");
+    const cudaError_t attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+    if (attr != cudaSuccess) return hybrid::launched(attr, "sigmoid_talk_kernel");
+    for (int64_t lo = 0; lo < a.T; lo += run) {
+        const int64_t hi = std::min(a.T, lo + run), rows = (std::min<int64_t>(hi - lo, a.max_query_len) + kStRows - 1) / kStRows + 1;
+        const dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>(a.B), static_cast<unsigned>(slots));
+        if (!hybrid::launched(launch_ex(kernel, grid, dim3(16 * static_cast<unsigned>(a.H)), smem, stream, a, static_cast<int>(lo), static_cast<int>(hi),
+                                        static_cast<int>(slots), partial),
+                              "sigmoid_talk_kernel"))
+            return false;
+        if (slots > 1 && !hybrid::launched(launch_ex(sigmoid_talk_sum_kernel, dim3(static_cast<unsigned>(std::min(a.T, hi + kStRows) - lo)), dim3(256), 0, stream, a,
+                                                    static_cast<const float *>(partial), static_cast<int>(lo), static_cast<int>(hi), static_cast<int>(slots)),
+                                          "sigmoid_talk_sum_kernel"))
+            return false;
+    }
+    return true;
 }
 
 }  // namespace atoma

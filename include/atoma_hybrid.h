@@ -105,7 +105,9 @@ void atoma_qk_norm_cache(const void *qkv, const float *bias, const float *q_weig
  *   s = (q_g . k_j) * scale;  s = softcap * tanh(s / softcap) (softcap > 0);  s -= slopes[g] * (p - j)
  *   a_g = sigmoid(s + head_bias[g]);   a'_h = sum_g talk[h, g] a_g  (talk NULL = identity)
  *   out[t, h, :] = sum_j a'_h(j) v_j[kv head of h, :]
- * Scores, weights and the sums are float32; keys are visited in position order whatever the batch looks like.
+ * Scores, weights and the sums are float32; keys are visited in position order whatever the batch looks like.  A position of a step that holds a
+ * portion of two tokens or more: where its keys' sums are cut (bfloat16 heads that talk: every 512 keys) depends on its keys alone, not on what
+ * else is in the step or how its sequence was cut into steps.  A step of decoded tokens alone: the cuts follow B and max_seq_len.
  */
 typedef struct atoma_sigmoid_attn_args {
     const void *q;                /* [T, H dim] */
@@ -120,7 +122,7 @@ typedef struct atoma_sigmoid_attn_args {
     float scale, softcap;
     uint32_t dtype;
     int32_t max_query_len;        /* longest portion of the batch (1 = decode only): selects the kernel */
-    int32_t max_seq_len;          /* longest sequence (context + portion) of the batch; 0 = unknown (keys are not split) */
+    int32_t max_seq_len;          /* longest sequence (context + portion) of the batch; 0 = unknown (decoded tokens' keys are not split) */
 } atoma_sigmoid_attn_args;
 void atoma_sigmoid_attention_paged(const atoma_sigmoid_attn_args *args, atoma_stream_t stream);
 

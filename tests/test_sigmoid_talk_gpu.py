@@ -84,6 +84,35 @@ def _compare(H, G, D, V, bs, seqs, cap, slopes, bias, edit, floor):
         t0 += n
 
 
+@pytest.mark.parametrize("H,D,others", [
+    (32, 64, ((4000, 3),)),                        # a longer sequence beside it
+    (16, 16, ((0, 4000), (0, 3000), (0, 3000))),   # a step of many tokens, whose CTAs take all segments of their rows
+    (32, 64, ((20000, 900),)),                     # sums that take more than one run of tokens
+])
+def test_a_position_does_not_depend_on_the_step(H, D, others):
+    """The same bits for a sequence alone, beside others, and read in two portions that end anywhere."""
+    G, bs, n = 8, 16, 1301
+    seqs = [(0, n)] + list(others)
+    each = [-(-(c + m) // bs) for c, m in seqs]
+    table, at = torch.zeros((len(seqs), max(each)), dtype=torch.int32), 0
+    for b, m in enumerate(each):
+        table[b, :m] = torch.arange(at, at + m)
+        at += m
+    kc, vc = (randn_t((at * bs, G, D), i, torch.bfloat16, DEV) for i in (1, 2))
+    q = randn_t((sum(m for _, m in seqs), H * D), 3, torch.bfloat16, DEV)
+    hb, talk = randn_t((H,), 4, torch.float32, DEV), torch.eye(H, device=DEV) + randn_t((H, H), 5, torch.float32, DEV, scale=0.3)
+
+    def run(rows, seqs, table):
+        pos = torch.cat([torch.arange(c, c + m) for c, m in seqs]).to(DEV)
+        tseq = torch.arange(len(seqs), dtype=torch.int32).repeat_interleave(torch.tensor([m for _, m in seqs])).to(DEV)
+        return ops.sigmoid_attention_paged(rows, kc, vc, pos, tseq, table.to(DEV), None, hb, talk, H, G, D, D, bs, D ** -0.5, 8.0, max(m for _, m in seqs))
+
+    alone = run(q[:n], seqs[:1], table[:1])
+    assert torch.equal(run(q, seqs, table)[:n], alone)
+    assert torch.equal(run(q[:701], [(0, 701)], table[:1]), alone[:701])
+    assert torch.equal(run(q[701:n], [(701, 600)], table[:1]), alone[701:])
+
+
 def test_capture_on_a_stream_without_scratch():
     """A long prompt captured on a stream that has run nothing: segments need scratch that cannot be had there, whole rows need none."""
     H, G, D, bs, n = 16, 2, 32, 16, 1100
