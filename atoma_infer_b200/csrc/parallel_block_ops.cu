@@ -272,30 +272,7 @@ __device__ __forceinline__ float softplusf_(float z) { return z > 20.f ? z : log
 // 16-byte aligned (float4 loads), and the PW lanes of a column read distinct banks.
 // Two splits per key size: many rows per lane (few instructions per state entry: steps with many CTAs) and 8 rows per lane (a
 // short chain per token and four times the warps: steps with few).  Both add in the same order, so they give the same bits.
-//
-// The delta rule's token is a chain: sums over the rows, a shuffle tree, the written row, the update, and the next token's sums wait for it (510
-// cycles a token where its instructions fill 200).  So whole blocks of four tokens (counted from the portion's first) are taken together, in
-// float32 as before: with G_i the product of the first i + 1 decays and d_ji that of the decays after token j up to i,
-//   u_i = beta_i (v_i - G_i S^T k_i - sum_{j<i} d_ji (k_j . k_i) u_j),   o_i = G_i S^T q_i + sum_{j<=i} d_ji (k_j . q_i) u_j,
-//   S' = G_3 S + sum_j d_j3 k_j u_j,
-// eight sums over the rows of the SAME state, one chain for four tokens, and one pass that writes the state.  The staging warps form the
-// dot products and decays of a block.  What is left of a portion goes token by token, so a decoded token's arithmetic is as it was.
 constexpr int kScanWarps = 4;
-constexpr int kScanBlock = 4, kBlockCoefs = 32;
-// a block's coefficients: 0 G_i, 4 beta_i, 8 d_ji (k_j . k_i) and 14 d_ji (k_j . q_i) for (i, j) = (1,0) (2,0) (2,1) (3,0) (3,1) (3,2), 20 k_i . q_i, 24 d_j3
-
-// 32 values per lane summed over the lanes: lane l gets the sum of value l, each by the xor tree 16, 8, 4, 2, 1.
-__device__ __forceinline__ float sum_each_32(float (&v)[32], int lane) {
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1)
-#pragma unroll
-        for (int i = 0; i < s; ++i) {
-            const bool up = lane & s;
-            const float send = up ? v[i] : v[i + s], keep = up ? v[i + s] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
-        }
-    return v[0];
-}
 
 template <int PW>
 __device__ __forceinline__ float parts_sum(float v) {
@@ -304,21 +281,10 @@ __device__ __forceinline__ float parts_sum(float v) {
     return v;
 }
 
-// BLOCKS: the form for steps with portions of four tokens and more.  NC: columns per lane.
-// Keys of 65 to 128 entries in steps of many CTAs run two columns of 16 rows a lane (one of 32 took three times the 16-byte loads of shared
-// memory): both columns share every load of keys and queries, and the keys stay in registers from the sums to the update.  The eight
-// lanes of a column pair are neighbours (different rows: no bank conflict), and each ends the sums' tree with one token's two sums of one
-// column.  A staging warp's chain (a round trip to memory, then the block's sums) was as long as the compute warps' (727 and 666 us run alone): it now
-// loads its next tokens ahead (434).  4096 tokens, 32 heads of 128 x 128: 1063 us token by token, 877 in blocks, 809 here; bound by the compute
-// warps' chain per block (736 us alone), one warp per scheduler.  Eight warps of each kind on 8 rows a lane: 871, or 1358 with loads
-// ahead (128 registers spill).
-template <typename T, int KIND, int RPT, int PW, bool BLOCKS, int NC>
-__global__ void __launch_bounds__(64 * kScanWarps, NC == 1 ? 2 : 1) state_scan_kernel(const atoma_state_scan_args a, int chunk) {
+template <typename T, int KIND, int RPT, int PW>
+__global__ void __launch_bounds__(64 * kScanWarps, 2) state_scan_kernel(const atoma_state_scan_args a, int chunk) {
     extern __shared__ __align__(16) float sm[];
-    constexpr int CW = 32 / PW, COLS = CW * NC * kScanWarps, DS = PW * (RPT + 4);
-    static_assert(NC == 1 || (NC == 2 && BLOCKS && RPT == 16 && PW == 8));
-    constexpr int kPart0 = NC == 1 ? CW : 1;                     // lanes of a column: every CW-th of the warp, or neighbours
-    static_assert(!BLOCKS || (KIND == 1 && RPT * PW <= 128));
+    constexpr int CW = 32 / PW, COLS = CW * kScanWarps, DS = PW * (RPT + 4);
     pdl_launch_dependents();
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -327,8 +293,6 @@ __global__ void __launch_bounds__(64 * kScanWarps, NC == 1 ? 2 : 1) state_scan_k
     const int q0 = a.query_start[b], n = a.query_start[b + 1] - q0;
     if (n <= 0) return;
     const int per_tok = (KIND == 0 ? 3 : 2) * DS + COLS + 4;     // q, k, (decay per channel), v of the CTA's columns, beta and decay
-    float *coefs = sm + 2 * chunk * per_tok;                     // [2][blocks of a chunk][kBlockCoefs]
-    const int coefs_per_buf = (chunk + kScanBlock - 1) / kScanBlock * kBlockCoefs;
     for (int i = threadIdx.x; i < 2 * chunk * per_tok; i += blockDim.x) sm[i] = 0.f;   // what lies beyond dim stays zero
     const int kvh = KIND != 0 ? h / (H / static_cast<int>(a.G)) : h;
     const T *qp = static_cast<const T *>(a.q), *kp = static_cast<const T *>(a.k), *vp = static_cast<const T *>(a.v);
@@ -353,118 +317,25 @@ __global__ void __launch_bounds__(64 * kScanWarps, NC == 1 ? 2 : 1) state_scan_k
         dtb = a.dt_bias[h];
     }
     const float inv_tau = 1.0f / a.tau;
-    // what a lane makes of a block's coefficients (kBlockCoefs): 0 .. 5 and 6 .. 11 the pairs (i, j), 12 .. 15 k_i . q_i, 16 .. 19 beta_i, 24 .. 26
-    // d_j3, 28 .. 31 G_i (20 .. 23 and 27 fill unused entries)
-    [[maybe_unused]] int co_lo = 4, co_hi = -1, co_f1 = 16, co_f2 = 16, co_to = lane;
-    if constexpr (BLOCKS) {
-        if (lane < 12) {
-            const int pr = lane % 6, i = pr == 0 ? 1 : (pr < 3 ? 2 : 3), j = pr - i * (i - 1) / 2;
-            co_lo = j + 1, co_hi = i, co_f1 = (lane < 6 ? 20 : 16) + i, co_f2 = 20 + j, co_to = 8 + lane;
-        } else if (lane < 16) {
-            co_f1 = 4 + lane, co_f2 = 8 + lane, co_to = 8 + lane;
-        } else if (lane < 20) {
-            co_to = lane - 12;
-        } else if (lane < 24) {
-            co_to = lane + 8;
-        } else if (lane < 28) {
-            co_lo = lane - 23, co_hi = 3;
-        } else {
-            co_lo = 0, co_hi = lane - 28, co_to = lane - 28;
-        }
-    }
-    struct Raw {
-        T q[TU][EPL], k[TU][EPL], z[KIND == 0 ? TU : 1][KIND == 0 ? EPL : 1], v[TU], b[TU], a[TU];
-    };
-    // every address is valid (a token beyond the portion reads its last, an element beyond dim reads element 0), so the loads carry no
-    // branches and all of them are in flight together
-    auto load = [&](Raw &r, int first) {
-#pragma unroll
-        for (int u = 0; u < TU; ++u) {
-            const int64_t t = q0 + min(first + u, n - 1);
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) {
-                const int i = lane + 32 * e < D ? lane + 32 * e : 0;
-                r.q[u][e] = qp[t * a.ld_q + kvh * D + i];
-                r.k[u][e] = kp[t * a.ld_k + kvh * D + i];
-                if (KIND == 0) r.z[u][e] = static_cast<const T *>(a.z)[t * a.ld_z + h * D + i];
-            }
-            r.v[u] = vp[t * a.ld_v + h * V + max(vcol, 0)];
-            if (KIND == 1) r.b[u] = static_cast<const T *>(a.b_pre)[t * a.ld_b + h];
-            if (KIND != 0) r.a[u] = static_cast<const T *>(a.a_pre)[t * a.ld_a + h];
-        }
-    };
-    // Two columns a lane leave registers to load a warp's next tokens, also of the next chunk, while it works on these.
-    constexpr bool kAhead = NC == 2;
-    [[maybe_unused]] Raw ahead;
-    auto stage = [&](int t0, float *buf, [[maybe_unused]] float *cbuf, int w, int nw) {
+    auto stage = [&](int t0, float *buf, int w, int nw) {
         const int nt = min(chunk, n - t0);
         for (int tk0 = w * TU; tk0 < nt; tk0 += nw * TU) {
-            Raw raw;
-            if constexpr (kAhead) {
-                raw = ahead;
-                load(ahead, tk0 + nw * TU < nt ? t0 + tk0 + nw * TU : t0 + chunk + w * TU);
-            } else {
-                load(raw, t0 + tk0);
-            }
-            auto &[qr, kr, zr, vr, br, ar] = raw;
-            if constexpr (BLOCKS) {
-                if (tk0 + kScanBlock <= nt) {   // a whole block: all its sums at once
-                    static_assert(TU == kScanBlock, "a warp stages whole blocks");
-                    float qv[4][EPL], kv[4][EPL], x[32];
+            // every address is valid (a token beyond the chunk reads the chunk's last, an element beyond dim reads element 0), so
+            // the loads carry no branches and all of them are in flight together
+            T qr[TU][EPL], kr[TU][EPL], zr[KIND == 0 ? TU : 1][KIND == 0 ? EPL : 1], vr[TU], br[TU], ar[TU];
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) x[i] = 0.f;
+            for (int u = 0; u < TU; ++u) {
+                const int64_t t = q0 + t0 + min(tk0 + u, nt - 1);
 #pragma unroll
-                    for (int e = 0; e < EPL; ++e) {
-                        const bool in = lane + 32 * e < D;
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            qv[i][e] = in ? to_f(qr[i][e]) : 0.f;
-                            kv[i][e] = in ? to_f(kr[i][e]) : 0.f;
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            x[16 + i] = fmaf(qv[i][e], qv[i][e], x[16 + i]);
-                            x[20 + i] = fmaf(kv[i][e], kv[i][e], x[20 + i]);
-                            x[12 + i] = fmaf(qv[i][e], kv[i][e], x[12 + i]);
-#pragma unroll
-                            for (int j = 0; j < i; ++j) {
-                                const int p = i * (i - 1) / 2 + j;
-                                x[p] = fmaf(kv[i][e], kv[j][e], x[p]);
-                                x[6 + p] = fmaf(qv[i][e], kv[j][e], x[6 + p]);
-                            }
-                        }
-                    }
-                    const float sum = sum_each_32(x, lane);
-                    // lanes 16 ..: what makes q_i (16 + i) and k_i (20 + i) unit length; lanes 0 .. 3: the tokens' decays and write strengths
-                    const float f = lane < 20 ? a.q_scale / sqrtf(sum + a.unit_eps) : 1.0f / sqrtf(sum + a.unit_eps);
-                    const T am = (lane & 3) == 0 ? ar[0] : (lane & 3) == 1 ? ar[1] : (lane & 3) == 2 ? ar[2] : ar[3];
-                    const T bm = (lane & 3) == 0 ? br[0] : (lane & 3) == 1 ? br[1] : (lane & 3) == 2 ? br[2] : br[3];
-                    const float g = expf(neg_rate * softplusf_(to_f(am) + dtb)), beta = sigmoidf_(to_f(bm));
-                    // every lane makes one coefficient: (a sum, times two lengths) times the decays lo .. hi, the last one first
-                    const float f1 = __shfl_sync(0xffffffffu, f, co_f1), f2 = __shfl_sync(0xffffffffu, f, co_f2);
-                    float d = 1.f;
-#pragma unroll
-                    for (int i = 3; i >= 0; --i) {
-                        const float gi = __shfl_sync(0xffffffffu, g, i);
-                        d *= i >= co_lo && i <= co_hi ? gi : 1.f;
-                    }
-                    cbuf[tk0 / kScanBlock * kBlockCoefs + co_to] = lane < 16 ? sum * f1 * f2 * d : (lane < 20 ? beta : d);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        float *row = buf + (tk0 + u) * per_tok;
-                        const float fq = __shfl_sync(0xffffffffu, f, 16 + u), fk = __shfl_sync(0xffffffffu, f, 20 + u);
-#pragma unroll
-                        for (int e = 0; e < EPL; ++e) {
-                            const int i = lane + 32 * e, o = (i / RPT) * (RPT + 4) + i % RPT;
-                            if (i < D) {
-                                row[o] = qv[u][e] * fq;
-                                row[DS + o] = kv[u][e] * fk;
-                            }
-                        }
-                        if (lane < COLS) row[2 * DS + lane] = vcol >= 0 ? to_f(vr[u]) : 0.f;
-                    }
-                    continue;
+                for (int e = 0; e < EPL; ++e) {
+                    const int i = lane + 32 * e < D ? lane + 32 * e : 0;
+                    qr[u][e] = qp[t * a.ld_q + kvh * D + i];
+                    kr[u][e] = kp[t * a.ld_k + kvh * D + i];
+                    if (KIND == 0) zr[u][e] = static_cast<const T *>(a.z)[t * a.ld_z + h * D + i];
                 }
+                vr[u] = vp[t * a.ld_v + h * V + max(vcol, 0)];
+                if (KIND == 1) br[u] = static_cast<const T *>(a.b_pre)[t * a.ld_b + h];
+                if (KIND != 0) ar[u] = static_cast<const T *>(a.a_pre)[t * a.ld_a + h];
             }
 #pragma unroll
             for (int u = 0; u < TU; ++u) {
@@ -526,223 +397,32 @@ __global__ void __launch_bounds__(64 * kScanWarps, NC == 1 ? 2 : 1) state_scan_k
         }
     };
     // ---- the state of this lane: rows part * RPT + r of column j ----
-    const int part = NC == 1 ? lane / CW : lane % PW;
-    const int col = ((warp % kScanWarps) * CW + (NC == 1 ? lane % CW : lane / PW)) * NC, j = jb + col;   // the lane's first column
+    const int part = lane / CW, j = jb + (warp % kScanWarps) * CW + lane % CW;
     float *S_g = a.state + static_cast<int64_t>(a.state_slots[b]) * a.state_stride + static_cast<int64_t>(h) * D * V;
-    float SS[NC][RPT];
+    float S[RPT];
     const bool fresh = a.context_lens[b] == 0;
     if (!loader) {
 #pragma unroll
         for (int r = 0; r < RPT; ++r) {
             const int i = part * RPT + r;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) SS[c][r] = (!fresh && i < D && j + c < V) ? S_g[static_cast<int64_t>(i) * V + j + c] : 0.f;
+            S[r] = (!fresh && i < D && j < V) ? S_g[static_cast<int64_t>(i) * V + j] : 0.f;
         }
     }
     __syncthreads();                                         // the zero fill is done
-    if constexpr (kAhead) load(ahead, warp * TU);
-    stage(0, sm, coefs, warp, 2 * kScanWarps);
-    if constexpr (kAhead)
-        if (loader) load(ahead, chunk + (warp - kScanWarps) * TU);
+    stage(0, sm, warp, 2 * kScanWarps);
     __syncthreads();
     int it = 0;
     for (int t0 = 0; t0 < n; t0 += chunk, ++it) {
         const float *buf = sm + (it & 1) * chunk * per_tok;
         if (loader) {
-            if (t0 + chunk < n) stage(t0 + chunk, sm + ((it + 1) & 1) * chunk * per_tok, coefs + ((it + 1) & 1) * coefs_per_buf, warp - kScanWarps, kScanWarps);
+            if (t0 + chunk < n) stage(t0 + chunk, sm + ((it + 1) & 1) * chunk * per_tok, warp - kScanWarps, kScanWarps);
         } else {
             const int nt = min(chunk, n - t0);
-            int tk = 0;
-            if constexpr (BLOCKS && NC == 2) {
-                uint64_t S2[2][RPT / 2];
-#pragma unroll
-                for (int c = 0; c < 2; ++c)
-#pragma unroll
-                    for (int r = 0; r < RPT / 2; ++r) S2[c][r] = pk2(SS[c][2 * r], SS[c][2 * r + 1]);
-                const int mine = lane & 1, tok = (lane & 7) >> 1;   // whose two sums this lane ends up with: its pair's column, the block's token
-                const bool mine_in = j + mine < V;
-                for (; tk + kScanBlock <= nt; tk += kScanBlock) {
-                    const float *row0 = buf + tk * per_tok;
-                    const float *co = coefs + (it & 1) * coefs_per_buf + tk / kScanBlock * kBlockCoefs;
-                    ulonglong2 kr[4][RPT / 4];
-#pragma unroll
-                    for (int r4 = 0; r4 < RPT / 4; ++r4)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) kr[i][r4] = *reinterpret_cast<const ulonglong2 *>(row0 + i * per_tok + DS + part * (RPT + 4) + 4 * r4);
-                    // the sums over the rows in the order of the token path, as below; x[w][c][i]: w 0 keys, 1 queries
-                    float x[2][2][4];
-#pragma unroll
-                    for (int w = 0; w < 2; ++w) {
-#pragma unroll
-                      for (int g8 = 0; g8 < RPT / 8; ++g8) {
-                        uint64_t acc[2][4] = {{0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull}};
-#pragma unroll
-                        for (int r4 = 2 * g8; r4 < 2 * g8 + 2; ++r4)
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                ulonglong2 y = kr[i][r4];
-                                if (w == 1) y = *reinterpret_cast<const ulonglong2 *>(row0 + i * per_tok + part * (RPT + 4) + 4 * r4);
-#pragma unroll
-                                for (int c = 0; c < 2; ++c) {
-                                    acc[c][i] = fma2(S2[c][2 * r4], y.x, acc[c][i]);
-                                    acc[c][i] = fma2(S2[c][2 * r4 + 1], y.y, acc[c][i]);
-                                }
-                            }
-#pragma unroll
-                        for (int c = 0; c < 2; ++c)
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                float lo, hi;
-                                upk2(acc[c][i], lo, hi);
-                                x[w][c][i] = g8 == 0 ? lo + hi : x[w][c][i] + (lo + hi);
-                            }
-                      }
-                    }
-                    // the tree over the eight lanes (xor 1, 2, 4): each step halves what a lane still adds, by its column, then its token
-                    float sk, sq;
-                    {
-                        float y1[2][4], y2[2][2];
-#pragma unroll
-                        for (int w = 0; w < 2; ++w)
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) y1[w][i] = (mine ? x[w][1][i] : x[w][0][i]) + __shfl_xor_sync(0xffffffffu, mine ? x[w][0][i] : x[w][1][i], 1);
-#pragma unroll
-                        for (int w = 0; w < 2; ++w)
-#pragma unroll
-                            for (int i = 0; i < 2; ++i)
-                                y2[w][i] = ((tok & 1) ? y1[w][2 * i + 1] : y1[w][2 * i]) + __shfl_xor_sync(0xffffffffu, (tok & 1) ? y1[w][2 * i] : y1[w][2 * i + 1], 2);
-                        sk = ((tok & 2) ? y2[0][1] : y2[0][0]) + __shfl_xor_sync(0xffffffffu, (tok & 2) ? y2[0][0] : y2[0][1], 4);
-                        sq = ((tok & 2) ? y2[1][1] : y2[1][0]) + __shfl_xor_sync(0xffffffffu, (tok & 2) ? y2[1][0] : y2[1][1], 4);
-                    }
-                    const float4 *cp = reinterpret_cast<const float4 *>(co);
-                    const float4 G = cp[0], be = cp[1], c2 = cp[2], c3 = cp[3], tail = cp[6];
-                    const float kk[6] = {c2.x, c2.y, c2.z, c2.w, c3.x, c3.y}, Gi[4] = {G.x, G.y, G.z, G.w}, bi[4] = {be.x, be.y, be.z, be.w};
-                    const float *vrow = row0 + 2 * DS + col + mine;
-                    float u[4], o = co[tok] * sq, oc[4], vv[4];      // oc: what the token's output takes of u_0 .. u_tok
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        oc[i] = co[i < tok ? 14 + tok * (tok - 1) / 2 + i : 20 + tok];
-                        vv[i] = vrow[i * per_tok];
-                    }
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        float r = fmaf(-Gi[i], __shfl_sync(0xffffffffu, sk, 2 * i + mine, 8), vv[i]);
-#pragma unroll
-                        for (int jj = 0; jj < i; ++jj) r = fmaf(-kk[i * (i - 1) / 2 + jj], u[jj], r);
-                        u[i] = bi[i] * r;
-                        o = i <= tok ? fmaf(oc[i], u[i], o) : o;
-                    }
-                    if (mine_in) a.out[static_cast<int64_t>(q0 + t0 + tk + tok) * H * V + h * V + j + mine] = o;
-                    const uint64_t G3 = pk2(Gi[3], Gi[3]);
-                    uint64_t wr[2][4];                               // the four written rows of both columns
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float m = (i == 0 ? tail.x : i == 1 ? tail.y : i == 2 ? tail.z : 1.f) * u[i], other = __shfl_xor_sync(0xffffffffu, m, 1);
-                        const float m0 = mine ? other : m, m1 = mine ? m : other;
-                        wr[0][i] = pk2(m0, m0);
-                        wr[1][i] = pk2(m1, m1);
-                    }
-#pragma unroll
-                    for (int r4 = 0; r4 < RPT / 4; ++r4)
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            S2[c][2 * r4] = fma2(kr[3][r4].x, wr[c][3], fma2(kr[2][r4].x, wr[c][2], fma2(kr[1][r4].x, wr[c][1], fma2(kr[0][r4].x, wr[c][0], fma2(S2[c][2 * r4], G3, 0ull)))));
-                            S2[c][2 * r4 + 1] =
-                                fma2(kr[3][r4].y, wr[c][3], fma2(kr[2][r4].y, wr[c][2], fma2(kr[1][r4].y, wr[c][1], fma2(kr[0][r4].y, wr[c][0], fma2(S2[c][2 * r4 + 1], G3, 0ull)))));
-                        }
-                }
-#pragma unroll
-                for (int c = 0; c < 2; ++c)
-#pragma unroll
-                    for (int r = 0; r < RPT / 2; ++r) upk2(S2[c][r], SS[c][2 * r], SS[c][2 * r + 1]);
-            } else if constexpr (BLOCKS) {
-                float (&S)[RPT] = SS[0];
-                uint64_t S2[RPT / 2];
-#pragma unroll
-                for (int r = 0; r < RPT / 2; ++r) S2[r] = pk2(S[2 * r], S[2 * r + 1]);
-                for (; tk + kScanBlock <= nt; tk += kScanBlock) {
-                    const float *row0 = buf + tk * per_tok;
-                    const float4 *cp = reinterpret_cast<const float4 *>(coefs + (it & 1) * coefs_per_buf + tk / kScanBlock * kBlockCoefs);
-                    // S^T k_i and S^T q_i: a sum over the rows in the order of the token path (groups of 8 rows, a tree over the groups, the lanes)
-                    float sums[2][4];
-#pragma unroll
-                    for (int w = 0; w < 2; ++w) {
-                        constexpr int G8 = RPT / 8;
-                        float gs[G8][4];
-#pragma unroll
-                        for (int g8 = 0; g8 < G8; ++g8) {
-                            uint64_t acc[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-                            for (int r4 = 2 * g8; r4 < 2 * g8 + 2; ++r4)
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(row0 + i * per_tok + (w == 0 ? DS : 0) + part * (RPT + 4) + 4 * r4);
-                                    acc[i] = fma2(S2[2 * r4], x.x, acc[i]);
-                                    acc[i] = fma2(S2[2 * r4 + 1], x.y, acc[i]);
-                                }
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                float lo, hi;
-                                upk2(acc[i], lo, hi);
-                                gs[g8][i] = lo + hi;
-                            }
-                        }
-#pragma unroll
-                        for (int s = 1; s < G8; s <<= 1)
-#pragma unroll
-                            for (int g8 = 0; g8 < G8; g8 += 2 * s)
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) gs[g8][i] += gs[g8 + s][i];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) sums[w][i] = gs[0][i];
-                    }
-#pragma unroll
-                    for (int s = 32 / PW; s < 32; s <<= 1)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            sums[0][i] += __shfl_xor_sync(0xffffffffu, sums[0][i], s);
-                            sums[1][i] += __shfl_xor_sync(0xffffffffu, sums[1][i], s);
-                        }
-                    const float4 G = cp[0], be = cp[1], c2 = cp[2], c3 = cp[3], c4 = cp[4], self = cp[5], tail = cp[6];
-                    const float kk[6] = {c2.x, c2.y, c2.z, c2.w, c3.x, c3.y}, qk[6] = {c3.z, c3.w, c4.x, c4.y, c4.z, c4.w};
-                    const float Gi[4] = {G.x, G.y, G.z, G.w}, bi[4] = {be.x, be.y, be.z, be.w}, qs[4] = {self.x, self.y, self.z, self.w};
-                    const float *vrow = row0 + 2 * DS + col;
-                    float u[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        float r = fmaf(-Gi[i], sums[0][i], vrow[i * per_tok]), o = Gi[i] * sums[1][i];
-#pragma unroll
-                        for (int jj = 0; jj < i; ++jj) {
-                            r = fmaf(-kk[i * (i - 1) / 2 + jj], u[jj], r);
-                            o = fmaf(qk[i * (i - 1) / 2 + jj], u[jj], o);
-                        }
-                        u[i] = bi[i] * r;
-                        o = fmaf(qs[i], u[i], o);
-                        if (part == 0 && j < V) a.out[static_cast<int64_t>(q0 + t0 + tk + i) * H * V + h * V + j] = o;
-                    }
-                    const uint64_t G3 = pk2(Gi[3], Gi[3]);
-                    const uint64_t w0 = pk2(tail.x * u[0], tail.x * u[0]), w1 = pk2(tail.y * u[1], tail.y * u[1]), w2 = pk2(tail.z * u[2], tail.z * u[2]),
-                                   w3 = pk2(u[3], u[3]);
-#pragma unroll
-                    for (int r4 = 0; r4 < RPT / 4; ++r4) {
-                        const float *kp_ = row0 + DS + part * (RPT + 4) + 4 * r4;
-                        const ulonglong2 k0 = *reinterpret_cast<const ulonglong2 *>(kp_), k1 = *reinterpret_cast<const ulonglong2 *>(kp_ + per_tok),
-                                         k2 = *reinterpret_cast<const ulonglong2 *>(kp_ + 2 * per_tok), k3 = *reinterpret_cast<const ulonglong2 *>(kp_ + 3 * per_tok);
-                        S2[2 * r4] = fma2(k3.x, w3, fma2(k2.x, w2, fma2(k1.x, w1, fma2(k0.x, w0, fma2(S2[2 * r4], G3, 0ull)))));
-                        S2[2 * r4 + 1] = fma2(k3.y, w3, fma2(k2.y, w2, fma2(k1.y, w1, fma2(k0.y, w0, fma2(S2[2 * r4 + 1], G3, 0ull)))));
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < RPT / 2; ++r) upk2(S2[r], S[2 * r], S[2 * r + 1]);
-            }
-            for (; tk < nt; ++tk) {
-#pragma unroll
-              for (int c_ = 0; c_ < NC; ++c_) {
-                float (&S)[RPT] = SS[c_];
+            for (int tk = 0; tk < nt; ++tk) {
                 const float *row = buf + tk * per_tok;
                 const float4 *qr = reinterpret_cast<const float4 *>(row + part * (RPT + 4));
                 const float4 *kr = reinterpret_cast<const float4 *>(row + DS + part * (RPT + 4));
-                const float vj = row[(KIND == 0 ? 3 : 2) * DS + col + c_];
+                const float vj = row[(KIND == 0 ? 3 : 2) * DS + (warp % kScanWarps) * CW + lane % CW];
                 float o;
                 // Both recurrences read the state AFTER the token's write.  With S' = A S + k w^T (A the decay, w the written row):
                 // S'^T q = S^T (A q) + (k . q) w, so the sums over the rows run on the state as the previous token left it and the
@@ -832,7 +512,7 @@ __global__ void __launch_bounds__(64 * kScanWarps, NC == 1 ? 2 : 1) state_scan_k
                         }
                     float sk = gk[0], sq = gq[0];
 #pragma unroll
-                    for (int x = kPart0; x < kPart0 * PW; x <<= 1) {
+                    for (int x = 32 / PW; x < 32; x <<= 1) {
                         sk += __shfl_xor_sync(0xffffffffu, sk, x);
                         sq += __shfl_xor_sync(0xffffffffu, sq, x);
                     }
@@ -847,8 +527,7 @@ __global__ void __launch_bounds__(64 * kScanWarps, NC == 1 ? 2 : 1) state_scan_k
                         S[4 * r4 + 3] = fmaf(g, S[4 * r4 + 3], k4.w * u);
                     }
                 }
-                if (part == 0 && j + c_ < V) a.out[static_cast<int64_t>(q0 + t0 + tk) * H * V + h * V + j + c_] = o;
-              }
+                if (part == 0 && j < V) a.out[static_cast<int64_t>(q0 + t0 + tk) * H * V + h * V + j] = o;
             }
         }
         __syncthreads();
@@ -857,9 +536,7 @@ __global__ void __launch_bounds__(64 * kScanWarps, NC == 1 ? 2 : 1) state_scan_k
 #pragma unroll
         for (int r = 0; r < RPT; ++r) {
             const int i = part * RPT + r;
-#pragma unroll
-            for (int c = 0; c < NC; ++c)
-                if (i < D && j + c < V) S_g[static_cast<int64_t>(i) * V + j + c] = SS[c][r];
+            if (i < D && j < V) S_g[static_cast<int64_t>(i) * V + j] = S[r];
         }
     }
 }
@@ -1303,36 +980,24 @@ bool hyb_state_scan(const atoma_state_scan_args &a, cudaStream_t stream) {
         pw = pw * rpt / 8;
         rpt = 8;
     }
+    const int cols = 32 / pw * kScanWarps;
+    const int per_tok = (gla ? 3 : 2) * pw * (rpt + 4) + cols + 4;
     int64_t longest = a.T;                                   // a bound of the longest portion: T tokens over B sequences, each has one at least
     longest = std::max<int64_t>(1, a.T - (a.B - 1));
-    // no portion of four tokens: the form without blocks; the results are the same
-    const bool blocks = delta && pw * rpt <= 128 && longest >= kScanBlock;
-    const bool pairs = blocks && rpt == 32;                  // 32 columns of a head per CTA all the same, two of 16 rows a lane
-    if (pairs) rpt = 16, pw = 8;
-    const int cols = 32 / pw * kScanWarps * (pairs ? 2 : 1);
-    const int per_tok = (gla ? 3 : 2) * pw * (rpt + 4) + cols + 4;
     // staged tokens per buffer: at most 32, no more than the longest portion, and two CTAs' buffers fit one SM
-    int chunk = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({32, longest, 96 * 1024 / (8 * per_tok)})));
-    if (chunk > kScanBlock) chunk -= chunk % kScanBlock;     // blocks are counted from the portion's first token, whatever the chunk
-    const size_t smem = static_cast<size_t>(2 * chunk * per_tok + 2 * ((chunk + kScanBlock - 1) / kScanBlock) * kBlockCoefs) * 4;
+    const int chunk = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({32, longest, 96 * 1024 / (8 * per_tok)})));
+    const size_t smem = static_cast<size_t>(2 * chunk * per_tok) * 4;
     const dim3 grid(static_cast<unsigned>((a.vdim + cols - 1) / cols), static_cast<unsigned>(a.H), static_cast<unsigned>(a.B));
     const dim3 block(64 * kScanWarps);
     cudaError_t e;
-#define SCAN_RUN(KERNEL)                                                                                                            \
+#define SCAN(TT, KIND, RPT, PW)                                                                                                    \
     do {                                                                                                                            \
-        auto kernel = KERNEL;                                                                                                       \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);                \
-        e = launch_ex(kernel, grid, block, smem, stream, a, chunk);                                                                 \
-    } while (0)
-#define SCAN(TT, KIND, RPT, PW)                                                                                                     \
-    do {                                                                                                                            \
-        constexpr bool kCan = KIND == 1 && RPT * PW <= 128 && RPT != 32;                                                            \
-        SCAN_RUN((blocks ? state_scan_kernel<TT, KIND, RPT, PW, kCan, 1> : state_scan_kernel<TT, KIND, RPT, PW, false, 1>));        \
+        if (smem > 48 * 1024) cudaFuncSetAttribute(state_scan_kernel<TT, KIND, RPT, PW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
+        e = launch_ex(state_scan_kernel<TT, KIND, RPT, PW>, grid, block, smem, stream, a, chunk);                                   \
     } while (0)
 #define SCAN_K(TT, KIND)                                \
     do {                                                \
-        if (pairs) SCAN_RUN((state_scan_kernel<TT, 1, 16, 8, true, 2>)); \
-        else if (rpt == 8 && pw == 8) SCAN(TT, KIND, 8, 8);  \
+        if (rpt == 8 && pw == 8) SCAN(TT, KIND, 8, 8);  \
         else if (rpt == 8 && pw == 16) SCAN(TT, KIND, 8, 16); \
         else if (rpt == 8) SCAN(TT, KIND, 8, 32);       \
         else if (rpt == 16) SCAN(TT, KIND, 16, 4);      \
@@ -1351,7 +1016,6 @@ bool hyb_state_scan(const atoma_state_scan_args &a, cudaStream_t stream) {
 #undef SCAN_T
 #undef SCAN_K
 #undef SCAN
-#undef SCAN_RUN
     return hybrid::launched(e, "state_scan_kernel");
 }
 
