@@ -114,8 +114,8 @@ __device__ __forceinline__ void exp2_poly2(uint64_t x2, float &p0, float &p1) {
     upk2(mul2_ftz(y, scale), p0, p1);
 }
 // P = 2^(s sc - m) of 32 scores as packed 16-bit pairs, and their sum.  MIX: every fourth pair leaves the special-function unit for the FMA
-// pipe (the unit's 16 results a cycle and SM are what bounds the softmax of heads of 64 and 128); tiles with masked scores take the
-// unit for all, which gives their exact zeros.
+// pipe (the unit's 16 results a cycle and SM are what bounds the softmax of heads of 64 and 128).  Tiles with masked scores, and kernels whose FMA pipe
+// adds a bias to every score, take the unit for all (4000 tokens in a window of 1024 with a distance table, heads of 128: 357 us, mixed 362).
 template <typename T, bool MIX>
 __device__ __forceinline__ void softmax_chunk(const uint32_t *sv, uint64_t sc2, uint64_t mm2, uint64_t (&ls)[2], uint32_t (&pk)[16]) {
 #pragma unroll
@@ -161,10 +161,10 @@ __device__ __forceinline__ PfSeq pf_seq(const MhaParams &p, int bidb) {
     return s;
 }
 
-// BIASED: a bias by query-key distance is added to the scaled scores (MhaParams::dist_bias); an instantiation of its own, so
+// BIAS: 1 or 2: a bias by query-key distance is added to the scaled scores (MhaParams::dist_bias); 2: the grid goes head by head.  Instantiations of their own, so
 // that the unbiased kernel keeps its register allocation.
 // PAGED: keys and values lie in pages behind a block table (MhaParams::block_table).
-template <typename T, int D, int KH, bool BIASED, bool PAGED>
+template <typename T, int D, int KH, int BIAS, bool PAGED>
 __global__ void __launch_bounds__(kPfThreads, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const MhaParams p) {
@@ -180,13 +180,16 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __shared__ uint32_t tmem_base_smem;
     __shared__ int late_s;
     volatile int *late = &late_s;
+    constexpr bool BIASED = BIAS != 0;
     __shared__ float bias_s[BIASED ? kPfBiasSmem : 1];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // Heads, then sequences, then query tiles from the last (causal: heaviest) one down, so that the SMs run out of light tiles together
-    // (head by head, one prompt of 8192 x 32 heads kept them 0.86 busy).  Tiles behind a sequence's end leave at once.
-    const int m_block = gridDim.z - 1 - blockIdx.z;
-    const int head = blockIdx.x, bidb = blockIdx.y;
+    // (head by head, one prompt of 8192 x 32 heads kept them 0.86 busy); head by head where a window makes the tiles alike (BIAS 2: chosen
+    // at compile time, as a choice at run time cost 4 to 7 us a call).  Tiles behind a sequence's end leave at once.
+    constexpr bool kByHead = BIAS == 2;
+    const int m_block = kByHead ? gridDim.x - 1 - blockIdx.x : gridDim.z - 1 - blockIdx.z;
+    const int head = kByHead ? blockIdx.y : blockIdx.x, bidb = kByHead ? blockIdx.z : blockIdx.y;
     pdl_wait();
     const PfSeq si = pf_seq(p, bidb);
     if (m_block * kQTiles * kPfM >= si.len_q) return;
@@ -212,7 +215,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tma_prefetch_desc(&map_k);
         tma_prefetch_desc(&map_v);
     }
-    const int bias_n = BIASED ? min(p.dist_rows, kPfBiasSmem) : 0;   // a constant table: read before the grid dependency resolves
+    const int bias_n = BIASED ? min(p.dist_rows, kPfBiasSmem) : 0;
     for (int i = tid; i < bias_n; i += kPfThreads) bias_s[i] = p.dist_bias[static_cast<int64_t>(i) * p.dist_heads + head] * 1.4426950408889634f;
     if (warp == 1) tmem_alloc(&tmem_base_smem, kTmemCols);
     tc_fence_before_sync();
@@ -565,7 +568,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         uint32_t pk[16];
-                        softmax_chunk<T, true>(sv_ + c * 32, sc2, mm2, ls, pk);
+                        softmax_chunk<T, !BIASED>(sv_ + c * 32, sc2, mm2, ls, pk);
                         tmem_st_32x32b_x16(tmem_s + c * 16, pk);
                     }
                 }
@@ -677,13 +680,13 @@ bool make_attn_map(CUtensorMap *out, const void *ptr, int d, int heads, int64_t 
     return true;
 }
 
-template <typename T, int D, int KH, bool BIASED, bool PAGED = false>
+template <typename T, int D, int KH, int BIAS, bool PAGED = false>
 bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const MhaParams &p, cudaStream_t stream) {
     constexpr size_t smem = PfCfg<D, KH>::kSmem;
     static thread_local int attr_dev = -1;
     const DeviceInfo &di = current_device_info();
     if (attr_dev != di.ordinal) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<T, D, KH, BIASED, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<T, D, KH, BIAS, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem));
         if (e != cudaSuccess) {
             set_status(static_cast<int>(e), "prefill: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -692,7 +695,8 @@ bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtens
         attr_dev = di.ordinal;
     }
     dim3 grid(p.h, p.b, (p.seqlen_q + kQTiles * kPfM - 1) / (kQTiles * kPfM));
-    prefill_attn_kernel<T, D, KH, BIASED, PAGED><<<grid, kPfThreads, smem, stream>>>(mq, mk, mv, p);
+    if (BIAS == 2) grid = dim3(grid.z, grid.x, grid.y);
+    prefill_attn_kernel<T, D, KH, BIAS, PAGED><<<grid, kPfThreads, smem, stream>>>(mq, mk, mv, p);
     note_launch();
     return check_launch("prefill_attn_kernel");
 }
@@ -700,8 +704,11 @@ bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtens
 template <typename T, int D>
 bool launch_prefill(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const MhaParams &p,
                     cudaStream_t stream) {
-    return (p.dist_bias && p.dist_rows > 0) ? launch_prefill_b<T, D, D / 64, true>(mq, mk, mv, p, stream)
-                                            : launch_prefill_b<T, D, D / 64, false>(mq, mk, mv, p, stream);
+    if (!p.dist_bias || p.dist_rows <= 0) return launch_prefill_b<T, D, D / 64, 0>(mq, mk, mv, p, stream);
+    // Window of 1024 over 4000 tokens, heads of 128: 340 us head by head, 360 over all heads, heads of 64 302 / 298; window of 256 266 / 278 and 225 / 229;
+    // window of 4096 342 / 311 and 308 / 265.
+    const bool narrow = p.window_left > 0 && static_cast<int64_t>(p.window_left) * (D == 128 ? 3 : 8) <= p.seqlen_q;
+    return narrow || p.seqlen_q <= kQTiles * kPfM ? launch_prefill_b<T, D, D / 64, 2>(mq, mk, mv, p, stream) : launch_prefill_b<T, D, D / 64, 1>(mq, mk, mv, p, stream);
 }
 
 }  // namespace
@@ -739,20 +746,20 @@ int try_launch_prefill_tc(const MhaParams &p, bool is_bf16, cudaStream_t stream)
     if (!make_attn_map(&mq, p.q, d_k, p.h, q_rows, q_b, p.q_hs, p.q_rs, q_bs, is_bf16)) return -1;
     if (p.block_table) {   // keys and values are not read through maps
         bool done;
-        if (is_bf16) done = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 2, false, true>(mq, mq, mq, p, stream)
-                                       : launch_prefill_b<__nv_bfloat16, 64, 1, false, true>(mq, mq, mq, p, stream);
-        else done = p.d == 128 ? launch_prefill_b<__half, 128, 2, false, true>(mq, mq, mq, p, stream)
-                               : launch_prefill_b<__half, 64, 1, false, true>(mq, mq, mq, p, stream);
+        if (is_bf16) done = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 2, 0, true>(mq, mq, mq, p, stream)
+                                       : launch_prefill_b<__nv_bfloat16, 64, 1, 0, true>(mq, mq, mq, p, stream);
+        else done = p.d == 128 ? launch_prefill_b<__half, 128, 2, 0, true>(mq, mq, mq, p, stream)
+                               : launch_prefill_b<__half, 64, 1, 0, true>(mq, mq, mq, p, stream);
         return done ? 1 : -1;
     }
     if (!make_attn_map(&mk, p.k, d_k, p.h_k, k_rows, k_b, p.k_hs, p.k_rs, k_bs, is_bf16)) return -1;
     if (!make_attn_map(&mv, p.v, p.d, p.v_share > 1 ? p.h_k / p.v_share : p.h_k, k_rows, k_b, p.v_hs, p.v_rs, v_bs, is_bf16)) return -1;
     bool ok;
     if (p.d == 128 && d_k <= 64 && is_bf16 && !p.dist_bias)   // shorter query / key heads: one 64-column piece
-        ok = launch_prefill_b<__nv_bfloat16, 128, 1, false>(mq, mk, mv, p, stream);
+        ok = launch_prefill_b<__nv_bfloat16, 128, 1, 0>(mq, mk, mv, p, stream);
     else if ((d_k + 63) / 64 > p.d / 64)   // longer query / key heads than value heads
-        ok = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 3, false>(mq, mk, mv, p, stream)
-                        : launch_prefill_b<__nv_bfloat16, 64, 2, false>(mq, mk, mv, p, stream);
+        ok = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 3, 0>(mq, mk, mv, p, stream)
+                        : launch_prefill_b<__nv_bfloat16, 64, 2, 0>(mq, mk, mv, p, stream);
     else if (is_bf16) ok = p.d == 128 ? launch_prefill<__nv_bfloat16, 128>(mq, mk, mv, p, stream)
                                  : launch_prefill<__nv_bfloat16, 64>(mq, mk, mv, p, stream);
     else ok = p.d == 128 ? launch_prefill<__half, 128>(mq, mk, mv, p, stream)
