@@ -506,9 +506,12 @@ bool launch_gemm_bf16_tn(const void *x, const void *w, void *y, int64_t T, int64
         a.ldy = ldy;
         return launch_skinny_gemm(a, x, w, static_cast<int>(T), K, ldx, ldw, 1, static_cast<int>(N), 1, 0, 0, true, stream);
     }
-    // Prompts go to the CTA pairs (gemm_pair.cu), which are faster from 129 tokens on (x 1.2 to 3 over six weight shapes) but for few tokens
-    // under a long K and few weight rows: 16 tiles of K = 14336 take 62 us at any width, the split-K kernel 54 at 132 tokens, 58 at 160, 77 at 256.
-    const bool few_long = T <= 192 && N <= 4096 && K >= 3 * N;
+    // Prompts go to the CTA pairs (gemm_pair.cu): over 42 weight shapes of 128 to 28672 rows and K of 2048 to 32768 they take 1.05 to 13 times less from
+    // 257 tokens on, and below that except where a wave of few wide tiles leaves pairs idle over a long K.  Split-K kernel / pairs, us: 4096 rows of
+    // K 18432, 129 and 192 tokens 49 / 57 and 59 / 59; 7168 of 18432 59 / 65 and 66 / 66; 6144 of 21504, 129 and 224 tokens 64 / 79 and 72 / 77; 10240 of
+    // 16384 76 / 101 and (208 tokens) 95 / 88.  On the pairs' side of the line: 4096 of 14336 45 / 46 and 54 / 47; 1024 of 8192 52 / 25 and 68 / 25; 16384 of
+    // 16384 105 / 95 and 114 / 101; against it (129 tokens) 2048 of 16384 44 / 46 and 28672 of 16384 170 / 183.
+    const bool few_long = K >= 16384 && T <= (K >= 20480 ? 240 : 192) && N >= 3072 && N <= 12288;
     if (g_gemm_algo != 2 && T > 128 && !few_long && gemm_pair_ok(x, w, N, K, ldx, ldw)) {
         GemmPairArgs a{};
         a.y = y;
