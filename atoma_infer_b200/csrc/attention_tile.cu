@@ -13,6 +13,8 @@
 #include "common.cuh"
 #include "mha_params.h"
 
+#include <algorithm>
+
 namespace atoma {
 namespace {
 
@@ -52,7 +54,7 @@ __global__ void __launch_bounds__(kThreads) attn_tile_kernel(const MhaParams p) 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int m_block = blockIdx.x, head = blockIdx.y, bidb = blockIdx.z;
     const SeqInfo si = seq_info(p, bidb);
-    if (m_block * kBM >= si.len_q) return;
+    if (m_block * kBM >= si.len_q || (p.split_short && !short_for_prefill(p.d, si.len_q, si.len_k))) return;
     const int kvh = head / (p.h / p.h_k);  // flash_fwd_kernel.h:593
     const int len_q = si.len_q, len_k = si.len_k;
     const int causal_shift = len_k - len_q;  // mask.h:171-172 (bottom-right aligned)
@@ -285,7 +287,8 @@ bool launch_tile(const MhaParams &p, cudaStream_t stream) {
                              static_cast<int>(smem));
         attr_dev = di.ordinal;
     }
-    dim3 grid((p.seqlen_q + kBM - 1) / kBM, p.h, p.b);
+    const int longest = p.split_short ? std::min(p.seqlen_q, 128) : p.seqlen_q;   // no longer portion is short
+    dim3 grid((longest + kBM - 1) / kBM, p.h, p.b);
     attn_tile_kernel<T, DP, BN><<<grid, kThreads, smem, stream>>>(p);
     note_launch();
     return check_launch("attn_tile_kernel");

@@ -44,6 +44,9 @@
 #include <vector>
 
 namespace atoma {
+
+bool launch_attention_tile(const MhaParams &p, bool is_bf16, cudaStream_t stream);   // attention_tile.cu
+
 namespace {
 
 constexpr int kPfThreads = 384;  // warpgroup 0: loads (warp 0) + MMA issue (warp 1); warpgroups 1, 2: softmax
@@ -192,7 +195,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int head = kByHead ? blockIdx.y : blockIdx.x, bidb = kByHead ? blockIdx.z : blockIdx.y;
     pdl_wait();
     const PfSeq si = pf_seq(p, bidb);
-    if (m_block * kQTiles * kPfM >= si.len_q) return;
+    if (m_block * kQTiles * kPfM >= si.len_q || (PAGED && p.split_short && short_for_prefill(D, si.len_q, si.len_k))) return;
 
     if (tid == 0) {
         late_s = 0;
@@ -725,6 +728,13 @@ int try_launch_prefill_tc(const MhaParams &p, bool is_bf16, cudaStream_t stream)
     if (p.gate && (!p.cu_q || p.gate_rs % 8 || (reinterpret_cast<uintptr_t>(p.gate) & 15))) return 0;
     const DeviceInfo &di = current_device_info();
     if (di.cc_major != 10) return 0;
+    // Pages: where all sequences are short (by the longest portion and the longest sequence), the tile kernel takes the step: from two pairs of a
+    // sequence and a head per SM on by short_for_prefill(), below that up to 64 keys (4 sequences of 8 heads of 64 over 32, 64, 96 keys, tiles /
+    // prefill kernel: 5 / 7, 6 / 8, 8 / 8 us).  Heads of 64 with six pairs per SM and more: each kernel takes its sequences of a mixed step.  A second
+    // launch costs 10 to 18 us there: one portion of 64 tokens beside 63 decoded ones over 128, 564 and 1064 keys, 32 heads, tiles alone / prefill kernel alone /
+    // both: 58 / 119 / 58, 168 / 220 / 168, 318 / 330 / 338 us.  With heads of 128 it gives back less than that (264 keys: 180 / 211 / 218).
+    const int64_t pairs = p.block_table ? static_cast<int64_t>(p.b) * p.h : 0;
+    if (p.block_table && (pairs >= 2 * di.sm_count ? short_for_prefill(p.d, p.seqlen_q, p.seqlen_k) : p.seqlen_k <= 64)) return 0;
     // TMA: 16-byte aligned bases and strides (run_mha already checked pointers and strides % 8)
     const bool q_varlen = p.cu_q != nullptr;
     const bool k_varlen = p.cu_k != nullptr && p.k_cumulative;
@@ -745,11 +755,14 @@ int try_launch_prefill_tc(const MhaParams &p, bool is_bf16, cudaStream_t stream)
     const int d_k = p.d_k > 0 ? p.d_k : p.d;
     if (!make_attn_map(&mq, p.q, d_k, p.h, q_rows, q_b, p.q_hs, p.q_rs, q_bs, is_bf16)) return -1;
     if (p.block_table) {   // keys and values are not read through maps
+        MhaParams pp = p;
+        pp.split_short = p.d == 64 && p.b > 1 && pairs >= 6 * di.sm_count ? 1 : 0;
         bool done;
-        if (is_bf16) done = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 2, 0, true>(mq, mq, mq, p, stream)
-                                       : launch_prefill_b<__nv_bfloat16, 64, 1, 0, true>(mq, mq, mq, p, stream);
-        else done = p.d == 128 ? launch_prefill_b<__half, 128, 2, 0, true>(mq, mq, mq, p, stream)
-                               : launch_prefill_b<__half, 64, 1, 0, true>(mq, mq, mq, p, stream);
+        if (is_bf16) done = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 2, 0, true>(mq, mq, mq, pp, stream)
+                                       : launch_prefill_b<__nv_bfloat16, 64, 1, 0, true>(mq, mq, mq, pp, stream);
+        else done = p.d == 128 ? launch_prefill_b<__half, 128, 2, 0, true>(mq, mq, mq, pp, stream)
+                               : launch_prefill_b<__half, 64, 1, 0, true>(mq, mq, mq, pp, stream);
+        if (done && pp.split_short) done = launch_attention_tile(pp, is_bf16, stream);
         return done ? 1 : -1;
     }
     if (!make_attn_map(&mk, p.k, d_k, p.h_k, k_rows, k_b, p.k_hs, p.k_rs, k_bs, is_bf16)) return -1;

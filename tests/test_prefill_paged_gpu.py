@@ -42,3 +42,47 @@ def test_same_bits_as_contiguous(D, dtype, H, G, page, news, contexts):
     assert ops.last_mha_path() == "prefill_tc"
     assert torch.equal(got, want)
     assert hybrid_ops.prefill_timeouts() == 0
+
+
+def _check(got, q, k, v, news, contexts):
+    """Against float64; k, v: the sequences' rows one after the other.  Bound: the weights are rounded to 16 bits (2^-8 or 2^-11 of the value at most), as is
+    the result; 1e-5 for the float32 sums."""
+    H, G, D = q.shape[1], k.shape[1], q.shape[2]
+    unit, at, row = 2.0 ** (-8 if q.dtype == torch.bfloat16 else -11), 0, 0
+    for b, (n, c) in enumerate(zip(news, contexts)):
+        i = torch.arange(n + c, device=DEV)
+        kb, vb = (t[row:row + n + c].double().transpose(0, 1).repeat_interleave(H // G, 0) for t in (k, v))
+        s = torch.bmm(q[at:at + n].double().transpose(0, 1), kb.transpose(1, 2)) * D ** -0.5
+        w = torch.softmax(s.masked_fill(i[None, None] > (c + torch.arange(n, device=DEV))[None, :, None], -float("inf")), 2)
+        want, mean = torch.bmm(w, vb).transpose(0, 1), torch.bmm(w, vb.abs()).transpose(0, 1)
+        diff = (got[at:at + n].double() - want).abs()
+        bound = (unit * 1.01 + 1e-5) * mean + unit * 1.01 * want.abs() + 1e-6
+        assert bool((diff <= bound).all()), f"sequence {b}: worst excess {float((diff - bound).max()):.3e}"
+        at, row = at + n, row + n + c
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("news,contexts,path", [
+    # 30 sequences of 32 heads, on both sides of every line of short_for_prefill
+    ((1, 64, 64, 65, 128, 128, 129, 1, 1, 300) * 3, (255, 192, 193, 0, 64, 65, 63, 1023, 1024, 0) * 3, "prefill_tc"),
+    ((33, 1, 64) * 4, (0, 200, 192) * 4, "tile"),      # nothing but short sequences
+])
+def test_short_sequences_of_a_wide_step(D, dtype, news, contexts, path):
+    """Steps of many sequences, whose short ones the tile kernel serves (heads of 64: beside the prefill kernel), against float64."""
+    H, G, page = 32, 8, 16
+    lens = [n + c for n, c in zip(news, contexts)]
+    T = sum(news)
+    q = randn_t((T, H, D), 1, dtype, DEV)
+    each = [-(-n // page) for n in lens]
+    pool = torch.randperm(sum(each), generator=torch.Generator().manual_seed(4)).to(torch.int32)
+    kc, vc = randn_t((sum(each), page, G, D), 2, dtype, DEV), randn_t((sum(each), page, G, D), 3, dtype, DEV)
+    table, used = torch.zeros((len(lens), max(each)), dtype=torch.int32), 0
+    for b, n in enumerate(each):
+        table[b, :n] = pool[used:used + n]
+        used += n
+    starts = lambda x: torch.tensor([sum(x[:i]) for i in range(len(x) + 1)], dtype=torch.int32, device=DEV)
+    got = ops.flash_attn_varlen_with_block_table(q, kc, vc, None, starts(news), starts(lens), max(news), max(lens), D ** -0.5, None, 0, table.to(DEV))
+    assert ops.last_mha_path() == path
+    rows = torch.cat([table[b].long()[torch.arange(n) // page] * page + torch.arange(n) % page for b, n in enumerate(lens)]).to(DEV)
+    _check(got, q, kc.reshape(-1, G, D)[rows], vc.reshape(-1, G, D)[rows], news, contexts)
