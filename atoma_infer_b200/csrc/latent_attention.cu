@@ -8,7 +8,9 @@
 // Softmax with a sink: the running maximum starts at the sink and the running denominator at one (exp(sink - sink)),
 // so the sink is one more term of the denominator that has no key and no value.  Sliding window: keys
 // [max(0, p - window + 1), p].  Scores, weights and sums are float32; keys are visited in position order in
-// tiles that start at the window's first key, so a query's result does not depend on the batch around it.
+// tiles that start at the window's first key.  A portion of two tokens and more goes through one chain of tiles, unless few CTAs have many keys
+// before them (below); a step of decoded tokens goes to the kernel that is faster for its number of sequences and its longest one, and
+// where a sequence's keys are cut there follows the whole step, so that its bits may differ between steps; its rounding error does not.
 #include "common.cuh"
 #include "hybrid_common.cuh"
 #include "mha_params.h"
@@ -728,6 +730,7 @@ bool hyb_head_project(const void *in, const void *w, void *out, int64_t T, int64
 // multiple of 64 up to 256 (four warps) or a multiple of 128 up to 512 (eight warps): at most 8 accumulator tiles per warp and row
 // tile.  Rows of up to 576 entries fit shared memory.  Everything else runs the general kernel.
 bool hyb_latent_decode_ok(const atoma_latent_attn_args &a);                        // latent_decode.cu
+bool hyb_latent_decode_better(const atoma_latent_attn_args &a);
 bool hyb_latent_decode(const atoma_latent_attn_args &a, cudaStream_t stream, bool &taken);
 
 bool hyb_latent_attention_tc(const atoma_latent_attn_args &a, cudaStream_t stream, bool *taken) {
@@ -739,9 +742,8 @@ bool hyb_latent_attention_tc(const atoma_latent_attn_args &a, cudaStream_t strea
         current_device_info().cc_major < 8)
         return true;
     *taken = true;
-    // Decoded tokens: tcgen05 with the cached rows as the wide operand, equal runs of key tiles over the SMs (latent_decode.cu; batch 32, contexts of 2048
-    // to 4096, 32 heads, rows of 576: 74 us; 168 with the kernels below, of which 20 merge the splits).
-    if (!(g_hybrid_debug & 32) && hyb_latent_decode_ok(a)) {
+    // Decoded tokens over many keys: tcgen05 with the cached rows as the wide operand, equal runs of key tiles over the SMs (latent_decode.cu)
+    if (!(g_hybrid_debug & 32) && hyb_latent_decode_ok(a) && ((g_hybrid_debug & 128) || hyb_latent_decode_better(a))) {
         bool has_room;
         const bool ok = hyb_latent_decode(a, stream, has_room);
         if (has_room) return ok;

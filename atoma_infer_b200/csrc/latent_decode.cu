@@ -33,8 +33,9 @@ constexpr int kLdKeys = 64, kLdStages = 2, kLdGroup = 8;   // keys per tile; key
 constexpr int kLdThreads = 192;                             // softmax 0-3, loads 4, products 5
 constexpr int kLdMaxSeqs = 512;
 constexpr int kLdTries = 1 << 18;
-constexpr int kLdOCol = 64, kLdTmem = 256;     // S^T: columns 0.. and 32..; O^T: 32 columns per 128 latent columns from 64 on
+constexpr int kLdPlain = 9;                    // 16-byte loads in flight per lane where a group goes by plain loads
 constexpr float kLdRescale = 8.f;
+constexpr int kLdOCol = 64, kLdTmem = 256;     // S^T: columns 0.. and 32..; O^T: 32 columns per 128 latent columns from 64 on
 
 __device__ unsigned int g_latent_late;
 
@@ -337,18 +338,34 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent
                     break;
                 }
                 unsigned char *dst = ring + st * stage_bytes;
-                // Groups [cut, whole) lie inside the keys that are seen.  The others go by plain loads, with zeros for what is not seen: a hidden row's
-                // weight is 0, which does not make a sum of a row that holds an infinity or NaN.
+                // Groups [cut, whole) lie inside the keys that are seen.  The first one of a window and the one that holds the end go by plain loads, with
+                // zeros for what is not seen (a hidden row's weight is 0, which does not make a sum of a row that holds an infinity or NaN), and what
+                // follows the end is zeros.
                 const int cut = j0 < k_lo ? 1 : 0, whole = max(cut, min(kLdKeys, k_hi - j0) / kLdGroup);
-                for (int g = cut ? 0 : whole; g < kLdKeys / kLdGroup; g = g == 0 && cut ? whole : g + 1) {
-                    const int64_t first = __shfl_sync(0xffffffffu, row, g);
-                    for (int i = lane; i < kLdGroup * pieces; i += 32) {
-                        const int r = i / pieces, c = i - r * pieces, key = j0 + g * kLdGroup + r;
-                        uint4 v = make_uint4(0, 0, 0, 0);
-                        if (key >= k_lo && key < k_hi) v = *reinterpret_cast<const uint4 *>(cache + (first + r) * R + c * 8);
-                        *reinterpret_cast<uint4 *>(dst + g * group_bytes + (c >> 3) * 1024 + r * 128 + (((c & 7) ^ r) << 4)) = v;
+                const int ends = (k_hi - j0 + kLdGroup - 1) / kLdGroup;   // groups from here on hold nothing
+                auto plain = [&](int g) {
+                    const int r = lane >> 2, key = j0 + g * kLdGroup + r;
+                    const bool seen = key >= k_lo && key < k_hi;
+                    const __nv_bfloat16 *src = cache + (static_cast<int64_t>(__shfl_sync(0xffffffffu, row, g)) + r) * R + (lane & 3) * 8;
+                    unsigned char *to = dst + g * group_bytes + r * 128;
+                    for (int k0 = 0; k0 < pieces / 4; k0 += kLdPlain) {
+                        uint4 v[kLdPlain];
+#pragma unroll
+                        for (int k = 0; k < kLdPlain; ++k) {
+                            v[k] = make_uint4(0, 0, 0, 0);
+                            if (seen && k0 + k < pieces / 4) v[k] = *reinterpret_cast<const uint4 *>(src + (k0 + k) * 32);
+                        }
+#pragma unroll
+                        for (int k = 0; k < kLdPlain; ++k) {
+                            const int c = 4 * (k0 + k) + (lane & 3);
+                            if (k0 + k < pieces / 4) *reinterpret_cast<uint4 *>(to + (c >> 3) * 1024 + (((c & 7) ^ r) << 4)) = v[k];
+                        }
                     }
-                }
+                };
+                if (cut) plain(0);
+                if (whole < min(ends, kLdKeys / kLdGroup)) plain(whole);
+                if (ends < kLdKeys / kLdGroup)
+                    for (int i = max(cut, ends) * group_bytes / 16 + lane; i < stage_bytes / 16; i += 32) reinterpret_cast<uint4 *>(dst)[i] = make_uint4(0, 0, 0, 0);
                 fence_proxy_async();   // generic-proxy writes -> visible to the tensor core's async reads
                 __syncwarp();
                 if (elect_one_sync()) mbar_arrive_expect_tx(&full[st], (whole - cut) * group_bytes);
@@ -486,6 +503,18 @@ bool hyb_latent_decode_ok(const atoma_latent_attn_args &a) {
     return a.dtype == ATOMA_DTYPE_BF16 && a.max_query_len == 1 && a.query_start && a.H <= 32 && a.B <= kLdMaxSeqs && a.R % 64 == 0 && a.R >= 128 && a.R <= 576 &&
            rv % 128 == 0 && rv <= 512 && al(a.latent_cache) && al(a.q_lat) && al(a.out) && a.max_blocks * a.block_size < (1ll << 30) && a.block_size % kLdGroup == 0 &&
            current_device_info().cc_major == 10;
+}
+
+// Where this kernel is the faster one, by the longest sequence's tiles.  A CTA pays some 8 us for a sequence's queries and sums whatever it reads, and holds one
+// sequence at a time, so many sequences want several tiles each; and few sequences of narrow rows are cut into so many runs that their merge
+// takes longer than the tiles.  Warp-level kernels / this one, us, 32 heads of 576: 96 sequences of 64, 128, 192 keys 17 / 19, 26 / 31, 35 / 33; 32 of 384
+// and 4096 33 / 28 and 196 / 52; one of 128, 1024, 8192 keys 26 / 15, 35 / 21, 82 / 80.  8 heads of 128: 256 of 192 and 384 keys 19 / 22 and 34 / 27; one of 1024, 2048
+// and 8192 keys 16 / 14, 18 / 20, 29 / 56, four of 8192 32 / 25.
+bool hyb_latent_decode_better(const atoma_latent_attn_args &a) {
+    int64_t span = a.max_seq_len > 0 ? a.max_seq_len : a.max_blocks * a.block_size;
+    if (a.window > 0) span = std::min<int64_t>(span, a.window);
+    const int64_t tiles = (span + kLdKeys - 1) / kLdKeys;
+    return tiles >= 2 + a.B / 96 && (tiles <= a.R / 8 || 2 * a.B * tiles >= 5 * current_device_info().sm_count);
 }
 
 // `taken`: false where there is no workspace for the runs' sums (the caller's other kernels may need none).

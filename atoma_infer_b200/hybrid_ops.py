@@ -32,7 +32,8 @@ def _check():
 def debug_flags(flags: int) -> None:
     """bit 0: plain float32 GEMM everywhere; bit 1: general attention kernel only; bit 2: sequential minGRU scan;
     bit 3: unused; bit 4: scans with many rows per lane; bit 5: latent attention of decoded tokens on the warp-level
-    kernel; bit 6: the talking heads' mix on CUDA cores."""
+    kernel; bit 6: the talking heads' mix on CUDA cores; bit 7: latent attention of decoded tokens on the tensor-memory
+    kernel."""
     _lib.lib().atoma_debug_hybrid(int(flags))
 
 

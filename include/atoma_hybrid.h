@@ -875,10 +875,11 @@ int64_t atoma_hybrid_scratch_bytes(const atoma_hybrid_model *model, int64_t num_
 void atoma_hybrid_step(const atoma_hybrid_model *model, const atoma_hybrid_batch *batch, atoma_stream_t stream);
 
 /* Diagnostics: bit 0 = every projection through the plain float32-FMA kernel; bit 1 = the general attention kernel
- * for every batch (no tensor-core prefill / split decode kernels); bit 2 = the sequential minGRU scan; bit 3 = the routed
- * experts' tensor-memory (tcgen05) products for steps of any size (they normally serve steps of 1024 pairs and more);
- * bit 4 = the matrix-state scans with many rows per lane whatever the step's size (they normally take 8 rows per lane when a
- * step has few CTAs; both add in the same order). */
+ * for every batch (no tensor-core prefill / split decode kernels, no row operators on 16-byte pieces); bit 2 = the sequential minGRU scan;
+ * bit 3: unused; bit 4 = the matrix-state scans with many rows per lane whatever the step's size (they normally take 8 rows per lane when a
+ * step has few CTAs; both add in the same order); bit 5 = latent attention of decoded tokens on the warp-level kernel whatever the step's size;
+ * bit 6 = the mix of talking heads on CUDA cores; bit 7 = latent attention of decoded tokens on the tensor-memory kernel whatever the step's
+ * size. */
 void atoma_debug_hybrid(int flags);
 
 /* CTAs of the tensor-memory prefill attention kernel that gave up a wait since the library was loaded (0 unless something is broken;
