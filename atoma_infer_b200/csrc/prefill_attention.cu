@@ -184,6 +184,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __shared__ int late_s;
     volatile int *late = &late_s;
     constexpr bool BIASED = BIAS != 0;
+    // Paged steps correct by every new maximum: a row's largest weight is then 1, which rounding to 16 bits leaves alone, as on the tile kernel, whose steps
+    // these are (error against 64 bits of bfloat16 portions, queries of 1 and 4 times unit size: 2.08e-3 and 1.73e-3 there, 2.09e-3 and 1.74e-3 here,
+    // 2.13e-3 and 2.09e-3 with corrections from 2^8 on; the portions of prompts over prefixes 180 -> 190 us).
+    constexpr float kThreshold = PAGED ? 0.f : kRescaleThreshold;
     __shared__ float bias_s[BIASED ? kPfBiasSmem : 1];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -533,8 +537,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 for (int i = 0; i < 8; ++i) mx8[i] = fmaxf(mx8[i], __uint_as_float(sv_[120 + i]));
                 const float mx = fmaxf(max3(mx8[0], mx8[1], mx8[2]), fmaxf(max3(mx8[3], mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7])));
                 const float m_tile = mx * sc;  // scale_log2 > 0 (checked on the host)
-                // ---- lazy running maximum ----
-                const bool need = m_tile > m_ref + kRescaleThreshold;  // also the first finite tile (m_ref = -inf)
+                // ---- running maximum ----
+                const bool need = m_tile > m_ref + kThreshold;  // also the first finite tile (m_ref = -inf)
                 if (__any_sync(0xffffffffu, need)) {
                     const float alpha = need ? (m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - m_tile)) : 1.f;
                     if (need) m_ref = m_tile;
