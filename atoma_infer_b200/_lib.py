@@ -412,6 +412,7 @@ SIGNATURES = {
     "atoma_set_launch_mode": (None, [C.c_int]),
     "atoma_get_launch_mode": (C.c_int, []),
     "atoma_last_status": (C.c_int, []),
+    "atoma_kernel_timeouts": (C.c_int, []),
     "atoma_last_error": (C.c_char_p, []),
     "atoma_last_mha_path": (C.c_char_p, []),
     "atoma_last_decode_mode": (C.c_int, []),

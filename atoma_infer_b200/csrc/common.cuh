@@ -47,6 +47,9 @@ enum : int { kWorkspaceDecode = 0, kWorkspaceSwapMap = 1, kWorkspaceGemm = 2, kW
 void *get_workspace(cudaStream_t stream, size_t bytes, int tag);
 // The same for a caller that can do without: nullptr and no error where there is none (no memory, or a stream being captured before the first call).
 void *try_workspace(cudaStream_t stream, size_t bytes, int tag);
+// A word in mapped host memory that a kernel sets to 1 when one of its waits ran out (atoma_kernel_timeouts reads it without a synchronisation); nullptr if
+// there is no such memory.
+unsigned int *late_word();
 
 // Launch mode (process-wide, atoma_set_launch_mode): programmatic dependent launch between this
 // library's kernels, "weights are immutable" (the GEMM may prefetch W before its grid dependency
@@ -329,9 +332,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
-// ---- packed float32 pairs: one issue slot for two operations ----
-__device__ __forceinline__ uint64_t pk2(float lo, float hi) {
-    uint64_t r;
 // n / (1 + e) for e >= 0 (inf and NaN included), 1 ulp: the reciprocal unit's estimate, one step of Newton's iteration, one product.  For
 // epilogues that divide per element, where the compiler's division takes three times the instructions and a branch.  Where e passes 2^126
 // it divides by 2^126 (the quotient is below n times the smallest normal number either way).
@@ -342,6 +342,9 @@ __device__ __forceinline__ float over_one_plus(float n, float e) {
     return n * fmaf(r, fmaf(-d, r, 1.f), r);
 }
 
+// ---- packed float32 pairs: one issue slot for two operations ----
+__device__ __forceinline__ uint64_t pk2(float lo, float hi) {
+    uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
     return r;
 }

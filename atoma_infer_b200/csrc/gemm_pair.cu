@@ -20,7 +20,7 @@
 // 4096 to 2 x 14336: 24 launches of 128 tokens 1400 / 480.
 //
 // Every wait is bounded: one that runs out raises a flag, the CTA's other roles stop waiting, the loads' warp waits (again with a bound)
-// for its copies, tensor memory is freed and a counter is raised (atoma_gemm_pair_timeouts).
+// for its copies, tensor memory is freed, a counter is raised (atoma_gemm_pair_timeouts) and the host is told (atoma_kernel_timeouts).
 #include "common.cuh"
 #include "gemm_pair.h"
 #include "hybrid_common.cuh"
@@ -371,7 +371,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
     if (tid == 0 && *late) {
         atomicAdd(&g_pair_late, 1u);
-        if (a.error) *a.error = 1;
+        if (a.late) *reinterpret_cast<volatile unsigned int *>(a.late) = 1;
     }
 }
 
@@ -458,6 +458,7 @@ int gemm_pair_width(int64_t T, int64_t N, int64_t K, bool glu) {
 // output, the activation and, when grouped, plan / tiles (an upper bound) filled in.
 bool launch_gemm_pair(GemmPairArgs a, const void *x, const void *w, int64_t rows, int64_t N, int64_t K, int64_t ldx, int64_t ldw, int64_t experts, bool glu,
                       bool is_bf16, cudaStream_t stream) {
+    a.late = late_word();
     a.N = static_cast<int>(N);
     a.K = static_cast<int>(K);
     a.is_bf16 = is_bf16 ? 1 : 0;

@@ -21,10 +21,10 @@ struct GemmPairArgs {
     const int32_t *plan;
     const int32_t *row_pair;      // with out_weight: row r is scaled by out_weight[row_pair[r]] (negative: zero)
     const float *out_weight;
-    int *error;                   // set to 1 when a wait ran out (may be null)
     int tiles, max_width;         // grouped: upper bounds of the tiles and of a chunk's width (a multiple of 32)
     int w_once;                   // the weights are read once: they need not stay in L2
     // filled in by launch_gemm_pair
+    unsigned int *late;           // set to 1 when a wait ran out (late_word())
     int T, N, K, is_bf16, w_tiles, stages, stage_bytes, kbs, k_blocked;
 };
 

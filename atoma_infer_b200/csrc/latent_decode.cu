@@ -17,7 +17,7 @@
 // 4096: 3.015e-3; rescaled from 2^8 on 3.061e-3 and 2 us less of 80).
 //
 // Every wait is bounded: one that runs out raises a flag, the other roles stop waiting, the loads land, tensor memory is freed and a
-// counter is raised (atoma_latent_decode_timeouts).
+// counter is raised (atoma_latent_decode_timeouts, atoma_kernel_timeouts).
 #include "common.cuh"
 #include "hybrid_common.cuh"
 
@@ -83,7 +83,8 @@ __device__ __forceinline__ int ld_span(const atoma_latent_attn_args &a, int b, i
 
 template <int NH>   // heads, padded: 16 or 32
 __global__ void __launch_bounds__(kLdThreads, 1)
-latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent_attn_args a, float *__restrict__ partial, float *__restrict__ partial_ml, int *__restrict__ prefix_out) {
+latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent_attn_args a, float *__restrict__ partial, float *__restrict__ partial_ml, int *__restrict__ prefix_out,
+                     unsigned int *late_out) {
     constexpr int kParts = 128 / NH, kPart = kLdKeys / kParts;   // keys of a tile per softmax thread: 8 or 16
     constexpr int kSLd = NH + 1;
     extern __shared__ unsigned char smem_dyn[];
@@ -446,7 +447,10 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, kLdTmem);
     }
-    if (tid == 0 && *late) atomicAdd(&g_latent_late, 1u);
+    if (tid == 0 && *late) {
+        atomicAdd(&g_latent_late, 1u);
+        if (late_out) *reinterpret_cast<volatile unsigned int *>(late_out) = 1;
+    }
 }
 
 // The runs of a sequence that several CTAs shared, in CTA order: M = max m, out = sum acc 2^(m - M) / sum l 2^(m - M).  A CTA takes 32 columns of
@@ -548,7 +552,7 @@ bool hyb_latent_decode(const atoma_latent_attn_args &a, cudaStream_t stream, boo
         set_status(static_cast<int>(e), "latent_decode_kernel: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         return false;
     }
-    if (!hybrid::launched(launch_ex(kernel, dim3(std::max(grid, 1)), dim3(kLdThreads), smem, stream, map, a, ws, ml, prefix), "latent_decode_kernel")) return false;
+    if (!hybrid::launched(launch_ex(kernel, dim3(std::max(grid, 1)), dim3(kLdThreads), smem, stream, map, a, ws, ml, prefix, late_word()), "latent_decode_kernel")) return false;
     const dim3 mgrid(static_cast<unsigned>(rv / 32), static_cast<unsigned>(a.B));
     return hybrid::launched(launch_ex(nh == 16 ? latent_decode_merge_kernel<16> : latent_decode_merge_kernel<32>, mgrid, dim3(nh * 8), 0, stream, a,
                                       static_cast<const float *>(ws), static_cast<const float *>(ml), static_cast<const int *>(prefix), std::max(grid, 1)),

@@ -54,6 +54,7 @@ struct MhaParams {
     int v_share;
     // a paged step that both prompt kernels serve: attn_tile_kernel the sequences with short_for_prefill(), prefill_attn_kernel the others
     int split_short;
+    unsigned int *late;   // set by the prefill kernel's launcher: where it says that a wait ran out (late_word())
 };
 
 // Sequences of a paged step of many (sequence, head) pairs that are faster on the 64-row tiles, several of which share an SM, than on

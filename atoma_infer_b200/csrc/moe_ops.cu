@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(32) moe_route_grouped_kernel(const float *__re
 
 // ---------------------------------------------------------------------------------------------
 // pairs -> expert segments (one CTA)
-// meta[0] = row tiles in use, meta[1] = rows in use (padded), meta[2] = error word of the grouped products (reset here)
+// meta[0] = row tiles in use, meta[1] = rows in use (padded)
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t *__restrict__ top_expert, int32_t *__restrict__ pair_row,
                                                         int32_t *__restrict__ row_pair, int32_t *__restrict__ tile_expert,
@@ -291,7 +291,6 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t *__restric
         }
         meta[0] = row / tile_rows;
         meta[1] = row;
-        meta[2] = 0;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
@@ -307,7 +306,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t *__restric
 }
 
 // The same for the CTA pairs' products: dense segments, and their chunks of up to chunk_rows rows (a multiple of 32), evenly cut (an
-// expert's 375 rows are chunks of 192 and 183).  plan[0] = chunks, plan[1] = error word (reset here); from plan[4] on
+// expert's 375 rows are chunks of 192 and 183).  plan[0] = chunks; from plan[4] on
 // {expert, first row, rows, width: rows rounded up to 32}.
 // One cluster of eight CTAs counts an eighth of the pairs each and reads the others' counts through distributed shared memory: what
 // bounds it is the latency of its few passes, not bytes (24000 pairs over 64 experts: one CTA 41 us, the cluster 13).
@@ -386,10 +385,7 @@ moe_plan_kernel(const int32_t *__restrict__ top_expert, int32_t *__restrict__ pa
             __syncthreads();
             base = base_s;
         }
-        if (tid == 0) {
-            plan[0] = base;
-            plan[1] = 0;
-        }
+        if (tid == 0) plan[0] = base;
     }
     __syncthreads();
     for (int i = p0 + tid; i < p1; i += 1024) {
@@ -675,14 +671,14 @@ bool hyb_moe_experts(const atoma_moe_args &a, const void **expert_out, const int
         GemmPairArgs g{};
         g.y = s.act, g.ldy = a.ff;
         g.act = kPairClamped, g.limit = a.limit, g.alpha = a.alpha, g.shift = a.up_shift;
-        g.plan = s.meta, g.error = s.meta + 1;
+        g.plan = s.meta;
         g.max_width = plan_chunk_rows(a.T);
         g.w_once = a.T <= 256;
         g.tiles = static_cast<int>(s.max_tiles) * gemm_pair_w_tiles(a.ff, true);
         if (!launch_gemm_pair(g, s.xs, a.w_gate_up, s.max_rows, a.ff, a.width, a.width, a.width, a.experts, true, true, stream)) return false;
         GemmPairArgs d{};
         d.y = s.y, d.ldy = a.width;
-        d.plan = s.meta, d.error = s.meta + 1;
+        d.plan = s.meta;
         d.row_pair = s.row_pair, d.out_weight = ow;
         d.max_width = g.max_width, d.w_once = g.w_once;
         d.tiles = static_cast<int>(s.max_tiles) * gemm_pair_w_tiles(a.width, false);

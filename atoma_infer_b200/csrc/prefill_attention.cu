@@ -25,7 +25,7 @@
 //    two query tiles, one key and two value stages take 208 KB of shared memory);
 //  * every wait is bounded: a wait that runs out stops the CTA's loads and lets its other roles run through,
 //    its copies in flight are waited for (again with a bound), tensor memory is freed and a counter is
-//    raised that the host can read (atoma_prefill_timeouts); the CTA's outputs mean nothing then.
+//    raised that the host can read (atoma_prefill_timeouts, atoma_kernel_timeouts); the CTA's outputs mean nothing then.
 //
 //  * paged keys and values (PAGED): two more warps look the pages up and copy rows of 16-byte pieces with cp.async into the same
 //    swizzled tiles (a page's rows of one head are strided: no box of a tensor map covers a tile of pages in any order);
@@ -641,7 +641,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, kTmemCols);
     }
-    if (tid == 0 && *late) atomicAdd(&g_prefill_late, 1u);
+    if (tid == 0 && *late) {
+        atomicAdd(&g_prefill_late, 1u);
+        if (p.late) *reinterpret_cast<volatile unsigned int *>(p.late) = 1;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -701,9 +704,11 @@ bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtens
         }
         attr_dev = di.ordinal;
     }
+    MhaParams pp = p;
+    pp.late = late_word();
     dim3 grid(p.h, p.b, (p.seqlen_q + kQTiles * kPfM - 1) / (kQTiles * kPfM));
     if (BIAS == 2) grid = dim3(grid.z, grid.x, grid.y);
-    prefill_attn_kernel<T, D, KH, BIAS, PAGED><<<grid, kPfThreads, smem, stream>>>(mq, mk, mv, p);
+    prefill_attn_kernel<T, D, KH, BIAS, PAGED><<<grid, kPfThreads, smem, stream>>>(mq, mk, mv, pp);
     note_launch();
     return check_launch("prefill_attn_kernel");
 }

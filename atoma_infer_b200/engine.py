@@ -13,7 +13,7 @@ from typing import Dict, Iterable, List, Optional, Sequence as Seq_, Tuple
 
 import torch
 
-from . import checkpoint, models
+from . import _lib, checkpoint, models
 from .cache import CacheManager
 from .models import CacheConfig
 from .ops import AtomaError
@@ -74,7 +74,13 @@ class Engine:
         return self.scheduler.has_work()
 
     # ---- steps ----
+    @staticmethod
+    def _check_waits() -> None:
+        if _lib.lib().atoma_kernel_timeouts():
+            raise AtomaError("a kernel gave up waiting for its data: the outputs of the steps since then mean nothing")
+
     def _run(self, plan: StepPlan, **kw):
+        self._check_waits()
         out = self.executor.execute(plan, **kw)
         self.scheduler.commit(plan)
         return out
@@ -90,6 +96,7 @@ class Engine:
         results: List[RequestOutput] = []
         if out.next_tokens is not None:
             toks = out.next_tokens.cpu().tolist()      # the step's one device-to-host read
+            self._check_waits()
             for (seq_id, _), tok in zip(out.rows, toks):
                 seq = self.sequences[seq_id]
                 seq.tokens.append(int(tok))

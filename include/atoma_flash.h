@@ -257,6 +257,9 @@ void atoma_debug_gemm_algo(int algo);
 int atoma_last_status(void);
 /* Human-readable text for the last non-zero status on this thread ("" if none). */
 const char *atoma_last_error(void);
+/* 1 once a kernel of this process has given up a bounded wait: outputs of the step it ran in mean nothing.  The kernel sets it in mapped host memory, so it
+ * is there when the step's results have been waited for; the call asks no device. */
+int atoma_kernel_timeouts(void);
 /* Name of the kernel path the last run_mha on this thread dispatched to (for tests/bench). */
 const char *atoma_last_mha_path(void);
 /* How the last paged decode launch of this thread ran: bit 0 = early KV streaming (ATOMA_CALL_STABLE_CACHE

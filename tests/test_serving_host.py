@@ -205,3 +205,28 @@ def test_engine_forced_steps_admit_extend_and_end():
     assert "a" not in eng.sequences and eng.cache.live == 1
     eng.step_forced([("c", [1] * 9, [])])
     assert eng.cache.get("c").state_slot == 0      # a's slot, used again
+
+
+def test_engine_stops_where_a_kernel_gave_up_waiting(monkeypatch):
+    """The step whose kernel ran out of a wait returns nothing, and no later one runs."""
+    from types import SimpleNamespace
+
+    from atoma_infer_b200 import engine
+
+    late = []
+    monkeypatch.setattr(engine._lib, "lib", lambda: SimpleNamespace(atoma_kernel_timeouts=lambda: len(late)))
+
+    class Executor(_CountingExecutor):
+        def execute(self, plan, **kw):
+            if len(self.batches) == 1:
+                late.append(1)
+            return super().execute(plan, **kw)
+
+    ex = Executor()
+    eng = Engine(ex, CacheManager(8, 4, 2))
+    eng.add_request([1, 2, 3], SamplingParams(5))
+    assert len(eng.step()) == 1
+    for _ in range(2):
+        with pytest.raises(AtomaError, match="gave up waiting"):
+            eng.step()
+    assert len(ex.batches) == 2 and len(next(iter(eng.sequences.values())).generated) == 1
