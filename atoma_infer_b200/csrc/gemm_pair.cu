@@ -499,7 +499,9 @@ bool launch_gemm_pair(GemmPairArgs a, const void *x, const void *w, int64_t rows
         if (!gp_map(&mx.m[i], kx)) return false;
     }
     if (is_bf16) return glu ? gp_launch<__nv_bfloat16, true>(mw, mx, a, stream) : gp_launch<__nv_bfloat16, false>(mw, mx, a, stream);
-    return glu ? gp_launch<__half, true>(mw, mx, a, stream) : gp_launch<__half, false>(mw, mx, a, stream);
+    if (glu) return gp_launch<__half, true>(mw, mx, a, stream);
+    set_status(kErrUnsupported, "gemm_pair: float16 with the gated activation only");
+    return false;
 }
 
 // Operands this path takes (strides in elements).
