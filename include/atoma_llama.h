@@ -31,7 +31,8 @@ extern "C" {
 /*
  * y[T,N] = x[T,K] w[N,K]^T for any 16-bit dtype (atoma_gemm_bf16_tn with a dtype argument).
  * T <= 128 with K % 64 == 0 runs the decode-time weight-streaming kernel (gemm_skinny.cu: no split-K,
- * tile width chosen to fill one wave of SMs); other shapes run the stream-K kernel (gemm_bf16.cu).
+ * tile width chosen to fill one wave of SMs).  bfloat16 beyond that: T > 128 with rows of whole 16-byte pieces and K >= 64 runs on CTA pairs
+ * (gemm_pair.cu) but for few tokens under a long K, everything else the stream-K kernel (gemm_bf16.cu).  float16 beyond it is refused.
  */
 void atoma_gemm_tn(const void *x, const void *w, void *y, int64_t T, int64_t N, int64_t K, int64_t ldx,
                    int64_t ldw, int64_t ldy, uint32_t dtype, atoma_stream_t stream);
@@ -46,7 +47,7 @@ void atoma_gemm_tn(const void *x, const void *w, void *y, int64_t T, int64_t N, 
  *   v of token t are also written to key_cache / value_cache [NB, block_size, Hkv, D] at
  *   slot_mapping[t] (slot < 0: skipped; slot_mapping or the caches may be NULL: no cache write) —
  *   bit-identical to atoma_gemm_tn + atoma_rope_reshape_and_cache.
- * T > 128: the CTA-pair GEMM with the activation in its epilogue.
+ * T > 128 is processed in 128-row passes.
  */
 void atoma_qkv_rope_cache(const void *x, const void *wqkv, void *qkv, int64_t T, int64_t K, int64_t ldx,
                           int64_t ldw, int64_t ldy, int64_t num_heads, int64_t num_kv_heads,
@@ -60,6 +61,7 @@ void atoma_qkv_rope_cache(const void *x, const void *wqkv, void *qkv, int64_t T,
  *   y[T, inter] = silu(x w_gate^T) * (x w_up^T), w_gate_up = [W_gate; W_up] stacked along N
  *   ([2 inter, K]); both projections are rounded to the model dtype first (the reference
  *   materialises them), silu(g) * u is evaluated in fp32 and rounded once.
+ * T > 128: the CTA-pair GEMM (gemm_pair.cu) with the activation in its epilogue, in all three forms.
  */
 void atoma_gate_up_silu(const void *x, const void *w_gate_up, void *y, int64_t T, int64_t inter, int64_t K,
                         int64_t ldx, int64_t ldw, int64_t ldy, uint32_t dtype, atoma_stream_t stream);
