@@ -160,12 +160,15 @@ void *workspace(cudaStream_t stream, size_t bytes, int tag, bool report) {
     static WorkspacePool pool;
     int dev = 0;
     cudaGetDevice(&dev);
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(stream, &cap);
-    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    bool capturing = false;
     cudaError_t e = cudaSuccess;
     size_t asked = bytes;
-    void *p = pool.get(WorkspacePool::Key(dev, tag, stream), bytes, !capturing, [&](size_t size) -> void * {
+    auto may_grow = [&] {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        cudaStreamIsCapturing(stream, &cap);
+        return !(capturing = cap != cudaStreamCaptureStatusNone);
+    };
+    void *p = pool.get(WorkspacePool::Key(dev, tag, stream), bytes, may_grow, [&](size_t size) -> void * {
         void *block = nullptr;
         asked = size;
         e = cudaMalloc(&block, size);

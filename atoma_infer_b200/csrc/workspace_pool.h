@@ -16,13 +16,14 @@ class WorkspacePool {
   public:
     using Key = std::tuple<int, int, const void *>;
 
-    // alloc(bytes) returns a new block or nullptr; may_grow: whether it may be called at all.  nullptr: there is no block of that size.
-    template <typename Alloc>
-    void *get(const Key &key, size_t bytes, bool may_grow, Alloc alloc) {
+    // alloc(bytes) returns a new block or nullptr; may_grow(), asked only where the block at hand is too small: whether it may be called at all.
+    // nullptr: there is no block of that size.
+    template <typename MayGrow, typename Alloc>
+    void *get(const Key &key, size_t bytes, MayGrow may_grow, Alloc alloc) {
         std::lock_guard<std::mutex> lock(mu_);
         Block &b = blocks_[key];
         if (b.size >= bytes && b.ptr) return b.ptr;
-        if (!may_grow) return nullptr;
+        if (!may_grow()) return nullptr;
         const size_t exact = round_up(std::max<size_t>(bytes, 1)), roomy = std::max(exact, round_up(b.size + b.size / 2));
         size_t size = roomy;
         void *p = alloc(size);

@@ -25,27 +25,31 @@ int main() {
         next += n;
         return next;
     };
-    void *first = pool.get(a, 9 * MB + 1, true, alloc);
+    int asked = 0;
+    auto yes = [&] { ++asked; return true; };
+    auto no = [&] { ++asked; return false; };
+    void *first = pool.get(a, 9 * MB + 1, yes, alloc);
     EXPECT(first && room == 30 * MB);
-    EXPECT(pool.get(a, 10 * MB, true, alloc) == first && calls == 1);       // rounded up to whole MiB
+    EXPECT(asked == 1);
+    EXPECT(pool.get(a, 10 * MB, yes, alloc) == first && calls == 1 && asked == 1);       // rounded up to whole MiB; a block that fits asks nothing
     // a growth that fails: the block that was there still serves what fits it, and nothing was lost
-    EXPECT(pool.get(a, 31 * MB, true, alloc) == nullptr && room == 30 * MB);
-    EXPECT(pool.get(a, 10 * MB, true, alloc) == first && room == 30 * MB);
+    EXPECT(pool.get(a, 31 * MB, yes, alloc) == nullptr && room == 30 * MB);
+    EXPECT(pool.get(a, 10 * MB, yes, alloc) == first && room == 30 * MB);
     for (int i = 0; i < 100; ++i) {
-        EXPECT(pool.get(a, 31 * MB, true, alloc) == nullptr);
-        EXPECT(pool.get(a, 5 * MB, true, alloc) == first);
+        EXPECT(pool.get(a, 31 * MB, yes, alloc) == nullptr);
+        EXPECT(pool.get(a, 5 * MB, yes, alloc) == first);
     }
     EXPECT(room == 30 * MB);
     // not allowed to grow (a stream that is being captured): the block as it is, or none; the allocator is not asked
     calls = 0;
-    EXPECT(pool.get(a, 10 * MB, false, alloc) == first && pool.get(a, 11 * MB, false, alloc) == nullptr && pool.get(b, 1, false, alloc) == nullptr && calls == 0);
+    EXPECT(pool.get(a, 10 * MB, no, alloc) == first && pool.get(a, 11 * MB, no, alloc) == nullptr && pool.get(b, 1, no, alloc) == nullptr && calls == 0);
     // a growth is by half at least, so that many small ones do not set many blocks aside; where that is too much, what is asked for
-    EXPECT(pool.get(a, 10 * MB + 1, true, alloc) != first && room == 15 * MB);
-    EXPECT(pool.get(a, 15 * MB, true, alloc) != nullptr && room == 15 * MB);
-    EXPECT(pool.get(b, 6 * MB, true, alloc) != nullptr && room == 9 * MB);
-    EXPECT(pool.get(b, 8 * MB, true, alloc) != nullptr && room == 0);
+    EXPECT(pool.get(a, 10 * MB + 1, yes, alloc) != first && room == 15 * MB);
+    EXPECT(pool.get(a, 15 * MB, yes, alloc) != nullptr && room == 15 * MB);
+    EXPECT(pool.get(b, 6 * MB, yes, alloc) != nullptr && room == 9 * MB);
+    EXPECT(pool.get(b, 8 * MB, yes, alloc) != nullptr && room == 0);
     room = 8 * MB + MB / 2;
-    EXPECT(pool.get(b, 9 * MB + 1, true, alloc) == nullptr && pool.get(b, 9 * MB, true, alloc) != nullptr && room == 8 * MB + MB / 2);
+    EXPECT(pool.get(b, 9 * MB + 1, yes, alloc) == nullptr && pool.get(b, 9 * MB, yes, alloc) != nullptr && room == 8 * MB + MB / 2);
     std::printf("ok\n");
     return 0;
 }
