@@ -1,10 +1,10 @@
-// One-shot all-reduce(sum) over NVLink peer memory for the tensor-parallel path (SURVEY §8 row f4).
+// One-shot all-reduce(sum) over NVLink peer memory for the tensor-parallel path.
 //
 // Replaces, for the [T, hidden] 16-bit payload that follows o_proj (and down_proj), the reference's
 // `comm.all_reduce(src, &mut dst, &ReduceOp::Sum)` through cudarc/NCCL (models/src/multi_gpu.rs:
 // 141-179).  The payload is 256 KiB at batch 32: a latency-bound collective (NVLink 5 moves it in
-// 0.3 us) for which ncclAllReduce measures 21.3 us on 2 x B200 inside a CUDA graph
-// (scripts/nccl_diag.py).  A flag handshake followed by remote loads (a first version of this file)
+// 0.3 us) for which ncclAllReduce measures 21.3 us on 2 x B200 inside a CUDA
+// graph.  A flag handshake followed by remote loads (a first version of this file)
 // costs three NVLink flights, 11.7 us.  This kernel needs ONE flight: data and flag travel in the
 // same store.
 //

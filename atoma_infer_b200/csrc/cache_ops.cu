@@ -226,7 +226,7 @@ __global__ void reshape_and_cache_flash_scalar_kernel(
 
 
 // ---------------------------------------------------------------------------------------------
-// Fused rotary embedding + cache write (SURVEY §8 row f1)
+// Fused rotary embedding + cache write
 // ---------------------------------------------------------------------------------------------
 // What the reference does with two index_select, two rope kernels, four transpose+contiguous copies
 // and reshape_and_cache_flash (models/src/llama.rs:218-251, 269-304; flash_attention.rs:361) in one

@@ -3,7 +3,7 @@
 // Replaces, for run_mha calls with a block table and seqlen_q == 1, the reference's
 // flash_fwd_splitkv_kernel + flash_fwd_splitkv_combine_kernel pair
 // (csrc/kernels/flash_fwd_kernel.h:504-1092, :1131-1313, launched from
-// flash_fwd_launch_template.h:105-177) — "paged attention v1/v2" in BASELINE.json's wording.
+// flash_fwd_launch_template.h:105-177) — paged attention v1 / v2.
 // Same contract: O[b,h,:] = softmax(scale * q[b,h,:] . K_b[:, h/G, :]^T) V_b over the first
 // seqlens_k[b] cached tokens, gathered through block_table[b, :]; fp32 scores/softmax, P rounded
 // to the 16-bit type before P.V, fp32 accumulation (flash_fwd_kernel.h:949-954).
@@ -17,13 +17,13 @@
 //    out of the reference's [num_blocks, block_size, num_kv_heads, head_size] cache layout.  For
 //    D = 128 the cache is described as a 5-D tensor {64 d, token, 2 halves of d, kv head, page}, so
 //    ONE op moves [HKT heads][2 halves][TB tokens][64 d] of a physical page — for Llama-3.1-8B one
-//    whole contiguous 32 KiB K page (all 8 kv heads).  Measured (scripts/tma_probe.cu): an SM
+//    whole contiguous 32 KiB K page (all 8 kv heads).  Measured: an SM
 //    sustains only ~5 tensor ops/us from one issuing warp (~10 from four), so the op size decides
 //    the bandwidth: 16-32 KiB ops reach the HBM limit from one warp, the 4 KiB ops of a
 //    tensor-parallel shard with one kv head need all four producer warps.  The ops of a stage are
 //    dealt round-robin to the four warps.  Page ids are prefetched 32 at a time from the block
 //    table with one coalesced load and never past ceil(len / page) (the reference reads up to 7
-//    entries past it, SURVEY appendix B).
+//    entries past it).
 //  * Eight consumer warps each own one (kv head, 16-token) slice of a stage and run the GQA group
 //    of that kv head as the M dimension of mma.sync m16n8k16 (all H/Hkv query heads share one pass
 //    over K/V; the reference re-streams K/V once per query head).

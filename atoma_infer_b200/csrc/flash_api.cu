@@ -248,7 +248,7 @@ void run_mha_impl(void *q_ptr, void *k_ptr, void *v_ptr, void *o_ptr, void *soft
     set_mha_path("none");
     if (b == 0 || h == 0 || seqlen_q == 0) return;
     // The reference compiles sliding windows and soft-capping OUT (FLASHATTENTION_DISABLE_LOCAL / _SOFTCAP,
-    // static_switch.h:7-11) and silently computes full attention for them; so did round 1 of this library.
+    // static_switch.h:7-11) and silently computes full attention for them.
     // A window that would actually mask something, or a soft cap, is refused instead of answered wrongly.
     // (The tuples the reference's wrappers build for plain causal / full attention — window (seqlen_k, 0)
     // or (-1, -1) — mask nothing beyond causality and pass.)

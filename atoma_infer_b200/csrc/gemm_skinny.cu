@@ -5,7 +5,7 @@
 //
 // Why a second GEMM kernel next to gemm_bf16.cu (stream-K): at T <= 128 the GEMM is a pure weight
 // stream (algorithmic bytes 2 (N K + T K + T N), ~T flop/byte) and what separates a kernel from the
-// HBM roofline is latency, not bandwidth: round 1's stream-K kernel streamed W at 6.9 TB/s but lost
+// HBM roofline is latency, not bandwidth: the stream-K kernel streamed W at 6.9 TB/s but lost
 // ~6.5 us per launch in its split reduction (fp32 partials through L2, fence, arrival counter,
 // last-arriver pass).  Here no tile is ever split:
 //  * the ACTIVATIONS are the M operand of tcgen05.mma (M = 64 for T <= 64 — rows >= T of the operand
@@ -18,13 +18,13 @@
 //    inside row group g (5-D tensor map {64 k, row, half, k block, group}; one TMA op moves
 //    [kbs k blocks][halves][np rows][128 B]): with halves = 2 an epilogue thread holds BOTH elements of
 //    a RoPE pair (d, d + D/2) or of a SwiGLU pair (gate_i, up_i), so RoPE + KV-cache scatter
-//    (llama.rs:218-304 + flash_attention.rs:361) and silu(gate) * up (llama.rs:364,
-//    f3) are applied to the accumulator before it is stored — no extra kernel, no extra pass;
+//    (llama.rs:218-304 + flash_attention.rs:361) and silu(gate) * up (llama.rs:364)
+//    are applied to the accumulator before it is stored — no extra kernel, no extra pass;
 //  * tensor-parallel row-parallel projections (o_proj, down_proj; multi_gpu.rs:141-179) can PUSH the
 //    bf16 partial tile straight into every peer's receive buffer over NVLink from the epilogue (8-byte
 //    units carrying their own epoch flag, the protocol of allreduce_p2p.cu) — the all-reduce kernel
 //    that followed the GEMM shrinks to the receive side, which is fused with residual + RMSNorm
-//    (llama_ops.cu), SURVEY §8 f4;
+//    (llama_ops.cu);
 //  * warp 0 = TMA producer (W evict-first, x evict-last; under programmatic dependent launch with
 //    immutable weights the ring is filled with W before the grid dependency resolves), warp 1 =
 //    tcgen05.mma issuer (accumulators double-buffered in TMEM so a multi-wave CTA's epilogue overlaps
@@ -47,9 +47,8 @@ constexpr int kSkSmemBudget = 200 * 1024;   // ring of a CTA that owns its SM; +
 // NEXT kernel of the stream (programmatic dependent launch) becomes resident and streams its weights while this
 // one drains: HBM does not idle across the kernel boundary.
 constexpr int kSkHalfBudget = 100 * 1024;
-// One thread issues only ~5 TMA tensor ops per microsecond whatever their size (measured: round 1's
-// tma_probe; here 0.25 us per stage with two ops per stage from one thread), so a stage is made of FEW,
-// LARGE ops — up to 96 KiB per stage, the weight box split over two issuing warps, x from a third.
+// One thread issues only ~5 TMA tensor ops per microsecond whatever their size (measured: 0.25 us per
+// stage with two ops per stage from one thread), so a stage is made of FEW, LARGE ops — up to 96 KiB per stage, the weight box split over two issuing warps, x from a third.
 constexpr int kSkStageTarget = 96 * 1024;
 constexpr int kSkDefaultBudget = kSkSmemBudget;
 
@@ -385,7 +384,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const bool is_w = warp == 0;
         // Release the dependent grid: at once, or (trigger_late) only when this CTA issues its last weight load —
         // a dependent grid that sits in the hardware queue for tens of microseconds waiting for SMs was measured
-        // to be placed several microseconds late once they free up (scripts/trace_step.py).
+        // to be placed several microseconds late once they free up.
         if (is_w && !a.trigger_late) pdl_launch_dependents();
         const int w_op_bytes = a.w_bytes / a.w_ops;
         // Under programmatic dependent launch with immutable weights the ring is filled with W while the
@@ -421,7 +420,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (a.trace && is_w && lane == 0 && n == 0) {
                     unsigned smid;
                     asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-                    a.trace[blockIdx.x * 8 + 4] = smid;   // which SM ran this CTA (hand-over analysis: scripts/trace_step.py)
+                    a.trace[blockIdx.x * 8 + 4] = smid;   // which SM ran this CTA (for the hand-over between kernels)
                 }
                 if (elect_one_sync()) {
                     // W is read exactly once by exactly one CTA: evict-first.  x is re-read by every CTA: keep it.
@@ -534,7 +533,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __syncthreads();
     if (a.trace && tid == 0) a.trace[blockIdx.x * 8 + 3] = sk_timer_ns();
     if (warp == 1) {
-        // Measured (scripts/trace_step.py, slot 5 - slot 3): this fence + release takes 1.1 us + 50 ns per accumulator
+        // Measured (trace slot 5 - slot 3): this fence + release takes 1.1 us + 50 ns per accumulator
         // column the tile used (2.7 us at 32 columns, 11.5 us at 208) — the fence is where the time goes, and dropping
         // it only moves the wait into tcgen05.dealloc.  It is the SM hand-over cost after every tensor-memory kernel.
         tc_fence_after_sync();
@@ -611,7 +610,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 // Two projections chained in ONE kernel: y1 = epi1( silu_mul(x0 . W0^T) . W1^T )  — the MLP of a Llama block
 // (gate_up + SwiGLU, then down_proj; models/src/llama.rs:362-366).
 //
-// Why: the step timeline (scripts/trace_step.py, per-SM hand-over) shows that an SM whose CTA used tensor memory
+// Why: the step's timeline (per-SM hand-over) shows that an SM whose CTA used tensor memory
 // takes 3.3 us (32 accumulator columns) to 12 us (208 columns: gate_up) to accept the next kernel's CTA, against
 // 0.5 us after the decode-attention kernel, which uses none — and down_proj's CTAs need exactly the SMs gate_up's
 // CTAs leave.  Here the CTA stays: phase 1 keeps the ring, the barriers and the tensor-memory allocation of phase 0,

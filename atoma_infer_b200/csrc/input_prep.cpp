@@ -1,4 +1,4 @@
-// Decode/prefill step input preparation (SURVEY §8 row f2): a C++ restatement of
+// Decode/prefill step input preparation: a C++ restatement of
 // `ModelWorker::prepare_input_tensors` (reference backends/vllm/src/worker.rs:224-460) that lays
 // every tensor of a step's `ModelInput` / `FlashAttentionMetadata` out in ONE host buffer, so that the
 // step's metadata reaches the GPU with ONE host-to-device copy.  The reference builds ten

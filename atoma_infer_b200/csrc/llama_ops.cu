@@ -1,10 +1,10 @@
-// The small kernels of a Llama decode step around the projections (SURVEY §8 row f3): token
+// The small kernels of a Llama decode step around the projections: token
 // embedding gather, residual add + RMSNorm (plain, and as the receive side of the tensor-parallel
 // all-reduce whose send side is the o_proj / down_proj GEMM epilogue, row f4), and greedy sampling
 // of the lm_head logits on the device.
 //
 // Reference behaviour restated (third-party arithmetic: candle-nn / candle-kernels 0.9.2-alpha.1 are
-// registry dependencies, not under /root/reference — parity for these ops is unpinned there; the
+// registry dependencies, not part of the reference's tree — parity for these ops is unpinned there; the
 // call sites are what is followed):
 //   * models/src/llama.rs:398-410  Block::forward:  x = attn(rms_1(x)) + residual;  x = mlp(rms_2(x)) + residual
 //     — the adds are in the model dtype (bf16), RMSNorm computes in fp32 on the bf16 input:

@@ -45,7 +45,7 @@ inline bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) =
 // is told what the NEXT one will stream first; bit i of the mask enables one edge (diagnostics: A/B runs).
 //   1: attention -> Wo    2: o_proj -> Wgate_up    4: gate_up -> Wdown    8: down_proj -> next layer's Wqkv / lm_head
 //  16: qkv -> Wo (instead of 1: the prefetch then sits in L2 through the attention kernel)
-// Default 0 (off): measured on a B200 (profiles/r02_step_prefetch_ab.json) every combination is within +-1 us per layer of
+// Default 0 (off): measured on a B200 every combination is within +-1 us per layer of
 // "off" — at a kernel boundary the dead time is control latency (CTA hand-over, set-up, descriptor fetch, first
 // HBM round trip), not bandwidth, and an L2 hit shortens only the last of those.
 int g_step_prefetch_mask = 0;
@@ -55,7 +55,7 @@ inline void hint(int bit, const void *w, long long bytes) {
     if (g_step_prefetch_mask & bit) set_next_kernel_prefetch(w, std::min(bytes, g_step_prefetch_cap));
 }
 
-// NVTX range for the lifetime of the object (SURVEY §5: the reference marks its forward passes with
+// NVTX range for the lifetime of the object (the reference marks its forward passes with
 // tracing spans — models/src/llama.rs:258, 363, 397; these are the profiler-visible equivalent).
 struct NvtxRange {
     explicit NvtxRange(const char *name) { nvtxRangePushA(name); }
@@ -251,8 +251,8 @@ NormArgs norm_tail_args(const void *residual, void *residual_out, const void *we
 }
 
 // 1: the add+RMSNorm after o_proj and after down_proj run in the tail of those GEMMs (5 launches per layer);
-// 0 (default): as separate kernels (7 launches per layer) — atoma_debug_step_fusion.  Measured on a B200
-// (profiles/r02_step_fusion_ab.json): the fused tail is 1.5 us per norm SLOWER (190.2 vs 187.1 us per layer at tp = 1,
+// 0 (default): as separate kernels (7 launches per layer) — atoma_debug_step_fusion.  Measured on a B200:
+// the fused tail is 1.5 us per norm SLOWER (190.2 vs 187.1 us per layer at tp = 1,
 // 66.5 vs 64.2 for a tp8 shard): the norm CTAs must first wait for the slowest CTA of the grid, whereas the separate
 // norm kernel is already resident (PDL) and its 32 CTAs start the moment the GEMM's grid completes.  Same bits.
 int g_step_norm_tail = 0;
@@ -451,7 +451,7 @@ extern "C" void atoma_llama_decode_step(const atoma_llama_model *model, const at
                             stream))
             return;
         // paged decode attention  (flash_attention.rs:455 -> flash_attn_kv_cache_full -> run_mha; the
-        // argument tuple of SURVEY appendix A.1 with q a strided view of the qkv buffer)
+        // argument tuple of that call with q a strided view of the qkv buffer)
         MhaParams p;
         std::memset(&p, 0, sizeof(p));
         p.q = s.qkv;

@@ -1,6 +1,6 @@
 // Residual add + RMSNorm of ONE token row by one CTA (models/src/llama.rs:398-410), shared by the standalone
 // kernel (llama_ops.cu: add_rmsnorm_kernel) and by the tail of the row-parallel projections (gemm_skinny.cu:
-// the CTAs that finish last normalise the rows of the output they have just completed — SURVEY §8 rows f3, f4).
+// the CTAs that finish last normalise the rows of the output they have just completed).
 //
 //   x        = the addend: a [T, hidden] tensor, or (W > 1) the rank-order fp32 sum of the W addends that the
 //              ranks pushed into this rank's receive buffers, rounded to the io type (multi_gpu.rs:141-179), or 0

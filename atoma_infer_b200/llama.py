@@ -1,4 +1,4 @@
-"""Host-side mirror of `models::llama` for the decode step (SURVEY §8 rows f2, f3): configuration,
+"""Host-side mirror of `models::llama` for the decode step: configuration,
 rotary tables, per-rank weight layout and the decode-step executor.
 
 What the reference assembles per step from candle calls (models/src/llama.rs:253-314, 362-366,

@@ -1,4 +1,4 @@
-"""Peer-to-peer all-reduce communicator over NVLink (SURVEY §8 row f4): the host side of
+"""Peer-to-peer all-reduce communicator over NVLink: the host side of
 `atoma_allreduce_sum_p2p` (csrc/allreduce_p2p.cu, include/atoma_flash.h).
 
 Serves the same call as the reference's `AllReduce` custom op (models/src/multi_gpu.rs:141-179:

@@ -1,5 +1,5 @@
 """Step input preparation: mirror of `ModelWorker::prepare_input_tensors` and `ModelInput`
-(reference backends/vllm/src/worker.rs:224-460, :24-40), SURVEY §8 row f2.
+(reference backends/vllm/src/worker.rs:224-460, :24-40).
 
 The host logic is C++ (`atoma_prepare_input`, csrc/input_prep.cpp); this module marshals sequences
 into it, owns the pinned staging buffer and its device image, and exposes the step's tensors as

@@ -162,7 +162,7 @@ void atoma_gemm_bf16_tn(const void *x, const void *w, void *y, int64_t T, int64_
                         int64_t ldx, int64_t ldw, int64_t ldy, atoma_stream_t stream);
 
 /*
- * One-shot all-reduce(sum) over NVLink peer memory for the tensor-parallel path (SURVEY §8 f4).
+ * One-shot all-reduce(sum) over NVLink peer memory for the tensor-parallel path.
  * The reference calls NCCL through cudarc (`comm.all_reduce(src, &mut dst, &ReduceOp::Sum)`,
  * models/src/multi_gpu.rs:141-179; one communicator per GPU thread) for the [T, hidden] payload after
  * o_proj / down_proj; these entries serve the same call behind `AllReduce::cuda_fwd`.

@@ -1,6 +1,5 @@
 /*
- * atoma_llama.h — the decode-step operators around the attention path and the step executor
- * (SURVEY §8 rows a11, f1, f2, f3, f4).
+ * atoma_llama.h — the decode-step operators around the attention path and the step executor.
  *
  * In the reference every one of these is a candle call issued from Rust: the projections are
  * `Linear::forward` -> cuBLAS (models/src/llama.rs:269-271, 311, 364-365, 476), RoPE is

@@ -179,7 +179,7 @@ const char *atoma_flash_attention_forward(const atoma_attention_config *cfg, con
 
 /*
  * Step input preparation — `ModelWorker::prepare_input_tensors`
- * (backends/vllm/src/worker.rs:224-460), SURVEY §8 row f2.  One flattened entry per sequence of
+ * (backends/vllm/src/worker.rs:224-460).  One flattened entry per sequence of
  * the scheduled sequence groups (group fields repeated per sequence), in the order the reference
  * iterates them.  Every tensor of the step's `ModelInput` / `FlashAttentionMetadata` is laid out in
  * ONE host buffer (16-byte aligned sections, offsets in `atoma_model_input_layout`), so one
