@@ -332,14 +332,15 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
-// n / (1 + e) for e >= 0 (inf and NaN included), 1 ulp: the reciprocal unit's estimate, one step of Newton's iteration, one product.  For
-// epilogues that divide per element, where the compiler's division takes three times the instructions and a branch.  Where e passes 2^126
-// it divides by 2^126 (the quotient is below n times the smallest normal number either way).
+// n / (1 + e) for e >= 0, within 1 ulp: the reciprocal unit's estimate of 4 / (1 + e), which is normal for every finite e, one step of Newton's
+// iteration, one product.  For epilogues that divide per element, where the compiler's division takes three times the instructions and a
+// branch.  e = inf gives 0 n, as division does: its estimate is 0, and the bound (2^126, past every finite e) keeps the step from 0 inf.
 __device__ __forceinline__ float over_one_plus(float n, float e) {
-    float d = 1.f + e, r;
-    d = d > 8.507059e37f ? 8.507059e37f : d;
+    const float d = fmaf(e, 0.25f, 0.25f);
+    float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    return n * fmaf(r, fmaf(-d, r, 1.f), r);
+    r = fmaf(r, fmaf(-fminf(d, 8.507059e37f), r, 1.f), r);
+    return 0.25f * n * r;
 }
 
 // ---- packed float32 pairs: one issue slot for two operations ----

@@ -95,6 +95,25 @@ def test_activation_is_float32(dtype):
     assert share < 2.2e-7 * 2.0 ** (7.5 if dtype == BF else 10.5), share
 
 
+def test_activation_of_extreme_gates():
+    """Gates whose exponential is huge, infinite or NaN: what float32 gives for g / (1 + e^-g) u, up to the exponential's 2 ulp and the rounding to bfloat16."""
+    gates = [-300.0, -100.0, -89.0, -88.5, -88.0, -87.5, -87.0, -60.0, -0.0, 60.0, 300.0, float("-inf"), float("inf"), float("nan")]
+    T, K, F = 129, 64, 16
+    x, w = torch.zeros((T, K), dtype=BF, device=DEV), torch.zeros((2 * F, K), dtype=BF, device=DEV)
+    for i, g in enumerate(gates):                  # column i of w alone meets row i of x; an infinity comes from a product that overflows
+        big = abs(g) == float("inf")
+        x[i, i] = 3e38 if big else 1.0
+        w[i, i] = (3.0 if g > 0 else -3.0) if big else g
+        w[F + i, i] = 2e-38 if big else 1.5
+    got = ops.gate_up_silu(x, w)
+    z = x.float() @ w.float().T
+    g, u = z[:, :F].to(BF).float(), z[:, F:].to(BF).float()
+    want = (g / (1 + torch.exp(-g)) * u).to(BF)
+    for i, name in enumerate(gates):
+        a, b = got[i, i].item(), want[i, i].item()
+        assert (a != a and b != b) or a == b or abs(a - b) <= abs(b) * 2.0 ** -7, (name, a, b)
+
+
 @pytest.mark.parametrize("scale_input", [False, True])
 @pytest.mark.parametrize("T,E,top,W,F", [
     (1, 3, 2, 64, 64),         # two chunks of one row
