@@ -25,6 +25,8 @@ BF = torch.bfloat16
     (513, 250, 1024),      # columns that miss the 4-wide stores
     (1023, 3000, 328),     # more tiles than pairs, every edge ragged
     (4097, 264, 64),       # more than 16 chunks: two groups of the raster
+    (192, 3072, 16384),    # the last tokens that a long K sends to the split-K kernel, and the first that it does not
+    (193, 3072, 16384),
 ])
 def test_against_float64(T, N, K):
     x = randn_t((T, K), 1, BF, DEV)
