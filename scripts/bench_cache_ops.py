@@ -138,8 +138,8 @@ def main():
             r.update({"per_block_memcpy_ms": t2 * 1e3, "per_block_memcpy_GBps": byts / t2 / 1e9})
             res[f"swap_{name}_{nseq}seq"] = r
             print(f"swap_{name}", json.dumps(r), flush=True)
-    (ROOT / "gpurun_out").mkdir(exist_ok=True)
-    (ROOT / "gpurun_out" / "bench_cache_ops.json").write_text(json.dumps(res, indent=1))
+    (ROOT / "build").mkdir(exist_ok=True)
+    (ROOT / "build" / "bench_cache_ops.json").write_text(json.dumps(res, indent=1))
 
 
 if __name__ == "__main__":

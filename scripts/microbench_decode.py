@@ -108,8 +108,8 @@ def main():
         torch.cuda.synchronize()
         res["max_abs_diff_vs_ref"] = float((out.float() - out2.float()).abs().max())
     print(json.dumps(res), flush=True)
-    Path(ROOT / "gpurun_out").mkdir(exist_ok=True)
-    (ROOT / "gpurun_out" / f"microbench_decode_{ctx}_hk{HK}.json").write_text(json.dumps(res, indent=1))
+    Path(ROOT / "build").mkdir(exist_ok=True)
+    (ROOT / "build" / f"microbench_decode_{ctx}_hk{HK}.json").write_text(json.dumps(res, indent=1))
 
 
 if __name__ == "__main__":

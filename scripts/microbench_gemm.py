@@ -55,8 +55,8 @@ def main():
                     "ours_GBps": byts / t_ours / 1e3, "cublas_GBps": byts / t_cublas / 1e3,
                     "ours_TFLOPs": flops / t_ours / 1e6, "cublas_TFLOPs": flops / t_cublas / 1e6})
         print(json.dumps(out[-1]), flush=True)
-    (ROOT / "gpurun_out").mkdir(exist_ok=True)
-    (ROOT / "gpurun_out" / "microbench_gemm.json").write_text(json.dumps(out, indent=1))
+    (ROOT / "build").mkdir(exist_ok=True)
+    (ROOT / "build" / "microbench_gemm.json").write_text(json.dumps(out, indent=1))
 
 
 if __name__ == "__main__":

@@ -51,8 +51,8 @@ def main():
             r.update({"ref_ms": t2 * 1e3, "ref_TFLOPs": flops / t2 / 1e12})
         print(json.dumps(r), flush=True)
         res.append(r)
-    (ROOT / "gpurun_out").mkdir(exist_ok=True)
-    (ROOT / "gpurun_out" / "microbench_prefill.json").write_text(json.dumps(res, indent=1))
+    (ROOT / "build").mkdir(exist_ok=True)
+    (ROOT / "build" / "microbench_prefill.json").write_text(json.dumps(res, indent=1))
 
 
 if __name__ == "__main__":

@@ -1,7 +1,7 @@
 """Decode-time GEMM (csrc/gemm_skinny.cu) at the shapes of a Llama decode step: quick numerics check
 against fp32 torch, then kernel timing vs cuBLAS (torch.matmul) — CUDA-graph loops over rotating
 weights so every launch streams W from HBM, CUDA events, programmatic dependent launch on for ours
-as in the step.  Writes gpurun_out/microbench_skinny.json.
+as in the step.  Writes build/microbench_skinny.json.
 
   python scripts/microbench_skinny.py [--quick] [--sweep]
 """
@@ -209,8 +209,8 @@ def main():
         ops.set_launch_mode(pdl=True, const_weights=True)
     ops.set_launch_mode()
     res["no_pdl"] = bench(shapes[:4], "no pdl")
-    (ROOT / "gpurun_out").mkdir(exist_ok=True)
-    (ROOT / "gpurun_out" / "microbench_skinny.json").write_text(json.dumps(res, indent=1))
+    (ROOT / "build").mkdir(exist_ok=True)
+    (ROOT / "build" / "microbench_skinny.json").write_text(json.dumps(res, indent=1))
 
 
 if __name__ == "__main__":

@@ -26,7 +26,7 @@ def main():
     ap.add_argument("--head", action="store_true")
     ap.add_argument("--tp", type=int, default=1, help="one rank's shard of a tp-N step, no all-reduce")
     ap.add_argument("--variants", default="default,b100,b80,default")
-    ap.add_argument("--out", default="gpurun_out/microbench_step.json")
+    ap.add_argument("--out", default="build/microbench_step.json")
     args = ap.parse_args()
     dev = torch.device("cuda", 0)
     torch.cuda.set_device(dev)

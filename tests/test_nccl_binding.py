@@ -84,7 +84,7 @@ def _worker(rank, world, port, out_dir):
 @pytest.mark.gpu
 def test_all_reduce_two_gpus_eager_and_captured(tmp_path):
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs 2 GPUs (gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     import torch.multiprocessing as mp
     mp.spawn(_worker, args=(2, _free_port(), str(tmp_path)), nprocs=2, join=True)
     for r in range(2):

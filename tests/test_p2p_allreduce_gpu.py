@@ -1,5 +1,5 @@
 """Peer-to-peer all-reduce over NVLink (csrc/allreduce_p2p.cu ≙ the reference's AllReduce op over
-NCCL, models/src/multi_gpu.rs:141-179).  Needs 2 GPUs (`gpurun --gpus 2`); skipped on a one-GPU
+NCCL, models/src/multi_gpu.rs:141-179).  Needs 2 GPUs; skipped on a one-GPU
 box.  Oracle: the fp32 sum of the ranks' addends in rank order, rounded once — the kernel must match
 it BIT FOR BIT on every rank, eagerly and replayed from a CUDA graph, for many consecutive
 all-reduces on alternating slots."""
@@ -114,7 +114,7 @@ def _worker(rank, world, port, out_dir):
 @pytest.mark.gpu
 def test_p2p_all_reduce_bit_exact_two_gpus(tmp_path):
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs 2 GPUs (gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     import torch.multiprocessing as mp
     n = torch.cuda.device_count()
     world = 8 if n >= 8 else 4 if n >= 4 else 2   # every world size the bench runs at, up to what the box has

@@ -8,7 +8,7 @@ kernel sums them (atoma_allreduce_recv_add_rmsnorm) — against
   * the tp=1 step of the same seeded model: after one layer within 8 bf16 ulps taken at the row's rms (one rounding per
     all-reduce + regrouped fp32 partial sums, then a norm and an MLP), after the whole step norm-wise.
 
-Needs >= 2 GPUs (`gpurun --gpus N`); world = min(8, device_count).  Skipped on a one-GPU box."""
+Needs >= 2 GPUs; world = min(8, device_count).  Skipped on a one-GPU box."""
 import os
 import socket
 import sys
@@ -195,7 +195,7 @@ def _worker(rank, world, port, out_dir):
 def test_tensor_parallel_step_matches_rank_order_sum_and_tp1(tmp_path):
     n = torch.cuda.device_count()
     if n < 2:
-        pytest.skip("needs >= 2 GPUs (gpurun --gpus N)")
+        pytest.skip("needs >= 2 GPUs")
     import torch.multiprocessing as mp
     world = 8 if n >= 8 else 4 if n >= 4 else 2
     mp.spawn(_worker, args=(world, _free_port(), str(tmp_path)), nprocs=world, join=True)
