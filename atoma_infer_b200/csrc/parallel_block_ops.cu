@@ -4,9 +4,7 @@
 // causal tap filter over time, and both results join the stream in one update (fused here with whatever precedes the next
 // layer and with its input norm).  The mixers that need more than attention kernels:
 //   - tap filters whose inputs before a portion come from a per-sequence history (the portion's last inputs replace it),
-//   - matrix-state recurrences (gated linear attention, gated delta rule, state-space recurrence): every head keeps S [dim, vdim] in float32; the
-//     columns of S are independent in all of them, so a CTA owns 32 columns of one head of one sequence, the rows
-//     of a column are spread over `parts` threads (registers), and the tokens are visited strictly in order,
+//   - matrix-state recurrences: state_scan.cu,
 //   - rotary positions on queries, keys and values with the cache write, the turn-back of a head's sum, and the
 //     latent-attention variants that keep one rotated key part beside the latent.
 // Statistics, angles, decays, gates of the recurrences and the state are float32 whatever the activation format; every
@@ -20,7 +18,7 @@
 
 namespace atoma {
 
-extern int g_hybrid_debug;   // bit 1: general kernels only; bit 4: scans with many rows per lane
+extern int g_hybrid_debug;   // bit 1: general kernels only
 bool hyb_head_project_ld(const void *, int64_t, int64_t, const void *, void *, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int32_t,
                          uint32_t, cudaStream_t, const void * = nullptr, int64_t = 0);   // latent_attention.cu
 
@@ -254,290 +252,6 @@ __global__ void __launch_bounds__(256) tap_history_kernel(const atoma_tap_filter
         if (k >= keep) break;
         const int rel = n - keep + k;
         hist[static_cast<int64_t>(k) * C + c] = rel >= 0 ? to_f(in[static_cast<int64_t>(q0 + rel) * a.ld_in + c]) + ib : old[k];
-    }
-}
-
-// ---------------------------------------------------------------------------------------------
-// matrix-state recurrences
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ float log_sigmoid(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
-__device__ __forceinline__ float softplusf_(float z) { return z > 20.f ? z : log1pf(expf(z)); }
-
-// One CTA = kScanWarps compute warps + kScanWarps staging warps for 32 * kScanWarps / PW columns of one head of one sequence.
-// A compute warp owns 32 / PW columns; the dim rows of a column are spread over PW lanes (RPT registers each), so the sums over
-// the rows are PW-lane shuffles in a fixed order and the token loop has no CTA-wide barrier.  While the compute warps walk through
-// one chunk of staged tokens, the staging warps load the next one (number-format conversion, the decays' exponentials, the unit
-// norms of q and k) into the other buffer; one barrier per chunk.
-// Staged row of a token: element i of q / k / decay at (i / RPT) * (RPT + 4) + i % RPT — a lane's RPT values are contiguous and
-// 16-byte aligned (float4 loads), and the PW lanes of a column read distinct banks.
-// Two splits per key size: many rows per lane (few instructions per state entry: steps with many CTAs) and 8 rows per lane (a
-// short chain per token and four times the warps: steps with few).  Both add in the same order, so they give the same bits.
-constexpr int kScanWarps = 4;
-
-template <int PW>
-__device__ __forceinline__ float parts_sum(float v) {
-#pragma unroll
-    for (int o = 32 / PW; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-template <typename T, int KIND, int RPT, int PW>
-__global__ void __launch_bounds__(64 * kScanWarps, 2) state_scan_kernel(const atoma_state_scan_args a, int chunk) {
-    extern __shared__ __align__(16) float sm[];
-    constexpr int CW = 32 / PW, COLS = CW * kScanWarps, DS = PW * (RPT + 4);
-    pdl_launch_dependents();
-    pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.y, b = blockIdx.z;
-    const int D = static_cast<int>(a.dim), V = static_cast<int>(a.vdim), H = static_cast<int>(a.H);
-    const int q0 = a.query_start[b], n = a.query_start[b + 1] - q0;
-    if (n <= 0) return;
-    const int per_tok = (KIND == 0 ? 3 : 2) * DS + COLS + 4;     // q, k, (decay per channel), v of the CTA's columns, beta and decay
-    for (int i = threadIdx.x; i < 2 * chunk * per_tok; i += blockDim.x) sm[i] = 0.f;   // what lies beyond dim stays zero
-    const int kvh = KIND != 0 ? h / (H / static_cast<int>(a.G)) : h;
-    const T *qp = static_cast<const T *>(a.q), *kp = static_cast<const T *>(a.k), *vp = static_cast<const T *>(a.v);
-    const int jb = blockIdx.x * COLS;
-    const bool loader = warp >= kScanWarps;
-    // ---- staging (all warps for the first chunk, the staging warps afterwards) ----
-    // A warp takes TU tokens at a time: every load of the TU tokens is issued before the first value is used, so a chunk costs a
-    // few round trips to memory, not one per token.  Lane l holds elements l, l + 32, ... of a token's q / k / decay rows; the sums
-    // of squares run over a lane's elements in index order, then over the lanes by xor-shuffles: the same order for every token,
-    // wherever it falls in a chunk or a batch.
-    constexpr int EPL = RPT * PW / 32;                           // elements of a row per lane
-    constexpr int TU = EPL <= 4 ? 4 : (EPL == 8 ? 2 : 1);
-    const int vcol = (lane < COLS && jb + lane < V) ? jb + lane : -1;
-    float zb[EPL];                                               // what does not change from token to token
-    float neg_rate = 0.f, dtb = 0.f;
-    const float skip = KIND == 2 && a.skip ? a.skip[h] : 0.f;
-    if (KIND == 0) {
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) zb[e] = lane + 32 * e < D ? a.z_bias[h * D + lane + 32 * e] : 0.f;
-    } else {
-        neg_rate = -expf(a.a_log[h]);
-        dtb = a.dt_bias[h];
-    }
-    const float inv_tau = 1.0f / a.tau;
-    auto stage = [&](int t0, float *buf, int w, int nw) {
-        const int nt = min(chunk, n - t0);
-        for (int tk0 = w * TU; tk0 < nt; tk0 += nw * TU) {
-            // every address is valid (a token beyond the chunk reads the chunk's last, an element beyond dim reads element 0), so
-            // the loads carry no branches and all of them are in flight together
-            T qr[TU][EPL], kr[TU][EPL], zr[KIND == 0 ? TU : 1][KIND == 0 ? EPL : 1], vr[TU], br[TU], ar[TU];
-#pragma unroll
-            for (int u = 0; u < TU; ++u) {
-                const int64_t t = q0 + t0 + min(tk0 + u, nt - 1);
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) {
-                    const int i = lane + 32 * e < D ? lane + 32 * e : 0;
-                    qr[u][e] = qp[t * a.ld_q + kvh * D + i];
-                    kr[u][e] = kp[t * a.ld_k + kvh * D + i];
-                    if (KIND == 0) zr[u][e] = static_cast<const T *>(a.z)[t * a.ld_z + h * D + i];
-                }
-                vr[u] = vp[t * a.ld_v + h * V + max(vcol, 0)];
-                if (KIND == 1) br[u] = static_cast<const T *>(a.b_pre)[t * a.ld_b + h];
-                if (KIND != 0) ar[u] = static_cast<const T *>(a.a_pre)[t * a.ld_a + h];
-            }
-#pragma unroll
-            for (int u = 0; u < TU; ++u) {
-                if (tk0 + u >= nt) break;
-                float *row = buf + (tk0 + u) * per_tok;
-                float qv[EPL], kv[EPL];
-                float sq = 0.f, sk = 0.f, dot = 0.f;
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) {
-                    const bool in = lane + 32 * e < D;
-                    qv[e] = in ? to_f(qr[u][e]) : 0.f;
-                    kv[e] = in ? to_f(kr[u][e]) : 0.f;
-                    sq = fmaf(qv[e], qv[e], sq);
-                    sk = fmaf(kv[e], kv[e], sk);
-                    dot = fmaf(qv[e], kv[e], dot);
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    if (KIND == 1) {
-                        sq += __shfl_xor_sync(0xffffffffu, sq, o);
-                        sk += __shfl_xor_sync(0xffffffffu, sk, o);
-                    }
-                    dot += __shfl_xor_sync(0xffffffffu, dot, o);
-                }
-                float fq = a.q_scale, fk = 1.f;
-                if (KIND == 1) {
-                    fq = a.q_scale / sqrtf(sq + a.unit_eps);     // unit length per head, the query scaled
-                    fk = 1.0f / sqrtf(sk + a.unit_eps);
-                }
-                if (lane == 0) {
-                    if (KIND == 1) {
-                        row[per_tok - 4] = sigmoidf_(to_f(br[u]));
-                        row[per_tok - 3] = expf(neg_rate * softplusf_(to_f(ar[u]) + dtb));
-                    }
-                    if (KIND == 2) {
-                        const float step = softplusf_(to_f(ar[u]) + dtb);
-                        row[per_tok - 4] = step;
-                        row[per_tok - 3] = expf(neg_rate * step);
-                    }
-                    row[per_tok - 2] = dot * fq * fk;            // q . k of the token as the recurrence sees them
-                }
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) {
-                    const int i = lane + 32 * e;
-                    if (i < D) {
-                        const int o = (i / RPT) * (RPT + 4) + i % RPT;
-                        if (KIND == 0) {
-                            const float decay = expf(log_sigmoid(to_f(zr[u][e]) + zb[e]) * inv_tau);
-                            row[o] = qv[e] * fq * decay;         // the read-out of the updated state, written on the old one (see below)
-                            row[2 * DS + o] = decay;
-                        } else {
-                            row[o] = qv[e] * fq;
-                        }
-                        row[DS + o] = kv[e] * fk;
-                    }
-                }
-                if (lane < COLS) row[(KIND == 0 ? 3 : 2) * DS + lane] = vcol >= 0 ? to_f(vr[u]) : 0.f;
-            }
-        }
-    };
-    // ---- the state of this lane: rows part * RPT + r of column j ----
-    const int part = lane / CW, j = jb + (warp % kScanWarps) * CW + lane % CW;
-    float *S_g = a.state + static_cast<int64_t>(a.state_slots[b]) * a.state_stride + static_cast<int64_t>(h) * D * V;
-    float S[RPT];
-    const bool fresh = a.context_lens[b] == 0;
-    if (!loader) {
-#pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-            const int i = part * RPT + r;
-            S[r] = (!fresh && i < D && j < V) ? S_g[static_cast<int64_t>(i) * V + j] : 0.f;
-        }
-    }
-    __syncthreads();                                         // the zero fill is done
-    stage(0, sm, warp, 2 * kScanWarps);
-    __syncthreads();
-    int it = 0;
-    for (int t0 = 0; t0 < n; t0 += chunk, ++it) {
-        const float *buf = sm + (it & 1) * chunk * per_tok;
-        if (loader) {
-            if (t0 + chunk < n) stage(t0 + chunk, sm + ((it + 1) & 1) * chunk * per_tok, warp - kScanWarps, kScanWarps);
-        } else {
-            const int nt = min(chunk, n - t0);
-            for (int tk = 0; tk < nt; ++tk) {
-                const float *row = buf + tk * per_tok;
-                const float4 *qr = reinterpret_cast<const float4 *>(row + part * (RPT + 4));
-                const float4 *kr = reinterpret_cast<const float4 *>(row + DS + part * (RPT + 4));
-                const float vj = row[(KIND == 0 ? 3 : 2) * DS + (warp % kScanWarps) * CW + lane % CW];
-                float o;
-                // Both recurrences read the state AFTER the token's write.  With S' = A S + k w^T (A the decay, w the written row):
-                // S'^T q = S^T (A q) + (k . q) w, so the sums over the rows run on the state as the previous token left it and the
-                // write is the only step between two tokens.
-                // Order of a sum over the rows, the same for every split of the rows over lanes: groups of 8 rows (four partial sums
-                // over rows m, m + 4, added as (0 + 1) + (2 + 3)), then a binary tree over the groups — inside a lane first, then by
-                // xor-shuffles over the lanes of the column.
-                constexpr int G8 = RPT / 8;
-                const float kq = row[per_tok - 2];
-                if (KIND == 0) {
-                    const float4 *ar = reinterpret_cast<const float4 *>(row + 2 * DS + part * (RPT + 4));
-                    float gs[G8];
-#pragma unroll
-                    for (int g8 = 0; g8 < G8; ++g8) {
-                        float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                        for (int r4 = 2 * g8; r4 < 2 * g8 + 2; ++r4) {
-                            const float4 a4 = ar[r4], k4 = kr[r4], q4 = qr[r4];     // q4: the query times the decay
-                            c[0] = fmaf(S[4 * r4], q4.x, c[0]);
-                            S[4 * r4] = fmaf(a4.x, S[4 * r4], k4.x * vj);
-                            c[1] = fmaf(S[4 * r4 + 1], q4.y, c[1]);
-                            S[4 * r4 + 1] = fmaf(a4.y, S[4 * r4 + 1], k4.y * vj);
-                            c[2] = fmaf(S[4 * r4 + 2], q4.z, c[2]);
-                            S[4 * r4 + 2] = fmaf(a4.z, S[4 * r4 + 2], k4.z * vj);
-                            c[3] = fmaf(S[4 * r4 + 3], q4.w, c[3]);
-                            S[4 * r4 + 3] = fmaf(a4.w, S[4 * r4 + 3], k4.w * vj);
-                        }
-                        gs[g8] = (c[0] + c[1]) + (c[2] + c[3]);
-                    }
-#pragma unroll
-                    for (int w = 1; w < G8; w <<= 1)
-#pragma unroll
-                        for (int g8 = 0; g8 < G8; g8 += 2 * w) gs[g8] += gs[g8 + w];
-                    o = fmaf(kq, vj, parts_sum<PW>(gs[0]));
-                } else if (KIND == 2) {
-                    const float g = row[per_tok - 3], u = row[per_tok - 4] * vj;   // decay, written row
-                    float gs[G8];
-#pragma unroll
-                    for (int g8 = 0; g8 < G8; ++g8) {
-                        float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                        for (int r4 = 2 * g8; r4 < 2 * g8 + 2; ++r4) {
-                            const float4 k4 = kr[r4], q4 = qr[r4];
-                            c[0] = fmaf(S[4 * r4], q4.x, c[0]);
-                            S[4 * r4] = fmaf(g, S[4 * r4], k4.x * u);
-                            c[1] = fmaf(S[4 * r4 + 1], q4.y, c[1]);
-                            S[4 * r4 + 1] = fmaf(g, S[4 * r4 + 1], k4.y * u);
-                            c[2] = fmaf(S[4 * r4 + 2], q4.z, c[2]);
-                            S[4 * r4 + 2] = fmaf(g, S[4 * r4 + 2], k4.z * u);
-                            c[3] = fmaf(S[4 * r4 + 3], q4.w, c[3]);
-                            S[4 * r4 + 3] = fmaf(g, S[4 * r4 + 3], k4.w * u);
-                        }
-                        gs[g8] = (c[0] + c[1]) + (c[2] + c[3]);
-                    }
-#pragma unroll
-                    for (int w = 1; w < G8; w <<= 1)
-#pragma unroll
-                        for (int g8 = 0; g8 < G8; g8 += 2 * w) gs[g8] += gs[g8 + w];
-                    o = fmaf(g, parts_sum<PW>(gs[0]), fmaf(kq, u, skip * vj));
-                } else {
-                    const float beta = row[per_tok - 4], g = row[per_tok - 3];
-                    float gk[G8], gq[G8];
-#pragma unroll
-                    for (int g8 = 0; g8 < G8; ++g8) {
-                        float c[4] = {0.f, 0.f, 0.f, 0.f}, d[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                        for (int r4 = 2 * g8; r4 < 2 * g8 + 2; ++r4) {
-                            const float4 k4 = kr[r4], q4 = qr[r4];
-                            c[0] = fmaf(S[4 * r4], k4.x, c[0]);
-                            d[0] = fmaf(S[4 * r4], q4.x, d[0]);
-                            c[1] = fmaf(S[4 * r4 + 1], k4.y, c[1]);
-                            d[1] = fmaf(S[4 * r4 + 1], q4.y, d[1]);
-                            c[2] = fmaf(S[4 * r4 + 2], k4.z, c[2]);
-                            d[2] = fmaf(S[4 * r4 + 2], q4.z, d[2]);
-                            c[3] = fmaf(S[4 * r4 + 3], k4.w, c[3]);
-                            d[3] = fmaf(S[4 * r4 + 3], q4.w, d[3]);
-                        }
-                        gk[g8] = (c[0] + c[1]) + (c[2] + c[3]);
-                        gq[g8] = (d[0] + d[1]) + (d[2] + d[3]);
-                    }
-#pragma unroll
-                    for (int w = 1; w < G8; w <<= 1)
-#pragma unroll
-                        for (int g8 = 0; g8 < G8; g8 += 2 * w) {
-                            gk[g8] += gk[g8 + w];
-                            gq[g8] += gq[g8 + w];
-                        }
-                    float sk = gk[0], sq = gq[0];
-#pragma unroll
-                    for (int x = 32 / PW; x < 32; x <<= 1) {
-                        sk += __shfl_xor_sync(0xffffffffu, sk, x);
-                        sq += __shfl_xor_sync(0xffffffffu, sq, x);
-                    }
-                    const float u = beta * (vj - g * sk);        // the decayed state's answer to k
-                    o = fmaf(g, sq, u * kq);
-#pragma unroll
-                    for (int r4 = 0; r4 < RPT / 4; ++r4) {
-                        const float4 k4 = kr[r4];
-                        S[4 * r4] = fmaf(g, S[4 * r4], k4.x * u);
-                        S[4 * r4 + 1] = fmaf(g, S[4 * r4 + 1], k4.y * u);
-                        S[4 * r4 + 2] = fmaf(g, S[4 * r4 + 2], k4.z * u);
-                        S[4 * r4 + 3] = fmaf(g, S[4 * r4 + 3], k4.w * u);
-                    }
-                }
-                if (part == 0 && j < V) a.out[static_cast<int64_t>(q0 + t0 + tk) * H * V + h * V + j] = o;
-            }
-        }
-        __syncthreads();
-    }
-    if (!loader) {
-#pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-            const int i = part * RPT + r;
-            if (i < D && j < V) S_g[static_cast<int64_t>(i) * V + j] = S[r];
-        }
     }
 }
 
@@ -954,71 +668,6 @@ bool hyb_tap_filter(const atoma_tap_filter_args &a, cudaStream_t stream) {
 #undef CALL
 }
 
-bool hyb_state_scan(const atoma_state_scan_args &a, cudaStream_t stream) {
-    if (a.T <= 0 || a.B <= 0) return true;
-    if (!hybrid::known_dtype(a.dtype, "atoma_state_scan")) return false;
-    const bool gla = a.kind == 0, delta = a.kind == 1, ssm = a.kind == 2;
-    if ((!gla && !delta && !ssm) || !a.q || !a.k || !a.v || !a.state || !a.state_slots || !a.query_start || !a.context_lens || !a.out || a.H <= 0 ||
-        a.dim <= 0 || a.vdim <= 0 || a.state_stride < a.H * a.dim * a.vdim || (gla && (!a.z || !a.z_bias || !(a.tau > 0.f))) ||
-        (delta && !a.b_pre) ||
-        (!gla && (!a.a_pre || !a.a_log || !a.dt_bias || a.G <= 0 || a.H % a.G))) {
-        set_status(kErrInvalidArg, "atoma_state_scan: null argument, unknown kind %d, or a state row shorter than heads * dim * vdim", a.kind);
-        return false;
-    }
-    // rows of a column per lane (RPT) and lanes per column (PW): dim <= RPT * PW
-    int rpt = a.dim <= 64 ? 16 : 32;
-    int pw = a.dim <= 128 ? 4 : (a.dim <= 256 ? 8 : 16);
-    if (a.dim > 512) {
-        set_status(kErrUnsupported, "atoma_state_scan: a key size of %lld exceeds 512", static_cast<long long>(a.dim));
-        return false;
-    }
-    // few CTAs (one long prompt, a handful of decoded tokens): 8 rows per lane, so that a token is a short chain and the state's
-    // entries are spread over more warps — as long as all CTAs are resident at once (two per SM): a second wave would walk the
-    // tokens a second time
-    const int64_t ctas_many = (a.vdim + 32 / pw * kScanWarps - 1) / (32 / pw * kScanWarps) * a.H * a.B;
-    if (a.dim <= 256 && !(g_hybrid_debug & 16) && ctas_many * (rpt / 8) <= 2 * current_device_info().sm_count) {
-        pw = pw * rpt / 8;
-        rpt = 8;
-    }
-    const int cols = 32 / pw * kScanWarps;
-    const int per_tok = (gla ? 3 : 2) * pw * (rpt + 4) + cols + 4;
-    int64_t longest = a.T;                                   // a bound of the longest portion: T tokens over B sequences, each has one at least
-    longest = std::max<int64_t>(1, a.T - (a.B - 1));
-    // staged tokens per buffer: at most 32, no more than the longest portion, and two CTAs' buffers fit one SM
-    const int chunk = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({32, longest, 96 * 1024 / (8 * per_tok)})));
-    const size_t smem = static_cast<size_t>(2 * chunk * per_tok) * 4;
-    const dim3 grid(static_cast<unsigned>((a.vdim + cols - 1) / cols), static_cast<unsigned>(a.H), static_cast<unsigned>(a.B));
-    const dim3 block(64 * kScanWarps);
-    cudaError_t e;
-#define SCAN(TT, KIND, RPT, PW)                                                                                                    \
-    do {                                                                                                                            \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(state_scan_kernel<TT, KIND, RPT, PW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
-        e = launch_ex(state_scan_kernel<TT, KIND, RPT, PW>, grid, block, smem, stream, a, chunk);                                   \
-    } while (0)
-#define SCAN_K(TT, KIND)                                \
-    do {                                                \
-        if (rpt == 8 && pw == 8) SCAN(TT, KIND, 8, 8);  \
-        else if (rpt == 8 && pw == 16) SCAN(TT, KIND, 8, 16); \
-        else if (rpt == 8) SCAN(TT, KIND, 8, 32);       \
-        else if (rpt == 16) SCAN(TT, KIND, 16, 4);      \
-        else if (pw == 4) SCAN(TT, KIND, 32, 4);        \
-        else if (pw == 8) SCAN(TT, KIND, 32, 8);        \
-        else SCAN(TT, KIND, 32, 16);                    \
-    } while (0)
-#define SCAN_T(TT)                                      \
-    do {                                                \
-        if (gla) SCAN_K(TT, 0);                         \
-        else if (ssm) SCAN_K(TT, 2);                    \
-        else SCAN_K(TT, 1);                             \
-    } while (0)
-    if (a.dtype == ATOMA_DTYPE_BF16) SCAN_T(__nv_bfloat16);
-    else SCAN_T(float);
-#undef SCAN_T
-#undef SCAN_K
-#undef SCAN
-    return hybrid::launched(e, "state_scan_kernel");
-}
-
 bool hyb_headnorm_gate(const float *o, const float *weight, const void *gate, int64_t ld_gate, void *out, int64_t T, int64_t H, int64_t vdim,
                        float eps, uint32_t dtype, cudaStream_t stream) {
     if (T <= 0) return true;
@@ -1155,15 +804,6 @@ extern "C" void atoma_tap_filter(const atoma_tap_filter_args *args, atoma_stream
         return;
     }
     hyb_tap_filter(*args, static_cast<cudaStream_t>(stream));
-}
-
-extern "C" void atoma_state_scan(const atoma_state_scan_args *args, atoma_stream_t stream) {
-    clear_status();
-    if (!args) {
-        set_status(kErrInvalidArg, "atoma_state_scan: args is NULL");
-        return;
-    }
-    hyb_state_scan(*args, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" void atoma_headnorm_gate(const float *o, const float *weight, const void *gate, int64_t ld_gate, void *out, int64_t T, int64_t H,

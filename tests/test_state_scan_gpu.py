@@ -1,0 +1,61 @@
+"""The matrix-state scans on every split of the state over lanes and warps, and on every way their rows are copied: the same bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def i32(xs):
+    return torch.tensor(xs, dtype=torch.int32, device=DEV)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("D,V", [(64, 128), (128, 64), (72, 8), (50, 34), (33, 7), (256, 16), (300, 24)])
+@pytest.mark.parametrize("rule", ["gla", "delta", "ssm"])
+def test_splits_and_copies_give_the_same_bits(rule, D, V, dtype):
+    """One sequence of 70 tokens (two chunks and a rest) alone, with sixteen rows a lane, among enough sequences for the CTAs of eight warps, and in
+    columns of a wider matrix that start at an odd element (value by value) or at an even one (pieces of four bytes)."""
+    from atoma_infer_b200 import hybrid_ops as ops
+
+    H, n, B = 4, 70, 90
+    G = H if rule == "gla" else 2
+    g = torch.Generator().manual_seed(D + V)
+    rnd = lambda c: torch.randn(n, c, generator=g).to(torch.bfloat16).to(dtype).to(DEV)
+    q, k, v, z, b, a = rnd(G * D), rnd(G * D), rnd(H * V), rnd(H * D), rnd(H), rnd(H)
+    k *= D ** -0.5 if rule != "delta" else 1.0
+    per_head = [torch.randn(H, generator=g).to(DEV) * 0.5 - 1.0 for _ in range(3)]
+    zb = torch.randn(H * D, generator=g).to(DEV)
+
+    def run(rows, starts, flags=0):
+        """Every sequence in its own slot, from zero; (outputs, states)."""
+        q, k, v, z, b, a = rows
+        S = len(starts) - 1
+        state = torch.full((S, H * D * V), 3.0, device=DEV)
+        at = (state, i32(list(range(S))), i32(starts), i32([0] * S), H)
+        ops.debug_flags(flags)
+        try:
+            if rule == "gla":
+                return ops.gla_scan(q, k, v, z, zb, 6.0, D ** -0.5, *at, D, V), state
+            if rule == "delta":
+                return ops.delta_rule_scan(q, k, v, b, a, per_head[0], per_head[1], D ** -0.5, *at, G, D, V), state
+            return ops.ssm_scan(v, k, q, a, per_head[0], per_head[1], per_head[2], *at, G, D, V), state
+        finally:
+            ops.debug_flags(0)
+
+    rows = [q, k, v, z, b, a]
+    out, state = run(rows, [0, n])
+    assert torch.isfinite(out).all() and torch.isfinite(state).all()
+    sixteen = run(rows, [0, n], 16)
+    assert torch.equal(sixteen[0], out) and torch.equal(sixteen[1], state)
+    short = [torch.cat([t] + [t[:1]] * (B - 1)) for t in rows]           # the portions of the others have one token
+    wide = run(short, [0] + list(range(n, n + B)))
+    assert torch.equal(wide[0][:n], out) and torch.equal(wide[1][0], state[0])
+    for shift in (1, 2):
+        padded = []
+        for t in rows:
+            m = torch.zeros(n, t.shape[1] + 3, dtype=dtype, device=DEV)
+            m[:, shift:shift + t.shape[1]] = t
+            padded.append(m[:, shift:shift + t.shape[1]])
+        moved = run(padded, [0, n])
+        assert torch.equal(moved[0], out) and torch.equal(moved[1], state), shift
