@@ -11,7 +11,7 @@
 //  * warp 1 issues S = Q K^T (tcgen05.mma, A and B from shared memory, 128x128 fp32 accumulator in
 //    TENSOR MEMORY, double buffered) and O += P V (A = P read from tensor memory, B = V from shared
 //    memory as an MN-major operand, 128 x D fp32 accumulator in tensor memory);
-//  * warps 2-5 own one query row per thread (TMEM lane = row): tcgen05.ld the 128 scores of the row,
+//  * the softmax warps own one query row per thread (TMEM lane = row), or half of its keys (SPLIT 2): tcgen05.ld the scores of the row,
 //    softmax them with a LAZY running maximum (the reference maximum is only moved, and O rescaled in
 //    tensor memory, when a row's maximum grows by more than 2^8 — otherwise exp2 stays in range and
 //    no correction pass is needed), write P back over S as packed 16-bit pairs (tcgen05.st);
@@ -27,15 +27,20 @@
 //    its copies in flight are waited for (again with a bound), tensor memory is freed and a counter is
 //    raised that the host can read (atoma_prefill_timeouts, atoma_kernel_timeouts); the CTA's outputs mean nothing then.
 //
-//  * paged keys and values (PAGED): two more warps look the pages up and copy rows of 16-byte pieces with cp.async into the same
+//  * paged keys and values (PAGED): three warps look the pages up and copy rows of 16-byte pieces with cp.async into the same
 //    swizzled tiles (a page's rows of one head are strided: no box of a tensor map covers a tile of pages in any order);
 //  * a quarter of the exponentials is a polynomial on the FMA pipe (exp2_poly2), and all heads' heaviest tiles start first;
 //  * an output gate is applied in the epilogue (fetched before the last P.V is waited for), so no pass over the outputs follows.
 //
-// Bound: the softmax warpgroups (exponentials and conversions) beside the tensor pipe.  Algorithmic flops: 4 * sum_b(visible
-// (q,k) pairs) * D per head.  Causal 8192 tokens, float16, 32 heads of 128: 627 -> 566 us by the share of polynomial
-// exponentials and the order of the tiles (none, 3/8 and 1/2 of them were slower).  Portions of 1500 tokens and less over
-// prefixes in pages: 765 us on the mma.sync tiles, 176 here.  Window of 4096 tokens with a distance table and a gate: 369 -> 301 us.
+// Bound: a tile's chain of products (S, then P V: 1300 to 1600 cycles, Q K^T at 100 instead of 64 per 128 x 128 x 16 since both operands come from
+// shared memory) and softmax (1700 to 2000), which the two query tiles of a CTA run in turn: 3500 cycles per 128 keys of 256 rows; without any
+// softmax the products alone take 3000.  Algorithmic flops: 4 * sum_b(visible (q,k) pairs) * D per head.
+//  * Causal 8192 tokens, float16, 32 heads of 128: 627 -> 566 us by the share of polynomial exponentials and the order of the tiles (none, 3/8 and 1/2
+//    of them were slower); 498 -> 479 (at higher clocks) with the maximum beside the exponentials (kEager).  Two threads a row: 488.
+//  * Portions of 1500 tokens and less over prefixes in pages: 765 us on the mma.sync tiles, 194 with two loading warps, 159 with three that hand a tile
+//    on at once; two threads a row, which halve the corrections: heads of 64 130 -> 126, others equal.
+//  * Window of 4096 tokens with a distance table and a gate: 324 -> 240 us with two threads a row (more of the biases' reads in flight), 216 with tiles on
+//    the diagonal and across the table's end on the path without clamps.
 #include "common.cuh"
 #include "mha_params.h"
 
@@ -49,15 +54,23 @@ bool launch_attention_tile(const MhaParams &p, bool is_bf16, cudaStream_t stream
 
 namespace {
 
-constexpr int kPfThreads = 384;  // warpgroup 0: loads (warp 0) + MMA issue (warp 1); warpgroups 1, 2: softmax
+// Threads: warpgroup 0 loads (warp 0) and issues the products (warp 1); then SPLIT softmax warpgroups per query tile, each of which takes 128 / SPLIT keys of a tile.
+template <int SPLIT>
+constexpr int kPfThreads = 128 + 256 * SPLIT;
 constexpr int kPfM = 128, kPfN = 128;
-constexpr int kQTiles = 2;       // two 128-row query tiles per CTA, one softmax warpgroup each
+constexpr int kQTiles = 2;       // two 128-row query tiles per CTA
 constexpr int kVStages = 2;
 constexpr int kPfWaitTries = 1 << 18;   // milliseconds at least (a try may also suspend the thread for a hardware-chosen time)
 constexpr int kTmemCols = 512;   // S_A 0..127 | S_B 128..255 | O_A 256.. | O_B 384..
-constexpr int kPfIssueRegs = 56, kPfSoftmaxRegs = 224;  // setmaxnreg: 168 * 384 = 56 * 128 + 224 * 256
+template <int SPLIT>
+constexpr int kPfIssueRegs = SPLIT == 1 ? 56 : 64;
+template <int SPLIT>
+constexpr int kPfSoftmaxRegs = SPLIT == 1 ? 224 : 104;  // setmaxnreg: 168 * 384 = 56 * 128 + 224 * 256; 96 * 640 = 64 * 128 + 104 * 512
 constexpr float kRescaleThreshold = 8.f;  // log2 units: P <= 2^8 between corrections
 constexpr int kPfBiasSmem = 2048;         // distances whose bias (this head's column of the table) is kept in shared memory
+// ... behind copies of its first row and in front of copies of its last, so that a tile on the diagonal (distances from -254 on) or across the table's end
+// reads its biases without a clamp: with one, such a tile took 9000 to 12000 cycles where others take 3000.
+constexpr int kPfBiasFront = 256, kPfBiasBack = 160;
 
 __device__ unsigned int g_prefill_late;   // CTAs that gave up waiting, since the library was loaded
 
@@ -119,10 +132,12 @@ __device__ __forceinline__ void exp2_poly2(uint64_t x2, float &p0, float &p1) {
 // P = 2^(s sc - m) of 32 scores as packed 16-bit pairs, and their sum.  MIX: every fourth pair leaves the special-function unit for the FMA
 // pipe (the unit's 16 results a cycle and SM are what bounds the softmax of heads of 64 and 128).  Tiles with masked scores, and kernels whose FMA pipe
 // adds a bias to every score, take the unit for all (4000 tokens in a window of 1024 with a distance table, heads of 128: 357 us, mixed 362).
-template <typename T, bool MIX>
-__device__ __forceinline__ void softmax_chunk(const uint32_t *sv, uint64_t sc2, uint64_t mm2, uint64_t (&ls)[2], uint32_t (&pk)[16]) {
+// MAX: the scores' maximum is taken beside them.
+template <typename T, bool MIX, bool MAX>
+__device__ __forceinline__ void softmax_chunk(const uint32_t *sv, uint64_t sc2, uint64_t mm2, uint64_t (&ls)[2], uint32_t (&pk)[16], float (&mx)[4]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
+        if (MAX) mx[i & 3] = max3(mx[i & 3], __uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1]));
         const uint64_t x2 = fma2(pk2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), sc2, mm2);
         float p0, p1;
         if (MIX && (i & 3) == 3) {
@@ -135,6 +150,20 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t *sv, uint64_t sc2, 
         ls[i & 1] = add2(ls[i & 1], pk2(p0, p1));
         pk[i] = pack2<T>(p0, p1);
     }
+}
+// ... of a thread's N scores, P to tensor memory.
+template <typename T, int N, bool MIX, bool MAX>
+__device__ __forceinline__ void softmax_scores(const uint32_t *sv, uint64_t sc2, uint64_t mm2, float &l, float (&mx)[4], uint32_t tmem_p) {
+    uint64_t ls[2] = {0ull, 0ull};
+#pragma unroll
+    for (int c = 0; c < N / 32; ++c) {
+        uint32_t pk[16];
+        softmax_chunk<T, MIX, MAX>(sv + c * 32, sc2, mm2, ls, pk, mx);
+        tmem_st_32x32b_x16(tmem_p + c * 16, pk);
+    }
+    float l0, l1;
+    upk2(add2(ls[0], ls[1]), l0, l1);
+    l = l0 + l1;
 }
 
 struct PfSeq {
@@ -164,11 +193,12 @@ __device__ __forceinline__ PfSeq pf_seq(const MhaParams &p, int bidb) {
     return s;
 }
 
+// SPLIT: softmax threads per query row.
 // BIAS: 1 or 2: a bias by query-key distance is added to the scaled scores (MhaParams::dist_bias); 2: the grid goes head by head.  Instantiations of their own, so
 // that the unbiased kernel keeps its register allocation.
 // PAGED: keys and values lie in pages behind a block table (MhaParams::block_table).
-template <typename T, int D, int KH, int BIAS, bool PAGED>
-__global__ void __launch_bounds__(kPfThreads, 1)
+template <typename T, int D, int KH, int BIAS, bool PAGED, int SPLIT>
+__global__ void __launch_bounds__(kPfThreads<SPLIT>, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const MhaParams p) {
     using C = PfCfg<D, KH>;
@@ -184,11 +214,16 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __shared__ int late_s;
     volatile int *late = &late_s;
     constexpr bool BIASED = BIAS != 0;
+    constexpr int N = kPfN / SPLIT;   // keys of a tile per softmax thread
     // Paged steps correct by every new maximum: a row's largest weight is then 1, which rounding to 16 bits leaves alone, as on the tile kernel, whose steps
     // these are (error against 64 bits of bfloat16 portions, queries of 1 and 4 times unit size: 2.08e-3 and 1.73e-3 there, 2.09e-3 and 1.74e-3 here,
     // 2.13e-3 and 2.09e-3 with corrections from 2^8 on; the portions of prompts over prefixes 180 -> 190 us).
     constexpr float kThreshold = PAGED ? 0.f : kRescaleThreshold;
-    __shared__ float bias_s[BIASED ? kPfBiasSmem : 1];
+    // Where most tiles correct nothing.  A thread of half the keys would have to learn of the other's maximum all the same; heads of 64 gain nothing (414 us, 428).
+        constexpr bool kEager = SPLIT == 1 && !PAGED && D == 128;
+    constexpr int kCorrect = SPLIT == 1 ? 32 : 16;   // columns of O that a correction holds
+    __shared__ float bias_s[BIASED ? kPfBiasFront + kPfBiasSmem + kPfBiasBack : 1];
+    __shared__ float swap_s[kQTiles][2][SPLIT == 2 ? kPfM : 1];            // a row's maximum (at the end: its sum) over either half of the keys
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // Heads, then sequences, then query tiles from the last (causal: heaviest) one down, so that the SMs run out of light tiles together
@@ -214,7 +249,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         for (int i = 0; i < kQTiles; ++i) {
             mbar_init(&q_full[i], 1);
             mbar_init(&s_full[i], 1);
-            mbar_init(&p_full[i], 4);  // one arrival per softmax warp
+            mbar_init(&p_full[i], 4 * SPLIT);  // one arrival per softmax warp
             mbar_init(&pv_done[i], 1);
         }
         fence_mbar_init();
@@ -223,7 +258,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tma_prefetch_desc(&map_v);
     }
     const int bias_n = BIASED ? min(p.dist_rows, kPfBiasSmem) : 0;
-    for (int i = tid; i < bias_n; i += kPfThreads) bias_s[i] = p.dist_bias[static_cast<int64_t>(i) * p.dist_heads + head] * 1.4426950408889634f;
+    if (BIASED)
+        for (int i = tid; i < kPfBiasFront + bias_n + kPfBiasBack; i += kPfThreads<SPLIT>)
+            bias_s[i] = p.dist_bias[static_cast<int64_t>(min(max(i - kPfBiasFront, 0), bias_n - 1)) * p.dist_heads + head] * 1.4426950408889634f;
     if (warp == 1) tmem_alloc(&tmem_base_smem, kTmemCols);
     tc_fence_before_sync();
     __syncthreads();
@@ -260,8 +297,49 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
     const int kvh = head / (p.h / p.h_k);  // flash_fwd_kernel.h:593
 
+    // ================================ paged loads: warps 2, 3 and, behind the queries, 0 ================================
+    // Pages are a few rows each, too small for a copy by the TMA unit each (a warp starts about six a microsecond); the 16-byte pieces of a tile of keys
+    // or values go by cp.async.  The tiles, K V K V .., go round the three warps; a warp hands a tile on as soon as its pieces have landed, while the
+    // others' tiles are under way (two warps that handed a tile on only behind their next one's copies, which wait for a free stage, made a tile
+    // of 128 keys cost 6700 cycles instead of 3500).  A lane looks up the rows 32 i + lane of a tile, and every piece asks for its row's place by shuffle.
+    [[maybe_unused]] auto paged_loads = [&](int worker) {
+        constexpr int kPieces = D / 8, kRowsPer = 32 / kPieces, kStages = 2;
+        static_assert(!PAGED || (kKStages == 2 && kVStages == 2 && KH == D / 64), "keys and values are loaded alike");
+        const int *table = p.block_table + static_cast<int64_t>(bidb) * p.bt_bs;
+        const int piece = lane % kPieces, sub = lane / kPieces;
+        for (int u = worker; u < 2 * (n_max - n_lo); u += 3) {
+            const bool keys = (u & 1) == 0;
+            const int jj = u >> 1, j = n_lo + jj, st = jj % kStages, left = len_k - j * kPfN;   // rows of the sequence from this tile on
+            const T *base = static_cast<const T *>(keys ? p.k : p.v) + static_cast<int64_t>(kvh) * (keys ? p.k_hs : p.v_hs) + piece * 8;
+            const int64_t bs = keys ? p.k_bs : p.v_bs, rs = keys ? p.k_rs : p.v_rs;
+            int64_t place[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = 32 * i + lane, key = j * kPfN + r;
+                const int pg = key / p.page;   // entries past the sequence's end are never read
+                place[i] = r < left ? static_cast<int64_t>(table[pg]) * bs + static_cast<int64_t>(key - pg * p.page) * rs : 0;
+            }
+            if (!pf_wait_all(keys ? &k_empty[st] : &v_empty[st], ((jj / kStages) & 1) ^ 1, late)) break;
+            const uint32_t dst = smem_u32((keys ? sk : sv) + st * C::kVBytes) + (piece >> 3) * C::kHalfBytes;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+#pragma unroll 4
+                for (int q = 0; q < kPieces; ++q) {
+                    const int rr = q * kRowsPer + sub, r = 32 * i + rr;
+                    const int64_t at = __shfl_sync(0xffffffffu, place[i], rr);
+                    cp_async_16(dst + r * 128 + (((piece & 7) ^ (r & 7)) << 4), base + at, r < left ? 16 : 0);
+                }
+            }
+            cp_async_commit();
+            cp_async_wait_all();
+            fence_proxy_async();       // generic-proxy writes -> visible to the tensor core's async reads
+            __syncwarp();
+            if (lane == 0) mbar_arrive(keys ? &k_full[st] : &v_full[st]);
+        }
+    };
+
     if (warp < 4) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfIssueRegs));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfIssueRegs<SPLIT>));
         if (warp == 0 && n_max > 0) {
             // ================================ loads ================================
             // A tile that lies completely inside its sequence is one TMA transaction (kHalves boxes);
@@ -307,6 +385,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     load_tile(QkPieces(), d_k, sq + t * C::kQkBytes, &map_q, &q_full[t], qg, p.q_rs, m0[t], len_q, si.q_row0 + m0[t],
                               head, si.q_batch, kL2EvictFirst);
             int k_issued = 0, v_issued = 0;
+            if constexpr (PAGED) paged_loads(2);
             for (int j = n_lo; !PAGED && j < n_max; ++j) {
                 const int jj = j - n_lo, ks = jj % kKStages, vs = jj % kVStages;
                 if (!pf_wait_all(&k_empty[ks], ((jj / kKStages) & 1) ^ 1, late)) break;
@@ -328,52 +407,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int i = max(0, k_issued - kKStages); i < k_issued; ++i) landed(&k_full[i % kKStages], (i / kKStages) & 1);
             for (int i = max(0, v_issued - kVStages); i < v_issued; ++i) landed(&v_full[i % kVStages], (i / kVStages) & 1);
         } else if (PAGED && warp >= 2 && n_max > 0) {
-            // ================================ paged loads: warp 2 the keys, warp 3 the values ================================
-            // Pages are a few rows each, too small for a copy by the TMA unit each (a warp starts about six a microsecond); one tile's 16-byte
-            // pieces go by cp.async while the tile before it lands and is handed on.  A lane looks up the rows 32 i + lane of a tile, and
-            // every piece asks for its row's place by shuffle.
-            const bool keys = warp == 2;
-            constexpr int kPieces = D / 8, kRowsPer = 32 / kPieces, kStages = kKStages < kVStages ? kKStages : kVStages;
-            static_assert(!PAGED || (kKStages == 2 && kVStages == 2 && KH == D / 64), "the two loading warps run alike");
-            const T *base = static_cast<const T *>(keys ? p.k : p.v) + static_cast<int64_t>(kvh) * (keys ? p.k_hs : p.v_hs);
-            const int64_t bs = keys ? p.k_bs : p.v_bs, rs = keys ? p.k_rs : p.v_rs;
-            const int *table = p.block_table + static_cast<int64_t>(bidb) * p.bt_bs;
-            unsigned char *ring = keys ? sk : sv;
-            uint64_t *full = keys ? k_full : v_full, *empty = keys ? k_empty : v_empty;
-            const int piece = lane % kPieces, sub = lane / kPieces;
-            auto hand_on = [&](int jj) {   // this lane's pieces of the tile have landed
-                fence_proxy_async();       // generic-proxy writes -> visible to the tensor core's async reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[jj % kStages]);
-            };
-            for (int j = n_lo; j < n_max; ++j) {
-                const int jj = j - n_lo, st = jj % kStages, left = len_k - j * kPfN;   // rows of the sequence from this tile on
-                int64_t place[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = 32 * i + lane, key = j * kPfN + r;
-                    const int pg = key / p.page;   // entries past the sequence's end are never read
-                    place[i] = r < left ? static_cast<int64_t>(table[pg]) * bs + static_cast<int64_t>(key - pg * p.page) * rs : 0;
-                }
-                if (!pf_wait_all(&empty[st], ((jj / kStages) & 1) ^ 1, late)) break;
-                const uint32_t dst = smem_u32(ring + st * C::kVBytes);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-#pragma unroll 4
-                    for (int q = 0; q < kPieces; ++q) {
-                        const int rr = q * kRowsPer + sub, r = 32 * i + rr;
-                        const int64_t at = __shfl_sync(0xffffffffu, place[i], rr);
-                        cp_async_16(dst + (piece >> 3) * C::kHalfBytes + r * 128 + (((piece & 7) ^ (r & 7)) << 4), base + at + piece * 8, r < left ? 16 : 0);
-                    }
-                }
-                cp_async_commit();
-                const bool now = jj == 0 || j + 1 == n_max;   // the first and the last tile have no other to overlap with
-                if (now) cp_async_wait_all();
-                else asm volatile("cp.async.wait_group 1;" ::: "memory");
-                if (jj > 1) hand_on(jj - 1);
-                if (now) hand_on(jj);
-            }
-            cp_async_wait_all();
+            paged_loads(warp - 2);
         } else if (warp == 1 && n_max > 0) {
             // ================================ MMA issue ================================
             // The whole warp runs this role converged on warp-uniform values; only the tcgen05
@@ -458,8 +492,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
     } else {
         // ================================ softmax / epilogue warpgroups ================================
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPfSoftmaxRegs));
-        const int t = (warp >> 2) - 1;          // query tile of this warpgroup
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPfSoftmaxRegs<SPLIT>));
+        const int t = (warp - 4) / (4 * SPLIT), half = SPLIT == 2 ? ((warp - 4) >> 2) & 1 : 0;   // query tile and half of its keys of this warpgroup
         const int quad = warp & 3;
         const int row = quad * 32 + lane;       // query row of this thread within the tile
         const int m0t = t ? m0[1] : m0[0];
@@ -467,121 +501,133 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int n_tiles = t ? nt[1] : nt[0];
         const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
         const uint32_t tmem_s = tmem_base + lane_addr + t * 128;
-        const uint32_t tmem_o = tmem_base + lane_addr + 256 + t * 128;
+        const uint32_t tmem_o = tmem_base + lane_addr + 256 + t * 128 + half * (D / SPLIT);   // this half corrects and stores half of O's columns
         T *og = static_cast<T *>(p.o) + si.o_off + static_cast<int64_t>(head) * p.o_hs +
-                static_cast<int64_t>(grow) * p.o_rs;
+                static_cast<int64_t>(grow) * p.o_rs + half * (D / SPLIT);
         int64_t lse_idx = 0;
         if (p.lse && grow < len_q) {
             if (p.unpadded_lse && p.cu_q) lse_idx = static_cast<int64_t>(head) * p.cu_q[p.b] + si.q_start + grow;
             else lse_idx = (static_cast<int64_t>(bidb) * p.h + head) * p.seqlen_q + grow;
         }
+        // the two warps of a row quad tell each other a value per row (both run the same tiles)
+        [[maybe_unused]] auto swap = [&](float mine) {
+            swap_s[t][half][row] = mine;
+            tc_fence_before_sync();
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + t * 4 + quad) : "memory");
+            tc_fence_after_sync();
+            return swap_s[t][half ^ 1][row];
+        };
         if (n_tiles > 0) {
             float m_ref = -INFINITY, l_run = 0.f;
             if (p.sink) {   // the sink is one more term of the denominator: the running state starts from it
                 m_ref = p.sink[head] * 1.4426950408889634f;
-                l_run = 1.f;
+                l_run = half ? 0.f : 1.f;
             }
             for (int j = n_lo; j < n_tiles; ++j) {
                 pf_wait(&s_full[t], (j - n_lo) & 1, late);
                 tc_fence_after_sync();
-                uint32_t sv_[128];
+                uint32_t sv_[N];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(tmem_s + c * 32, sv_ + c * 32);
+                for (int c = 0; c < N / 32; ++c) tmem_ld_32x32b_x32(tmem_s + half * N + c * 32, sv_ + c * 32);
                 tmem_ld_wait();
-                // ---- bias by distance: the scores move to the scaled log2 domain here, and `sc` below becomes 1 ----
+                const int col0 = j * kPfN + half * N;
+                // ---- bias by distance: the scores move to the scaled log2 domain here, and `sc` below becomes 1; where all of the warp's keys lie
+                // beyond the table's last row the bias is one value, which goes into the exponent with the maximum ----
+                float sc = p.scale_log2, far_bias = 0.f;
+                bool far = !BIASED;
                 if constexpr (BIASED) {
-                    const int d0 = grow + shift - j * kPfN, last = p.dist_rows - 1;   // distance of this row to the tile's first key
-                    const float sl2 = p.scale_log2;
-                    if (__all_sync(0xffffffffu, d0 - 127 >= last) && last < bias_n) {
-                        // the whole tile lies beyond the table's last row for every row of the warp: one value
-                        const float bv = bias_s[last];
-#pragma unroll
-                        for (int c = 0; c < 128; ++c) sv_[c] = __float_as_uint(fmaf(__uint_as_float(sv_[c]), sl2, bv));
-                    } else if (__all_sync(0xffffffffu, d0 - 127 >= 0 && d0 < bias_n && d0 <= last)) {
+                    const int d0 = grow + shift - col0, last = p.dist_rows - 1;   // distance of this row to the half's first key
+                    const float sl2 = sc;
+                    if (__all_sync(0xffffffffu, d0 - (N - 1) >= last) && last < bias_n) {
+                        far = true;
+                        far_bias = bias_s[kPfBiasFront + last];
+                    } else if (__all_sync(0xffffffffu, d0 - (N - 1) >= -kPfBiasFront && d0 < last + kPfBiasBack) && last < bias_n) {
                         // every distance of the tile is a row of the shared-memory copy: no clamps, constant offsets from one address
-                        const float *bp = bias_s + d0;
+                        const float *bp = bias_s + kPfBiasFront + d0;
 #pragma unroll
-                        for (int c = 0; c < 128; ++c) sv_[c] = __float_as_uint(fmaf(__uint_as_float(sv_[c]), sl2, bp[-c]));
+                        for (int c = 0; c < N; ++c) sv_[c] = __float_as_uint(fmaf(__uint_as_float(sv_[c]), sl2, bp[-c]));
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 128; ++c) {
+                        for (int c = 0; c < N; ++c) {
                             const int dist = min(max(d0 - c, 0), last);
-                            const float bv = dist < bias_n ? bias_s[dist]
+                            const float bv = dist < bias_n ? bias_s[kPfBiasFront + dist]
                                                            : __ldg(p.dist_bias + static_cast<int64_t>(dist) * p.dist_heads + head) * 1.4426950408889634f;
                             sv_[c] = __float_as_uint(fmaf(__uint_as_float(sv_[c]), sl2, bv));
                         }
                     }
                 }
-                const float sc = BIASED ? 1.f : p.scale_log2;
+                if (!far) sc = 1.f;
                 // ---- masks: only tiles that touch the sequence end or the causal diagonal ----
-                const int col0 = j * kPfN;
-                const bool tail = col0 + kPfN > len_k;
-                const bool diag = p.is_causal && (col0 + kPfN - 1 > m0t + shift);
+                const bool tail = col0 + N > len_k;
+                const bool diag = p.is_causal && (col0 + N - 1 > m0t + shift);
                 const bool low = window > 0 && col0 < m0t + kPfM + shift - window;   // some row's window starts inside or after this tile
                 if (tail || diag || low) {
                     const int lim = p.is_causal ? min(len_k, grow + shift + 1) : len_k;  // first masked column
                     const int lb = window > 0 ? grow + shift - window + 1 : -(1 << 30);  // first visible column
 #pragma unroll
-                    for (int c = 0; c < 128; ++c)
+                    for (int c = 0; c < N; ++c)
                         if (col0 + c >= lim || col0 + c < lb) sv_[c] = 0xff800000u;  // -inf
                 }
-                // eight independent chains: a single running max / sum is 128 dependent operations
-                float mx8[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) mx8[i] = __uint_as_float(sv_[i]);
-#pragma unroll
-                for (int c = 8; c + 15 < 128; c += 16)
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) mx8[i] = max3(mx8[i], __uint_as_float(sv_[c + i]), __uint_as_float(sv_[c + 8 + i]));
-#pragma unroll
-                for (int i = 0; i < 8; ++i) mx8[i] = fmaxf(mx8[i], __uint_as_float(sv_[120 + i]));
-                const float mx = fmaxf(max3(mx8[0], mx8[1], mx8[2]), fmaxf(max3(mx8[3], mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7])));
-                const float m_tile = mx * sc;  // scale_log2 > 0 (checked on the host)
-                // ---- running maximum ----
-                const bool need = m_tile > m_ref + kThreshold;  // also the first finite tile (m_ref = -inf)
-                if (__any_sync(0xffffffffu, need)) {
-                    const float alpha = need ? (m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - m_tile)) : 1.f;
-                    if (need) m_ref = m_tile;
-                    l_run *= alpha;
-                    if (j > n_lo) {
-                        // O of this row lives in tensor memory: wait until P.V of the previous tile has
-                        // been accumulated, rescale, write back.  Rare after the first tiles.
-                        pf_wait(&pv_done[t], (j - 1 - n_lo) & 1, late);
-                        tc_fence_after_sync();
-#pragma unroll
-                        for (int c = 0; c < D / 32; ++c) {
-                            uint32_t ov[32];
-                            tmem_ld_32x32b_x32(tmem_o + c * 32, ov);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-                            tmem_st_32x32b_x32(tmem_o + c * 32, ov);
-                        }
-                        tmem_st_wait();
-                    }
-                }
-                const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+                const bool masked = tail || diag || low;
+                const uint64_t sc2 = pk2(sc, sc);
+                const uint32_t tmem_p = tmem_s + half * (N / 2);
                 // ---- P = exp2(S * scale - m), row sum, packed 16-bit pairs back over S ----
-                uint64_t ls[2] = {0ull, 0ull};
-                const uint64_t sc2 = pk2(sc, sc), mm2 = pk2(-m_use, -m_use);
-                if (tail || diag || low) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t pk[16];
-                        softmax_chunk<T, false>(sv_ + c * 32, sc2, mm2, ls, pk);
-                        tmem_st_32x32b_x16(tmem_s + c * 16, pk);
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t pk[16];
-                        softmax_chunk<T, !BIASED>(sv_ + c * 32, sc2, mm2, ls, pk);
-                        tmem_st_32x32b_x16(tmem_s + c * 16, pk);
-                    }
+                // Most tiles move no row's reference maximum: the exponentials start from the one at hand and the tile's maximum is taken beside them.
+                float l_tile = 0.f, mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                bool done = false;
+                if (kEager && j > n_lo && !masked) {
+                    const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+                    softmax_scores<T, N, true, true>(sv_, sc2, pk2(-m_use, -m_use), l_tile, mx4, tmem_p);
+                    const float m_tile = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sc;
+                    done = !__any_sync(0xffffffffu, m_tile > m_ref + kThreshold);
+                    if (!done) tmem_st_wait();   // P is written once more
                 }
-                float l0, l1;
-                upk2(add2(ls[0], ls[1]), l0, l1);
-                l_run += l0 + l1;
+                if (!done) {
+                    // eight independent chains: a single running maximum is a chain of dependent operations
+                    float mx8[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) mx8[i] = max3(__uint_as_float(sv_[i]), __uint_as_float(sv_[8 + i]), __uint_as_float(sv_[16 + i]));
+#pragma unroll
+                    for (int c = 24; c + 15 < N; c += 16)
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) mx8[i] = max3(mx8[i], __uint_as_float(sv_[c + i]), __uint_as_float(sv_[c + 8 + i]));
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) mx8[i] = fmaxf(mx8[i], __uint_as_float(sv_[N - 8 + i]));
+                    const float mx = fmaxf(max3(mx8[0], mx8[1], mx8[2]), fmaxf(max3(mx8[3], mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7])));
+                    float m_tile = BIASED ? fmaf(mx, sc, far_bias) : mx * sc;  // scale_log2 > 0 (checked on the host)
+                    if constexpr (SPLIT == 2) m_tile = fmaxf(m_tile, swap(m_tile));   // both halves' scores are in registers: P may be written over them
+                    // ---- running maximum ----
+                    const bool need = m_tile > m_ref + kThreshold;  // also the first finite tile (m_ref = -inf)
+                    if (__any_sync(0xffffffffu, need)) {
+                        const float alpha = need ? (m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - m_tile)) : 1.f;
+                        if (need) m_ref = m_tile;
+                        l_run *= alpha;
+                        if (j > n_lo) {
+                            // O of this row lives in tensor memory: wait until P.V of the previous tile has
+                            // been accumulated, rescale, write back.  Rare after the first tiles.
+                            pf_wait(&pv_done[t], (j - 1 - n_lo) & 1, late);
+                            tc_fence_after_sync();
+#pragma unroll 1
+                            for (int c = 0; c < D / SPLIT; c += kCorrect) {       // the scores hold most registers
+                                uint32_t ov[kCorrect];
+#pragma unroll
+                                for (int i = 0; i < kCorrect; i += 16) tmem_ld_32x32b_x16(tmem_o + c + i, *reinterpret_cast<uint32_t (*)[16]>(ov + i));
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int i = 0; i < kCorrect; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+#pragma unroll
+                                for (int i = 0; i < kCorrect; i += 16) tmem_st_32x32b_x16(tmem_o + c + i, ov + i);
+                            }
+                            tmem_st_wait();
+                        }
+                    }
+                    const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+                    const float off = BIASED ? far_bias - m_use : -m_use;
+                    const uint64_t mm2 = pk2(off, off);
+                    if (masked || !far) softmax_scores<T, N, false, false>(sv_, sc2, mm2, l_tile, mx4, tmem_p);
+                    else softmax_scores<T, N, true, false>(sv_, sc2, mm2, l_tile, mx4, tmem_p);
+                }
+                l_run += l_tile;
                 tmem_st_wait();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -589,18 +635,23 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             // ---- epilogue: O / rowsum -> global ----
             const bool gated = p.gate && grow < len_q && (p.gate_below <= 0 || grow + shift + (p.key_lo ? p.key_lo[bidb] : 0) < p.gate_below);
-            uint4 gv[D / 8];   // the row's gate: under way while the last products run
+            if constexpr (SPLIT == 2) {   // both halves' sums of a row, in the same order on both sides
+                const float other = swap(l_run);
+                l_run = half ? other + l_run : l_run + other;
+            }
+            // this half's part of the row's gate, 32 columns at a time: the first are under way while the last products run
+            const T *gg = gated ? static_cast<const T *>(p.gate) + static_cast<int64_t>(si.q_row0 + grow) * p.gate_rs + static_cast<int64_t>(head) * D + half * (D / SPLIT) : nullptr;
+            uint4 gv[4];
             if (gated) {
-                const T *gg = static_cast<const T *>(p.gate) + static_cast<int64_t>(si.q_row0 + grow) * p.gate_rs + static_cast<int64_t>(head) * D;
 #pragma unroll
-                for (int i = 0; i < D / 8; ++i) gv[i] = *reinterpret_cast<const uint4 *>(gg + i * 8);
+                for (int i = 0; i < 4; ++i) gv[i] = *reinterpret_cast<const uint4 *>(gg + i * 8);
             }
             pf_wait(&pv_done[t], (n_tiles - 1 - n_lo) & 1, late);
             tc_fence_after_sync();
             const bool empty = (l_run == 0.f || l_run != l_run);
             const float inv = empty ? 0.f : 1.f / l_run;
 #pragma unroll
-            for (int c = 0; c < D / 32; ++c) {
+            for (int c = 0; c < D / 32 / SPLIT; ++c) {
                 uint32_t ov[32];
                 tmem_ld_32x32b_x32(tmem_o + c * 32, ov);
                 tmem_ld_wait();
@@ -608,10 +659,11 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     if (gated) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            const T *ge = reinterpret_cast<const T *>(&gv[c * 4 + i]);
+                            const T *ge = reinterpret_cast<const T *>(&gv[i]);
 #pragma unroll
                             for (int e = 0; e < 8; ++e)
                                 ov[8 * i + e] = __float_as_uint(over_one_plus(__uint_as_float(ov[8 * i + e]), expf(-static_cast<float>(ge[e]))));
+                            if (c + 1 < D / 32 / SPLIT) gv[i] = *reinterpret_cast<const uint4 *>(gg + (c + 1) * 32 + i * 8);
                         }
                     }
 #pragma unroll
@@ -625,13 +677,13 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     }
                 }
             }
-            if (p.lse && grow < len_q)
+            if (p.lse && half == 0 && grow < len_q)
                 p.lse[lse_idx] = empty ? INFINITY : m_ref * 0.6931471805599453f + __logf(l_run);
         } else if (grow < len_q && !skip) {
             // No visible key for any row of this tile: O = 0, LSE = +inf (flash_fwd_kernel.h:543-582).
 #pragma unroll
-            for (int c = 0; c < D / 8; ++c) *reinterpret_cast<uint4 *>(og + c * 8) = make_uint4(0, 0, 0, 0);
-            if (p.lse) p.lse[lse_idx] = INFINITY;
+            for (int c = 0; c < D / 8 / SPLIT; ++c) *reinterpret_cast<uint4 *>(og + c * 8) = make_uint4(0, 0, 0, 0);
+            if (p.lse && half == 0) p.lse[lse_idx] = INFINITY;
         }
     }
 
@@ -692,11 +744,12 @@ bool make_attn_map(CUtensorMap *out, const void *ptr, int d, int heads, int64_t 
 
 template <typename T, int D, int KH, int BIAS, bool PAGED = false>
 bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const MhaParams &p, cudaStream_t stream) {
+    constexpr int SPLIT = BIAS || PAGED ? 2 : 1;
     constexpr size_t smem = PfCfg<D, KH>::kSmem;
     static thread_local int attr_dev = -1;
     const DeviceInfo &di = current_device_info();
     if (attr_dev != di.ordinal) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<T, D, KH, BIAS, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<T, D, KH, BIAS, PAGED, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem));
         if (e != cudaSuccess) {
             set_status(static_cast<int>(e), "prefill: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -708,7 +761,7 @@ bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtens
     pp.late = late_word();
     dim3 grid(p.h, p.b, (p.seqlen_q + kQTiles * kPfM - 1) / (kQTiles * kPfM));
     if (BIAS == 2) grid = dim3(grid.z, grid.x, grid.y);
-    prefill_attn_kernel<T, D, KH, BIAS, PAGED><<<grid, kPfThreads, smem, stream>>>(mq, mk, mv, pp);
+    prefill_attn_kernel<T, D, KH, BIAS, PAGED, SPLIT><<<grid, kPfThreads<SPLIT>, smem, stream>>>(mq, mk, mv, pp);
     note_launch();
     return check_launch("prefill_attn_kernel");
 }
