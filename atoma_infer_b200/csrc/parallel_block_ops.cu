@@ -364,14 +364,23 @@ __global__ void __launch_bounds__(256) qkv_headnorm_rope_cache_kernel(const atom
 // The same for bfloat16 heads of whole 16-byte pieces: L lanes own a head, each two runs of four entries that stay in registers from the load
 // to the store.  A lane's runs are the two halves of its four pairs (or, pairs of neighbours, eight entries in a row), so it turns
 // them without asking another lane, and its sines and cosines serve every head of the token; entries behind the turned ones go to the lanes that
-// are left, eight in a row.  A lane issues the loads of up to four heads before it uses the first; values that only move are one run of bytes.
-// Bound: HBM, then instruction issue (0.74 of the slots).  8192 tokens of 32 + 16 heads of 128, 201 MB: a warp per head, element by element
-// through shared memory 147 us (latency of six dependent rounds per token); eight entries in a row per lane, the other half of a pair by
-// shuffles 99; this 61; four tokens a CTA, one pass over their angles, 93 (the loads of a token wait for the one before).
+// are left, eight in a row.  A warp takes one of `parts` equal shares of a token's heads, 32 / L at a time, forms the token's angles itself (each group of
+// L lanes some of them, the others by shuffles) and issues the loads of up to four rounds before it uses the first; no shared memory, no barrier.
+// Values that only move are one run of bytes.
+// Bound: HBM.  8192 tokens of 32 + 16 heads of 128, 201 MB: a warp per head, element by element through shared memory 147 us; a CTA per token
+// 65.6 (0.73 of the issue slots: 47 M instructions, weights read and addresses formed per head, angles behind a barrier); this 46.1 (20 M); 8000 tokens of
+// 32 + 16 heads of 64 51.3 and 29.3.  24 warps an SM without spilled registers 51.2, 40 with loads of three heads 71.8.
 constexpr int kQkvHeads = 4;
-__device__ __forceinline__ void unpack4(uint2 r, float (&v)[4]) {
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&r.x)), y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&r.y));
-    v[0] = x.x, v[1] = x.y, v[2] = y.x, v[3] = y.y;
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t unpack2(uint32_t w) { return pk2(__uint_as_float(__byte_perm(w, 0u, 0x1044)), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ uint32_t repack2(uint64_t v) {
+    float lo, hi;
+    upk2(v, lo, hi);
+    return pack2<__nv_bfloat16>(lo, hi);
 }
 struct HeadRuns {   // a lane's two runs of four entries in a head of n with `pairs` turned pairs (-1: none)
     int a, b;
@@ -386,133 +395,163 @@ __device__ __forceinline__ HeadRuns head_runs(int l, int n, int pairs, bool inte
     if (8 * l >= n) r.a = r.b = -1;
     return r;
 }
+// What turns a lane's pairs: halves (0, 1), (2, 3): cosines, sines and their negatives of two pairs at a time; neighbours: (cos, cos) and (-sin, sin) of each.
 struct HeadTurns {
-    float4 s0, s1;   // sin, cos of a lane's four pairs
+    uint64_t c[4], s[4];
 };
-// One head's two runs in a lane: bias, norm (mul > 0: over the L lanes of `group`, 1 / n = mul), weight, turn, back to bfloat16.
+// The angles of a lane's four pairs (4 l .. 4 l + 3 of `pairs`): the groups of L lanes take turns, and every lane asks for what it needs.
 template <int L, bool IL>
-__device__ __forceinline__ void head_finish(uint2 &ra, uint2 &rb, const HeadRuns &r, const float *bias, float mul, float eps, float head_scale, const float *w,
-                                            const HeadTurns &turns, unsigned group) {
-    float x[4], y[4];
-    unpack4(ra, x);
-    unpack4(rb, y);
-    if (bias && r.a >= 0) {
-        const float4 b0 = *reinterpret_cast<const float4 *>(bias + r.a), b1 = *reinterpret_cast<const float4 *>(bias + r.b);
-        x[0] += b0.x, x[1] += b0.y, x[2] += b0.z, x[3] += b0.w, y[0] += b1.x, y[1] += b1.y, y[2] += b1.z, y[3] += b1.w;
+__device__ __forceinline__ HeadTurns head_turns(float pos, const float *freq, const float *freq_lo, float amplitude, int pairs) {
+    constexpr int NG = 32 / L, OWN = NG >= 4 ? 1 : 4 / NG;
+    const int lane = threadIdx.x & 31, l = lane % L, g = lane / L;
+    float sn[OWN], cs[OWN];
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+        const int i = 4 * l + k * NG + g;
+        sn[k] = 0.f, cs[k] = 1.f;
+        if (i < pairs && k * NG + g < 4) turn(pos, freq[i], freq_lo ? freq_lo[i] : 0.f, amplitude, sn[k], cs[k]);
     }
-    if (mul > 0.f) {
-        float ss = 0.f;
+    float s4[4], c4[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) ss = fmaf(x[j], x[j], fmaf(y[j], y[j], ss));
+    for (int j = 0; j < 4; ++j) {
+        s4[j] = __shfl_sync(0xffffffffu, sn[j / NG], j % NG * L + l);
+        c4[j] = __shfl_sync(0xffffffffu, cs[j / NG], j % NG * L + l);
+    }
+    HeadTurns t;
 #pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(group, ss, o);
-        const float inv = rsqrtf(fmaf(ss, mul, eps)) * head_scale;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) x[j] *= inv, y[j] *= inv;
-        if (w && r.a >= 0) {
-            const float4 w0 = *reinterpret_cast<const float4 *>(w + r.a), w1 = *reinterpret_cast<const float4 *>(w + r.b);
-            x[0] *= w0.x, x[1] *= w0.y, x[2] *= w0.z, x[3] *= w0.w, y[0] *= w1.x, y[1] *= w1.y, y[2] *= w1.z, y[3] *= w1.w;
+    for (int j = 0; j < 4; ++j) {
+        if (IL) {
+            t.c[j] = pk2(c4[j], c4[j]);
+            t.s[j] = pk2(-s4[j], s4[j]);
+        } else if (j < 2) {
+            t.c[j] = pk2(c4[2 * j], c4[2 * j + 1]);
+            t.s[j] = pk2(s4[2 * j], s4[2 * j + 1]);
+            t.c[j + 2] = 0;
+            t.s[j + 2] = pk2(-s4[2 * j], -s4[2 * j + 1]);
         }
     }
-    if (r.turned) {
-        auto rotate = [](float &u, float &v, float sn, float cs) {
-            const float p = u * cs - v * sn;
-            v = v * cs + u * sn;
-            u = p;
-        };
-        rotate(x[0], IL ? x[1] : y[0], turns.s0.x, turns.s0.y);
-        rotate(IL ? x[2] : x[1], IL ? x[3] : y[1], turns.s0.z, turns.s0.w);
-        rotate(IL ? y[0] : x[2], IL ? y[1] : y[2], turns.s1.x, turns.s1.y);
-        rotate(IL ? y[2] : x[3], y[3], turns.s1.z, turns.s1.w);
-    }
-    ra = make_uint2(pack2<__nv_bfloat16>(x[0], x[1]), pack2<__nv_bfloat16>(x[2], x[3]));
-    rb = make_uint2(pack2<__nv_bfloat16>(y[0], y[1]), pack2<__nv_bfloat16>(y[2], y[3]));
+    return t;
 }
-template <int L, bool IL, int NT>   // NT: threads (0: fewer than 256, as launched)
-__global__ void __launch_bounds__(256, 4) qkv_headnorm_rope_cache_vec_kernel(const atoma_qkv_rope_args a) {
-    extern __shared__ __align__(16) float sm[];
+// Rounds of 32 / L heads from head u0 on, to n, of a token: src, dst and bias point to head 0; norm over the head's L lanes (mul = 1 / size; 0: none),
+// weight w, scale per head, turn, back to bfloat16.  Every lane of a warp makes the same rounds, since a head's sum is asked for by shuffles.
+// WHOLE: heads of 8 L entries, all of them turned, so that every lane has its eight and all distances are constants.
+template <int L, bool IL, bool WHOLE>
+__device__ __forceinline__ void heads_finish(const __nv_bfloat16 *src, __nv_bfloat16 *dst, int u0, int n, int size, const HeadRuns &r, const float *bias, float mul, float eps,
+                                             const float *head_scale, const float *w, const HeadTurns &turns) {
+    constexpr int NG = 32 / L;
+    const int lane = threadIdx.x & 31, g = lane / L, l = lane % L;
+    const bool mine = WHOLE || r.a >= 0, turned = WHOLE || r.turned;
+    const int at = WHOLE ? (IL ? 8 : 4) * l : max(r.a, 0), gap = WHOLE ? (IL ? 4 : 4 * L) : r.b - r.a, stride = WHOLE ? 256 : NG * size;
+    const int64_t begin = static_cast<int64_t>(u0 + g) * (WHOLE ? 8 * L : size) + at;
+    src += begin, dst += begin;
+    if (bias) bias += begin;
+    ulonglong2 w0 = make_ulonglong2(0, 0), w1 = w0;
+    if (w && mine) {
+        w0 = *reinterpret_cast<const ulonglong2 *>(w + at);
+        w1 = *reinterpret_cast<const ulonglong2 *>(w + at + gap);
+    }
+    for (; u0 < n; u0 += kQkvHeads * NG) {
+        const int left = n - u0 - g;             // heads from this lane's on
+        uint2 ra[kQkvHeads], rb[kQkvHeads];
+#pragma unroll
+        for (int i = 0; i < kQkvHeads; ++i) {
+            ra[i] = rb[i] = make_uint2(0, 0);
+            if (left > i * NG && mine) {
+                ra[i] = *reinterpret_cast<const uint2 *>(src + i * stride);
+                rb[i] = *reinterpret_cast<const uint2 *>(src + i * stride + gap);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kQkvHeads; ++i) {
+            if (u0 + i * NG >= n) break;
+            uint64_t v[4] = {unpack2(ra[i].x), unpack2(ra[i].y), unpack2(rb[i].x), unpack2(rb[i].y)};
+            const bool live = left > i * NG && mine;
+            if (bias && live) {
+                const ulonglong2 b0 = *reinterpret_cast<const ulonglong2 *>(bias + i * stride), b1 = *reinterpret_cast<const ulonglong2 *>(bias + i * stride + gap);
+                v[0] = add2(v[0], b0.x), v[1] = add2(v[1], b0.y), v[2] = add2(v[2], b1.x), v[3] = add2(v[3], b1.y);
+            }
+            if (mul > 0.f) {
+                float lo, hi;
+                upk2(fma2(v[0], v[0], fma2(v[1], v[1], fma2(v[2], v[2], mul2(v[3], v[3])))), lo, hi);
+                float ss = lo + hi;
+#pragma unroll
+                for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                float inv = rsqrtf(fmaf(ss, mul, eps));
+                if (head_scale && left > i * NG) inv *= head_scale[u0 + g + i * NG];
+                const uint64_t inv2 = pk2(inv, inv);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = mul2(v[j], inv2);
+                if (w) v[0] = mul2(v[0], w0.x), v[1] = mul2(v[1], w0.y), v[2] = mul2(v[2], w1.x), v[3] = mul2(v[3], w1.y);
+            }
+            if (turned) {
+                if (IL) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float lo, hi;
+                        upk2(v[j], lo, hi);
+                        v[j] = fma2(v[j], turns.c[j], mul2(pk2(hi, lo), turns.s[j]));
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const uint64_t u = v[j];
+                        v[j] = fma2(u, turns.c[j], mul2(v[2 + j], turns.s[2 + j]));
+                        v[2 + j] = fma2(v[2 + j], turns.c[j], mul2(u, turns.s[j]));
+                    }
+                }
+            }
+            if (live) {
+                *reinterpret_cast<uint2 *>(dst + i * stride) = make_uint2(repack2(v[0]), repack2(v[1]));
+                *reinterpret_cast<uint2 *>(dst + i * stride + gap) = make_uint2(repack2(v[2]), repack2(v[3]));
+            }
+        }
+        src += kQkvHeads * stride;
+        dst += kQkvHeads * stride;
+        if (bias) bias += kQkvHeads * stride;
+    }
+}
+constexpr int kQkvWarps = 4, kQkvResident = 32;   // warps of a CTA, of an SM
+template <int L, bool IL, bool WHOLE>
+__global__ void __launch_bounds__(32 * kQkvWarps, kQkvResident / kQkvWarps) qkv_headnorm_rope_cache_vec_kernel(const atoma_qkv_rope_args a, int parts) {
     using bf16 = __nv_bfloat16;
+    constexpr int NG = 32 / L;
     pdl_launch_dependents();
     pdl_wait();
-    const int64_t t = blockIdx.x;
+    const unsigned job = blockIdx.x * kQkvWarps + threadIdx.x / 32;
+    const int t = static_cast<int>(job / static_cast<unsigned>(parts)), part = static_cast<int>(job % static_cast<unsigned>(parts));
+    if (t >= a.T) return;
     const int H = static_cast<int>(a.H), G = static_cast<int>(a.G), D = static_cast<int>(a.dim), V = static_cast<int>(a.vdim);
     const int Gv = a.v_heads > 0 ? static_cast<int>(a.v_heads) : G;
+    const int lane = threadIdx.x & 31, l = lane % L;
     const int64_t slot = a.slot_mapping ? a.slot_mapping[t] : -1;
-    const int units = slot >= 0 ? H + G : H;
-    const int l = threadIdx.x % L, first = threadIdx.x / L;
-    const int nt = NT ? NT : static_cast<int>(blockDim.x), step = nt / L;
-    const unsigned group = L == 32 ? 0xffffffffu : ((1u << (L & 31)) - 1u) << (threadIdx.x & 31 & ~(L - 1));   // a head's lanes go the same way
     const int qk_pairs = a.qk_freq ? static_cast<int>(a.rot_pairs) : 0, v_pairs = a.v_freq ? static_cast<int>(a.v_pairs) : 0;
     const HeadRuns qk = head_runs(l, D, qk_pairs, IL);
     const bf16 *row = static_cast<const bf16 *>(a.proj) + t * a.ld;
-    const int q_off = static_cast<int>(a.q_off), k_off = static_cast<int>(a.k_off) - H * D;   // of unit 0, so that unit u lies at + u D
-    uint2 ra[kQkvHeads], rb[kQkvHeads];
-    auto fetch = [&](int u0) {
-#pragma unroll
-        for (int i = 0; i < kQkvHeads; ++i) {
-            const int u = u0 + first + i * step;
-            ra[i] = rb[i] = make_uint2(0, 0);
-            if (u < units && qk.a >= 0) {
-                const bf16 *p = row + (u < H ? q_off : k_off) + u * D;
-                ra[i] = *reinterpret_cast<const uint2 *>(p + qk.a);
-                rb[i] = *reinterpret_cast<const uint2 *>(p + qk.b);
-            }
-        }
-    };
-    fetch(0);
     const bool v_plain = v_pairs == 0 && !a.bias;
     if (slot >= 0 && v_plain) {   // values as projected: one run of bytes
         const uint4 *src = reinterpret_cast<const uint4 *>(row + a.v_off);
         uint4 *dst = reinterpret_cast<uint4 *>(static_cast<bf16 *>(a.v_cache) + slot * Gv * V);
-        for (int i = threadIdx.x; i < Gv * V / 8; i += nt) dst[i] = src[i];
+#pragma unroll 2
+        for (int i = part * 32 + lane; i < Gv * V / 8; i += parts * 32) dst[i] = src[i];
     }
-    const float amplitude = a.qk_amplitude != 0.f ? a.qk_amplitude : 1.f;
-    float *turns = sm, *v_turns = sm + 2 * qk_pairs;
-    const float pos = static_cast<float>(a.positions[t]);
-    for (int i = threadIdx.x; i < qk_pairs; i += nt)
-        turn(pos, a.qk_freq[i], a.qk_freq_lo ? a.qk_freq_lo[i] : 0.f, amplitude, turns[2 * i], turns[2 * i + 1]);
-    for (int i = threadIdx.x; i < v_pairs; i += nt) turn(pos, a.v_freq[i], 0.f, 1.f, v_turns[2 * i], v_turns[2 * i + 1]);
-    __syncthreads();
+    // this warp's share of the token's rounds: query heads, key heads, values
+    const int rq = (H + NG - 1) / NG, rk = a.slot_mapping ? (G + NG - 1) / NG : 0, rv = a.slot_mapping && !v_plain ? (Gv + NG - 1) / NG : 0;
+    const int each = (rq + rk + rv + parts - 1) / parts, from = part * each, to = from + each;
+    const float amplitude = a.qk_amplitude != 0.f ? a.qk_amplitude : 1.f, pos = static_cast<float>(a.positions[t]), mul = 1.f / static_cast<float>(D);
     HeadTurns tr;
-    tr.s0 = tr.s1 = make_float4(0.f, 1.f, 0.f, 1.f);
-    if (qk.turned) {
-        tr.s0 = *reinterpret_cast<const float4 *>(turns + 8 * l);
-        tr.s1 = *reinterpret_cast<const float4 *>(turns + 8 * l + 4);
-    }
-    bf16 *qd = static_cast<bf16 *>(a.q_out) + t * H * D, *kd = static_cast<bf16 *>(a.k_cache) + (slot * G - H) * D;
-    const float mul = 1.f / static_cast<float>(D);
-    for (int u0 = 0; u0 < units; u0 += kQkvHeads * step) {
-        if (u0 > 0) fetch(u0);
-#pragma unroll
-        for (int i = 0; i < kQkvHeads; ++i) {
-            const int u = u0 + first + i * step;
-            if (u >= units) break;
-            const bool is_q = u < H;
-            const float *w = is_q ? a.q_weight : a.k_weight;
-            head_finish<L, IL>(ra[i], rb[i], qk, a.bias ? a.bias + (is_q ? q_off : k_off) + u * D : nullptr, w || a.unit_norm ? mul : 0.f, a.eps,
-                               is_q && a.q_head_scale ? a.q_head_scale[u] : 1.f, w, tr, group);
-            if (qk.a >= 0) {
-                bf16 *dst = (is_q ? qd : kd) + u * D;
-                *reinterpret_cast<uint2 *>(dst + qk.a) = ra[i];
-                *reinterpret_cast<uint2 *>(dst + qk.b) = rb[i];
-            }
-        }
-    }
-    if (slot < 0 || v_plain) return;
+    if (from < rq + rk) tr = head_turns<L, IL>(pos, a.qk_freq, a.qk_freq_lo, amplitude, qk_pairs);
+    if (from < rq)
+        heads_finish<L, IL, WHOLE>(row + a.q_off, static_cast<bf16 *>(a.q_out) + static_cast<int64_t>(t) * H * D, from * NG, min(H, to * NG), D, qk, a.bias ? a.bias + a.q_off : nullptr,
+                                   a.q_weight || a.unit_norm ? mul : 0.f, a.eps, a.q_head_scale, a.q_weight, tr);
+    if (slot < 0) return;
+    if (from < rq + rk && to > rq)
+        heads_finish<L, IL, WHOLE>(row + a.k_off, static_cast<bf16 *>(a.k_cache) + slot * G * D, max(0, from - rq) * NG, min(G, (to - rq) * NG), D, qk, a.bias ? a.bias + a.k_off : nullptr,
+                                   a.k_weight || a.unit_norm ? mul : 0.f, a.eps, nullptr, a.k_weight, tr);
+    if (v_plain || to <= rq + rk) return;
     const HeadRuns vr = head_runs(l, V, v_pairs, IL);
-    if (vr.a < 0) return;
-    if (vr.turned) {
-        tr.s0 = *reinterpret_cast<const float4 *>(v_turns + 8 * l);
-        tr.s1 = *reinterpret_cast<const float4 *>(v_turns + 8 * l + 4);
-    }
-    for (int u = first; u < Gv; u += step) {
-        const int64_t col = a.v_off + u * V;
-        uint2 x = *reinterpret_cast<const uint2 *>(row + col + vr.a), y = *reinterpret_cast<const uint2 *>(row + col + vr.b);
-        head_finish<L, IL>(x, y, vr, a.bias ? a.bias + col : nullptr, 0.f, 0.f, 1.f, nullptr, tr, group);
-        bf16 *dst = static_cast<bf16 *>(a.v_cache) + (slot * Gv + u) * V;
-        *reinterpret_cast<uint2 *>(dst + vr.a) = x;
-        *reinterpret_cast<uint2 *>(dst + vr.b) = y;
-    }
+    tr = head_turns<L, IL>(pos, a.v_freq, nullptr, 1.f, v_pairs);
+    heads_finish<L, IL, false>(row + a.v_off, static_cast<bf16 *>(a.v_cache) + slot * Gv * V, max(0, from - rq - rk) * NG, min(Gv, (to - rq - rk) * NG), V, vr, a.bias ? a.bias + a.v_off : nullptr,
+                               0.f, 0.f, nullptr, nullptr, tr);
 }
 
 template <typename T>
@@ -704,17 +743,21 @@ bool hyb_qkv_headnorm_rope_cache(const atoma_qkv_rope_args &a, cudaStream_t stre
     const bool pieces = a.dtype == ATOMA_DTYPE_BF16 && !(g_hybrid_debug & 2) && a.dim % 8 == 0 && a.vdim % 8 == 0 && std::max(a.dim, a.vdim) <= 256 && a.ld % 8 == 0 &&
                         a.q_off % 8 == 0 && (!a.slot_mapping || (a.k_off % 8 == 0 && a.v_off % 8 == 0)) && al(a.proj) && al(a.q_out) &&
                         (!a.slot_mapping || (al(a.k_cache) && al(a.v_cache))) && al(a.q_weight) && al(a.k_weight) && al(a.bias) &&
-                        a.rot_pairs % 4 == 0 && a.v_pairs % 4 == 0;
+                        a.rot_pairs % 4 == 0 && a.v_pairs % 4 == 0 && a.T < (1ll << 24);
     if (pieces) {
-        const size_t turns = static_cast<size_t>(2 * (a.rot_pairs + a.v_pairs)) * 4;
-        const int64_t n = std::max(a.dim, a.vdim);
-        // no more lanes than the heads take (12000 tokens of 1 + 1 heads of 128: 46 us with 256 threads, 18.7 on the general kernel)
-        const int64_t lanes = (a.H + a.G) * (n <= 64 ? 8 : n <= 128 ? 16 : 32);
-        const dim3 grid(static_cast<unsigned>(a.T)), block(static_cast<unsigned>(std::min<int64_t>(256, (lanes + 31) / 32 * 32)));
-#define PICK(IL, NT) (n <= 64 ? qkv_headnorm_rope_cache_vec_kernel<8, IL, NT> : n <= 128 ? qkv_headnorm_rope_cache_vec_kernel<16, IL, NT> : qkv_headnorm_rope_cache_vec_kernel<32, IL, NT>)
-        auto kernel = block.x == 256 ? (a.interleaved ? PICK(true, 256) : PICK(false, 256)) : (a.interleaved ? PICK(true, 0) : PICK(false, 0));
+        const int64_t n = std::max(a.dim, a.vdim), groups = n <= 64 ? 4 : n <= 128 ? 2 : 1;
+        const int64_t heads = a.H + (a.slot_mapping ? a.G + (a.bias || (a.v_freq && a.v_pairs > 0) ? (a.v_heads > 0 ? a.v_heads : a.G) : 0) : 0), rounds = (heads + groups - 1) / groups;
+        // shares of a token: so many that the warps fill the SMs once, and no more than there are rounds (twice as many: 8192 tokens 47.3 us, 1000 17.2; once:
+        // 46.1 and 15.4)
+        const int64_t want = (kQkvResident * current_device_info().sm_count + a.T - 1) / a.T;
+        const int parts = static_cast<int>(std::max<int64_t>(1, std::min(rounds, want)));
+        const dim3 grid(static_cast<unsigned>((a.T * parts + kQkvWarps - 1) / kQkvWarps)), block(32 * kQkvWarps);
+        const bool whole = a.dim == 256 / groups && a.qk_freq && 2 * a.rot_pairs == a.dim;
+#define PICK_L(IL, WHOLE) (n <= 64 ? qkv_headnorm_rope_cache_vec_kernel<8, IL, WHOLE> : n <= 128 ? qkv_headnorm_rope_cache_vec_kernel<16, IL, WHOLE> : qkv_headnorm_rope_cache_vec_kernel<32, IL, WHOLE>)
+#define PICK(IL) (whole ? PICK_L(IL, true) : PICK_L(IL, false))
+        const cudaError_t e = launch_ex(a.interleaved ? PICK(true) : PICK(false), grid, block, 0, stream, a, parts);
 #undef PICK
-        const cudaError_t e = launch_ex(kernel, grid, block, turns, stream, a);
+#undef PICK_L
         return hybrid::launched(e, "qkv_headnorm_rope_cache_vec_kernel");
     }
 #define CALL(TT) launch_ex(qkv_headnorm_rope_cache_kernel<TT>, dim3(static_cast<unsigned>(a.T)), dim3(warps * 32), smem, stream, a)
