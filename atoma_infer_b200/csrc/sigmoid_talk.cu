@@ -14,14 +14,18 @@
 // segment is 512 keys from a multiple of 512 on whatever the step looks like, so a position's sums depend on its keys alone.  A CTA takes one
 // segment, or, in steps whose row blocks fill the SMs without, all of its rows' segments one after the other; the sums between take at most 256 MiB
 // (kStScratch), and longer steps go in runs of tokens.  Keys of the next tile are copied under the mix, values under the scores.
-// 2048 tokens, 32 heads of 64 on 8: 1218 us on the CUDA-core mix (hybrid_attention.cu), 506 here; 8000 tokens before 17 new ones 3308 and 250.  A prompt of one to
-// sixteen row blocks and few keys is slower than there (64 tokens: 31 and 38 us): all heads wait for each other in one CTA.
+// A tile of 2048 tokens, 32 heads of 64 on 8, takes 14000 cycles: scores and weights 6000 (four results of the special-function unit per weight are 4100 of them),
+// the mix 5000 (3100 of the tensor pipe), values 2000.  With 27000: every copy waited for its own block-table entry (5000), a branch per weight kept
+// their chains from overlapping, quotients and exponentials took denormal numbers into account, and registers spilled.
+// 2048 tokens, 32 heads of 64 on 8: 1218 us on the CUDA-core mix (hybrid_attention.cu), 511 with those, 286 here; 2000 tokens of 16 heads 328 and 169.  A prompt of
+// a few row blocks and few keys stays as fast as on CUDA cores (64 tokens: 31 us): all heads wait for each other in one CTA.
 #include "common.cuh"
 #include "hybrid_common.cuh"
 
 #include "atoma_hybrid.h"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace atoma {
 namespace {
@@ -31,11 +35,22 @@ using namespace hybrid;
 constexpr int kStRows = 16, kStKeys = 32, kStSegKeys = 512, kStPieces = 3;
 constexpr int64_t kStScratch = 256ll << 20;
 
-__device__ __forceinline__ float st_weight(float dot, float scale, float softcap, float inv_cap, float slope, float dist, float head_bias) {
-    float s = dot * scale;
-    if (softcap > 0.f) s = softcap * (1.f - __fdividef(2.f, __expf(2.f * s * inv_cap) + 1.f));
-    s = s - slope * dist + head_bias;
-    return __fdividef(1.f, 1.f + __expf(-s));
+// sigmoid(cap tanh(s / cap) - slope dist + bias), tanh(y) = 1 - 2 / (1 + e^2y).  The unit's estimates of 2^x and of the reciprocal are within 2 and 1 units of the last
+// place.  The logit keeps its own unit until it is whole: slopes in units of log 2 would carry their rounding times the distance (rms 1.4e-7 off where this is 4e-8).
+template <bool CAP>
+__device__ __forceinline__ float st_weight(float dot, float scale, float in, float cap, float slope, float dist, float head_bias) {
+    auto ex2 = [](float x) {
+        float y;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    };
+    auto rcp = [](float x) {
+        float y;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    };
+    const float s = CAP ? fmaf(-2.f, rcp(1.f + ex2(dot * in)), 1.f) * cap : dot * scale;
+    return rcp(1.f + ex2(-1.4426950408889634f * (fmaf(-slope, dist, s) + head_bias)));
 }
 
 template <int HT>   // heads = 16 HT
@@ -81,15 +96,23 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
     __nv_bfloat16 *Ks = reinterpret_cast<__nv_bfloat16 *>(sm + L::kv_off), *Vs = Ks + G * kStKeys * (D + 8);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t4 = lane & 3, rq = lane >> 2;
     const __nv_bfloat16 *kc = static_cast<const __nv_bfloat16 *>(a.k_cache), *vc = static_cast<const __nv_bfloat16 *>(a.v_cache);
-    // rows past the sequence's end are zero-filled; a thread's piece of a row is the same for all its keys when the CTA takes whole rows at a time
+    // Cache rows of a tile's keys (-1: behind the sequence's end, zero-filled), looked up one tile ahead by one warp: a copy that waits for its own table
+    // entry costs a round trip to memory.
+    __shared__ int32_t slot_s[2][kStKeys];
     const int bs_shift = (bs & (bs - 1)) == 0 ? __ffs(bs) - 1 : -1;
-    auto stage = [&](const __nv_bfloat16 *cache, __nv_bfloat16 *dst, int n, int j0) {
+    auto look_up = [&](int j) {
+        const int pg = bs_shift >= 0 ? j >> bs_shift : j / bs;
+        return j < total ? bt[pg] * bs + (j - pg * bs) : -1;
+    };
+    static_assert(kStKeys == 32, "a lane per key");
+    if (warp == 0) slot_s[0][lane] = look_up(j_begin + lane);
+    __syncthreads();
+    // a thread's piece of a row is the same for all its keys when the CTA takes whole rows at a time
+    auto stage = [&](const __nv_bfloat16 *cache, __nv_bfloat16 *dst, int n, const int32_t *slots) {
         const int pieces = G * n / 8;
         auto put = [&](int jj, int e, int g) {
-            const int j = j0 + jj, pg = bs_shift >= 0 ? j >> bs_shift : j / bs;
-            const bool ok = j < total;
-            const int64_t slot = ok ? static_cast<int64_t>(bt[pg]) * bs + (j - pg * bs) : 0;
-            cp_async_16(smem_u32(dst + (g * kStKeys + jj) * (n + 8) + e * 8 - g * n), cache + slot * G * n + e * 8, ok ? 16 : 0);
+            const int slot = slots[jj];
+            cp_async_16(smem_u32(dst + (g * kStKeys + jj) * (n + 8) + e * 8 - g * n), cache + static_cast<int64_t>(max(slot, 0)) * G * n + e * 8, slot >= 0 ? 16 : 0);
         };
         if (NT % pieces == 0) {
             const int e = tid % pieces, g = e * 8 / n;
@@ -102,7 +125,7 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
         }
         cp_async_commit();
     };
-    stage(kc, Ks, D, j_begin);
+    stage(kc, Ks, D, slot_s[0]);
     // ---- the talk matrix in three pieces ----
     for (int i = tid; i < H * H; i += NT) {
         float piece[kStPieces];
@@ -113,7 +136,7 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
     }
     // ---- this warp's heads: query fragments, constants ----
     const int h0 = 2 * warp, rep = H / G;
-    uint32_t qf[2][4][4];
+    uint32_t qf[32];   // [head][16 of its entries][fragment]
     float slope[2], hb[2];
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
@@ -125,15 +148,33 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int row = rq + (e & 1) * 8, col = kk * 16 + 2 * t4 + (e >> 1) * 8;
-                qf[x][kk][e] = kk * 16 < D && row < rows ? *reinterpret_cast<const uint32_t *>(q + static_cast<int64_t>(row) * H * D + col) : 0u;
+                qf[x * 16 + kk * 4 + e] = kk * 16 < D && row < rows ? *reinterpret_cast<const uint32_t *>(q + static_cast<int64_t>(row) * H * D + col) : 0u;
             }
     }
+    // Of 32 heads, a thread's 64 sums, 32 queries and the mix do not fit its 128 registers (spilled, 81 KB a tile passed through an L1 of 28 KB: 386 us, 308 without):
+    // the queries and, between tiles, the sums lie in tensor memory, from where a phase takes them in one or two loads.
+    __shared__ uint32_t tmem_base_s;
+    uint32_t tmem_q = 0, tmem_o = 0;
+    if constexpr (HT == 2) {
+        if (warp == 0) tmem_alloc(&tmem_base_s, 512);
+        tc_fence_before_sync();
+        __syncthreads();
+        tc_fence_after_sync();
+        tmem_q = tmem_base_s + (static_cast<uint32_t>((warp & 3) * 32) << 16) + (warp >> 2) * 32;
+        tmem_o = tmem_base_s + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 128 + (warp >> 2) * 64;
+        tmem_st_32x32b_x32(tmem_q, qf);
+        tmem_st_wait();
+    }
     float o[2][8][4];
+    auto clear = [&] {
 #pragma unroll
-    for (int x = 0; x < 2; ++x)
+        for (int x = 0; x < 2; ++x)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[x][i][0] = o[x][i][1] = o[x][i][2] = o[x][i][3] = 0.f;
-    const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
+            for (int i = 0; i < 8; ++i) o[x][i][0] = o[x][i][1] = o[x][i][2] = o[x][i][3] = 0.f;
+    };
+    clear();
+    bool fresh = true;   // nothing has been summed since the start, or since a segment went out
+    const float in = a.softcap > 0.f ? a.scale * 2.8853900817779268f / a.softcap : 0.f;   // e^(2 s / cap) = 2^(in dot)
     // the sums of a segment, out of the accumulators: into its place, onto the running sum, or, where no other segment follows or precedes, out
     bool more = false;   // a running sum waits in this token's place
     auto put = [&](bool last) {
@@ -159,41 +200,63 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
     for (int j0 = j_begin; j0 < j_end; j0 += kStKeys) {
         cp_async_wait_all();
         __syncthreads();   // the keys are there; everyone is done with the last tile's values and mixed weights
-        stage(vc, Vs, DV, j0);
+        const int cur = (j0 - j_begin) / kStKeys & 1;
+        stage(vc, Vs, DV, slot_s[cur]);
+        int next_slot = 0;
+        if (warp == 0) next_slot = look_up(j0 + kStKeys + lane);
         // ---- 1. scores and weights of two heads; both heads' weights of a pair go out together ----
-        float w0[4][4];
+        if constexpr (HT == 2) {
+            tmem_ld_32x32b_x32(tmem_q, qf);
+            tmem_ld_wait();
+        }
+        // 16 keys at a time: the accumulators of the values and the queries leave few registers
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-            float s[4][4];
+        for (int np = 0; np < 2; ++np) {
+            float w0[2][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
-            const __nv_bfloat16 *kb = Ks + ((h0 + x) / rep * kStKeys + (lane >> 4) * 8 + (lane & 7)) * (D + 8) + ((lane >> 3) & 1) * 8;
+            for (int x = 0; x < 2; ++x) {
+                float s[2][4];
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-                if (kk * 16 < D) {
+                for (int i = 0; i < 2; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+                const __nv_bfloat16 *kb = Ks + ((h0 + x) / rep * kStKeys + (lane >> 4) * 8 + (lane & 7)) * (D + 8) + ((lane >> 3) & 1) * 8;
 #pragma unroll
-                    for (int np = 0; np < 2; ++np) {
+                for (int kk = 0; kk < 4; ++kk)
+                    if (kk * 16 < D) {
                         uint32_t r[4];
                         ldmatrix_x4(r, smem_u32(kb + np * 16 * (D + 8) + kk * 16));
-                        Mma16816<__nv_bfloat16>::run(s[2 * np], qf[x][kk], r[0], r[1]);
-                        Mma16816<__nv_bfloat16>::run(s[2 * np + 1], qf[x][kk], r[2], r[3]);
+                        const uint32_t(&qk)[4] = *reinterpret_cast<const uint32_t(*)[4]>(qf + x * 16 + kk * 4);
+                        Mma16816<__nv_bfloat16>::run(s[0], qk, r[0], r[1]);
+                        Mma16816<__nv_bfloat16>::run(s[1], qk, r[2], r[3]);
                     }
-                }
+                // weights of hidden pairs are formed too and dropped: without a branch per weight their chains of exponentials and quotients overlap
+                const float base = static_cast<float>(p0 + rq - j0 - 2 * t4);
+                auto weigh = [&](auto with_cap) {
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
+                    for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int row = rq + (e >> 1) * 8, key = nt * 8 + 2 * t4 + (e & 1), dist = p0 + row - (j0 + key);
-                    const float w = row < rows && dist >= 0 ? st_weight(s[nt][e], a.scale, a.softcap, inv_cap, slope[x], static_cast<float>(dist), hb[x]) : 0.f;
-                    if (x == 0) w0[nt][e] = w;
-                    else *reinterpret_cast<float2 *>(weights + row * L::kRow + key * L::kPair + h0 * 4) = make_float2(w0[nt][e], w);
-                }
+                        for (int e = 0; e < 4; ++e)
+                            s[nt][e] = st_weight<decltype(with_cap)::value>(s[nt][e], a.scale, in, a.softcap, slope[x],
+                                                                            base - static_cast<float>((2 * np + nt) * 8 + (e & 1) - (e >> 1) * 8), hb[x]);
+                };
+                if (a.softcap > 0.f) weigh(std::true_type{});
+                else weigh(std::false_type{});
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int row = rq + (e >> 1) * 8, key = (2 * np + nt) * 8 + 2 * t4 + (e & 1);
+                        const float w = row < rows && p0 + row >= j0 + key ? s[nt][e] : 0.f;
+                        if (x == 0) w0[nt][e] = w;
+                        else *reinterpret_cast<float2 *>(weights + row * L::kRow + key * L::kPair + h0 * 4) = make_float2(w0[nt][e], w);
+                    }
+            }
         }
+        if (warp == 0) slot_s[cur ^ 1][lane] = next_slot;
         __syncthreads();   // all heads' weights are there, and the keys are done with
-        if (j0 + kStKeys < j_end) stage(kc, Ks, D, j0 + kStKeys);
+        if (j0 + kStKeys < j_end) stage(kc, Ks, D, slot_s[cur ^ 1]);
         else cp_async_commit();   // an empty group: the values' is always the one before the last
-        // ---- 2. the heads talk: a warp takes whole query rows, eight (32 heads: registers) or sixteen keys at a time ----
-        constexpr int kN = HT == 2 ? 1 : 2;
+        // ---- 2. the heads talk: a warp takes whole query rows, eight (32 heads; thirty-two: 286 us for 286) or thirty-two (16 heads; eight: 179 us for 169) keys at a time ----
+        constexpr int kN = HT == 2 ? 1 : 4;
         for (int row = warp; row < kStRows; row += NW)
 #pragma unroll 1
             for (int n2 = 0; n2 < kStKeys / 8; n2 += kN) {
@@ -205,29 +268,43 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
                             const float2 w = *reinterpret_cast<const float2 *>(weights + row * L::kRow + ((n2 + i) * 8 + rq) * L::kPair + (kk * 16 + 8 * e + 2 * t4) * 4);
-                            float px[kStPieces], py[kStPieces];
-                            st_split(w.x, px);
-                            st_split(w.y, py);
+                            float x = w.x, y = w.y;   // two values' pieces at a time
 #pragma unroll
-                            for (int k = 0; k < kStPieces; ++k) wb[i][k][kk][e] = pack2<__nv_bfloat16>(px[k], py[k]);
+                            for (int k = 0; k < kStPieces; ++k) {
+                                const uint32_t piece = pack2<__nv_bfloat16>(x, y);
+                                wb[i][k][kk][e] = piece;
+                                x -= __uint_as_float(piece << 16);
+                                y -= __uint_as_float(piece & 0xffff0000u);
+                            }
                         }
 #pragma unroll
                 for (int mt = 0; mt < HT; ++mt) {
-                    uint32_t ta[kStPieces][HT][4];
+                    // products of one order in a sum of their own, a shorter chain; the smallest are added first
+                    float co[kN][kStPieces][4];
 #pragma unroll
-                    for (int k = 0; k < kStPieces; ++k)
+                    for (int i = 0; i < kN; ++i)
+#pragma unroll
+                        for (int order = 0; order < kStPieces; ++order)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) co[i][order][e] = 0.f;
+#pragma unroll
+                    for (int k = 0; k < kStPieces; ++k) {
+                        uint32_t ta[HT][4];
 #pragma unroll
                         for (int kk = 0; kk < HT; ++kk)
-                            ldmatrix_x4(ta[k][kk], smem_u32(talk + k * L::kTalk + (mt * 16 + (lane & 15)) * L::kTalkRow + (kk * 16 + (lane >> 4) * 8) * 2));
+                            ldmatrix_x4(ta[kk], smem_u32(talk + k * L::kTalk + (mt * 16 + (lane & 15)) * L::kTalkRow + (kk * 16 + (lane >> 4) * 8) * 2));
+#pragma unroll
+                        for (int i = 0; i < kN; ++i)
+#pragma unroll
+                            for (int kk = 0; kk < HT; ++kk)
+#pragma unroll
+                                for (int order = k; order < kStPieces; ++order) Mma16816<__nv_bfloat16>::run(co[i][order], ta[kk], wb[i][order - k][kk][0], wb[i][order - k][kk][1]);
+                    }
 #pragma unroll
                     for (int i = 0; i < kN; ++i) {
-                        float c[4] = {0.f, 0.f, 0.f, 0.f};
+                        float c[4];
 #pragma unroll
-                        for (int order = kStPieces - 1; order >= 0; --order)   // the smallest products first
-#pragma unroll
-                            for (int k = 0; k <= order; ++k)
-#pragma unroll
-                                for (int kk = 0; kk < HT; ++kk) Mma16816<__nv_bfloat16>::run(c, ta[k][kk], wb[i][order - k][kk][0], wb[i][order - k][kk][1]);
+                        for (int e = 0; e < 4; ++e) c[e] = co[i][0][e] + (co[i][1][e] + co[i][2][e]);
                         unsigned char *m = mix + (mt * 16 + rq) * L::kMixHead + row * L::kMixRow + ((n2 + i) * 8 + 2 * t4) * 2;
                         *reinterpret_cast<uint32_t *>(m) = pack2<__nv_bfloat16>(c[0], c[1]);
                         *reinterpret_cast<uint32_t *>(m + 8 * L::kMixHead) = pack2<__nv_bfloat16>(c[2], c[3]);
@@ -237,6 +314,18 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
         asm volatile("cp.async.wait_group 1;" ::: "memory");   // the values
         __syncthreads();
         // ---- 3. values ----
+        if constexpr (HT == 2) {
+            if (fresh) {
+                clear();
+            } else {
+                uint32_t *r = reinterpret_cast<uint32_t *>(&o[0][0][0]);
+                tmem_st_wait();
+                tmem_ld_32x32b_x32(tmem_o, r);
+                tmem_ld_32x32b_x32(tmem_o + 32, r + 32);
+                tmem_ld_wait();
+            }
+        }
+        fresh = false;
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             const __nv_bfloat16 *vb = Vs + ((h0 + x) / rep * kStKeys + ((lane >> 3) & 1) * 8 + (lane & 7)) * (DV + 8) + (lane >> 4) * 8;
@@ -257,14 +346,23 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
         if (slots == 1 && partial && j0 + kStKeys < j_end && (j0 + kStKeys) % kStSegKeys == 0) {   // a segment ends here
             put(false);
             more = true;
-#pragma unroll
-            for (int x = 0; x < 2; ++x)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o[x][i][0] = o[x][i][1] = o[x][i][2] = o[x][i][3] = 0.f;
+            fresh = true;
+            clear();
+        } else if constexpr (HT == 2) {
+            const uint32_t *r = reinterpret_cast<const uint32_t *>(&o[0][0][0]);
+            tmem_st_32x32b_x32(tmem_o, r);
+            tmem_st_32x32b_x32(tmem_o + 32, r + 32);
         }
     }
     cp_async_wait_all();
     put(true);
+    if constexpr (HT == 2) {
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncthreads();
+        tc_fence_after_sync();
+        if (warp == 0) tmem_dealloc(tmem_base_s, 512);
+    }
 }
 
 // A token's segments, in order; tokens of one segment are out already.
