@@ -76,7 +76,8 @@ struct DecodeArgs {
     int early;       // PDL + the caller's per-call promise: stream older pages before the grid dependency resolves
     int late_trigger;  // a cache-maintenance op is in flight on the stream: wait BEFORE releasing dependents
     int merged;      // map_k describes K AND V (one allocation, contiguous heads): one op moves both
-    int *counters;   // [b * hg], zero between launches
+    int *counters;   // [b * hg] or [b * h_k], zero between launches
+    int *group_counters;   // [cta][2][8 warps]: of the groups of partials that start there, zero between launches
     float *ws_ml;    // [cta][2][8 warps][16 rows][2]
     float *ws_o;     // [cta][2][8 warps][16 rows][D]
     unsigned long long *trace;  // diagnostics (atoma_debug_decode_trace): [cta][4] or null
@@ -113,10 +114,10 @@ __device__ __forceinline__ int cta_of_unit(long long units, long long u, int num
     return static_cast<int>(((u + 1) * num_ctas + units - 1) / units - 1);
 }
 
-// Reduction of every partial of one (sequence, kv head) by ONE warp (the last to arrive for that
+// Reduction of a few partials of one (sequence, kv head) by ONE warp (the last to arrive for that
 // head).  Partials are merged in CTA-index order whoever arrives last, four outputs per lane and
 // four partials in flight at a time (16-byte loads), so the result is bit-reproducible and the cost
-// is a few L2 round trips.
+// is one or two L2 round trips; more partials go through merge_parts.
 template <typename T, int D>
 __device__ __forceinline__ void combine_head(const DecodeArgs &a, long long units, int ncta, int fc, int lc,
                                              long long ub, long long ue, int b, int kvh, int hh, int G,
@@ -204,7 +205,137 @@ __device__ __forceinline__ void combine_head(const DecodeArgs &a, long long unit
     }
 }
 
+// Merge of up to kMergeParts partials of one kv head by ONE warp: lane j < n holds partial j's workspace index.  The outputs of two chunks of 128 (all of them for
+// 4 query heads of 64) are asked for first; under their way the maxima and sums of all rows, a lane per partial and two
+// rows at a time, become weights in shared memory.  A few round trips, however many partials.  put(row, d, acc, m, l) takes four outputs of a row, not yet
+// divided.
+constexpr int kMergeParts = 16, kMergeRows = 8;   // partials; rows whose weights are at hand
+constexpr int kFewUnits = 8, kFewParts = 8, kManyParts = 24;
+struct MergeRow {
+    float w[kMergeParts];
+    float m, l, pad[2];
+};
+template <int D, typename Put>
+__device__ __forceinline__ void merge_parts(const DecodeArgs &a, MergeRow *rows, int n, int mybase, int G, int lane, Put put) {
+    constexpr int C4 = D / 4, NC = 2, NP = kMergeParts;
+    for (int c0 = 0; c0 * 32 < G * C4; c0 += NC) {
+        float4 ov[NC][NP];
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            const float *o = a.ws_o + static_cast<int64_t>(__shfl_sync(0xffffffffu, mybase, min(j, n - 1))) * (kPartRows * D) + (c0 * 32 + lane) * 4;
+#pragma unroll
+            for (int k = 0; k < NC; ++k) {
+                ov[k][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j < n) ov[k][j] = __ldcg(reinterpret_cast<const float4 *>(o + k * 128));   // rows from G on: of the workspace, not used
+            }
+        }
+        const int r0 = c0 * 32 / C4;
+        if (r0 % kMergeRows == 0) {
+            const int j = lane & 15;
+            const float *ml = a.ws_ml + static_cast<int64_t>(__shfl_sync(0xffffffffu, mybase, min(j, n - 1))) * (kPartRows * 2);
+            float2 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int row = r0 + 2 * i + (lane >> 4);
+                v[i] = make_float2(-INFINITY, 0.f);
+                if (row < G && j < n) v[i] = __ldcg(reinterpret_cast<const float2 *>(ml + row * 2));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int row = r0 + 2 * i + (lane >> 4);
+                float m = v[i].x;
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+                const float w = m == -INFINITY ? 0.f : fast_exp2(v[i].x - m);   // empty partial: exp2(-inf) = 0
+                float l = w * v[i].y;
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+                if (row < G) {
+                    rows[row % kMergeRows].w[j] = w;
+                    if (j == 0) rows[row % kMergeRows].m = m, rows[row % kMergeRows].l = l;
+                }
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+            const int idx = (c0 + k) * 32 + lane;
+            const MergeRow &row = rows[min(idx / C4, G - 1) % kMergeRows];
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < NP; ++j) {
+                if (j < n) {
+                    acc.x = fmaf(row.w[j], ov[k][j].x, acc.x);
+                    acc.y = fmaf(row.w[j], ov[k][j].y, acc.y);
+                    acc.z = fmaf(row.w[j], ov[k][j].z, acc.z);
+                    acc.w = fmaf(row.w[j], ov[k][j].w, acc.w);
+                }
+            }
+            if (idx < G * C4) put(idx / C4, idx % C4 * 4, acc, row.m, row.l);
+        }
+        __syncwarp();   // the rows may be written again
+    }
+}
+
+// Contributors of one (sequence, kv head) are the CTAs fc .. lc, a partial each; merged in CTA-index order whoever arrives last, so the result is
+// bit-reproducible.  A few: combine_head (32 sequences, five partials each, 0.8 us less than merge_parts).  Up to kMergeParts: by the warp that arrives last.  More: groups of equal size first, each by its last arriver into its first contributor's
+// place, then the groups (one user at 4000 keys, 148 partials: 53 us of 60 were one warp's chain of round trips, four partials each).
 template <typename T, int D>
+__device__ __forceinline__ void arrive_and_merge(const DecodeArgs &a, long long units, int ncta, int fc, int lc, long long ub, long long ue, int b, int kvh, int hh,
+                                                 int G, int lane, int cta, MergeRow *rows) {
+    const MhaParams &p = a.p;
+    const int nparts = lc - fc + 1;
+    auto place = [&](int c) {   // workspace index of contributor c
+        const long long cs = cta_start(units, c, ncta);
+        return (c * 2 + ((cs >= ub && cs < ue) ? 0 : 1)) * kConsumerWarps + hh;
+    };
+    auto last_of = [&](int *ctr, int n) {
+        __threadfence();
+        __syncwarp();
+        int old = 0;
+        if (lane == 0) old = atomicAdd(ctr, 1);
+        if (__shfl_sync(0xffffffffu, old, 0) != n - 1) return false;
+        __threadfence();
+        return true;
+    };
+    const bool grouped = nparts > kMergeParts;
+    const int step = grouped ? max(8, (nparts + kMergeParts - 1) / kMergeParts) : 1;
+    const int first = grouped ? fc + (cta - fc) / step * step : fc, at = grouped ? place(first) : 0;
+    float *po = a.ws_o + static_cast<int64_t>(at) * (kPartRows * D), *pml = a.ws_ml + static_cast<int64_t>(at) * (kPartRows * 2);
+    for (int level = grouped ? 0 : 1; level < 2; ++level) {
+        const int n = level == 0 ? min(step, lc + 1 - first) : (nparts + step - 1) / step;
+        int *ctr = level == 0 ? a.group_counters + at : &a.counters[b * p.h_k + kvh];
+        if (!last_of(ctr, n)) return;
+        if (a.trace && lane == 0) a.trace[blockIdx.x * 8 + 6] = global_timer_ns();
+        if (nparts <= kFewParts) {
+            combine_head<T, D>(a, units, ncta, fc, lc, ub, ue, b, kvh, hh, G, lane);
+            if (lane == 0) *ctr = 0;
+            break;
+        }
+        const int base = place(lane < n ? (level == 0 ? first + lane : fc + lane * step) : fc);
+        auto put = [&](int row, int d, float4 acc, float m, float l) {
+            if (level == 0) {
+                __stcg(reinterpret_cast<float4 *>(po + row * D + d), acc);
+                if (d == 0) __stcg(reinterpret_cast<float2 *>(pml + row * 2), make_float2(m, l));
+                return;
+            }
+            const bool empty = (l == 0.f || l != l);
+            const float inv = empty ? 1.f : 1.f / l;
+            const int head = kvh * G + row;
+            uint2 packed;
+            packed.x = pack2<T>(acc.x * inv, acc.y * inv);
+            packed.y = pack2<T>(acc.z * inv, acc.w * inv);
+            *reinterpret_cast<uint2 *>(static_cast<T *>(p.o) + b * p.o_bs + static_cast<int64_t>(head) * p.o_hs + d) = packed;
+            if (d == 0 && p.lse) p.lse[static_cast<int64_t>(b) * p.h + head] = empty ? INFINITY : m * 0.6931471805599453f + __logf(l);
+        };
+        merge_parts<D>(a, rows, n, base, G, lane, put);
+        if (lane == 0) *ctr = 0;   // self-cleaning for the next launch (a store in front of the fence above would be waited for)
+    }
+    if (a.trace && lane == 0) a.trace[blockIdx.x * 8 + 7] = global_timer_ns();
+}
+
+// MANY: a sequence may have many partials (few sequences of many keys).  A kernel of its own: a full batch of 32 lost 0.5 % of a step to the merge's code.
+template <typename T, int D, bool MANY>
 __global__ void __launch_bounds__(kDecodeThreads, 1)
 decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const DecodeArgs a) {
@@ -215,7 +346,9 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
     unsigned char *tiles = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
     __shared__ __align__(8) uint64_t full_k[C::kStages], full_v[C::kStages], empty[C::kStages];
     __shared__ int cum[kMaxBatch + 2];  // cum[b] = first unit of sequence b
+    __shared__ __align__(16) MergeRow merge_s[MANY ? kConsumerWarps : 1][MANY ? kMergeRows : 1];
     __shared__ int combine_flag;
+    [[maybe_unused]] __shared__ int longest_s;   // longest_s: units of the longest sequence and head group
     __shared__ int part_base[kMaxCtas];  // combine: workspace index of each contributing CTA's partial
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -261,10 +394,11 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
     if (tid == 0) cum[0] = 0;
     __syncthreads();
     if (warp == 0) {
-        int carry = 0;
+        int carry = 0, longest = 0;
         for (int base = 0; base < B; base += 32) {
             const int i = base + lane;
             int v = i < B ? cum[i + 1] : 0;
+            if (MANY) longest = max(longest, v);
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int n = __shfl_up_sync(0xffffffffu, v, o);
@@ -272,6 +406,11 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
             }
             if (i < B) cum[i + 1] = v + carry;
             carry += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if constexpr (MANY) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+            if (lane == 0) longest_s = longest / a.hg;
         }
     }
     __syncthreads();
@@ -297,7 +436,13 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
     // The grid was sized from the host-side upper bound of the unit count; only the first
     // min(grid, units) CTAs take part in the partition, so that every participant owns >= 1 unit
     // (the arrival-count logic below relies on it).
-    const int ncta = static_cast<int>(min(static_cast<long long>(gridDim.x), units));
+    int ncta = static_cast<int>(min(static_cast<long long>(gridDim.x), units));
+    // Few keys: a sequence on no more CTAs than one merge takes, as long as that leaves a CTA no more than kFewUnits units (one user at 1000 keys of
+    // heads of 128: 15 CTAs of four or five units 21.2 us, 63 of one and a merge in two levels 25.3; twelve units instead of eight are as fast).
+    if (MANY && units <= kFewUnits * ncta) {
+        const int few = static_cast<int>(units) * (kMergeParts - 1) / max(longest_s, 1);
+        if (few < ncta && few * kFewUnits >= units) ncta = max(1, few);
+    }
     if (cta >= ncta) return;
     const long long u_begin = cta_start(units, cta, ncta), u_end = cta_start(units, cta + 1, ncta);
 
@@ -647,6 +792,12 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
                 u += n;
                 continue;
             }
+            if constexpr (MANY) {
+                if (a.trace && tid == 0) a.trace[blockIdx.x * 8 + 4] = global_timer_ns();
+                arrive_and_merge<T, D>(a, units, ncta, fc, lc, ub, ue, b, kvh, hh, G, lane, cta, merge_s[warp]);
+                u += n;
+                continue;
+            }
             __threadfence();
             __syncwarp();
             if (a.trace && tid == 0) a.trace[blockIdx.x * 8 + 4] = global_timer_ns();
@@ -826,27 +977,37 @@ inline bool box_lines_ok(int hkt, int d) { return hkt * (d / 64) <= 256; }
 void *g_decode_trace = nullptr;
 int g_decode_no_merge = 0;  // diagnostics (atoma_debug_decode_merge): 1 = always two tensor maps
 
-template <typename T, int D>
-bool launch_decode(const CUtensorMap &mk, const CUtensorMap &mv, const DecodeArgs &a,
+template <typename T, int D, bool MANY>
+bool launch_decode_as(const CUtensorMap &mk, const CUtensorMap &mv, const DecodeArgs &a,
                    cudaStream_t stream) {
     constexpr size_t smem = Cfg<D>::kStages * Cfg<D>::kStageBytes + 1024 + Cfg<D>::kTreeBytes;
     static thread_local int attr_dev = -1;
     const DeviceInfo &di = current_device_info();
     if (attr_dev != di.ordinal) {
-        cudaFuncSetAttribute(decode_paged_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(decode_paged_kernel<T, D, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(smem));
         // the same (maximum) carve-out as every other kernel of the decode step: see gemm_skinny.cu
-        cudaFuncSetAttribute(decode_paged_kernel<T, D>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        cudaFuncSetAttribute(decode_paged_kernel<T, D, MANY>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
         attr_dev = di.ordinal;
     }
-    cudaError_t e = launch_ex(decode_paged_kernel<T, D>, dim3(a.num_ctas), dim3(kDecodeThreads), smem, stream, mk, mv, a);
+    cudaError_t e = launch_ex(decode_paged_kernel<T, D, MANY>, dim3(a.num_ctas), dim3(kDecodeThreads), smem, stream, mk, mv, a);
     note_launch();
     if (e != cudaSuccess) {
         set_status(static_cast<int>(e), "decode_paged_kernel: %s", cudaGetErrorString(e));
         return false;
     }
     return check_launch("decode_paged_kernel");
+}
+
+template <typename T, int D>
+bool launch_decode(const CUtensorMap &mk, const CUtensorMap &mv, const DecodeArgs &a, cudaStream_t stream) {
+    // Many partials per sequence: by the CTAs there are for it, and by its stages of a.tok keys (the longest it can have).  Steps of a model with 2048-wide layers,
+    // one partial at a time / in groups, us: one user at 4000 keys 335 / 272, 777 keys 280 / 267, 100 keys (7 partials) 120.7 / 123.0; eight sequences of
+    // 500 keys (18 partials) 187.6 / 190.6.
+    const int64_t stages = (a.p.seqlen_k + a.tok - 1) / a.tok, share = current_device_info().sm_count / std::max<int64_t>(1, static_cast<int64_t>(a.p.b) * a.hg);
+    const bool many = std::min(stages, share) >= kManyParts;
+    return many ? launch_decode_as<T, D, true>(mk, mv, a, stream) : launch_decode_as<T, D, false>(mk, mv, a, stream);
 }
 
 }  // namespace
@@ -898,12 +1059,13 @@ int try_launch_decode_paged(const MhaParams &p, bool is_bf16, int64_t max_units_
     (void)max_units_hint;
     a.num_ctas = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::min(di.sm_count, kMaxCtas), units_ub)));
 
-    const size_t counters_bytes = kMaxCounters * sizeof(int);
+    const size_t counters_bytes = (kMaxCounters + kMaxCtas * 2 * kConsumerWarps) * sizeof(int);
     const size_t ml_bytes = static_cast<size_t>(di.sm_count) * 2 * kConsumerWarps * kPartRows * 2 * sizeof(float);
     const size_t o_bytes = static_cast<size_t>(di.sm_count) * 2 * kConsumerWarps * kPartRows * 128 * sizeof(float);
     char *ws = static_cast<char *>(get_workspace(stream, counters_bytes + ml_bytes + o_bytes, kWorkspaceDecode));
     if (!ws) return -1;
     a.counters = reinterpret_cast<int *>(ws);
+    a.group_counters = a.counters + kMaxCounters;
     a.ws_ml = reinterpret_cast<float *>(ws + counters_bytes);
     a.ws_o = reinterpret_cast<float *>(ws + counters_bytes + ml_bytes);
     a.trace = static_cast<unsigned long long *>(g_decode_trace);
