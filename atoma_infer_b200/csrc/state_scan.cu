@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
     }
 }
 
-// a bound of the longest portion: T tokens over B sequences, each has one at least
+// the longest portion where every one of the B sequences has a token (one without makes another longer: nothing but speed may depend on this)
 int64_t longest_portion(const atoma_state_scan_args &a) { return std::max<int64_t>(1, a.T - (a.B - 1)); }
 
 template <typename T, int KIND, int R, int PW, int NW, int NB>
@@ -484,7 +484,7 @@ cudaError_t launch_scan(const atoma_state_scan_args &a, cudaStream_t stream) {
     // staged tokens per buffer: at most 32, no more than the longest portion can have, and NB CTAs' buffers fit one SM
     const int64_t fit = 200 * 1024 / NB / (kScanBuffers * L::kBytes);
     const int chunk = static_cast<int>(std::max<int64_t>(4, std::min<int64_t>({32, (longest_portion(a) + 3) / 4 * 4, fit / 4 * 4})));
-    const int buffers = longest_portion(a) <= chunk ? 1 : kScanBuffers;   // portions of one chunk fill the first only
+    const int buffers = a.T <= chunk ? 1 : kScanBuffers;   // a step of one chunk fills the first only (whatever share of it is whose: a sequence may have no token)
     const size_t smem = static_cast<size_t>(buffers) * chunk * L::kBytes;
     if (smem > 48 * 1024) cudaFuncSetAttribute(state_scan_kernel<T, KIND, R, PW, NW, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
     // copies in pieces of 16 bytes where every row and size allows it, else of 4, else value by value

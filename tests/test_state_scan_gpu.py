@@ -59,3 +59,22 @@ def test_splits_and_copies_give_the_same_bits(rule, D, V, dtype):
             padded.append(m[:, shift:shift + t.shape[1]])
         moved = run(padded, [0, n])
         assert torch.equal(moved[0], out) and torch.equal(moved[1], state), shift
+
+
+@pytest.mark.parametrize("n,empty", [(10, 2), (5, 3), (33, 30)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_sequences_without_a_token(n, empty, D):
+    """A portion that is longer than the step's tokens shared out, one to every sequence, would allow."""
+    from atoma_infer_b200 import hybrid_ops as ops
+
+    H, V = 4, 64
+    g = torch.Generator().manual_seed(n)
+    q, k, v, z = (torch.randn(n, c, generator=g).to(torch.bfloat16).to(DEV) for c in (H * D, H * D, H * V, H * D))
+    zb = torch.randn(H * D, generator=g).to(DEV)
+    outs = []
+    for starts in ([0, n], [0] + [n] * (empty + 1), [0] * (empty + 1) + [n]):
+        S = len(starts) - 1
+        state = torch.zeros((S, H * D * V), device=DEV)
+        out = ops.gla_scan(q, k, v, z, zb, 6.0, D ** -0.5, state, i32(list(range(S))), i32(starts), i32([0] * S), H, D, V)
+        outs.append((out, state[starts.index(n) - 1]))
+    assert all(torch.equal(o, outs[0][0]) and torch.equal(s, outs[0][1]) for o, s in outs[1:])
