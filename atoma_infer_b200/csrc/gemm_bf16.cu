@@ -110,8 +110,8 @@ gemm_tn_stream_kernel(const __grid_constant__ CUtensorMap map_w,
     const int KB = a.kb_per_tile;
 
     // Producer and MMA warps run converged on warp-uniform values with only the asynchronous instructions
-    // under elect.sync (see gemm_skinny.cu: inside `if (lane == 0)` every UTMALDG / UTCHMMA is wrapped in
-    // an R2UR + ELECT waterfall loop, ~70 cycles per MMA — more than a 128x128x16 MMA occupies the pipe).
+    // under elect.sync (under `if (lane == 0)` the loop took ~70 cycles per product — more than a 128x128x16
+    // product occupies the pipe).
     if (warp == 0) {
         // ============================ TMA producer ============================
         pdl_launch_dependents();

@@ -373,10 +373,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int total = my_tiles * a.chunks;   // (tile, k chunk) stages this CTA streams
 
     // The producer and MMA warps run their loops CONVERGED, all 32 lanes, on warp-uniform values; only the
-    // asynchronous instructions themselves sit under elect.sync.  (Inside an `if (lane == 0)` region the
-    // compiler keeps every operand in vector registers and wraps each UTMALDG / UTCHMMA — which take uniform
-    // registers — in an R2UR + ELECT waterfall loop: ~70 cycles per tcgen05.mma and ~0.2 us per TMA op,
-    // measured; that, not HBM, bounded the first version of this kernel.)
+    // asynchronous instructions themselves sit under elect.sync.  (Under `if (lane == 0)` the loops took
+    // ~70 cycles per tcgen05.mma and ~0.2 us per TMA op; that, not HBM, bounded the first version of this
+    // kernel.)
     if (warp == 0 || warp == 7) {
         // ============================ TMA producers ============================
         // warp 0: the weight op(s) of every stage; warp 7: the x op.  Each arrives on the stage's full

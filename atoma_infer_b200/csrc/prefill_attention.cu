@@ -411,10 +411,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         } else if (warp == 1 && n_max > 0) {
             // ================================ MMA issue ================================
             // The whole warp runs this role converged on warp-uniform values; only the tcgen05
-            // instructions sit under elect.sync.  (Inside an `if (lane == 0)` region the compiler keeps
-            // the operands in vector registers and wraps every UTCHMMA in an R2UR + ELECT waterfall loop,
-            // ~70 cycles per MMA against the 64 cycles a 128x128x16 MMA occupies the tensor pipe — the
-            // issue thread, not the pipe, was the limit of a first version: tensor pipe 49 % active.)
+            // instructions sit under elect.sync.  (Under `if (lane == 0)` the loop took ~70 cycles per
+            // product against the 64 cycles a 128x128x16 product occupies the tensor pipe — the issue
+            // thread, not the pipe, was the limit of a first version: tensor pipe 49 % active.)
             // Order per key tile j:  P.V(A,j)  QK(A,j+1)  P.V(B,j)  QK(B,j+1)
             // so while one query tile is being exponentiated the tensor pipe works for the other.
             constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
