@@ -114,11 +114,12 @@ __device__ __forceinline__ int cta_of_unit(long long units, long long u, int num
     return static_cast<int>(((u + 1) * num_ctas + units - 1) / units - 1);
 }
 
-// Reduction of a few partials of one (sequence, kv head) by ONE warp (the last to arrive for that
-// head).  Partials are merged in CTA-index order whoever arrives last, four outputs per lane and
-// four partials in flight at a time (16-byte loads), so the result is bit-reproducible and the cost
-// is one or two L2 round trips; more partials go through merge_parts.
-template <typename T, int D>
+// Reduction of the partials of one (sequence, kv head) by ONE warp (the last to arrive for that
+// head).  Partials are merged in CTA-index order whoever arrives last, NK float4 per lane and
+// NS partials in flight at a time (16-byte loads), so the result is bit-reproducible; the running
+// maximum moves every four partials whatever NS, and no sum is left to the compiler's choice of
+// contraction, so that all forms give the same bits.
+template <typename T, int D, int NK, int NS>
 __device__ __forceinline__ void combine_head(const DecodeArgs &a, long long units, int ncta, int fc, int lc,
                                              long long ub, long long ue, int b, int kvh, int hh, int G,
                                              int lane) {
@@ -126,13 +127,13 @@ __device__ __forceinline__ void combine_head(const DecodeArgs &a, long long unit
     constexpr int C4 = D / 4;
     const int nparts = lc - fc + 1;
     const int total = G * C4;
-    for (int g0 = 0; g0 < total; g0 += 128) {
-        bool ok[4];
-        int rr[4], d4[4];
-        float m_run[4], l_run[4];
-        float4 acc[4];
+    for (int g0 = 0; g0 < total; g0 += 32 * NK) {
+        bool ok[NK];
+        int rr[NK], d4[NK];
+        float m_run[NK], l_run[NK];
+        float4 acc[NK];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < NK; ++k) {
             const int idx = g0 + lane + 32 * k;
             ok[k] = idx < total;
             rr[k] = ok[k] ? idx / C4 : 0;
@@ -149,46 +150,48 @@ __device__ __forceinline__ void combine_head(const DecodeArgs &a, long long unit
                 mybase = (c * 2 + ((cs >= ub && cs < ue) ? 0 : 1)) * kConsumerWarps + hh;
             }
             const int nchunk = min(32, nparts - pc);
-            for (int s0 = 0; s0 < nchunk; s0 += 4) {
-                float2 ml[4][4];
-                float4 ov[4][4];
+            for (int s0 = 0; s0 < nchunk; s0 += NS) {
+                float2 ml[NS][NK];
+                float4 ov[NS][NK];
 #pragma unroll
-                for (int ss = 0; ss < 4; ++ss) {
-                    // Loads are unconditional (clamped to a valid partial) so that all 32 of them are
+                for (int ss = 0; ss < NS; ++ss) {
+                    // Loads are unconditional (clamped to a valid partial) so that all of them are
                     // in flight together; out-of-range ones get weight exp2(-inf) = 0 below.
                     const int64_t base = __shfl_sync(0xffffffffu, mybase, min(s0 + ss, nchunk - 1));
                     const bool pv = s0 + ss < nchunk;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
+                    for (int k = 0; k < NK; ++k) {
                         ml[ss][k] = __ldcg(reinterpret_cast<const float2 *>(a.ws_ml + base * (kPartRows * 2) + rr[k] * 2));
                         ov[ss][k] = __ldcg(reinterpret_cast<const float4 *>(a.ws_o + base * (kPartRows * D) + rr[k] * D + d4[k] * 4));
                         if (!(pv && ok[k])) ml[ss][k].x = -INFINITY;
                     }
                 }
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    float m_new = m_run[k];
+                for (int k = 0; k < NK; ++k) {
 #pragma unroll
-                    for (int ss = 0; ss < 4; ++ss) m_new = fmaxf(m_new, ml[ss][k].x);
-                    if (m_new == -INFINITY) continue;  // nothing but empty partials so far
-                    const float c0 = fast_exp2(m_run[k] - m_new);  // m_run = -inf -> 0
-                    acc[k].x *= c0; acc[k].y *= c0; acc[k].z *= c0; acc[k].w *= c0;
-                    l_run[k] *= c0;
+                    for (int s4 = 0; s4 < NS; s4 += 4) {
+                        float m_new = m_run[k];
 #pragma unroll
-                    for (int ss = 0; ss < 4; ++ss) {
-                        const float wgt = fast_exp2(ml[ss][k].x - m_new);  // empty partial: exp2(-inf) = 0
-                        acc[k].x += wgt * ov[ss][k].x;
-                        acc[k].y += wgt * ov[ss][k].y;
-                        acc[k].z += wgt * ov[ss][k].z;
-                        acc[k].w += wgt * ov[ss][k].w;
-                        l_run[k] += wgt * ml[ss][k].y;
+                        for (int ss = s4; ss < s4 + 4; ++ss) m_new = fmaxf(m_new, ml[ss][k].x);
+                        if (m_new == -INFINITY || s0 + s4 >= nchunk) continue;  // nothing but empty partials so far
+                        const float c0 = fast_exp2(m_run[k] - m_new);  // m_run = -inf -> 0
+#pragma unroll
+                        for (int ss = s4; ss < s4 + 4; ++ss) {
+                            const float wgt = fast_exp2(ml[ss][k].x - m_new);  // empty partial: exp2(-inf) = 0
+                            auto add = [&](float sum, float x) { return ss == s4 ? fmaf(sum, c0, __fmul_rn(wgt, x)) : fmaf(wgt, x, sum); };
+                            acc[k].x = add(acc[k].x, ov[ss][k].x);
+                            acc[k].y = add(acc[k].y, ov[ss][k].y);
+                            acc[k].z = add(acc[k].z, ov[ss][k].z);
+                            acc[k].w = add(acc[k].w, ov[ss][k].w);
+                            l_run[k] = add(l_run[k], ml[ss][k].y);
+                        }
+                        m_run[k] = m_new;
                     }
-                    m_run[k] = m_new;
                 }
             }
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < NK; ++k) {
             if (!ok[k]) continue;
             const bool empty = (l_run[k] == 0.f || l_run[k] != l_run[k]);
             const float inv = empty ? 1.f : 1.f / l_run[k];
@@ -200,17 +203,17 @@ __device__ __forceinline__ void combine_head(const DecodeArgs &a, long long unit
             *reinterpret_cast<uint2 *>(op) = packed;
             if (d4[k] == 0 && p.lse)
                 p.lse[static_cast<int64_t>(b) * p.h + head] =
-                    empty ? INFINITY : m_run[k] * 0.6931471805599453f + __logf(l_run[k]);
+                    empty ? INFINITY : fmaf(__log2f(l_run[k]), 0.6931471805599453f, __fmul_rn(m_run[k], 0.6931471805599453f));
         }
     }
 }
 
-// Merge of up to kMergeParts partials of one kv head by ONE warp: lane j < n holds partial j's workspace index.  The outputs of two chunks of 128 (all of them for
+// Merge of a group of up to kMergeParts partials of one kv head by ONE warp: lane j < n holds partial j's workspace index.  The outputs of two chunks of 128 (all of them for
 // 4 query heads of 64) are asked for first; under their way the maxima and sums of all rows, a lane per partial and two
 // rows at a time, become weights in shared memory.  A few round trips, however many partials.  put(row, d, acc, m, l) takes four outputs of a row, not yet
 // divided.
-constexpr int kMergeParts = 16, kMergeRows = 8;   // partials; rows whose weights are at hand
-constexpr int kFewUnits = 8, kFewParts = 8, kManyParts = 24;
+constexpr int kMergeParts = 16, kMergeRows = 8;   // partials of a group; rows whose weights are at hand
+constexpr int kManyParts = 24, kInOrder = 64 * 256;   // partials from which a step takes the kernel for many; floats of a kv head's partials up to which they are merged in order
 struct MergeRow {
     float w[kMergeParts];
     float m, l, pad[2];
@@ -278,8 +281,11 @@ __device__ __forceinline__ void merge_parts(const DecodeArgs &a, MergeRow *rows,
 }
 
 // Contributors of one (sequence, kv head) are the CTAs fc .. lc, a partial each; merged in CTA-index order whoever arrives last, so the result is
-// bit-reproducible.  A few: combine_head (32 sequences, five partials each, 0.8 us less than merge_parts).  Up to kMergeParts: by the warp that arrives last.  More: groups of equal size first, each by its last arriver into its first contributor's
-// place, then the groups (one user at 4000 keys, 148 partials: 53 us of 60 were one warp's chain of round trips, four partials each).
+// bit-reproducible.  Up to kInOrder floats: in order, by the warp that arrives last, which is bound by what one SM reads from L2 (its eight warps merge a head
+// each): steps of small models with one user and 38, 49 and 64 partials of 4 x 64 floats, in order / in groups, us: 244.0 / 245.1, 247.0 / 244.4, 250.4 /
+// 245.2; 32 and 49 of 4 x 128 442.3 / 443.6, 453.1 / 444.2.  More: groups of equal size first, each by its last arriver into its first contributor's place, then the
+// groups (one user at 4000 keys, 148 partials: 280 and 249 us, with four partials in flight 310).  The line lies where the two meet, but for 49 to 64 partials of
+// small heads, which keep the bits of the merge in order.
 template <typename T, int D>
 __device__ __forceinline__ void arrive_and_merge(const DecodeArgs &a, long long units, int ncta, int fc, int lc, long long ub, long long ue, int b, int kvh, int hh,
                                                  int G, int lane, int cta, MergeRow *rows) {
@@ -298,7 +304,7 @@ __device__ __forceinline__ void arrive_and_merge(const DecodeArgs &a, long long 
         __threadfence();
         return true;
     };
-    const bool grouped = nparts > kMergeParts;
+    const bool grouped = nparts >= kManyParts && nparts * G * D > kInOrder;
     const int step = grouped ? max(8, (nparts + kMergeParts - 1) / kMergeParts) : 1;
     const int first = grouped ? fc + (cta - fc) / step * step : fc, at = grouped ? place(first) : 0;
     float *po = a.ws_o + static_cast<int64_t>(at) * (kPartRows * D), *pml = a.ws_ml + static_cast<int64_t>(at) * (kPartRows * 2);
@@ -307,8 +313,9 @@ __device__ __forceinline__ void arrive_and_merge(const DecodeArgs &a, long long 
         int *ctr = level == 0 ? a.group_counters + at : &a.counters[b * p.h_k + kvh];
         if (!last_of(ctr, n)) return;
         if (a.trace && lane == 0) a.trace[blockIdx.x * 8 + 6] = global_timer_ns();
-        if (nparts <= kFewParts) {
-            combine_head<T, D>(a, units, ncta, fc, lc, ub, ue, b, kvh, hh, G, lane);
+        if (!grouped) {
+            if (D == 64 && G * D <= 256) combine_head<T, D, 2, 8>(a, units, ncta, fc, lc, ub, ue, b, kvh, hh, G, lane);
+            else combine_head<T, D, 4, 4>(a, units, ncta, fc, lc, ub, ue, b, kvh, hh, G, lane);
             if (lane == 0) *ctr = 0;
             break;
         }
@@ -348,7 +355,6 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
     __shared__ int cum[kMaxBatch + 2];  // cum[b] = first unit of sequence b
     __shared__ __align__(16) MergeRow merge_s[MANY ? kConsumerWarps : 1][MANY ? kMergeRows : 1];
     __shared__ int combine_flag;
-    [[maybe_unused]] __shared__ int longest_s;   // longest_s: units of the longest sequence and head group
     __shared__ int part_base[kMaxCtas];  // combine: workspace index of each contributing CTA's partial
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -394,11 +400,10 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
     if (tid == 0) cum[0] = 0;
     __syncthreads();
     if (warp == 0) {
-        int carry = 0, longest = 0;
+        int carry = 0;
         for (int base = 0; base < B; base += 32) {
             const int i = base + lane;
             int v = i < B ? cum[i + 1] : 0;
-            if (MANY) longest = max(longest, v);
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int n = __shfl_up_sync(0xffffffffu, v, o);
@@ -406,11 +411,6 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
             }
             if (i < B) cum[i + 1] = v + carry;
             carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if constexpr (MANY) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
-            if (lane == 0) longest_s = longest / a.hg;
         }
     }
     __syncthreads();
@@ -436,13 +436,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
     // The grid was sized from the host-side upper bound of the unit count; only the first
     // min(grid, units) CTAs take part in the partition, so that every participant owns >= 1 unit
     // (the arrival-count logic below relies on it).
-    int ncta = static_cast<int>(min(static_cast<long long>(gridDim.x), units));
-    // Few keys: a sequence on no more CTAs than one merge takes, as long as that leaves a CTA no more than kFewUnits units (one user at 1000 keys of
-    // heads of 128: 15 CTAs of four or five units 21.2 us, 63 of one and a merge in two levels 25.3; twelve units instead of eight are as fast).
-    if (MANY && units <= kFewUnits * ncta) {
-        const int few = static_cast<int>(units) * (kMergeParts - 1) / max(longest_s, 1);
-        if (few < ncta && few * kFewUnits >= units) ncta = max(1, few);
-    }
+    const int ncta = static_cast<int>(min(static_cast<long long>(gridDim.x), units));
     if (cta >= ncta) return;
     const long long u_begin = cta_start(units, cta, ncta), u_end = cta_start(units, cta + 1, ncta);
 
@@ -809,7 +803,7 @@ decode_paged_kernel(const __grid_constant__ CUtensorMap map_k,
             if (old == lc - fc) {
                 __threadfence();
                 if (a.trace && lane == 0) a.trace[blockIdx.x * 8 + 6] = global_timer_ns();
-                combine_head<T, D>(a, units, ncta, fc, lc, ub, ue, b, kvh, hh, G, lane);
+                combine_head<T, D, 4, 4>(a, units, ncta, fc, lc, ub, ue, b, kvh, hh, G, lane);
                 if (lane == 0) *ctr = 0;  // self-cleaning for the next launch
                 if (a.trace && lane == 0) a.trace[blockIdx.x * 8 + 7] = global_timer_ns();
             }
@@ -1002,9 +996,8 @@ bool launch_decode_as(const CUtensorMap &mk, const CUtensorMap &mv, const Decode
 
 template <typename T, int D>
 bool launch_decode(const CUtensorMap &mk, const CUtensorMap &mv, const DecodeArgs &a, cudaStream_t stream) {
-    // Many partials per sequence: by the CTAs there are for it, and by its stages of a.tok keys (the longest it can have).  Steps of a model with 2048-wide layers,
-    // one partial at a time / in groups, us: one user at 4000 keys 335 / 272, 777 keys 280 / 267, 100 keys (7 partials) 120.7 / 123.0; eight sequences of
-    // 500 keys (18 partials) 187.6 / 190.6.
+    // Many partials per sequence: by the CTAs there are for it, and by its stages of a.tok keys (the longest it can have).  Up to kManyParts - 1 partials both
+    // kernels merge in order and give the same bits, so a sequence's do not follow the width of its table.
     const int64_t stages = (a.p.seqlen_k + a.tok - 1) / a.tok, share = current_device_info().sm_count / std::max<int64_t>(1, static_cast<int64_t>(a.p.b) * a.hg);
     const bool many = std::min(stages, share) >= kManyParts;
     return many ? launch_decode_as<T, D, true>(mk, mv, a, stream) : launch_decode_as<T, D, false>(mk, mv, a, stream);
