@@ -108,6 +108,13 @@ struct Staged {
     static constexpr int kBytes = kEnd / 16 % 2 ? kEnd : kEnd + 16;
 };
 
+// The state of a CTA's columns in shared memory, where it passes through on its way (SHORT): the rows of a lane apart by what lets a column's lanes hit distinct banks.
+template <int R, int PW, int NW>
+struct StateTile {
+    static constexpr int kCols = 64 * NW / PW, kPad = 128 / PW > 4 ? 64 / PW : 4, kPart = R * kCols + kPad, kBytes = PW * kPart * 4;
+    static __device__ __forceinline__ int at(int row, int col) { return row / R * kPart + row % R * kCols + col; }
+};
+
 __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -124,8 +131,12 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
 // Rows kept as bfloat16 in shared memory and converted per warp beat float32 rows (718 us against 729 for 4096 tokens of 32 heads of 128 x 128),
 // one column a lane loses to two (924 to 1330 us).  Against one column a lane, 32 rows, rows converted and normed by the staging warps: delta
 // rule 1064 -> 729 us (that case), 504 -> 289 (16 heads, 2000 tokens); state space 794 -> 365 (32 heads of 128 x 64, 4000 tokens); gated linear
-// attention 752 -> 421 (32 heads of 64 x 128, 4000 tokens); one token of 32 sequences 70 -> 51, 62 -> 48, 45 -> 31.
-template <typename T, int KIND, int R, int PW, int NW, int NB>
+// attention 752 -> 421 (32 heads of 64 x 128, 4000 tokens).
+// SHORT: steps of a few tokens a sequence are bound by the states, read and written once.  What counts there is bytes on their way: four CTAs an SM (no token ahead
+// in registers), and the state through shared memory in pieces of 16 bytes, since the 8 to 32 bytes of a row that a warp's columns are touch as many
+// lines.  One token of 32 sequences, one column a lane / wide CTAs without this / this, us: delta rule, 32 heads of 128 x 128 (134 MB), 78 / 113 / 60; state space,
+// 128 x 64, 37 / 57 / 27; gated linear attention, 64 x 128, 49 / 56 / 29; 64 heads of 64 x 64 47 / 104 / 29; of 128 sequences, 32 heads of 64 x 32, 57 / 203 / 32.
+template <typename T, int KIND, int R, int PW, int NW, int NB, bool SHORT>
 __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(const atoma_state_scan_args a, int chunk, int buffers, int piece, int v_piece) {
     using L = Staged<T, KIND, R, PW, NW>;
     extern __shared__ __align__(16) unsigned char sm[];
@@ -325,10 +336,38 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
     const float skip = KIND == 2 && a.skip ? a.skip[h] : 0.f;
     float *S_g = a.state + static_cast<int64_t>(a.state_slots[b]) * a.state_stride + static_cast<int64_t>(h) * D * V;
     const bool pair_ok = V % 2 == 0 && reinterpret_cast<uintptr_t>(S_g) % 8 == 0;
+    using Tile = StateTile<R, PW, NW>;
+    const bool through = SHORT && V % 4 == 0 && reinterpret_cast<uintptr_t>(S_g) % 16 == 0;
+    float *tile = reinterpret_cast<float *>(sm + buffers * chunk_bytes);
+    // the compute warps' pieces of 16 bytes of the CTA's columns, a row's one after the other
+    auto each_piece = [&](auto f) {
+        constexpr int kPer = COLS / 4;
+        for (int i = threadIdx.x; i < D * kPer; i += 32 * NW) {
+            const int row = i / kPer, c = i % kPer * 4;
+            if (jb + c < V) f(tile + Tile::at(row, c), S_g + static_cast<int64_t>(row) * V + jb + c);
+        }
+    };
     uint64_t Sa[R / 2], Sb[R / 2];
     if (a.context_lens[b] == 0) {
 #pragma unroll
         for (int i = 0; i < R / 2; ++i) Sa[i] = Sb[i] = 0;
+    } else if (through) {
+        each_piece([](float *t, const float *g) { cp_async_16(smem_u32(t), g, 16); });
+        cp_async_commit();
+        cp_async_wait_all();
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory");
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) {
+            float2 x[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int row = part * R + 2 * i + e;
+                x[e] = make_float2(0.f, 0.f);
+                if (row < D && j < V) x[e] = *reinterpret_cast<const float2 *>(tile + Tile::at(row, jl));
+            }
+            Sa[i] = pk2(x[0].x, x[1].x);
+            Sb[i] = pk2(x[0].y, x[1].y);
+        }
     } else {
 #pragma unroll
         for (int i = 0; i < R / 2; ++i) {
@@ -385,10 +424,11 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
             if (KIND == 1) tk.s1 = *reinterpret_cast<const float2 *>(row + L::kScalars + 16);
             fetch_pair(reinterpret_cast<const T *>(row + L::kV) + jl, tk.va, tk.vb);
         };
-        fetch(0);
-        constexpr int kUnroll = 4;
+        if (!SHORT) fetch(0);
+        constexpr int kUnroll = SHORT ? 1 : 4;
 #pragma unroll kUnroll
         for (int i = 0; i < nt; ++i) {
+            if (SHORT) fetch(i);   // registers for more warps instead of a token ahead
             uint64_t k2[R / 2], q2[R / 2], d2[KIND == 0 ? R / 2 : 1];
             unpack<R>(tk.k, k2, T{});
             unpack<R>(tk.q, q2, T{});
@@ -402,7 +442,7 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
             const float4 s0 = tk.s0;
             const float2 s1 = tk.s1;
             const float va = tk.va, vb = tk.vb;
-            fetch(min(i + 1, nt - 1));
+            if (!SHORT) fetch(min(i + 1, nt - 1));
             float o = o_mine;
             float ua, ub, wa, wb;                                  // written rows of both columns, before and with the key's length
             uint64_t g2 = 0;
@@ -464,7 +504,9 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
             const int row = part * R + 2 * i + e;
             float *p = S_g + static_cast<int64_t>(row) * V + j;
             if (row < D) {
-                if (pair_ok) {
+                if (through) {
+                    *reinterpret_cast<float2 *>(tile + Tile::at(row, jl)) = x[e];
+                } else if (pair_ok) {
                     if (j < V) *reinterpret_cast<float2 *>(p) = x[e];
                 } else {
                     if (j < V) p[0] = x[e].x;
@@ -473,20 +515,24 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
             }
         }
     }
+    if (through) {   // a warp stores other warps' entries
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory");
+        each_piece([](const float *t, float *g) { *reinterpret_cast<float4 *>(g) = *reinterpret_cast<const float4 *>(t); });
+    }
 }
 
 // the longest portion where every one of the B sequences has a token (one without makes another longer: nothing but speed may depend on this)
 int64_t longest_portion(const atoma_state_scan_args &a) { return std::max<int64_t>(1, a.T - (a.B - 1)); }
 
-template <typename T, int KIND, int R, int PW, int NW, int NB>
+template <typename T, int KIND, int R, int PW, int NW, int NB, bool SHORT = false>
 cudaError_t launch_scan(const atoma_state_scan_args &a, cudaStream_t stream) {
     using L = Staged<T, KIND, R, PW, NW>;
     // staged tokens per buffer: at most 32, no more than the longest portion can have, and NB CTAs' buffers fit one SM
     const int64_t fit = 200 * 1024 / NB / (kScanBuffers * L::kBytes);
-    const int chunk = static_cast<int>(std::max<int64_t>(4, std::min<int64_t>({32, (longest_portion(a) + 3) / 4 * 4, fit / 4 * 4})));
+    const int chunk = SHORT ? 4 : static_cast<int>(std::max<int64_t>(4, std::min<int64_t>({32, (longest_portion(a) + 3) / 4 * 4, fit / 4 * 4})));
     const int buffers = a.T <= chunk ? 1 : kScanBuffers;   // a step of one chunk fills the first only (whatever share of it is whose: a sequence may have no token)
-    const size_t smem = static_cast<size_t>(buffers) * chunk * L::kBytes;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(state_scan_kernel<T, KIND, R, PW, NW, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
+    const size_t smem = static_cast<size_t>(buffers) * chunk * L::kBytes + (SHORT ? StateTile<R, PW, NW>::kBytes : 0);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(state_scan_kernel<T, KIND, R, PW, NW, NB, SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
     // copies in pieces of 16 bytes where every row and size allows it, else of 4, else value by value
     const int64_t size = sizeof(T);
     auto row = [&](const void *p, int64_t ld, int64_t cols, int64_t piece) {
@@ -495,19 +541,26 @@ cudaError_t launch_scan(const atoma_state_scan_args &a, cudaStream_t stream) {
     auto rows = [&](int64_t piece) { return row(a.q, a.ld_q, a.dim, piece) && row(a.k, a.ld_k, a.dim, piece) && (KIND != 0 || row(a.z, a.ld_z, a.dim, piece)); };
     const int piece = rows(16) ? 16 : (rows(4) ? 4 : 0), v_piece = row(a.v, a.ld_v, a.vdim, 16) ? 16 : (row(a.v, a.ld_v, a.vdim, 4) ? 4 : 0);
     const dim3 grid(static_cast<unsigned>((a.vdim + L::kCols - 1) / L::kCols), static_cast<unsigned>(a.H), static_cast<unsigned>(a.B));
-    return launch_ex(state_scan_kernel<T, KIND, R, PW, NW, NB>, grid, dim3(32 * (NW + kStagers)), smem, stream, a, chunk, buffers, piece, v_piece);
+    return launch_ex(state_scan_kernel<T, KIND, R, PW, NW, NB, SHORT>, grid, dim3(32 * (NW + kStagers)), smem, stream, a, chunk, buffers, piece, v_piece);
 }
 
 // How the state is split.  Sixteen rows a lane need the fewest instructions per entry and one shuffle fewer; eight rows a lane put the state on
 // twice the warps, and serve steps that leave half of the SMs idle (us, eight / sixteen: delta rule of 16 heads, 2000 tokens 289 / 363; state space of
-// 32 heads, 4000 tokens 365 / 518; where sixteen fill the SMs once it is 876 / 727, 301 / 266).  CTAs of eight warps share the staging and keep
-// two warps a scheduler: for more than a wave of CTAs (one token of 32 sequences 96 / 51, 500 + 500 tokens 194 / 164); between one and two waves a long
+// 32 heads, 4000 tokens 365 / 518; where sixteen fill the SMs once it is 876 / 727, 301 / 266), and steps of more than a wave whose heads are too narrow
+// for the columns of eight warps (32 sequences of 40 tokens, 16 heads of 64 x 64, eight rows / sixteen in wide CTAs 41 / 66, 32 heads of 64 x 32 41 / 117).  CTAs of eight
+// warps share the staging and keep two warps a scheduler: for more than a wave of CTAs (500 + 500 tokens 194 / 164); between one and two waves a long
 // portion stays with the narrow CTAs, since the sequences' lengths, which only the device knows, may leave wide ones alone on an SM (900, 700, 300 and 105
-// tokens of 16 heads 193 / 285, 500 + 500 tokens of 32 heads the other way round).
-enum class Split { kEight, kSixteen, kSixteenWide };
+// tokens of 16 heads 193 / 285, 500 + 500 tokens of 32 heads the other way round).  Steps of four tokens a sequence and less in the mean go by kShort, though one of them
+// may be long (32 sequences of 1, 2, 4 tokens, eight rows or wide CTAs / short, us: 113 / 60, 117 / 68, 125 / 80; 31 of one token beside one of 60 129 / 97).
+enum class Split { kEight, kSixteen, kSixteenWide, kShort };
 
 template <typename T, int KIND>
 cudaError_t launch_split(const atoma_state_scan_args &a, Split split, cudaStream_t stream) {
+    if (split == Split::kShort)
+        return a.dim <= 64    ? launch_scan<T, KIND, 8, 8, 4, 4, true>(a, stream)
+               : a.dim <= 128 ? launch_scan<T, KIND, 8, 16, 4, 4, true>(a, stream)
+               : a.dim <= 256 ? launch_scan<T, KIND, 8, 32, 4, 4, true>(a, stream)
+                              : launch_scan<T, KIND, 16, 32, 4, 2, true>(a, stream);
     if (split == Split::kEight)
         return a.dim <= 64 ? launch_scan<T, KIND, 8, 8, 4, 2>(a, stream) : a.dim <= 128 ? launch_scan<T, KIND, 8, 16, 4, 2>(a, stream) : launch_scan<T, KIND, 8, 32, 4, 2>(a, stream);
     if (split == Split::kSixteenWide)
@@ -546,7 +599,8 @@ bool hyb_state_scan(const atoma_state_scan_args &a, cudaStream_t stream) {
     const int pw = a.dim <= 64 ? 4 : (a.dim <= 128 ? 8 : (a.dim <= 256 ? 16 : 32)), cols = 256 / pw, sms = current_device_info().sm_count;
     const int64_t ctas = (a.vdim + cols - 1) / cols * a.H * a.B;
     Split split = Split::kSixteen;
-    if (a.dim <= 256 && ctas * 2 <= sms && !(g_hybrid_debug & 16)) split = Split::kEight;
+    if (a.T <= 4 * a.B && !(g_hybrid_debug & 16)) split = Split::kShort;
+    else if (a.dim <= 256 && (ctas * 2 <= sms || (ctas > sms && a.vdim <= cols)) && !(g_hybrid_debug & 16)) split = Split::kEight;
     else if (ctas > (a.dim > 256 || longest_portion(a) <= 256 ? sms : 2 * sms)) split = Split::kSixteenWide;
     const cudaError_t e = a.dtype == ATOMA_DTYPE_BF16 ? launch_kind<__nv_bfloat16>(a, split, stream) : launch_kind<float>(a, split, stream);
     return hybrid::launched(e, "state_scan_kernel");

@@ -78,3 +78,55 @@ def test_sequences_without_a_token(n, empty, D):
         out = ops.gla_scan(q, k, v, z, zb, 6.0, D ** -0.5, state, i32(list(range(S))), i32(starts), i32([0] * S), H, D, V)
         outs.append((out, state[starts.index(n) - 1]))
     assert all(torch.equal(o, outs[0][0]) and torch.equal(s, outs[0][1]) for o, s in outs[1:])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("D,V", [(64, 128), (64, 64), (64, 32), (128, 64), (72, 8), (50, 34), (33, 7), (256, 16), (300, 24), (512, 12)])
+@pytest.mark.parametrize("rule", ["gla", "delta", "ssm"])
+def test_short_steps_give_the_bits_of_long_ones(rule, D, V, dtype):
+    """A portion of 23 tokens at once, among enough others for the wide CTAs, and in steps of one to four tokens, whose states pass through shared memory where
+    their rows are whole pieces of 16 bytes; states of an odd pitch, which are not."""
+    from atoma_infer_b200 import hybrid_ops as ops
+
+    H, n, B = 4, 23, 80
+    G = H if rule == "gla" else 2
+    g = torch.Generator().manual_seed(D + V)
+    rnd = lambda c: torch.randn(n, c, generator=g).to(torch.bfloat16).to(dtype).to(DEV)
+    rows = [rnd(G * D), rnd(G * D), rnd(H * V), rnd(H * D), rnd(H), rnd(H)]
+    rows[1] *= D ** -0.5 if rule != "delta" else 1.0
+    per_head = [torch.randn(H, generator=g).to(DEV) * 0.5 - 1.0 for _ in range(3)]
+    zb = torch.randn(H * D, generator=g).to(DEV)
+    before = torch.randn(H * D * V, generator=g).to(DEV)
+
+    def step(rows, state, slots, starts, contexts):
+        q, k, v, z, b, a = rows
+        at = (state, i32(slots), i32(starts), i32(contexts), H)
+        if rule == "gla":
+            return ops.gla_scan(q, k, v, z, zb, 6.0, D ** -0.5, *at, D, V)
+        if rule == "delta":
+            return ops.delta_rule_scan(q, k, v, b, a, per_head[0], per_head[1], D ** -0.5, *at, G, D, V)
+        return ops.ssm_scan(v, k, q, a, per_head[0], per_head[1], per_head[2], *at, G, D, V)
+
+    def states(count, pitch=0):
+        s = torch.full((count, H * D * V + pitch), 3.0, device=DEV)
+        s[:, :H * D * V] = before
+        return s
+
+    state = states(1)
+    out = step(rows, state, [0], [0, n], [7])
+    assert torch.isfinite(out).all() and torch.isfinite(state).all()
+    many = [torch.cat([t] + [t[:6]] * (B - 1)) for t in rows]            # six tokens a sequence: no short step
+    wide = states(B)
+    assert torch.equal(step(many, wide, list(range(B)), [0] + [n + 6 * b for b in range(B)], [7] * B)[:n], out) and torch.equal(wide[0], state[0])
+    for pitch in (0, 1):
+        cut, t0, k = states(2, pitch), 0, 0
+        while t0 < n:
+            m = min(1 + k % 4, n - t0)
+            part = step([t[t0:t0 + m].contiguous() for t in rows], cut, [1], [0, m], [7 + t0])
+            assert torch.equal(part, out[t0:t0 + m]), (t0, m, pitch)
+            t0, k = t0 + m, k + 1
+        assert torch.equal(cut[1, :H * D * V], state[0]) and bool((cut[:, H * D * V:] == 3.0).all()) and torch.equal(cut[0, :H * D * V], before)
+    fresh = states(1)                                                     # no context: what the slot held does not count
+    whole = states(1)
+    a, b = step(rows, whole, [0], [0, n], [0]), step([t[:1] for t in rows], fresh, [0], [0, 1], [0])
+    assert torch.equal(a[:1], b)
