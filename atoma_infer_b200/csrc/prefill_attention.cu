@@ -223,7 +223,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         constexpr bool kEager = SPLIT == 1 && !PAGED && D == 128;
     constexpr int kCorrect = SPLIT == 1 ? 32 : 16;   // columns of O that a correction holds
     __shared__ float bias_s[BIASED ? kPfBiasFront + kPfBiasSmem + kPfBiasBack : 1];
-    __shared__ float swap_s[kQTiles][2][SPLIT == 2 ? kPfM : 1];            // a row's maximum (at the end: its sum) over either half of the keys
+    __shared__ float swap_s[2][kQTiles][2][SPLIT == 2 ? kPfM : 1];         // a row's maximum (at the end: its sum) over either half of the keys
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // Heads, then sequences, then query tiles from the last (causal: heaviest) one down, so that the SMs run out of light tiles together
@@ -508,13 +508,14 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (p.unpadded_lse && p.cu_q) lse_idx = static_cast<int64_t>(head) * p.cu_q[p.b] + si.q_start + grow;
             else lse_idx = (static_cast<int64_t>(bidb) * p.h + head) * p.seqlen_q + grow;
         }
-        // the two warps of a row quad tell each other a value per row (both run the same tiles)
-        [[maybe_unused]] auto swap = [&](float mine) {
-            swap_s[t][half][row] = mine;
+        // The two warps of a row quad tell each other a value per row (both run the same tiles).  The exchanges of a row take two cells in turn: a cell is stored
+        // to again behind the barrier of the exchange between, where the other warp arrives with the value that it read.
+        [[maybe_unused]] auto swap = [&](int turn, float mine) {
+            swap_s[turn & 1][t][half][row] = mine;
             tc_fence_before_sync();
             asm volatile("bar.sync %0, 64;" ::"r"(1 + t * 4 + quad) : "memory");
             tc_fence_after_sync();
-            return swap_s[t][half ^ 1][row];
+            return swap_s[turn & 1][t][half ^ 1][row];
         };
         if (n_tiles > 0) {
             float m_ref = -INFINITY, l_run = 0.f;
@@ -594,7 +595,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     for (int i = 0; i < 8; ++i) mx8[i] = fmaxf(mx8[i], __uint_as_float(sv_[N - 8 + i]));
                     const float mx = fmaxf(max3(mx8[0], mx8[1], mx8[2]), fmaxf(max3(mx8[3], mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7])));
                     float m_tile = BIASED ? fmaf(mx, sc, far_bias) : mx * sc;  // scale_log2 > 0 (checked on the host)
-                    if constexpr (SPLIT == 2) m_tile = fmaxf(m_tile, swap(m_tile));   // both halves' scores are in registers: P may be written over them
+                    if constexpr (SPLIT == 2) m_tile = fmaxf(m_tile, swap(j - n_lo, m_tile));   // both halves' scores are in registers: P may be written over them
                     // ---- running maximum ----
                     const bool need = m_tile > m_ref + kThreshold;  // also the first finite tile (m_ref = -inf)
                     if (__any_sync(0xffffffffu, need)) {
@@ -635,7 +636,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             // ---- epilogue: O / rowsum -> global ----
             const bool gated = p.gate && grow < len_q && (p.gate_below <= 0 || grow + shift + (p.key_lo ? p.key_lo[bidb] : 0) < p.gate_below);
             if constexpr (SPLIT == 2) {   // both halves' sums of a row, in the same order on both sides
-                const float other = swap(l_run);
+                const float other = swap(n_tiles - n_lo, l_run);
                 l_run = half ? other + l_run : l_run + other;
             }
             // this half's part of the row's gate, 32 columns at a time: the first are under way while the last products run

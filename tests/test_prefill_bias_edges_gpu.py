@@ -64,3 +64,43 @@ def test_scores_that_grow_from_tile_to_tile(D, step):
     w = torch.softmax(s, 2)
     check(got, *(torch.bmm(w, x).transpose(0, 1) for x in (rep(v), rep(v).abs())), score=float(s[s > -math.inf].abs().max()))
     assert ho.prefill_timeouts() == 0
+
+
+def halves(case, n, step, dev):
+    """What 64 keys at a time (a thread's share of a tile) add to the score, in units of log 2."""
+    h = torch.arange(n, device=dev) // 64
+    if case == "rising":
+        return step * h.float()
+    low = (h % 2 == 1) if case == "first" else (h % 2 == 0) if case == "second" else ((h // 2 + h) % 2 == 1)   # the half that never holds the largest score
+    return step * (h // 2).float() - 24.0 * low.float()
+
+
+@pytest.mark.parametrize("case", ["rising", "first", "second", "alternate"])
+@pytest.mark.parametrize("D,step,form", [(64, 3.0, "paged"), (128, 12.0, "paged"), (64, 12.0, "bias"), (128, 3.0, "bias"), (128, 12.0, "bias")])
+def test_largest_scores_in_one_half_of_the_tiles(D, step, form, case):
+    """Two threads share a row's scores where pages or a distance table are read: each has to learn of the other's maximum, in every tile and behind the last."""
+    H, G, n, bs = 4, 2, 900, 16
+    pages = -(-n // bs)
+    q = 0.3 * randn_t((n, H, D), 1, torch.bfloat16, DEV)
+    kc = 0.3 * randn_t((pages, bs, G, D), 2, torch.bfloat16, DEV)
+    vc = randn_t((pages, bs, G, D), 3, torch.bfloat16, DEV)
+    order = torch.randperm(pages, generator=torch.Generator().manual_seed(4)).to(DEV)
+    slot = order[torch.arange(n, device=DEV) // bs] * bs + torch.arange(n, device=DEV) % bs
+    q[:, :, 0] = (torch.arange(n, device=DEV) % 3 != 1).to(q.dtype)[:, None] * 4.0
+    kc.view(-1, G, D)[slot, :, 0] = (halves(case, n, step, DEV) * math.log(2.0) * D ** 0.5 / 4.0)[:, None].to(kc.dtype)
+    k, v = (x.reshape(-1, G, D)[slot].double().transpose(0, 1).repeat_interleave(H // G, 0) for x in (kc, vc))
+    i, j = torch.arange(n, device=DEV)[:, None], torch.arange(n, device=DEV)[None]
+    s = torch.bmm(q.double().transpose(0, 1), k.transpose(1, 2)) * D ** -0.5
+    table = order.to(torch.int32)[None].contiguous()
+    if form == "paged":
+        start = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+        got = ops.flash_attn_varlen_with_block_table(q, kc, vc, None, start, start, n, n, D ** -0.5, None, 0, table)
+    else:
+        dist = randn_t((300, H), 5, torch.float32, DEV)
+        pos, tseq = torch.arange(n, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+        got = ho.softmax_attention_paged(q.reshape(n, H * D), kc.view(-1, G, D), vc.view(-1, G, D), pos, tseq, table, H, G, D, D, bs, D ** -0.5, dist_bias=dist, long_min_q=128)
+        s = s + dist.double()[(i - j).clamp(0, 299)].permute(2, 0, 1)
+    s = s.masked_fill((j > i)[None], -math.inf)
+    w = torch.softmax(s, 2)
+    check(got.reshape(n, H, D), *(torch.bmm(w, x).transpose(0, 1) for x in (v, v.abs())), score=float(s[s > -math.inf].abs().max()))
+    assert ho.prefill_timeouts() == 0
