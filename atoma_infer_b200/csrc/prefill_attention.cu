@@ -68,8 +68,9 @@ template <int SPLIT>
 constexpr int kPfSoftmaxRegs = SPLIT == 1 ? 224 : 104;  // setmaxnreg: 168 * 384 = 56 * 128 + 224 * 256; 96 * 640 = 64 * 128 + 104 * 512
 constexpr float kRescaleThreshold = 8.f;  // log2 units: P <= 2^8 between corrections
 constexpr int kPfBiasSmem = 2048;         // distances whose bias (this head's column of the table) is kept in shared memory
-// ... behind copies of its first row and in front of copies of its last, so that a tile on the diagonal (distances from -254 on) or across the table's end
-// reads its biases without a clamp: with one, such a tile took 9000 to 12000 cycles where others take 3000.
+// ... behind copies of its first row and in front of copies of its last (of a longer table: the rows that follow), so that a tile on the diagonal (distances
+// from -254 on), across the table's end or within a longer table's first rows reads its biases without a clamp: with one, such a tile took 9000 to 12000
+// cycles where others take 3000 (4000 tokens under a table of 4096 rows, heads of 64 and 128: 651 and 686 us with clamps in all tiles, 432 and 471).
 constexpr int kPfBiasFront = 256, kPfBiasBack = 160;
 
 __device__ unsigned int g_prefill_late;   // CTAs that gave up waiting, since the library was loaded
@@ -260,7 +261,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int bias_n = BIASED ? min(p.dist_rows, kPfBiasSmem) : 0;
     if (BIASED)
         for (int i = tid; i < kPfBiasFront + bias_n + kPfBiasBack; i += kPfThreads<SPLIT>)
-            bias_s[i] = p.dist_bias[static_cast<int64_t>(min(max(i - kPfBiasFront, 0), bias_n - 1)) * p.dist_heads + head] * 1.4426950408889634f;
+            bias_s[i] = p.dist_bias[static_cast<int64_t>(min(max(i - kPfBiasFront, 0), p.dist_rows - 1)) * p.dist_heads + head] * 1.4426950408889634f;
     if (warp == 1) tmem_alloc(&tmem_base_smem, kTmemCols);
     tc_fence_before_sync();
     __syncthreads();
@@ -541,7 +542,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     if (__all_sync(0xffffffffu, d0 - (N - 1) >= last) && last < bias_n) {
                         far = true;
                         far_bias = bias_s[kPfBiasFront + last];
-                    } else if (__all_sync(0xffffffffu, d0 - (N - 1) >= -kPfBiasFront && d0 < last + kPfBiasBack) && last < bias_n) {
+                    } else if (__all_sync(0xffffffffu, d0 - (N - 1) >= -kPfBiasFront && d0 < bias_n + kPfBiasBack)) {
                         // every distance of the tile is a row of the shared-memory copy: no clamps, constant offsets from one address
                         const float *bp = bias_s + kPfBiasFront + d0;
 #pragma unroll

@@ -66,6 +66,23 @@ def test_scores_that_grow_from_tile_to_tile(D, step):
     assert ho.prefill_timeouts() == 0
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("rows,n,context", [(2210, 300, 2100), (2049, 200, 2250), (4096, 700, 3700), (3000, 400, 1900)])
+def test_tables_longer_than_their_copy(D, rows, n, context):
+    """Tiles whose distances lie within the copy of the first rows and the rows behind it, across their end, between there and the table's end, and beyond that."""
+    H, G, bs, m = 4, 2, 16, n + context
+    kc, vc = randn_t((-(-m // bs) * bs, G, D), 1, torch.bfloat16, DEV), randn_t((-(-m // bs) * bs, G, D), 2, torch.bfloat16, DEV)
+    q, dist = randn_t((n, H * D), 3, torch.bfloat16, DEV), randn_t((rows, H), 5, torch.float32, DEV)
+    table, pos = torch.arange(-(-m // bs), dtype=torch.int32, device=DEV)[None], context + torch.arange(n, device=DEV)
+    got = ho.softmax_attention_paged(q, kc, vc, pos, torch.zeros(n, dtype=torch.int32, device=DEV), table, H, G, D, D, bs, D ** -0.5, dist_bias=dist, long_min_q=128)
+    k, v = (x[:m].double().transpose(0, 1).repeat_interleave(H // G, 0) for x in (kc, vc))
+    i, j = pos[:, None], torch.arange(m, device=DEV)[None]
+    s = torch.bmm(q.double().reshape(n, H, D).transpose(0, 1), k.transpose(1, 2)) * D ** -0.5
+    w = torch.softmax((s + dist.double()[(i - j).clamp(0, rows - 1)].permute(2, 0, 1)).masked_fill((j > i)[None], -math.inf), 2)
+    check(got, *((torch.bmm(w, x).transpose(0, 1).reshape(n, H * D)) for x in (v, v.abs())))
+    assert ho.prefill_timeouts() == 0
+
+
 def halves(case, n, step, dev):
     """What 64 keys at a time (a thread's share of a tile) add to the score, in units of log 2."""
     h = torch.arange(n, device=dev) // 64
