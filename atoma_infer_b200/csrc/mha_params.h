@@ -58,10 +58,9 @@ struct MhaParams {
 };
 
 // Sequences of a paged step of many (sequence, head) pairs that are faster on the 64-row tiles, several of which share an SM, than on
-// prefill_attn_kernel, whose CTA fills one: few query rows over few keys (no longer sequence is short if one is not).  64 and 128 sequences of 32 heads,
-// tiles / prefill kernel, us: heads of 128, 64 rows over 64 keys 58 / 111, 264 keys 186 / 216, 564 keys 337 / 298; one row over 32, 232, 532 keys
-// 48 / 110, 153 / 150, 327 / 297; heads of 64, 64 rows over 64, 564, 1064, 2064 keys 29 / 92, 176 / 235, 324 / 341, 614 / 553; 128 rows over 128, 192, 328 keys
-// 76 / 101, 111 / 131, 213 / 179.
+// prefill_attn_kernel, whose CTA fills one: few query rows over few keys (no longer sequence is short if one is not).  64 sequences of 32 heads,
+// tiles / prefill kernel, us: heads of 128, 64 rows over 64, 164, 264, 364 keys 64 / 115, 127 / 164, 188 / 195, 235 / 191, 100 rows over 100 and 200 keys 146 / 129,
+// 277 / 172; heads of 64, 64 rows over 64, 564, 1064 keys 36 / 98, 180 / 210, 328 / 306, 128 rows over 128, 192, 328 keys 82 / 109, 116 / 139, 217 / 164.
 __host__ __device__ inline bool short_for_prefill(int d, int len_q, int len_k) {
     return d <= 64 ? (len_q <= 64 ? len_k <= 1024 : len_q <= 128 && len_k <= 192) : len_q <= 64 && len_k <= 256;
 }

@@ -35,12 +35,12 @@
 // Bound: a tile's chain of products (S, then P V: 1300 to 1600 cycles, Q K^T at 100 instead of 64 per 128 x 128 x 16 since both operands come from
 // shared memory) and softmax (1700 to 2000), which the two query tiles of a CTA run in turn: 3500 cycles per 128 keys of 256 rows; without any
 // softmax the products alone take 3000.  Algorithmic flops: 4 * sum_b(visible (q,k) pairs) * D per head.
-//  * Causal 8192 tokens, float16, 32 heads of 128: 627 -> 566 us by the share of polynomial exponentials and the order of the tiles (none, 3/8 and 1/2
-//    of them were slower); 498 -> 479 (at higher clocks) with the maximum beside the exponentials (kEager).  Two threads a row: 488.
-//  * Portions of 1500 tokens and less over prefixes in pages: 765 us on the mma.sync tiles, 194 with two loading warps, 159 with three that hand a tile
-//    on at once; two threads a row, which halve the corrections: heads of 64 130 -> 126, others equal.
-//  * Window of 4096 tokens with a distance table and a gate: 324 -> 240 us with two threads a row (more of the biases' reads in flight), 216 with tiles on
-//    the diagonal and across the table's end on the path without clamps.
+//  * Causal 8192 tokens, float16, 32 heads of 128: 627 -> 576 us by the share of polynomial exponentials and the order of the tiles (none, 3/8 and 1/2
+//    of them were slower), 575 -> 562 with the maximum beside the exponentials (kEager).
+//  * Portions of 1500 tokens and less over prefixes in pages: 765 us on the mma.sync tiles, 190 with one thread a row and two loading warps, 154 with two threads a
+//    row, which halve the corrections, and three loading warps that hand a tile on at once.
+//  * Window of 4096 tokens with a distance table and a gate: 310 us with one thread a row and clamps on the diagonal and across the table's end, 208 with two (more
+//    of the biases' reads in flight) and none.
 #include "common.cuh"
 #include "mha_params.h"
 
@@ -131,8 +131,8 @@ __device__ __forceinline__ void exp2_poly2(uint64_t x2, float &p0, float &p1) {
     upk2(mul2_ftz(y, scale), p0, p1);
 }
 // P = 2^(s sc - m) of 32 scores as packed 16-bit pairs, and their sum.  MIX: every fourth pair leaves the special-function unit for the FMA
-// pipe (the unit's 16 results a cycle and SM are what bounds the softmax of heads of 64 and 128).  Tiles with masked scores, and kernels whose FMA pipe
-// adds a bias to every score, take the unit for all (4000 tokens in a window of 1024 with a distance table, heads of 128: 357 us, mixed 362).
+// pipe (the unit's 16 results a cycle and SM are what bounds the softmax of heads of 64 and 128).  Tiles with masked scores, and tiles whose FMA pipe
+// adds a bias to every score, take the unit for all.
 // MAX: the scores' maximum is taken beside them.
 template <typename T, bool MIX, bool MAX>
 __device__ __forceinline__ void softmax_chunk(const uint32_t *sv, uint64_t sc2, uint64_t mm2, uint64_t (&ls)[2], uint32_t (&pk)[16], float (&mx)[4]) {
@@ -195,10 +195,10 @@ __device__ __forceinline__ PfSeq pf_seq(const MhaParams &p, int bidb) {
 }
 
 // SPLIT: softmax threads per query row.
-// BIAS: 1 or 2: a bias by query-key distance is added to the scaled scores (MhaParams::dist_bias); 2: the grid goes head by head.  Instantiations of their own, so
+// BIASED: a bias by query-key distance is added to the scaled scores (MhaParams::dist_bias).  Instantiations of their own, so
 // that the unbiased kernel keeps its register allocation.
 // PAGED: keys and values lie in pages behind a block table (MhaParams::block_table).
-template <typename T, int D, int KH, int BIAS, bool PAGED, int SPLIT>
+template <typename T, int D, int KH, bool BIASED, bool PAGED, int SPLIT>
 __global__ void __launch_bounds__(kPfThreads<SPLIT>, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const MhaParams p) {
@@ -214,25 +214,23 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __shared__ uint32_t tmem_base_smem;
     __shared__ int late_s;
     volatile int *late = &late_s;
-    constexpr bool BIASED = BIAS != 0;
     constexpr int N = kPfN / SPLIT;   // keys of a tile per softmax thread
     // Paged steps correct by every new maximum: a row's largest weight is then 1, which rounding to 16 bits leaves alone, as on the tile kernel, whose steps
     // these are (error against 64 bits of bfloat16 portions, queries of 1 and 4 times unit size: 2.08e-3 and 1.73e-3 there, 2.09e-3 and 1.74e-3 here,
     // 2.13e-3 and 2.09e-3 with corrections from 2^8 on; the portions of prompts over prefixes 180 -> 190 us).
     constexpr float kThreshold = PAGED ? 0.f : kRescaleThreshold;
-    // Where most tiles correct nothing.  A thread of half the keys would have to learn of the other's maximum all the same; heads of 64 gain nothing (414 us, 428).
-        constexpr bool kEager = SPLIT == 1 && !PAGED && D == 128;
+    // Where most tiles correct nothing (8192 tokens of 32 heads, float16: 575 us without, 562 so).  A thread of half the keys would have to learn of the other's
+    // maximum all the same; heads of 64 gain nothing (414 us, 428).
+    constexpr bool kEager = SPLIT == 1 && !PAGED && D == 128;
     constexpr int kCorrect = SPLIT == 1 ? 32 : 16;   // columns of O that a correction holds
     __shared__ float bias_s[BIASED ? kPfBiasFront + kPfBiasSmem + kPfBiasBack : 1];
     __shared__ float swap_s[2][kQTiles][2][SPLIT == 2 ? kPfM : 1];         // a row's maximum (at the end: its sum) over either half of the keys
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // Heads, then sequences, then query tiles from the last (causal: heaviest) one down, so that the SMs run out of light tiles together
-    // (head by head, one prompt of 8192 x 32 heads kept them 0.86 busy); head by head where a window makes the tiles alike (BIAS 2: chosen
-    // at compile time, as a choice at run time cost 4 to 7 us a call).  Tiles behind a sequence's end leave at once.
-    constexpr bool kByHead = BIAS == 2;
-    const int m_block = kByHead ? gridDim.x - 1 - blockIdx.x : gridDim.z - 1 - blockIdx.z;
-    const int head = kByHead ? blockIdx.y : blockIdx.x, bidb = kByHead ? blockIdx.z : blockIdx.y;
+    // (head by head, one prompt of 8192 x 32 heads kept them 0.86 busy; under a window of 256, 1024 and 4096 4000 tokens of 32 heads of 128 take 108,
+    // 154 and 242 us head by head, 105, 145 and 206 so).  Tiles behind a sequence's end leave at once.
+    const int m_block = gridDim.z - 1 - blockIdx.z, head = blockIdx.x, bidb = blockIdx.y;
     pdl_wait();
     const PfSeq si = pf_seq(p, bidb);
     if (m_block * kQTiles * kPfM >= si.len_q || (PAGED && p.split_short && short_for_prefill(D, si.len_q, si.len_k))) return;
@@ -743,14 +741,14 @@ bool make_attn_map(CUtensorMap *out, const void *ptr, int d, int heads, int64_t 
     return true;
 }
 
-template <typename T, int D, int KH, int BIAS, bool PAGED = false>
+template <typename T, int D, int KH, bool BIASED, bool PAGED = false>
 bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const MhaParams &p, cudaStream_t stream) {
-    constexpr int SPLIT = BIAS || PAGED ? 2 : 1;
+    constexpr int SPLIT = BIASED || PAGED ? 2 : 1;
     constexpr size_t smem = PfCfg<D, KH>::kSmem;
     static thread_local int attr_dev = -1;
     const DeviceInfo &di = current_device_info();
     if (attr_dev != di.ordinal) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<T, D, KH, BIAS, PAGED, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<T, D, KH, BIASED, PAGED, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem));
         if (e != cudaSuccess) {
             set_status(static_cast<int>(e), "prefill: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -760,9 +758,8 @@ bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtens
     }
     MhaParams pp = p;
     pp.late = late_word();
-    dim3 grid(p.h, p.b, (p.seqlen_q + kQTiles * kPfM - 1) / (kQTiles * kPfM));
-    if (BIAS == 2) grid = dim3(grid.z, grid.x, grid.y);
-    prefill_attn_kernel<T, D, KH, BIAS, PAGED, SPLIT><<<grid, kPfThreads<SPLIT>, smem, stream>>>(mq, mk, mv, pp);
+    const dim3 grid(p.h, p.b, (p.seqlen_q + kQTiles * kPfM - 1) / (kQTiles * kPfM));
+    prefill_attn_kernel<T, D, KH, BIASED, PAGED, SPLIT><<<grid, kPfThreads<SPLIT>, smem, stream>>>(mq, mk, mv, pp);
     note_launch();
     return check_launch("prefill_attn_kernel");
 }
@@ -770,11 +767,7 @@ bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtens
 template <typename T, int D>
 bool launch_prefill(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const MhaParams &p,
                     cudaStream_t stream) {
-    if (!p.dist_bias || p.dist_rows <= 0) return launch_prefill_b<T, D, D / 64, 0>(mq, mk, mv, p, stream);
-    // Window of 1024 over 4000 tokens, heads of 128: 340 us head by head, 360 over all heads, heads of 64 302 / 298; window of 256 266 / 278 and 225 / 229;
-    // window of 4096 342 / 311 and 308 / 265.
-    const bool narrow = p.window_left > 0 && static_cast<int64_t>(p.window_left) * (D == 128 ? 3 : 8) <= p.seqlen_q;
-    return narrow || p.seqlen_q <= kQTiles * kPfM ? launch_prefill_b<T, D, D / 64, 2>(mq, mk, mv, p, stream) : launch_prefill_b<T, D, D / 64, 1>(mq, mk, mv, p, stream);
+    return p.dist_bias && p.dist_rows > 0 ? launch_prefill_b<T, D, D / 64, true>(mq, mk, mv, p, stream) : launch_prefill_b<T, D, D / 64, false>(mq, mk, mv, p, stream);
 }
 
 }  // namespace
@@ -794,8 +787,8 @@ int try_launch_prefill_tc(const MhaParams &p, bool is_bf16, cudaStream_t stream)
     // Pages: where all sequences are short (by the longest portion and the longest sequence), the tile kernel takes the step: from two pairs of a
     // sequence and a head per SM on by short_for_prefill(), below that up to 64 keys (4 sequences of 8 heads of 64 over 32, 64, 96 keys, tiles /
     // prefill kernel: 5 / 7, 6 / 8, 8 / 8 us).  Heads of 64 with six pairs per SM and more: each kernel takes its sequences of a mixed step.  A second
-    // launch costs 10 to 18 us there: one portion of 64 tokens beside 63 decoded ones over 128, 564 and 1064 keys, 32 heads, tiles alone / prefill kernel alone /
-    // both: 58 / 119 / 58, 168 / 220 / 168, 318 / 330 / 338 us.  With heads of 128 it gives back less than that (264 keys: 180 / 211 / 218).
+    // launch costs 10 to 18 us there: one portion of 64 tokens beside 63 decoded ones over 64, 264 and 564 keys, 32 heads, tiles alone / prefill kernel alone:
+    // 30 / 90, 82 / 123, 160 / 171 us.  With heads of 128 it gives back less than that (41 / 107, 152 / 145, 302 / 210).
     const int64_t pairs = p.block_table ? static_cast<int64_t>(p.b) * p.h : 0;
     if (p.block_table && (pairs >= 2 * di.sm_count ? short_for_prefill(p.d, p.seqlen_q, p.seqlen_k) : p.seqlen_k <= 64)) return 0;
     // TMA: 16-byte aligned bases and strides (run_mha already checked pointers and strides % 8)
@@ -821,10 +814,10 @@ int try_launch_prefill_tc(const MhaParams &p, bool is_bf16, cudaStream_t stream)
         MhaParams pp = p;
         pp.split_short = p.d == 64 && p.b > 1 && pairs >= 6 * di.sm_count ? 1 : 0;
         bool done;
-        if (is_bf16) done = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 2, 0, true>(mq, mq, mq, pp, stream)
-                                       : launch_prefill_b<__nv_bfloat16, 64, 1, 0, true>(mq, mq, mq, pp, stream);
-        else done = p.d == 128 ? launch_prefill_b<__half, 128, 2, 0, true>(mq, mq, mq, pp, stream)
-                               : launch_prefill_b<__half, 64, 1, 0, true>(mq, mq, mq, pp, stream);
+        if (is_bf16) done = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 2, false, true>(mq, mq, mq, pp, stream)
+                                       : launch_prefill_b<__nv_bfloat16, 64, 1, false, true>(mq, mq, mq, pp, stream);
+        else done = p.d == 128 ? launch_prefill_b<__half, 128, 2, false, true>(mq, mq, mq, pp, stream)
+                               : launch_prefill_b<__half, 64, 1, false, true>(mq, mq, mq, pp, stream);
         if (done && pp.split_short) done = launch_attention_tile(pp, is_bf16, stream);
         return done ? 1 : -1;
     }
@@ -832,10 +825,10 @@ int try_launch_prefill_tc(const MhaParams &p, bool is_bf16, cudaStream_t stream)
     if (!make_attn_map(&mv, p.v, p.d, p.v_share > 1 ? p.h_k / p.v_share : p.h_k, k_rows, k_b, p.v_hs, p.v_rs, v_bs, is_bf16)) return -1;
     bool ok;
     if (p.d == 128 && d_k <= 64 && is_bf16 && !p.dist_bias)   // shorter query / key heads: one 64-column piece
-        ok = launch_prefill_b<__nv_bfloat16, 128, 1, 0>(mq, mk, mv, p, stream);
+        ok = launch_prefill_b<__nv_bfloat16, 128, 1, false>(mq, mk, mv, p, stream);
     else if ((d_k + 63) / 64 > p.d / 64)   // longer query / key heads than value heads
-        ok = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 3, 0>(mq, mk, mv, p, stream)
-                        : launch_prefill_b<__nv_bfloat16, 64, 2, 0>(mq, mk, mv, p, stream);
+        ok = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 3, false>(mq, mk, mv, p, stream)
+                        : launch_prefill_b<__nv_bfloat16, 64, 2, false>(mq, mk, mv, p, stream);
     else if (is_bf16) ok = p.d == 128 ? launch_prefill<__nv_bfloat16, 128>(mq, mk, mv, p, stream)
                                  : launch_prefill<__nv_bfloat16, 64>(mq, mk, mv, p, stream);
     else ok = p.d == 128 ? launch_prefill<__half, 128>(mq, mk, mv, p, stream)
