@@ -18,13 +18,11 @@ namespace {
 using namespace hybrid;
 
 // log(sigmoid(z)) = min(z, 0) - log(1 + x) with x = exp(-|z|) in [0, 1], without a branch, so that a lane's tokens overlap:
-// log(1 + x) = 2 artanh(s) = 2 s (1 + s^2 / 3 + s^4 / 5 + ...), s = x / (2 + x) <= 1/3; the terms from s^16 / 17 on are below 2^-29.
+// log(1 + x) = 2 artanh(s) = 2 s (1 + s^2 / 3 + s^4 / 5 + ...), s = x / (2 + x) <= 1/3; the terms from s^16 / 17 on are below 2^-29.  The decay that comes of it is
+// off by 5.2e-7 at most (tau = 1, z in [-85, 85]; 1.3e-7 with tau = 16), as it is with log1pf.  With a rounded division 4000 tokens of 32 heads take 484 us for 418.
 __device__ __forceinline__ float log_sigmoid(float z) {
-    const float x = expf(-fabsf(z)), d = 2.f + x;
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    float s = x * r;
-    s = fmaf(fmaf(-d, s, x), r, s);
+    const float x = expf(-fabsf(z));
+    float s = __fdividef(x, 2.f + x);
     const float y = s * s;
     float p = 1.f / 15.f;
     p = fmaf(p, y, 1.f / 13.f);

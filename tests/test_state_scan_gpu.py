@@ -130,3 +130,23 @@ def test_short_steps_give_the_bits_of_long_ones(rule, D, V, dtype):
     whole = states(1)
     a, b = step(rows, whole, [0], [0, n], [0]), step([t[:1] for t in rows], fresh, [0], [0, 1], [0])
     assert torch.equal(a[:1], b)
+
+
+def test_gla_decay_against_float64():
+    """One token with k = 0 on a state of ones: the state that is left is the decay, sigmoid(z)^(1 / tau)."""
+    from atoma_infer_b200 import hybrid_ops as ho
+
+    H, D, V = 64, 64, 64
+    z = torch.linspace(-85.0, 85.0, H * D, device=DEV)
+    z[:7] = torch.tensor([0.0, -0.0, 1e-6, -1e-6, 1e-30, -17.3, 17.3], device=DEV)
+    zeros = lambda n: torch.zeros((1, n), device=DEV)
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    for tau in (1.0, 16.0):
+        state = torch.ones((1, H * D * V), device=DEV)
+        ho.gla_scan(zeros(H * D), zeros(H * D), zeros(H * V), z[None].contiguous(), torch.zeros(H * D, device=DEV), tau, 1.0, state, i32(0), i32(0, 1), i32(5), H, D, V)
+        log = torch.nn.functional.logsigmoid(z.double()) / tau
+        got, want = state.reshape(H * D, V)[:, 0].double(), torch.exp(log)
+        # the logarithm and its quotient by tau are rounded to float32 each, its term log(1 + x) <= log 2 is within three units, the exponential within two
+        bound = log.abs() * 2.0 ** -23 + 2.1 * 2.0 ** -24 / tau + 2.0 ** -22
+        assert bool(((got / want - 1.0).abs() <= bound).all())
+        assert torch.equal(state.reshape(H * D, V), state.reshape(H * D, V)[:, :1].expand(-1, V))
