@@ -45,7 +45,7 @@ def main():
         L.atoma_debug_step_prefetch(0, 32)
         L.atoma_debug_step_fusion(0)
         L.atoma_debug_skinny_mode(0, 1)
-        if v == "dbuf":             # two accumulator buffers even for single-tile CTAs (the round-2 default before)
+        if v == "dbuf":             # two accumulator buffers even for single-tile CTAs (an earlier default)
             L.atoma_debug_skinny_mode(8, 1)
         elif v.startswith("late"):    # late<N>: GEMMs release their dependents N stages before their last weight load
             L.atoma_debug_skinny_mode(int(v[4:]) << 8, 1)

@@ -79,7 +79,7 @@ def test_library_matches_the_source_tree():
 
 def test_ctypes_struct_mirrors_have_the_library_layout():
     """include/atoma_llama.h's structs as the library was compiled against the ctypes mirrors in _lib.py (the
-    vocab-parallel fields were appended to atoma_llama_model in round 2: a stale mirror would silently misread)."""
+    vocab-parallel fields were appended to atoma_llama_model later: a stale mirror would silently misread)."""
     lib = _lib.load()
     assert lib.atoma_llama_abi_sizeof(0) == C.sizeof(_lib.LlamaLayer)
     assert lib.atoma_llama_abi_sizeof(1) == C.sizeof(_lib.LlamaModel)

@@ -490,7 +490,7 @@ def test_peaky_softmax_range():
 
 def test_sliding_window_and_softcap_are_refused_not_silently_ignored():
     """The reference compiles LOCAL and SOFTCAP out (static_switch.h:7-11) and computes full attention for
-    them; round 1 did the same silently.  A window that would mask something, or a soft cap, now raises."""
+    them; so did the first form of this library, silently.  A window that would mask something, or a soft cap, now raises."""
     q = randn_t((1, 64, 4, 64), 1, torch.bfloat16, DEV)
     k = randn_t((1, 64, 2, 64), 2, torch.bfloat16, DEV)
     v = randn_t((1, 64, 2, 64), 3, torch.bfloat16, DEV)

@@ -68,7 +68,7 @@ def test_committed_bench_lines_follow_the_contract():
     for name in ("r01_bench_reference.json", "r02_bench_reference.json"):
         ref = json.loads((ROOT / "profiles" / name).read_text())
         assert ref["impl"] == "reference" and ref["e2e"]["h2d_bytes_per_step"] == 0
-    # round 2: the metric is BASELINE.json's, without a scope qualifier, and the step holds no library kernel
+    # the metric is the headline one, without a scope qualifier, and the step holds no library kernel
     ours = json.loads((ROOT / "profiles" / "r02_bench_ours.json").read_text())
     assert ours["metric"] == json.loads((ROOT / "BASELINE.json").read_text()).get("metric", ours["metric"]) or "(" not in ours["metric"]
     assert ours["gpu_launches"] == ours["launches_per_step"] * ours["steps"] and "cuBLAS" not in ours["config"]["gemm"]
@@ -85,7 +85,7 @@ def test_tp_roofline_is_the_slower_of_hbm_and_nvlink():
     # a step that streams almost nothing per rank is bound by the link
     r = bench.tp_roofline(1.0, 1_000_000, 6542.4, 8, payload, ars, fused_push=False)
     assert r["bound"] == "nvlink" and r["target_ms"] == r["nvlink_ms"] == r["nvlink_ms_as_sent"]
-    # derived from the committed round-2 lines (measured step times): the strong-scaling curve against this roofline
+    # derived from the committed lines (measured step times): the strong-scaling curve against this roofline
     for n in (2, 4, 8):
         d = json.loads((ROOT / "profiles" / f"r02_bench_tp{n}_ours.json").read_text())
         c = d["config"]

@@ -146,7 +146,7 @@ def test_one_copy_ships_the_step_to_the_gpu():
 
 
 def test_refresh_never_reallocates_the_staging_image():
-    """Round-1 advisor (medium): refresh() used to swap the host / device images when a step outgrew them,
+    """refresh() used to swap the host / device images when a step outgrew them,
     leaving views handed out earlier (and graphs captured over them) pointing at a dead image.  Now only
     prepare_input_tensors() may grow (new views, `generation` bumped); refresh() raises."""
     from atoma_infer_b200.ops import AtomaError

@@ -113,7 +113,7 @@ def test_gemm_is_deterministic_and_graph_capturable():
 
 
 def test_stream_k_gemm_counters_survive_interleaved_shapes():
-    """Regression (round-1 advisor, high): the stream-K kernel's arrival counters and fp32 partials shared
+    """Regression: the stream-K kernel's arrival counters and fp32 partials shared
     one workspace whose split moved with the shape, so a launch with more than 64 tiles after a small one
     found partials where it expected zeroed counters and silently skipped its split reductions."""
     L = _lib.lib()
@@ -168,7 +168,7 @@ def test_qkv_rope_cache_fused_is_bit_identical_to_unfused_and_matches_oracle(T, 
     kv2 = kv1.clone()
     fused = ops.qkv_rope_cache(x, w, H, HK, D, pos, cos, sin, kv1[0], kv1[1], slots)
     # unfused: plain projection (in the same 128-row passes: beyond 128 rows gemm_tn switches to the stream-K
-    # kernel, whose accumulation order differs), then the RoPE + cache-write kernel of round 1
+    # kernel, whose accumulation order differs), then the RoPE + cache-write kernel
     qkv = torch.cat([ops.gemm_tn(x[t0:t0 + 128], w) for t0 in range(0, T, 128)], dim=0)
     plain = qkv.clone()
     nq, nkv = H * D, HK * D
