@@ -368,8 +368,9 @@ __global__ void __launch_bounds__(256) qkv_headnorm_rope_cache_kernel(const atom
 // L lanes some of them, the others by shuffles) and issues the loads of up to four rounds before it uses the first; no shared memory, no barrier.
 // Values that only move are one run of bytes.
 // Bound: HBM.  8192 tokens of 32 + 16 heads of 128, 201 MB: a warp per head, element by element through shared memory 147 us; a CTA per token
-// 65.6 (0.73 of the issue slots: 47 M instructions, weights read and addresses formed per head, angles behind a barrier); this 46.1 (20 M); 8000 tokens of
-// 32 + 16 heads of 64 51.3 and 29.3.  24 warps an SM without spilled registers 51.2, 40 with loads of three heads 71.8.
+// 61.5 (0.73 of the issue slots: 47 M instructions, weights read and addresses formed per head, angles behind a barrier); this 41.0 (20 M); 3000 tokens of
+// 32 + 16 heads of 64 24.6 and 17.0.  At 32 warps an SM a lane's 64 registers spill 8 to 88 bytes; 24 warps without spills took 51.2 us where this took 46.1 (at
+// lower clocks), 40 with loads of three heads 71.8.
 constexpr int kQkvHeads = 4;
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
     uint64_t r;
@@ -747,8 +748,8 @@ bool hyb_qkv_headnorm_rope_cache(const atoma_qkv_rope_args &a, cudaStream_t stre
     if (pieces) {
         const int64_t n = std::max(a.dim, a.vdim), groups = n <= 64 ? 4 : n <= 128 ? 2 : 1;
         const int64_t heads = a.H + (a.slot_mapping ? a.G + (a.bias || (a.v_freq && a.v_pairs > 0) ? (a.v_heads > 0 ? a.v_heads : a.G) : 0) : 0), rounds = (heads + groups - 1) / groups;
-        // shares of a token: so many that the warps fill the SMs once, and no more than there are rounds (twice as many: 8192 tokens 47.3 us, 1000 17.2; once:
-        // 46.1 and 15.4)
+        // shares of a token: so many that the warps fill the SMs once, and no more than there are rounds (twice as many: 8192 tokens 47.3 us, 1000 17.2; once,
+        // in the same run: 46.1 and 15.4)
         const int64_t want = (kQkvResident * current_device_info().sm_count + a.T - 1) / a.T;
         const int parts = static_cast<int>(std::max<int64_t>(1, std::min(rounds, want)));
         const dim3 grid(static_cast<unsigned>((a.T * parts + kQkvWarps - 1) / kQkvWarps)), block(32 * kQkvWarps);

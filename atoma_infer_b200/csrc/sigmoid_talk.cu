@@ -17,8 +17,9 @@
 // A tile of 2048 tokens, 32 heads of 64 on 8, takes 14000 cycles: scores and weights 6000 (four results of the special-function unit per weight are 4100 of them),
 // the mix 5000 (3100 of the tensor pipe), values 2000.  With 27000: every copy waited for its own block-table entry (5000), a branch per weight kept
 // their chains from overlapping, quotients and exponentials took denormal numbers into account, and registers spilled.
-// 2048 tokens, 32 heads of 64 on 8: 1218 us on the CUDA-core mix (hybrid_attention.cu), 511 with those, 286 here; 2000 tokens of 16 heads 328 and 169.  A prompt of
-// a few row blocks and few keys stays as fast as on CUDA cores (64 tokens: 31 us): all heads wait for each other in one CTA.
+// 2048 tokens, 32 heads of 64 on 8: 1218 us on the CUDA-core mix (hybrid_attention.cu), 507 with those, 283 here; 2000 tokens of 16 heads 328 and 169.  Prompts of up to
+// some 40 tokens are slower than on CUDA cores, since all heads wait for each other in one CTA (33 tokens of 16 and 32 heads 15.9 and 24.2 us, there 14.3 and 19.1;
+// 64 tokens 16.4 and 26.6, there 22.6 and 32.8); they stay here, so that a position's bits do not follow the step.
 #include "common.cuh"
 #include "hybrid_common.cuh"
 
