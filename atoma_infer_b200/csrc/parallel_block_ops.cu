@@ -748,9 +748,10 @@ bool hyb_qkv_headnorm_rope_cache(const atoma_qkv_rope_args &a, cudaStream_t stre
     if (pieces) {
         const int64_t n = std::max(a.dim, a.vdim), groups = n <= 64 ? 4 : n <= 128 ? 2 : 1;
         const int64_t heads = a.H + (a.slot_mapping ? a.G + (a.bias || (a.v_freq && a.v_pairs > 0) ? (a.v_heads > 0 ? a.v_heads : a.G) : 0) : 0), rounds = (heads + groups - 1) / groups;
-        // shares of a token: so many that the warps fill the SMs once, and no more than there are rounds (twice as many: 8192 tokens 47.3 us, 1000 17.2; once,
-        // in the same run: 46.1 and 15.4)
-        const int64_t want = (kQkvResident * current_device_info().sm_count + a.T - 1) / a.T;
+        // shares of a token: so many that the warps stay within the SMs once, and no more than there are rounds (a share more, which starts a second wave / this, us:
+        // 1000 tokens of 32 + 32 + 32 heads, values of 128 rotated, 17.5 / 14.5, a CTA per token 16.4; 1700 tokens of 32 + 16 of 128, half of them turned, 18.4 / 16.5, 16.4;
+        // 2200 tokens of 32 + 16 of 128 17.8 / 14.5; twice as many shares, 8192 tokens, 47.3 where once took 46.1)
+        const int64_t want = kQkvResident * current_device_info().sm_count / a.T;
         const int parts = static_cast<int>(std::max<int64_t>(1, std::min(rounds, want)));
         const dim3 grid(static_cast<unsigned>((a.T * parts + kQkvWarps - 1) / kQkvWarps)), block(32 * kQkvWarps);
         const bool whole = a.dim == 256 / groups && a.qk_freq && 2 * a.rot_pairs == a.dim;
