@@ -465,6 +465,7 @@ SIGNATURES = {
     "atoma_group_rmsnorm_rows": (None, [C.c_void_p] * 3 + [C.c_float, C.c_int64, C.c_void_p, C.c_int64, C.c_int64, C.c_float, C.c_uint32,
                                         C.c_void_p]),
     "atoma_gated_residual_norm": (None, [C.POINTER(GatedResidualArgs), C.c_void_p]),
+    "atoma_expert_rows_sum": (None, [C.c_void_p] * 3 + [C.c_int64] * 3 + [C.c_uint32, C.c_void_p]),
     "atoma_side_gate": (None, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_int64, C.c_int64,
                                C.c_int64, C.c_uint32, C.c_void_p]),
     "atoma_unitnorm_add_norm": (None, [C.c_void_p] * 5 + [C.c_int64] * 3 + [C.c_float, C.c_float, C.c_uint32, C.c_void_p]),

@@ -267,11 +267,8 @@ def moe_experts(h, top_expert, top_weight, w_gate_up, w_down, limit, alpha, up_s
     eo, pr = C.c_void_p(), C.c_void_p()
     _lib.lib().atoma_moe_experts(C.byref(a), C.byref(eo), C.byref(pr), _s())
     _check()
-    x = torch.zeros((T, W), dtype=torch.float32, device=h.device)
-    ga = _lib.GatedResidualArgs()
-    ga.expert_out, ga.pair_row, ga.top, ga.x = eo.value, pr.value, top, _p(x)
-    ga.T, ga.width, ga.groups, ga.eps, ga.dtype = T, W, 1, 1e-5, code
-    _lib.lib().atoma_gated_residual_norm(C.byref(ga), _s())
+    x = torch.empty((T, W), dtype=torch.float32, device=h.device)
+    _lib.lib().atoma_expert_rows_sum(eo, pr, _p(x), T, top, W, code, _s())
     _check()
     x._workspace = ws             # the kernels may still be running: the workspace lives as long as the result
     return x

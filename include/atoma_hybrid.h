@@ -191,6 +191,11 @@ typedef struct atoma_gated_residual_args {
 } atoma_gated_residual_args;
 void atoma_gated_residual_norm(const atoma_gated_residual_args *args, atoma_stream_t stream);
 
+/* out[t, c] = sum_{k < top} rows[pair_row[t top + k], c] in float32, in the order k = 0 .. top - 1: the same sum without a residual.
+ * rows [.., width] in `dtype`, out [T, width] float32. */
+void atoma_expert_rows_sum(const void *rows, const int32_t *pair_row, float *out, int64_t T, int64_t top, int64_t width, uint32_t dtype,
+                           atoma_stream_t stream);
+
 /* Token side input, gate part: out[t, j] = gelu_tanh(a[t, j]) * side_table[tokens[t], part * dim + j], j < dim.
  * a (row stride ld_a) and out [T, dim] in `dtype`; side_table [vocab, table_width] in `dtype`. */
 void atoma_side_gate(const void *a, int64_t ld_a, const uint32_t *tokens, const void *side_table, int64_t table_width, int64_t part,
