@@ -43,7 +43,7 @@ const DeviceInfo &current_device_info();
 // Library-owned scratch, one per (device, stream, tag); grows monotonically, zero-initialised
 // when (re)allocated.  Used for the decode kernel's split partials + arrival counters and for the
 // device copy of a swap mapping.
-enum : int { kWorkspaceDecode = 0, kWorkspaceSwapMap = 1, kWorkspaceGemm = 2, kWorkspaceGemmCounters = 3, kWorkspaceSkinnyTail = 4, kWorkspaceHybridAttn = 5, kWorkspaceMoeRoute = 6, kWorkspaceLatentExpand = 7, kWorkspaceTags = 8 };
+enum : int { kWorkspaceDecode = 0, kWorkspaceSwapMap = 1, kWorkspaceGemm = 2, kWorkspaceGemmCounters = 3, kWorkspaceSkinnyTail = 4, kWorkspaceHybridAttn = 5, kWorkspaceMoeRoute = 6, kWorkspaceLatentExpand = 7, kWorkspacePrefillKeys = 8, kWorkspaceTags = 9 };
 void *get_workspace(cudaStream_t stream, size_t bytes, int tag);
 // The same for a caller that can do without: nullptr and no error where there is none (no memory, or a stream being captured before the first call).
 void *try_workspace(cudaStream_t stream, size_t bytes, int tag);

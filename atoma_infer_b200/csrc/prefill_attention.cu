@@ -28,7 +28,8 @@
 //    raised that the host can read (atoma_prefill_timeouts, atoma_kernel_timeouts); the CTA's outputs mean nothing then.
 //
 //  * paged keys and values (PAGED): three warps look the pages up and copy rows of 16-byte pieces with cp.async into the same
-//    swizzled tiles (a page's rows of one head are strided: no box of a tensor map covers a tile of pages in any order);
+//    swizzled tiles (a page's rows of one head are strided: no box of a tensor map covers a tile of pages in any order), or, in long steps, all keys and values are
+//    gathered first (try_launch_gathered);
 //  * a quarter of the exponentials is a polynomial on the FMA pipe (exp2_poly2), and all heads' heaviest tiles start first;
 //  * an output gate is applied in the epilogue (fetched before the last P.V is waited for), so no pass over the outputs follows.
 //
@@ -45,6 +46,7 @@
 #include "mha_params.h"
 
 #include <cstring>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -180,9 +182,10 @@ __device__ __forceinline__ PfSeq pf_seq(const MhaParams &p, int bidb) {
     // reference block_info.h:14-36
     s.q_start = p.cu_q ? p.cu_q[bidb] : -1;
     s.len_q = p.cu_q ? p.cu_q[bidb + 1] - s.q_start : p.seqlen_q;
-    const int k_start = (p.cu_k && p.k_cumulative) ? p.cu_k[bidb] : -1;
-    const int len_k_cache = p.cu_k ? (p.k_cumulative ? p.cu_k[bidb + 1] - k_start : p.cu_k[bidb]) : p.seqlen_k;
+    const int k_first = (p.cu_k && p.k_cumulative) ? p.cu_k[bidb] : -1, k_start = p.k_batched ? -1 : k_first;
+    const int len_k_cache = p.cu_k ? (p.k_cumulative ? p.cu_k[bidb + 1] - k_first : p.cu_k[bidb]) : p.seqlen_k;
     s.len_k = p.seqused_k ? p.seqused_k[bidb] : len_k_cache;
+    if (p.k_batched) s.len_k = min(s.len_k, p.seqlen_k);   // the rows that there are
     s.q_off = s.q_start < 0 ? bidb * p.q_bs : static_cast<int64_t>(s.q_start) * p.q_rs;
     s.o_off = s.q_start < 0 ? bidb * p.o_bs : static_cast<int64_t>(s.q_start) * p.o_rs;
     s.k_off = k_start < 0 ? bidb * p.k_bs : static_cast<int64_t>(k_start) * p.k_rs;
@@ -198,7 +201,8 @@ __device__ __forceinline__ PfSeq pf_seq(const MhaParams &p, int bidb) {
 // BIASED: a bias by query-key distance is added to the scaled scores (MhaParams::dist_bias).  Instantiations of their own, so
 // that the unbiased kernel keeps its register allocation.
 // PAGED: keys and values lie in pages behind a block table (MhaParams::block_table).
-template <typename T, int D, int KH, bool BIASED, bool PAGED, int SPLIT>
+// EXACT: the results of a paged step, to the bit, where its keys and values have been gathered (paged_rows_kernel).
+template <typename T, int D, int KH, bool BIASED, bool PAGED, int SPLIT, bool EXACT>
 __global__ void __launch_bounds__(kPfThreads<SPLIT>, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const MhaParams p) {
@@ -218,10 +222,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // Paged steps correct by every new maximum: a row's largest weight is then 1, which rounding to 16 bits leaves alone, as on the tile kernel, whose steps
     // these are (error against 64 bits of bfloat16 portions, queries of 1 and 4 times unit size: 2.08e-3 and 1.73e-3 there, 2.09e-3 and 1.74e-3 here,
     // 2.13e-3 and 2.09e-3 with corrections from 2^8 on; the portions of prompts over prefixes 180 -> 190 us).
-    constexpr float kThreshold = PAGED ? 0.f : kRescaleThreshold;
+    constexpr float kThreshold = PAGED || EXACT ? 0.f : kRescaleThreshold;
     // Where most tiles correct nothing (8192 tokens of 32 heads, float16: 575 us without, 562 so).  A thread of half the keys would have to learn of the other's
     // maximum all the same; heads of 64 gain nothing (414 us, 428).
-    constexpr bool kEager = SPLIT == 1 && !PAGED && D == 128;
+    constexpr bool kEager = SPLIT == 1 && !PAGED && !EXACT && D == 128;
     constexpr int kCorrect = SPLIT == 1 ? 32 : 16;   // columns of O that a correction holds
     __shared__ float bias_s[BIASED ? kPfBiasFront + kPfBiasSmem + kPfBiasBack : 1];
     __shared__ float swap_s[2][kQTiles][2][SPLIT == 2 ? kPfM : 1];         // a row's maximum (at the end: its sum) over either half of the keys
@@ -518,6 +522,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         };
         if (n_tiles > 0) {
             float m_ref = -INFINITY, l_run = 0.f;
+            [[maybe_unused]] float l_high = 0.f;   // EXACT: the second half of the keys apart, as two threads sum them
             if (p.sink) {   // the sink is one more term of the denominator: the running state starts from it
                 m_ref = p.sink[head] * 1.4426950408889634f;
                 l_run = half ? 0.f : 1.f;
@@ -601,6 +606,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         const float alpha = need ? (m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - m_tile)) : 1.f;
                         if (need) m_ref = m_tile;
                         l_run *= alpha;
+                        if (EXACT) l_high *= alpha;
                         if (j > n_lo) {
                             // O of this row lives in tensor memory: wait until P.V of the previous tile has
                             // been accumulated, rescale, write back.  Rare after the first tiles.
@@ -623,7 +629,17 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
                     const float off = BIASED ? far_bias - m_use : -m_use;
                     const uint64_t mm2 = pk2(off, off);
-                    if (masked || !far) softmax_scores<T, N, false, false>(sv_, sc2, mm2, l_tile, mx4, tmem_p);
+                    if constexpr (EXACT) {   // half by half, each by its own masks, as two threads a row have it
+                        static_assert(SPLIT == 1 && !BIASED, "one thread a row");
+                        constexpr int M = N / 2;
+                        const bool diag0 = p.is_causal && (col0 + M - 1 > m0t + shift), masked0 = col0 + M > len_k || diag0 || low, masked1 = tail || diag || (window > 0 && col0 + M < m0t + kPfM + shift - window);
+                        float l_half = 0.f;
+                        if (masked0) softmax_scores<T, M, false, false>(sv_, sc2, mm2, l_tile, mx4, tmem_p);
+                        else softmax_scores<T, M, true, false>(sv_, sc2, mm2, l_tile, mx4, tmem_p);
+                        if (masked1) softmax_scores<T, M, false, false>(sv_ + M, sc2, mm2, l_half, mx4, tmem_p + M / 2);
+                        else softmax_scores<T, M, true, false>(sv_ + M, sc2, mm2, l_half, mx4, tmem_p + M / 2);
+                        l_high += l_half;
+                    } else if (masked || !far) softmax_scores<T, N, false, false>(sv_, sc2, mm2, l_tile, mx4, tmem_p);
                     else softmax_scores<T, N, true, false>(sv_, sc2, mm2, l_tile, mx4, tmem_p);
                 }
                 l_run += l_tile;
@@ -638,6 +654,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 const float other = swap(n_tiles - n_lo, l_run);
                 l_run = half ? other + l_run : l_run + other;
             }
+            if (EXACT) l_run += l_high;
             // this half's part of the row's gate, 32 columns at a time: the first are under way while the last products run
             const T *gg = gated ? static_cast<const T *>(p.gate) + static_cast<int64_t>(si.q_row0 + grow) * p.gate_rs + static_cast<int64_t>(head) * D + half * (D / SPLIT) : nullptr;
             uint4 gv[4];
@@ -698,6 +715,26 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
 }
 
+// Keys and values of a paged step into rows of their own: sequence b's from b * pitch on, all heads of a row together.  One warp per key; bound by the bytes (16-byte pieces).
+constexpr int kPfGatherWarps = 8;
+__global__ void __launch_bounds__(32 * kPfGatherWarps) paged_rows_kernel(const MhaParams p, uint4 *__restrict__ k_out, uint4 *__restrict__ v_out, int pitch) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int b = blockIdx.y, key = blockIdx.x * kPfGatherWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const PfSeq si = pf_seq(p, b);
+    if (key >= min(si.len_k, pitch) || si.len_q <= 0) return;
+    const int pg = key / p.page, per = p.d / 8, pieces = p.h_k * per;
+    const int64_t page = p.block_table[static_cast<int64_t>(b) * p.bt_bs + pg], in = key - pg * p.page, row = (static_cast<int64_t>(b) * pitch + key) * pieces;
+    const uint16_t *k = static_cast<const uint16_t *>(p.k) + page * p.k_bs + in * p.k_rs, *v = static_cast<const uint16_t *>(p.v) + page * p.v_bs + in * p.v_rs;
+#pragma unroll 4
+    for (int c = lane; c < pieces; c += 32) {
+        const int g = c / per, at = (c - g * per) * 8;
+        const uint4 kv = *reinterpret_cast<const uint4 *>(k + g * p.k_hs + at), vv = *reinterpret_cast<const uint4 *>(v + g * p.v_hs + at);
+        k_out[row + c] = kv;
+        v_out[row + c] = vv;
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 struct Map4Key {
     const void *ptr;
@@ -741,14 +778,14 @@ bool make_attn_map(CUtensorMap *out, const void *ptr, int d, int heads, int64_t 
     return true;
 }
 
-template <typename T, int D, int KH, bool BIASED, bool PAGED = false>
+template <typename T, int D, int KH, bool BIASED, bool PAGED = false, bool EXACT = false>
 bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const MhaParams &p, cudaStream_t stream) {
     constexpr int SPLIT = BIASED || PAGED ? 2 : 1;
     constexpr size_t smem = PfCfg<D, KH>::kSmem;
     static thread_local int attr_dev = -1;
     const DeviceInfo &di = current_device_info();
     if (attr_dev != di.ordinal) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<T, D, KH, BIASED, PAGED, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(prefill_attn_kernel<T, D, KH, BIASED, PAGED, SPLIT, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem));
         if (e != cudaSuccess) {
             set_status(static_cast<int>(e), "prefill: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -759,7 +796,7 @@ bool launch_prefill_b(const CUtensorMap &mq, const CUtensorMap &mk, const CUtens
     MhaParams pp = p;
     pp.late = late_word();
     const dim3 grid(p.h, p.b, (p.seqlen_q + kQTiles * kPfM - 1) / (kQTiles * kPfM));
-    prefill_attn_kernel<T, D, KH, BIASED, PAGED, SPLIT><<<grid, kPfThreads<SPLIT>, smem, stream>>>(mq, mk, mv, pp);
+    prefill_attn_kernel<T, D, KH, BIASED, PAGED, SPLIT, EXACT><<<grid, kPfThreads<SPLIT>, smem, stream>>>(mq, mk, mv, pp);
     note_launch();
     return check_launch("prefill_attn_kernel");
 }
@@ -768,6 +805,41 @@ template <typename T, int D>
 bool launch_prefill(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const MhaParams &p,
                     cudaStream_t stream) {
     return p.dist_bias && p.dist_rows > 0 ? launch_prefill_b<T, D, D / 64, true>(mq, mk, mv, p, stream) : launch_prefill_b<T, D, D / 64, false>(mq, mk, mv, p, stream);
+}
+
+// A paged step whose keys and values are gathered first, so that the kernel for contiguous ones serves it, with the same bits: 1 = launched, 0 = not taken, -1 = error.
+// A tile of keys that TMA copies and one thread a row works on takes 4700 cycles, one that three warps copy and two threads a row work on 5100; the gather reads and
+// writes every key once (8 us for 5100 keys of 8 heads).  32 query heads of 128 on 8, pages / rows, us: 2048, 1500 and 531 tokens behind 0, 1003 and 37 155 / 146, 3000
+// tokens 124 / 119, 1024 behind 8000 203 / 194, 512 behind 4000 108 / 104, 256 behind 3000 80 / 78; 1024 tokens 32.8 / 33.8, 129 behind 1000 34.8 / 39.9: what is
+// short pays for the second launch.  Heads of 64 gain nothing (123 / 123, 99 / 102).
+constexpr int64_t kPfGatherBytes = 256ll << 20;   // of scratch at most; longer steps stay with the pages
+constexpr int kPfGatherQ = 256, kPfGatherK = 2048;
+int try_launch_gathered(const MhaParams &p, bool is_bf16, const CUtensorMap &mq, cudaStream_t stream) {
+    const int64_t row = static_cast<int64_t>(p.h_k) * p.d, bytes = static_cast<int64_t>(p.b) * p.seqlen_k * row * 2;
+    if (p.d != 128 || p.seqlen_q < kPfGatherQ || p.seqlen_k < kPfGatherK || 2 * bytes > kPfGatherBytes) return 0;
+    // The copy and the kernel that reads it are enqueued together: another thread may use this stream and its scratch.
+    static std::mutex together;
+    std::lock_guard<std::mutex> lock(together);
+    unsigned char *space = static_cast<unsigned char *>(try_workspace(stream, static_cast<size_t>(2 * bytes), kWorkspacePrefillKeys));
+    if (!space) return 0;
+    MhaParams pp = p;
+    pp.block_table = nullptr;
+    pp.k = space, pp.v = space + bytes;
+    pp.k_hs = pp.v_hs = p.d, pp.k_rs = pp.v_rs = row, pp.k_bs = pp.v_bs = p.seqlen_k * row;
+    pp.k_batched = 1;
+    CUtensorMap mk, mv;
+    if (!make_attn_map(&mk, pp.k, p.d, p.h_k, p.seqlen_k, p.b, pp.k_hs, pp.k_rs, pp.k_bs, is_bf16)) return -1;
+    if (!make_attn_map(&mv, pp.v, p.d, p.h_k, p.seqlen_k, p.b, pp.v_hs, pp.v_rs, pp.v_bs, is_bf16)) return -1;
+    const dim3 grid(static_cast<unsigned>((p.seqlen_k + kPfGatherWarps - 1) / kPfGatherWarps), static_cast<unsigned>(p.b));
+    const cudaError_t e = launch_ex(paged_rows_kernel, grid, dim3(32 * kPfGatherWarps), 0, stream, p, reinterpret_cast<uint4 *>(space), reinterpret_cast<uint4 *>(space + bytes), p.seqlen_k);
+    note_launch();
+    if (e != cudaSuccess) {
+        set_status(static_cast<int>(e), "paged_rows_kernel: %s", cudaGetErrorString(e));
+        return -1;
+    }
+    const bool done = is_bf16 ? launch_prefill_b<__nv_bfloat16, 128, 2, false, false, true>(mq, mk, mv, pp, stream)
+                              : launch_prefill_b<__half, 128, 2, false, false, true>(mq, mk, mv, pp, stream);
+    return done ? 1 : -1;
 }
 
 }  // namespace
@@ -810,10 +882,12 @@ int try_launch_prefill_tc(const MhaParams &p, bool is_bf16, cudaStream_t stream)
     const int64_t v_bs = (k_varlen || p.b == 1 || p.v_bs == 0) ? p.v_rs : p.v_bs;
     const int d_k = p.d_k > 0 ? p.d_k : p.d;
     if (!make_attn_map(&mq, p.q, d_k, p.h, q_rows, q_b, p.q_hs, p.q_rs, q_bs, is_bf16)) return -1;
-    if (p.block_table) {   // keys and values are not read through maps
+    if (p.block_table) {
         MhaParams pp = p;
         pp.split_short = p.d == 64 && p.b > 1 && pairs >= 6 * di.sm_count ? 1 : 0;
         bool done;
+        const int gathered = try_launch_gathered(pp, is_bf16, mq, stream);
+        if (gathered != 0) return gathered;
         if (is_bf16) done = p.d == 128 ? launch_prefill_b<__nv_bfloat16, 128, 2, false, true>(mq, mq, mq, pp, stream)
                                        : launch_prefill_b<__nv_bfloat16, 64, 1, false, true>(mq, mq, mq, pp, stream);
         else done = p.d == 128 ? launch_prefill_b<__half, 128, 2, false, true>(mq, mq, mq, pp, stream)

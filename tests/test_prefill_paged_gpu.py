@@ -50,6 +50,36 @@ def test_same_bits_whatever_the_pages(D, dtype, H, G, page, news, contexts):
     assert hybrid_ops.prefill_timeouts() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,G,page,news,contexts", [
+    (4, 2, 16, (256,), (1792,)),                        # the shortest step that is gathered
+    (3, 1, 48, (300, 1, 33), (2100, 0, 1991)),          # pages that straddle tiles, a decoded token, a sequence shorter than a tile
+    (2, 2, 256, (1000, 640), (1100, 1408)),
+])
+def test_gathered_steps_give_the_bits_of_pages(dtype, H, G, page, news, contexts):
+    """A bound on the longest sequence that would take too much scratch leaves the step on its pages; rows behind a sequence's end and unused pages hold NaN."""
+    D, lens = 128, [n + c for n, c in zip(news, contexts)]
+    q = randn_t((sum(news), H, D), 1, dtype, DEV)
+    each = [-(-n // page) for n in lens]
+    pool = torch.randperm(sum(each) + 2, generator=torch.Generator().manual_seed(4)).to(torch.int32)
+    kc, vc = (torch.full((sum(each) + 2, page, G, D), float("nan"), dtype=dtype, device=DEV) for _ in range(2))
+    k, v = randn_t((sum(lens), G, D), 2, dtype, DEV), randn_t((sum(lens), G, D), 3, dtype, DEV)
+    table, used, row = torch.zeros((len(lens), max(each)), dtype=torch.int32), 0, 0
+    for b, n in enumerate(lens):
+        table[b, :each[b]] = pool[used:used + each[b]]
+        at = torch.arange(n)
+        slot = (table[b].long()[at // page] * page + at % page).to(DEV)
+        kc.view(-1, G, D)[slot], vc.view(-1, G, D)[slot] = k[row:row + n], v[row:row + n]
+        used, row = used + each[b], row + n
+    starts = lambda x: torch.tensor([sum(x[:i]) for i in range(len(x) + 1)], dtype=torch.int32, device=DEV)
+    run = lambda longest: ops.flash_attn_varlen_with_block_table(q, kc, vc, None, starts(news), starts(lens), max(news), longest, D ** -0.5, None, 0, table.to(DEV))
+    got = run(max(lens))
+    assert ops.last_mha_path() == "prefill_tc"
+    assert torch.equal(got, run(1 << 22))
+    _check(got, q, k, v, news, contexts)
+    assert hybrid_ops.prefill_timeouts() == 0
+
+
 def _check(got, q, k, v, news, contexts):
     """Against float64; k, v: the sequences' rows one after the other.  Bound: the weights are rounded to 16 bits (2^-8 or 2^-11 of the value at most), as is
     the result; 1e-5 for the float32 sums."""
