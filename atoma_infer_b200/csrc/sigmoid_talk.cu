@@ -8,13 +8,13 @@
 // What bounded the mix on CUDA cores was shared memory (32 float32 weights read per pair and head; 4000 warp instructions per tile and
 // warp), so it runs on the tensor cores too, at float32's precision: weights and talk are each split into three bfloat16 pieces of 8 bits, which
 // hold all of a float32's 24 and its whole range, and the six products of pieces down to 2^-16 of a term are summed in float32 (what is dropped is
-// 2^-25 of a term).  mma.sync and not tcgen05: the products per tile are 16 rows or one head-square deep.
+// 2^-25 of a term).
 // One CTA holds all heads (64 accumulator registers per thread for two heads), so there is no cluster exchange, and the keys are cut into segments,
 // whose float32 sums simply add (no softmax): 128 row blocks of one prompt over 74 CTA pairs left the SMs idle half of the time.  A
 // segment is 512 keys from a multiple of 512 on whatever the step looks like, so a position's sums depend on its keys alone.  A CTA takes one
 // segment, or, in steps whose row blocks fill the SMs without, all of its rows' segments one after the other; the sums between take at most 256 MiB
 // (kStScratch), and longer steps go in runs of tokens.  Keys of the next tile are copied under the mix, values under the scores.
-// A tile of 2048 tokens, 32 heads of 64 on 8, takes 14000 cycles: scores and weights 6000 (four results of the special-function unit per weight are 4100 of them),
+// A tile of 2048 tokens, 32 heads of 64 on 8, takes 14000 cycles here (sigmoid_talk32_kernel serves 32 heads where its tiles fit): scores and weights 6000 (four results of the special-function unit per weight are 4100 of them),
 // the mix 5000 (3100 of the tensor pipe), values 2000.  With 27000: every copy waited for its own block-table entry (5000), a branch per weight kept
 // their chains from overlapping, quotients and exponentials took denormal numbers into account, and registers spilled.
 // 2048 tokens, 32 heads of 64 on 8: 1218 us on the CUDA-core mix (hybrid_attention.cu), 507 with those, 283 here; 2000 tokens of 16 heads 328 and 169.  Prompts of up to
@@ -366,6 +366,395 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
     }
 }
 
+// The same for 32 heads, with the mix on tcgen05: a pair's weights of all heads are a row of 32, so that 128 pairs are the wide operand, in tensor memory, and the
+// talk matrix's pieces the narrow one: 12 products of 128 x 32 x 16 stand for the six products of pieces, where mma.sync took 1536 at a quarter of the rate.
+//   split    a thread takes 16 heads of a pair: float32 weights from shared memory, three bfloat16 pieces into tensor memory
+//   mix      D0 = a0 t0; D12 = a2 t0 + a1 t1 + a0 t2 + a1 t0 + a0 t1 (the smallest first), added in float32 and rounded into shared memory
+//   weights  of the next tile, and values of the last one, while the mix runs; one barrier of the CTA a tile of 16 keys
+// Queries lie in tensor memory, the sums in registers; keys are copied two tiles ahead, values one.
+// Bound: latencies.  A tile takes 5500 cycles: weights 2400 (2050 of the special-function unit), values 1000, the split 700, mixed weights 600, the rest waits; 42 % of
+// the issue slots.  2048 tokens, 32 heads of 64 on 8: 283 us with the mix on mma.sync in tiles of 32 keys, 242 so.  Tried: an exponential of each weight as a polynomial 258;
+// sums in tensor memory and queries in registers 248; queries in shared memory and three barriers a tile 275.
+constexpr int kS3Keys = 16, kS3Tries = 1 << 18;
+struct S3Layout {
+    static constexpr int kPair = 4 * 32 + 16, kRow = kS3Keys * kPair + 16, kW = kStRows * kRow;      // bytes: a pair's weights, a query row's, a tile's
+    static constexpr int kMixRow = 2 * kS3Keys + 16, kMixHead = kStRows * kMixRow + 16, kMix = 32 * kMixHead;
+    static constexpr int t_off = 0, kv_off = 8192;   // t, and keys and values by TMA: rows of 128 swizzled bytes
+    __host__ __device__ static constexpr int k_tile(int G, int D, bool tma) { return G * kS3Keys * (tma ? 64 : D + 8); }   // elements
+    __host__ __device__ static size_t total(int G, int D, int DV, bool tma) { return 1024 + kv_off + 2 * kW + 2 * kMix + 4 * (static_cast<size_t>(k_tile(G, D, tma)) + k_tile(G, DV, tma)); }
+};
+constexpr int kS3Smem = 226 * 1024;
+constexpr int kS3Block = 112, kS3D = 48, kS3D12 = 80, kS3Q = 224;   // tensor-memory columns of 128 pairs: pieces, D0, D12; behind both blocks': the queries
+
+__device__ __forceinline__ void s3_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]),
+                 "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ void s3_load(void *dst, const CUtensorMap *map, uint64_t *bar, int row) {   // 16 rows of all heads
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(0), "r"(row), "r"(0)
+                 : "memory");
+}
+
+// TMA: heads of 64 whose pages are whole tiles: a tile's keys are neighbours in the cache and go by one copy each of keys and values.  The cp.async pieces of other
+// shapes cost a tile 1100 to 1700 cycles of issue.
+template <bool TMA>
+__global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const atoma_sigmoid_attn_args a, int lo, int hi, int slots, float *__restrict__ partial, unsigned int *late_out) {
+    using L = S3Layout;
+    constexpr int H = 32, NT = 512;
+    extern __shared__ unsigned char sm_raw[];
+    unsigned char *sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int G = static_cast<int>(a.G), D = TMA ? 64 : static_cast<int>(a.dim), DV = TMA ? 64 : static_cast<int>(a.vdim), bs = static_cast<int>(a.block_size);
+    const int b = blockIdx.y, seg = blockIdx.z;
+    const int t_begin = a.query_start[b], n_q = a.query_start[b + 1] - t_begin;
+    const int first = max(0, lo - t_begin + kStRows - 1) / kStRows, last = (min(n_q, hi - t_begin) + kStRows - 1) / kStRows - 1;   // this run's row blocks
+    const int blk = last - static_cast<int>(blockIdx.x);   // the rows with the most keys first
+    if (n_q <= 0 || blk < first) return;
+    const int r0 = blk * kStRows, rows = min(kStRows, n_q - r0), tok0 = t_begin + r0;
+    const int ctx = static_cast<int>(a.positions[t_begin]), p0 = ctx + r0, total = ctx + n_q;
+    const int all_end = p0 + rows, j_begin = seg * kStSegKeys, j_end = seg == slots - 1 ? all_end : min(all_end, j_begin + kStSegKeys);
+    if (j_begin >= all_end) return;
+    const int32_t *bt = a.block_tables + static_cast<int64_t>(b) * a.max_blocks;
+    unsigned char *talk = sm + L::t_off;
+    const int k_tile = L::k_tile(G, D, TMA), v_tile = L::k_tile(G, DV, TMA);
+    __nv_bfloat16 *Ks = reinterpret_cast<__nv_bfloat16 *>(sm + L::kv_off), *Vs = Ks + 2 * k_tile;
+    unsigned char *weights = reinterpret_cast<unsigned char *>(Vs + 2 * v_tile), *mix = weights + 2 * L::kW;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t4 = lane & 3, rq = lane >> 2;
+    const __nv_bfloat16 *kc = static_cast<const __nv_bfloat16 *>(a.k_cache), *vc = static_cast<const __nv_bfloat16 *>(a.v_cache);
+    __shared__ int32_t slot_s[4][kS3Keys];   // cache rows of a tile's keys (-1: behind the sequence's end), looked up three tiles ahead
+    __shared__ __align__(8) uint64_t split[2], mixed[2], k_full[2], v_full[2];   // split, mixed: of 128 pairs each
+    __shared__ uint32_t tmem_base_s;
+    __shared__ int late_s;
+    volatile int *late = &late_s;
+    const int bs_shift = (bs & (bs - 1)) == 0 ? __ffs(bs) - 1 : -1;
+    auto look_up = [&](int j) {
+        const int pg = bs_shift >= 0 ? j >> bs_shift : j / bs;
+        return j < total ? bt[pg] * bs + (j - pg * bs) : -1;
+    };
+    if (tid < 3 * kS3Keys) slot_s[tid / kS3Keys][tid % kS3Keys] = look_up(j_begin + tid);
+    if (tid == 0) {
+        late_s = 0;
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&split[i], 8);
+            mbar_init(&mixed[i], 1);
+            mbar_init(&k_full[i], 1);
+            mbar_init(&v_full[i], 1);
+        }
+        fence_mbar_init();
+    }
+    if (warp == 0) tmem_alloc(&tmem_base_s, 512);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = tmem_base_s;
+    // A thread's piece of a row is the same for all its keys where the CTA takes whole rows at a time; what it takes to find it is worked out once.
+    struct Piece {
+        int key, step, src, dst;   // first key, keys apart; elements into a key's row of the cache, into the tile
+    };
+    auto piece_of = [&](int n) {
+        const int pieces = G * n / 8, e = tid % pieces, g = e * 8 / n;
+        return NT % pieces == 0 ? Piece{tid / pieces, NT / pieces, e * 8, g * kS3Keys * (n + 8) + e * 8 - g * n} : Piece{0, 0, 0, 0};
+    };
+    const Piece k_piece = TMA ? Piece{} : piece_of(D), v_piece = TMA ? Piece{} : piece_of(DV);
+    auto stage = [&](const __nv_bfloat16 *cache, __nv_bfloat16 *dst, int n, const Piece &pc, const int32_t *at) {
+        if constexpr (TMA) {
+            if (tid == 0) {
+                uint64_t *bar = cache == kc ? &k_full[dst != Ks] : &v_full[dst != Vs];
+                mbar_arrive_expect_tx(bar, G * kS3Keys * 128);
+                s3_load(dst, cache == kc ? &map_k : &map_v, bar, max(at[0], 0));
+            }
+        } else if (pc.step) {
+            for (int jj = pc.key; jj < kS3Keys; jj += pc.step) {
+                const int slot = at[jj];
+                cp_async_16(smem_u32(dst + pc.dst + jj * (n + 8)), cache + static_cast<int64_t>(max(slot, 0)) * (G * n) + pc.src, slot >= 0 ? 16 : 0);
+            }
+        } else {
+            const int pieces = G * n / 8;
+            for (int i = tid; i < kS3Keys * pieces; i += NT) {
+                const int jj = i / pieces, e = i - jj * pieces, g = e * 8 / n, slot = at[jj];
+                cp_async_16(smem_u32(dst + (g * kS3Keys + jj) * (n + 8) + e * 8 - g * n), cache + static_cast<int64_t>(max(slot, 0)) * (G * n) + e * 8, slot >= 0 ? 16 : 0);
+            }
+        }
+    };
+    const int tiles = (j_end - j_begin + kS3Keys - 1) / kS3Keys;
+    stage(kc, Ks, D, k_piece, slot_s[0]);
+    if (tiles > 1) stage(kc, Ks + k_tile, D, k_piece, slot_s[1]);
+    cp_async_commit();
+    // ---- the talk matrix in three pieces, rows of heads h: [t0 | t1], then [t2 | -] ----
+    for (int i = tid; i < H * H; i += NT) {
+        const int h = i / H, g = i % H;
+        float piece[kStPieces];
+        st_split(a.talk[i], piece);
+#pragma unroll
+        for (int k = 0; k < kStPieces; ++k) {
+            const int col = (k & 1) * 64 + g * 2;
+            *reinterpret_cast<__nv_bfloat16 *>(talk + (k >> 1) * 4096 + h * 128 + (((col >> 4) ^ (h & 7)) << 4) + (col & 15)) = __float2bfloat16_rn(piece[k]);
+        }
+    }
+    fence_proxy_async();   // generic-proxy writes -> visible to the tensor core's asynchronous reads
+    const int h0 = 2 * warp, kv_head[2] = {h0 / (H / G), (h0 + 1) / (H / G)};
+    float slope[2], hb[2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        slope[x] = a.slopes ? a.slopes[h0 + x] : 0.f;
+        hb[x] = a.head_bias[h0 + x];
+    }
+    // ---- this warp's queries as the products take them, in tensor memory: [head][16 of its entries][fragment] ----
+    const uint32_t tmem_q = tmem_base + kS3Q + (warp >> 2) * 32 + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    {
+        uint32_t qf[32];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const __nv_bfloat16 *q = static_cast<const __nv_bfloat16 *>(a.q) + static_cast<int64_t>(tok0) * H * D + (h0 + x) * D;
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int row = rq + (e & 1) * 8, col = kk * 16 + 2 * t4 + (e >> 1) * 8;
+                    qf[x * 16 + kk * 4 + e] = kk * 16 < D && row < rows ? *reinterpret_cast<const uint32_t *>(q + static_cast<int64_t>(row) * H * D + col) : 0u;
+                }
+        }
+        tmem_st_32x32b_x32(tmem_q, qf);
+        tmem_st_wait();
+    }
+    float o[2][8][4];
+    auto clear = [&] {
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[x][i][0] = o[x][i][1] = o[x][i][2] = o[x][i][3] = 0.f;
+    };
+    clear();
+    const float in = a.softcap > 0.f ? a.scale * 2.8853900817779268f / a.softcap : 0.f;   // e^(2 s / cap) = 2^(in dot)
+    bool more = false;   // a running sum waits in this token's place
+    // the sums of a segment, out of the accumulators: into its place, onto the running sum, or, where no other segment follows or precedes, out
+    auto put = [&](bool end) {
+        const bool out = end && (slots == 1 || all_end <= kStSegKeys);
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt) {
+                if (nt * 8 >= DV) continue;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int row = rq + 8 * e, col = (h0 + x) * DV + nt * 8 + 2 * t4;
+                    if (row >= rows) continue;
+                    float2 s = make_float2(o[x][nt][2 * e], o[x][nt][2 * e + 1]);
+                    float2 *place = reinterpret_cast<float2 *>(partial + (static_cast<int64_t>(tok0 + row - lo) * slots + seg) * H * DV + col);
+                    if (more) s = make_float2(place->x + s.x, place->y + s.y);
+                    if (out) *reinterpret_cast<uint32_t *>(static_cast<__nv_bfloat16 *>(a.out) + static_cast<int64_t>(tok0 + row) * H * DV + col) = pack2<__nv_bfloat16>(s.x, s.y);
+                    else *place = s;
+                }
+            }
+    };
+    auto wait = [&](uint64_t *bar, uint32_t parity) {   // bounded, for a whole warp
+#pragma unroll 1
+        for (int i = 0; !mbar_try_wait(bar, parity);) {
+            if (*late) break;
+            if (++i == kS3Tries) {
+                *late = 1;
+                break;
+            }
+        }
+        __syncwarp();
+    };
+    // ---- scores and weights of this warp's two heads for tile j ----
+    auto form_weights_as = [&](auto all_seen, int j) {
+        const int j0 = j_begin + j * kS3Keys;
+        const __nv_bfloat16 *kt = Ks + (j & 1) * k_tile;
+        unsigned char *wt = weights + (j & 1) * L::kW;
+        const float base = static_cast<float>(p0 + rq - j0 - 2 * t4);
+        float w0[2][4];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            float s[2][4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+            const int key = kv_head[x] * kS3Keys + (lane >> 4) * 8 + (lane & 7), odd = (lane >> 3) & 1;
+            const uint32_t kb = smem_u32(kt + key * (TMA ? 64 : D + 8));
+            uint32_t qf[16];
+            tmem_ld_32x32b_x16(tmem_q + x * 16, qf);
+            tmem_ld_wait();
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+                if (kk * 16 < D) {
+                    uint32_t r[4];
+                    const uint32_t(&qk)[4] = *reinterpret_cast<const uint32_t(*)[4]>(qf + kk * 4);
+                    ldmatrix_x4(r, kb + (TMA ? ((2 * kk + odd) ^ (lane & 7)) << 4 : kk * 32 + odd * 16));
+                    Mma16816<__nv_bfloat16>::run(s[0], qk, r[0], r[1]);
+                    Mma16816<__nv_bfloat16>::run(s[1], qk, r[2], r[3]);
+                }
+            // weights of hidden pairs are formed too and dropped: without a branch per weight their chains of exponentials and quotients overlap
+            auto weigh = [&](auto with_cap) {
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        s[nt][e] = st_weight<decltype(with_cap)::value>(s[nt][e], a.scale, in, a.softcap, slope[x], base - static_cast<float>(nt * 8 + (e & 1) - (e >> 1) * 8), hb[x]);
+            };
+            if (a.softcap > 0.f) weigh(std::true_type{});
+            else weigh(std::false_type{});
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int row = rq + (e >> 1) * 8, key = nt * 8 + 2 * t4 + (e & 1);
+                    const float w = decltype(all_seen)::value || (row < rows && p0 + row >= j0 + key) ? s[nt][e] : 0.f;
+                    if (x == 0) w0[nt][e] = w;
+                    else *reinterpret_cast<float2 *>(wt + row * L::kRow + key * L::kPair + h0 * 4) = make_float2(w0[nt][e], w);
+                }
+        }
+    };
+    auto form_weights = [&](int j) {
+        if (TMA) wait(&k_full[j & 1], (j >> 1) & 1);
+        if (rows == kStRows && j_begin + (j + 1) * kS3Keys - 1 <= p0) form_weights_as(std::true_type{}, j);
+        else form_weights_as(std::false_type{}, j);
+    };
+    // this thread's pair: block of 128 pairs (8 query rows x 16 keys), and which 16 of its heads
+    const int block = warp >> 3, half = (warp >> 2) & 1, pair = (warp & 3) * 32 + lane, prow = 8 * block + pair / kS3Keys, pkey = pair % kS3Keys;
+    const uint32_t tmem_block = tmem_base + block * kS3Block, tmem_lane = tmem_block + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    cp_async_wait_all();
+    __syncthreads();
+    form_weights(0);
+    // The sequence ends inside tile j (its last one): what follows in the page is not multiplied in.  Every warp zeroes what it reads.
+    auto hide_rows = [&](int j) {
+        for (int x = 0; x < 2; ++x)
+            for (int i = lane; i < kS3Keys * 8; i += 32)
+                if (j_begin + j * kS3Keys + i / 8 >= total) *reinterpret_cast<uint4 *>(Vs + (j & 1) * v_tile + (kv_head[x] * kS3Keys + i / 8) * 64 + i % 8 * 8) = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+    };
+    // ---- values of tile j: what the mix of all heads has given this warp's two ----
+    auto add_values = [&](int j) {
+        if (TMA) wait(&v_full[j & 1], (j >> 1) & 1);
+        if (TMA && j_begin + (j + 1) * kS3Keys > total) hide_rows(j);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const uint32_t vb = smem_u32(Vs + (j & 1) * v_tile + (kv_head[x] * kS3Keys + ((lane >> 3) & 1) * 8 + (lane & 7)) * (TMA ? 64 : DV + 8));
+            uint32_t af[4];
+            ldmatrix_x4(af, smem_u32(mix + (j & 1) * L::kMix + (h0 + x) * L::kMixHead + (lane & 15) * L::kMixRow + (lane >> 4) * 16));
+#pragma unroll
+            for (int n2 = 0; n2 < 4; ++n2)
+                if (n2 * 16 < DV) {
+                    uint32_t r[4];
+                    ldmatrix_x4_trans(r, vb + (TMA ? ((2 * n2 + (lane >> 4)) ^ (lane & 7)) << 4 : n2 * 32 + (lane >> 4) * 16));
+                    Mma16816<__nv_bfloat16>::run(o[x][2 * n2], af, r[0], r[1]);
+                    Mma16816<__nv_bfloat16>::run(o[x][2 * n2 + 1], af, r[2], r[3]);
+                }
+        }
+        if (slots == 1 && partial && j + 1 < tiles && (j_begin + (j + 1) * kS3Keys) % kStSegKeys == 0) {   // a segment ends here
+            put(false);
+            more = true;
+            clear();
+        }
+    };
+    for (int j = 0; j < tiles; ++j) {
+        // The one barrier of a tile: its weights, the mixed weights of the tile before, its values and the next tile's keys are there.  What follows, a warp does at
+        // its own pace, so that one's exponentials run beside another's products.
+        cp_async_wait_all();
+        __syncthreads();
+        stage(vc, Vs + (j & 1) * v_tile, DV, v_piece, slot_s[j & 3]);
+        if (j + 2 < tiles) stage(kc, Ks + (j & 1) * k_tile, D, k_piece, slot_s[(j + 2) & 3]);
+        cp_async_commit();
+        int next_slot = 0;
+        if (tid < kS3Keys) next_slot = look_up(j_begin + (j + 3) * kS3Keys + tid);
+        // ---- split ----
+        {
+            const float4 *w = reinterpret_cast<const float4 *>(weights + (j & 1) * L::kW + prow * L::kRow + pkey * L::kPair + half * 64);
+            uint32_t piece[kStPieces][8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 v = w[i];
+                float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int k = 0; k < kStPieces; ++k) {
+                        const uint32_t two = pack2<__nv_bfloat16>(x[2 * e], x[2 * e + 1]);
+                        piece[k][2 * i + e] = two;
+                        x[2 * e] -= __uint_as_float(two << 16);
+                        x[2 * e + 1] -= __uint_as_float(two & 0xffff0000u);
+                    }
+            }
+#pragma unroll
+            for (int k = 0; k < kStPieces; ++k) s3_st8(tmem_lane + k * 16 + half * 8, piece[k]);
+            tmem_st_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&split[block]);
+        }
+        // ---- mix: issued by the block's first warp ----
+        if ((warp & 7) == 0) {
+            wait(&split[block], j & 1);
+            tc_fence_after_sync();
+            const uint32_t id = umma_idesc_f16(128, H, true);
+            const uint64_t t01 = umma_desc_k_sw128(smem_u32(talk)), t2 = umma_desc_k_sw128(smem_u32(talk) + 4096);
+            if (elect_one_sync()) {
+                auto product = [&](int pa, uint64_t t, uint32_t d, bool fresh) {   // both steps of 16 heads
+                    umma_f16_ts(tmem_block + d, tmem_block + pa * 16, t, id, fresh ? 0u : 1u);
+                    umma_f16_ts(tmem_block + d, tmem_block + pa * 16 + 8, t + 2, id, 1u);
+                };
+                product(2, t01, kS3D12, true);
+                product(1, t01 + 4, kS3D12, false);
+                product(0, t2, kS3D12, false);
+                product(1, t01, kS3D12, false);
+                product(0, t01 + 4, kS3D12, false);
+                product(0, t01, kS3D, true);
+                umma_commit(&mixed[block]);
+            }
+            __syncwarp();
+        }
+        // Half of every scheduler's warps form weights (special functions) while the others apply the last tile's (tensor pipe, shared memory): 255 us without, 242 so.
+#pragma unroll 1
+        for (int step = 0; step < 2; ++step) {
+            if (step == ((warp >> 2) & 1)) {
+                if (j > 0) add_values(j - 1);
+            } else {
+                if (j + 1 < tiles) form_weights(j + 1);
+            }
+        }
+        // ---- the mixed weights of this thread's pair, rounded, to where the values' warps read them ----
+        wait(&mixed[block], j & 1);
+        tc_fence_after_sync();
+        {
+            uint32_t d0[16], d1[16];
+            tmem_ld_32x32b_x16(tmem_lane + kS3D + half * 16, d0);
+            tmem_ld_32x32b_x16(tmem_lane + kS3D12 + half * 16, d1);
+            tmem_ld_wait();
+            unsigned char *m = mix + (j & 1) * L::kMix + half * 16 * L::kMixHead + prow * L::kMixRow + pkey * 2;
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+                const uint32_t two = pack2<__nv_bfloat16>(__uint_as_float(d0[i]) + __uint_as_float(d1[i]), __uint_as_float(d0[i + 1]) + __uint_as_float(d1[i + 1]));
+                *reinterpret_cast<uint16_t *>(m + i * L::kMixHead) = static_cast<uint16_t>(two);
+                *reinterpret_cast<uint16_t *>(m + (i + 1) * L::kMixHead) = static_cast<uint16_t>(two >> 16);
+            }
+        }
+        tc_fence_before_sync();
+        if (tid < kS3Keys) slot_s[(j + 3) & 3][tid] = next_slot;
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    add_values(tiles - 1);
+    put(true);
+    if (TMA && tid == 0) {   // whatever happened to the waits, the copies have landed before the CTA leaves
+        auto landed = [&](uint64_t *bar, int uses) {
+            for (int i = 0; uses > 0 && i < kS3Tries && !mbar_try_wait(bar, (uses - 1) & 1); ++i) {
+            }
+        };
+        for (int i = 0; i < 2; ++i) {
+            landed(&k_full[i], (tiles + 1 - i) / 2);
+            landed(&v_full[i], (tiles + 1 - i) / 2);
+        }
+    }
+    __syncthreads();
+    tc_fence_after_sync();
+    if (warp == 0) tmem_dealloc(tmem_base, 512);
+    if (tid == 0 && *late && late_out) *reinterpret_cast<volatile unsigned int *>(late_out) = 1;
+}
+
 // A token's segments, in order; tokens of one segment are out already.
 __global__ void __launch_bounds__(256) sigmoid_talk_sum_kernel(const atoma_sigmoid_attn_args a, const float *__restrict__ partial, int lo, int hi, int segs) {
     pdl_launch_dependents();
@@ -398,6 +787,21 @@ bool hyb_sigmoid_talk_ok(const atoma_sigmoid_attn_args &a) {
     return (a.H == 16 ? StLayout<1>::total(G, D, DV) : StLayout<2>::total(G, D, DV)) <= 225 * 1024;
 }
 
+namespace {
+// A cache of rows of G heads of 64: 16 rows of all heads a copy, head by head.
+bool s3_map(CUtensorMap *out, const void *cache, int G) {
+    EncodeTiledFn enc = get_encode_tiled();
+    if (!enc) return false;
+    const cuuint64_t dims[3] = {64, 1ull << 31, static_cast<cuuint64_t>(G)}, strides[2] = {static_cast<cuuint64_t>(G) * 128, 128};
+    const cuuint32_t box[3] = {64, kS3Keys, static_cast<cuuint32_t>(G)}, estr[3] = {1, 1, 1};
+    const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(cache), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r == CUDA_SUCCESS) return true;
+    set_status(kErrDriver, "sigmoid_talk: cuTensorMapEncodeTiled failed (CUresult %d)", static_cast<int>(r));
+    return false;
+}
+}  // namespace
+
 bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
     const int64_t longest = a.max_seq_len > 0 ? a.max_seq_len : a.max_blocks * a.block_size;
     const int64_t segs = std::min<int64_t>(65535, (longest + kStSegKeys - 1) / kStSegKeys), blocks = (a.T + kStRows - 1) / kStRows;
@@ -414,15 +818,23 @@ bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
         if (!partial) slots = 1, run = a.T;   // no scratch: one chain needs none
     }
     const int G = static_cast<int>(a.G), D = static_cast<int>(a.dim), DV = static_cast<int>(a.vdim);
+    const bool tma = D == 64 && DV == 64 && a.block_size % kS3Keys == 0;
+    const bool on_tcgen05 = a.H == 32 && S3Layout::total(G, D, DV, tma) <= kS3Smem;   // by the model's sizes alone: a position's bits do not follow the step
+    auto kernel32 = tma ? sigmoid_talk32_kernel<true> : sigmoid_talk32_kernel<false>;
+    CUtensorMap map_k{}, map_v{};
+    if (on_tcgen05 && tma && (!s3_map(&map_k, a.k_cache, G) || !s3_map(&map_v, a.v_cache, G))) return false;
     auto kernel = a.H == 16 ? sigmoid_talk_kernel<1> : sigmoid_talk_kernel<2>;
-    const size_t smem = a.H == 16 ? StLayout<1>::total(G, D, DV) : StLayout<2>::total(G, D, DV);
-    const cudaError_t attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+    const size_t smem = a.H == 16 ? StLayout<1>::total(G, D, DV) : on_tcgen05 ? S3Layout::total(G, D, DV, tma) : StLayout<2>::total(G, D, DV);
+    const cudaError_t attr = on_tcgen05 ? cudaFuncSetAttribute(kernel32, cudaFuncAttributeMaxDynamicSharedMemorySize, kS3Smem)
+                                        : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
     if (attr != cudaSuccess) return hybrid::launched(attr, "sigmoid_talk_kernel");
     for (int64_t lo = 0; lo < a.T; lo += run) {
         const int64_t hi = std::min(a.T, lo + run), rows = (std::min<int64_t>(hi - lo, a.max_query_len) + kStRows - 1) / kStRows + 1;
         const dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>(a.B), static_cast<unsigned>(slots));
-        if (!hybrid::launched(launch_ex(kernel, grid, dim3(16 * static_cast<unsigned>(a.H)), smem, stream, a, static_cast<int>(lo), static_cast<int>(hi),
-                                        static_cast<int>(slots), partial),
+        const dim3 block(16 * static_cast<unsigned>(a.H));
+        const int from = static_cast<int>(lo), to = static_cast<int>(hi), places = static_cast<int>(slots);
+        if (!hybrid::launched(on_tcgen05 ? launch_ex(kernel32, grid, block, smem, stream, map_k, map_v, a, from, to, places, partial, late_word())
+                                         : launch_ex(kernel, grid, block, smem, stream, a, from, to, places, partial),
                               "sigmoid_talk_kernel"))
             return false;
         if (slots > 1 && !hybrid::launched(launch_ex(sigmoid_talk_sum_kernel, dim3(static_cast<unsigned>(std::min(a.T, hi + kStRows) - lo)), dim3(256), 0, stream, a,

@@ -113,6 +113,33 @@ def test_a_position_does_not_depend_on_the_step(H, D, others):
     assert torch.equal(run(q[701:n], [(701, 600)], table[:1]), alone[701:])
 
 
+@pytest.mark.parametrize("G", [1, 2, 8])
+def test_same_bits_whatever_the_pages(G):
+    """32 heads of 64: pages of whole 16-key tiles go by TMA, others by pieces; cache rows that belong to no sequence hold NaN."""
+    H, D, seqs = 32, 64, ((0, 49), (30, 2), (1007, 17), (512, 16), (495, 1))
+    lens = [c + n for c, n in seqs]
+    T = sum(n for _, n in seqs)
+    q, talk = randn_t((T, H * D), 3, torch.bfloat16, DEV), torch.eye(H, device=DEV) + randn_t((H, H), 5, torch.float32, DEV, scale=0.3)
+    k, v = (randn_t((sum(lens), G, D), i, torch.bfloat16, DEV) for i in (1, 2))
+    hb = randn_t((H,), 4, torch.float32, DEV)
+    pos = torch.cat([torch.arange(c, c + n) for c, n in seqs]).to(DEV)
+    tseq = torch.arange(len(seqs), dtype=torch.int32).repeat_interleave(torch.tensor([n for _, n in seqs])).to(DEV)
+    outs = []
+    for bs in (16, 24, 48, 8):
+        each = [-(-n // bs) for n in lens]
+        pool = torch.randperm(sum(each), generator=torch.Generator().manual_seed(bs)).to(torch.int32)
+        kc, vc = (torch.full((sum(each) * bs, G, D), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        table, used, row = torch.zeros((len(seqs), max(each)), dtype=torch.int32), 0, 0
+        for b, n in enumerate(lens):
+            table[b, :each[b]] = pool[used:used + each[b]]
+            at = torch.arange(n)
+            slot = (table[b].long()[at // bs] * bs + at % bs).to(DEV)
+            kc[slot], vc[slot] = k[row:row + n], v[row:row + n]
+            used, row = used + each[b], row + n
+        outs.append(ops.sigmoid_attention_paged(q, kc, vc, pos, tseq, table.to(DEV), None, hb, talk, H, G, D, D, bs, D ** -0.5, 8.0, 49))
+    assert torch.isfinite(outs[0]).all() and all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
 def test_capture_on_a_stream_without_scratch():
     """A long prompt captured on a stream that has run nothing: segments need scratch that cannot be had there, whole rows need none."""
     H, G, D, bs, n = 16, 2, 32, 16, 1100
