@@ -11,9 +11,9 @@
 // 2^-25 of a term).
 // One CTA holds all heads (64 accumulator registers per thread for two heads), so there is no cluster exchange, and the keys are cut into segments,
 // whose float32 sums simply add (no softmax): 128 row blocks of one prompt over 74 CTA pairs left the SMs idle half of the time.  A
-// segment is 512 keys from a multiple of 512 on whatever the step looks like, so a position's sums depend on its keys alone.  A CTA takes one
-// segment, or, in steps whose row blocks fill the SMs without, all of its rows' segments one after the other; the sums between take at most 256 MiB
-// (kStScratch), and longer steps go in runs of tokens.  Keys of the next tile are copied under the mix, values under the scores.
+// segment is 256 or 512 keys (by the heads) from a multiple of that on whatever the step looks like, so a position's sums depend on its keys alone.  A CTA takes one
+// segment, two neighbours in steps of many, or, in steps whose row blocks fill the SMs without, all of its rows' segments one after the other; the sums between take
+// at most 256 MiB (kStScratch), and longer steps go in runs of tokens.  Keys of the next tile are copied under the mix, values under the scores.
 // A tile of 2048 tokens, 32 heads of 64 on 8, takes 14000 cycles here (sigmoid_talk32_kernel serves 32 heads where its tiles fit): scores and weights 6000 (four results of the special-function unit per weight are 4100 of them),
 // the mix 5000 (3100 of the tensor pipe), values 2000.  With 27000: every copy waited for its own block-table entry (5000), a branch per weight kept
 // their chains from overlapping, quotients and exponentials took denormal numbers into account, and registers spilled.
@@ -33,7 +33,10 @@ namespace {
 
 using namespace hybrid;
 
-constexpr int kStRows = 16, kStKeys = 32, kStSegKeys = 512, kStPieces = 3;
+constexpr int kStRows = 16, kStKeys = 32, kStPieces = 3;
+// Keys of a segment.  Shorter ones put short prompts on more SMs (32 heads, 600 and 1000 tokens, 512 / 256: 117 / 66, 119 / 68 us; 128 lose from 1000 tokens on) and
+// cost long ones more sums (16 heads, 2000 tokens: 166 / 171).
+constexpr int st_seg_keys(int heads) { return heads == 32 ? 256 : 512; }
 constexpr int64_t kStScratch = 256ll << 20;
 
 // sigmoid(cap tanh(s / cap) - slope dist + bias), tanh(y) = 1 - 2 / (1 + e^2y).  The unit's estimates of 2^x and of the reciprocal are within 2 and 1 units of the last
@@ -76,21 +79,22 @@ __device__ __forceinline__ void st_split(float x, float (&piece)[kStPieces]) {
 // (blockIdx.z: which segment this CTA takes; sigmoid_talk_sum_kernel adds them), or 1: this CTA takes them all and keeps the running sum there.  Both add the
 // segments in order, so they give the same bits.  No scratch: one chain over all keys.
 template <int HT>
-__global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_sigmoid_attn_args a, int lo, int hi, int slots, float *__restrict__ partial) {
+__global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_sigmoid_attn_args a, int lo, int hi, int slots, int per, float *__restrict__ partial) {
     using L = StLayout<HT>;
-    constexpr int H = L::H, NW = 8 * HT, NT = 256 * HT;
+    constexpr int kStSegKeys = st_seg_keys(L::H), H = L::H, NW = 8 * HT, NT = 256 * HT;
     extern __shared__ __align__(16) unsigned char sm[];
     pdl_launch_dependents();
     pdl_wait();
     const int G = static_cast<int>(a.G), D = static_cast<int>(a.dim), DV = static_cast<int>(a.vdim), bs = static_cast<int>(a.block_size);
-    const int b = blockIdx.y, seg = blockIdx.z;
+    const int b = blockIdx.y;
+    int seg = blockIdx.z * per;   // the segment in hand
     const int t_begin = a.query_start[b], n_q = a.query_start[b + 1] - t_begin;
     const int first = max(0, lo - t_begin + kStRows - 1) / kStRows, last = (min(n_q, hi - t_begin) + kStRows - 1) / kStRows - 1;   // this run's row blocks
     const int blk = last - static_cast<int>(blockIdx.x);   // the rows with the most keys first
     if (n_q <= 0 || blk < first) return;
     const int r0 = blk * kStRows, rows = min(kStRows, n_q - r0), tok0 = t_begin + r0;
     const int ctx = static_cast<int>(a.positions[t_begin]), p0 = ctx + r0, total = ctx + n_q;
-    const int all_end = p0 + rows, j_begin = seg * kStSegKeys, j_end = seg == slots - 1 ? all_end : min(all_end, j_begin + kStSegKeys);
+    const int all_end = p0 + rows, j_begin = seg * kStSegKeys, j_end = seg + per >= slots ? all_end : min(all_end, j_begin + per * kStSegKeys);
     if (j_begin >= all_end) return;
     const int32_t *bt = a.block_tables + static_cast<int64_t>(b) * a.max_blocks;
     unsigned char *weights = sm + L::w_off, *mix = sm + L::m_off, *talk = sm + L::t_off;
@@ -344,9 +348,10 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
                     }
             }
         }
-        if (slots == 1 && partial && j0 + kStKeys < j_end && (j0 + kStKeys) % kStSegKeys == 0) {   // a segment ends here
+        if (partial && j0 + kStKeys < j_end && (j0 + kStKeys) % kStSegKeys == 0 && (slots == 1 || seg + 1 < slots)) {   // a segment ends here
             put(false);
-            more = true;
+            if (slots == 1) more = true;
+            else ++seg;
             fresh = true;
             clear();
         } else if constexpr (HT == 2) {
@@ -401,22 +406,23 @@ __device__ __forceinline__ void s3_load(void *dst, const CUtensorMap *map, uint6
 // TMA: heads of 64 whose pages are whole tiles: a tile's keys are neighbours in the cache and go by one copy each of keys and values.  The cp.async pieces of other
 // shapes cost a tile 1100 to 1700 cycles of issue.
 template <bool TMA>
-__global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const atoma_sigmoid_attn_args a, int lo, int hi, int slots, float *__restrict__ partial, unsigned int *late_out) {
+__global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const atoma_sigmoid_attn_args a, int lo, int hi, int slots, int per, float *__restrict__ partial, unsigned int *late_out) {
     using L = S3Layout;
-    constexpr int H = 32, NT = 512;
+    constexpr int H = 32, NT = 512, kStSegKeys = st_seg_keys(32);
     extern __shared__ unsigned char sm_raw[];
     unsigned char *sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
     pdl_launch_dependents();
     pdl_wait();
     const int G = static_cast<int>(a.G), D = TMA ? 64 : static_cast<int>(a.dim), DV = TMA ? 64 : static_cast<int>(a.vdim), bs = static_cast<int>(a.block_size);
-    const int b = blockIdx.y, seg = blockIdx.z;
+    const int b = blockIdx.y;
+    int seg = blockIdx.z * per;   // the segment in hand
     const int t_begin = a.query_start[b], n_q = a.query_start[b + 1] - t_begin;
     const int first = max(0, lo - t_begin + kStRows - 1) / kStRows, last = (min(n_q, hi - t_begin) + kStRows - 1) / kStRows - 1;   // this run's row blocks
     const int blk = last - static_cast<int>(blockIdx.x);   // the rows with the most keys first
     if (n_q <= 0 || blk < first) return;
     const int r0 = blk * kStRows, rows = min(kStRows, n_q - r0), tok0 = t_begin + r0;
     const int ctx = static_cast<int>(a.positions[t_begin]), p0 = ctx + r0, total = ctx + n_q;
-    const int all_end = p0 + rows, j_begin = seg * kStSegKeys, j_end = seg == slots - 1 ? all_end : min(all_end, j_begin + kStSegKeys);
+    const int all_end = p0 + rows, j_begin = seg * kStSegKeys, j_end = seg + per >= slots ? all_end : min(all_end, j_begin + per * kStSegKeys);
     if (j_begin >= all_end) return;
     const int32_t *bt = a.block_tables + static_cast<int64_t>(b) * a.max_blocks;
     unsigned char *talk = sm + L::t_off;
@@ -645,9 +651,10 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
                     Mma16816<__nv_bfloat16>::run(o[x][2 * n2 + 1], af, r[2], r[3]);
                 }
         }
-        if (slots == 1 && partial && j + 1 < tiles && (j_begin + (j + 1) * kS3Keys) % kStSegKeys == 0) {   // a segment ends here
+        if (partial && j + 1 < tiles && (j_begin + (j + 1) * kS3Keys) % kStSegKeys == 0 && (slots == 1 || seg + 1 < slots)) {   // a segment ends here
             put(false);
-            more = true;
+            if (slots == 1) more = true;
+            else ++seg;
             clear();
         }
     };
@@ -756,13 +763,13 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
 }
 
 // A token's segments, in order; tokens of one segment are out already.
-__global__ void __launch_bounds__(256) sigmoid_talk_sum_kernel(const atoma_sigmoid_attn_args a, const float *__restrict__ partial, int lo, int hi, int segs) {
+__global__ void __launch_bounds__(256) sigmoid_talk_sum_kernel(const atoma_sigmoid_attn_args a, const float *__restrict__ partial, int lo, int hi, int segs, int seg_keys) {
     pdl_launch_dependents();
     pdl_wait();
     const int64_t t = lo + static_cast<int64_t>(blockIdx.x);
     const int b = a.token_seq[t], t_begin = a.query_start[b], n_q = a.query_start[b + 1] - t_begin;
     const int r0 = static_cast<int>(t - t_begin) / kStRows * kStRows, end = static_cast<int>(a.positions[t_begin]) + min(r0 + kStRows, n_q);
-    const int n = min(segs, (end + kStSegKeys - 1) / kStSegKeys), row = static_cast<int>(a.H * a.vdim);
+    const int n = min(segs, (end + seg_keys - 1) / seg_keys), row = static_cast<int>(a.H * a.vdim);
     if (n < 2 || t_begin + r0 < lo || t_begin + r0 >= hi) return;
     const float *p = partial + (t - lo) * segs * row;
     for (int i = threadIdx.x * 4; i < row; i += 1024) {
@@ -804,7 +811,7 @@ bool s3_map(CUtensorMap *out, const void *cache, int G) {
 
 bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
     const int64_t longest = a.max_seq_len > 0 ? a.max_seq_len : a.max_blocks * a.block_size;
-    const int64_t segs = std::min<int64_t>(65535, (longest + kStSegKeys - 1) / kStSegKeys), blocks = (a.T + kStRows - 1) / kStRows;
+    const int64_t seg_keys = st_seg_keys(static_cast<int>(a.H)), segs = std::min<int64_t>(65535, (longest + seg_keys - 1) / seg_keys), blocks = (a.T + kStRows - 1) / kStRows;
     const int64_t place = a.H * a.vdim * 4;   // bytes of a token's sums
     int64_t slots = 1, run = a.T;
     float *partial = nullptr;
@@ -817,6 +824,8 @@ bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
         partial = static_cast<float *>(try_workspace(stream, static_cast<size_t>((run + kStRows) * slots * place), kWorkspaceHybridAttn));   // a run's last row block may end behind it
         if (!partial) slots = 1, run = a.T;   // no scratch: one chain needs none
     }
+    // two segments a CTA where the row blocks have many: a CTA's start and end cost some four tiles
+    const int per = seg_keys < 512 && slots > 1 && blocks * slots >= 4 * current_device_info().sm_count ? 2 : 1;
     const int G = static_cast<int>(a.G), D = static_cast<int>(a.dim), DV = static_cast<int>(a.vdim);
     const bool tma = D == 64 && DV == 64 && a.block_size % kS3Keys == 0;
     const bool on_tcgen05 = a.H == 32 && S3Layout::total(G, D, DV, tma) <= kS3Smem;   // by the model's sizes alone: a position's bits do not follow the step
@@ -830,15 +839,15 @@ bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
     if (attr != cudaSuccess) return hybrid::launched(attr, "sigmoid_talk_kernel");
     for (int64_t lo = 0; lo < a.T; lo += run) {
         const int64_t hi = std::min(a.T, lo + run), rows = (std::min<int64_t>(hi - lo, a.max_query_len) + kStRows - 1) / kStRows + 1;
-        const dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>(a.B), static_cast<unsigned>(slots));
+        const dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>(a.B), static_cast<unsigned>((slots + per - 1) / per));
         const dim3 block(16 * static_cast<unsigned>(a.H));
         const int from = static_cast<int>(lo), to = static_cast<int>(hi), places = static_cast<int>(slots);
-        if (!hybrid::launched(on_tcgen05 ? launch_ex(kernel32, grid, block, smem, stream, map_k, map_v, a, from, to, places, partial, late_word())
-                                         : launch_ex(kernel, grid, block, smem, stream, a, from, to, places, partial),
+        if (!hybrid::launched(on_tcgen05 ? launch_ex(kernel32, grid, block, smem, stream, map_k, map_v, a, from, to, places, per, partial, late_word())
+                                         : launch_ex(kernel, grid, block, smem, stream, a, from, to, places, per, partial),
                               "sigmoid_talk_kernel"))
             return false;
         if (slots > 1 && !hybrid::launched(launch_ex(sigmoid_talk_sum_kernel, dim3(static_cast<unsigned>(std::min(a.T, hi + kStRows) - lo)), dim3(256), 0, stream, a,
-                                                    static_cast<const float *>(partial), static_cast<int>(lo), static_cast<int>(hi), static_cast<int>(slots)),
+                                                    static_cast<const float *>(partial), static_cast<int>(lo), static_cast<int>(hi), static_cast<int>(slots), static_cast<int>(seg_keys)),
                                           "sigmoid_talk_sum_kernel"))
             return false;
     }
