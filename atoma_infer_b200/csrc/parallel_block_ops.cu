@@ -650,6 +650,74 @@ __global__ void __launch_bounds__(256) latent_query_rope_kernel(const T *__restr
     }
 }
 
+// Queries of a few tokens into the latent space, their rotated part beside them: q_lat[t, h, :kv_rank] = q[t, h, :dim] . w_uk[h] and the rotation of what follows, by one
+// launch.  Bound: latency (32 tokens of 32 heads move 9 MB).  A CTA takes 32 tokens x 64 columns of one head with all of its operands in flight at once, or, the last
+// of a head, that head's rotations.  32 tokens of 32 heads of 128 + 64 on 512: a product in 64-token tiles and a rotation behind it 16.3 us a call, this 12.9.
+constexpr int kAbsorbTokens = 32, kAbsorbCols = 64;
+__global__ void __launch_bounds__(128) latent_absorb_few_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restrict__ w, const float *__restrict__ freq,
+                                                                const float *__restrict__ freq_lo, float amplitude, int pairs, int interleaved,
+                                                                const int64_t *__restrict__ positions, float *__restrict__ q_lat, int T, int H, int dim, int rot_dim, int kv_rank) {
+    extern __shared__ __align__(16) unsigned char absorb_sm[];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.z, t0 = blockIdx.y * kAbsorbTokens, n = min(kAbsorbTokens, T - t0);
+    const int hs = dim + rot_dim, row = kv_rank + rot_dim;
+    const __nv_bfloat16 *qh = q + (static_cast<int64_t>(t0) * H + h) * hs;
+    float *oh = q_lat + (static_cast<int64_t>(t0) * H + h) * row;
+    if (blockIdx.x == gridDim.x - 1 && rot_dim > 0) {
+        for (int i = tid; i < n * pairs; i += 128) {
+            const int t = i / pairs, c = i - t * pairs, ia = interleaved ? 2 * c : c, ib = interleaved ? 2 * c + 1 : c + pairs;
+            const __nv_bfloat16 *src = qh + static_cast<int64_t>(t) * H * hs + dim;
+            float sn, cs;
+            turn(static_cast<float>(positions[t0 + t]), freq[c], freq_lo ? freq_lo[c] : 0.f, amplitude, sn, cs);
+            const float u = to_f(src[ia]), v = to_f(src[ib]);
+            float *dst = oh + static_cast<int64_t>(t) * H * row + kv_rank;
+            dst[ia] = u * cs - v * sn;
+            dst[ib] = v * cs + u * sn;
+        }
+        const int rest = rot_dim - 2 * pairs;
+        for (int i = tid; i < n * rest; i += 128) {
+            const int t = i / rest, c = 2 * pairs + i - t * rest;
+            oh[static_cast<int64_t>(t) * H * row + kv_rank + c] = to_f(qh[static_cast<int64_t>(t) * H * hs + dim + c]);
+        }
+        return;
+    }
+    const int n0 = blockIdx.x * kAbsorbCols, q_row = dim * 2 + 16, pieces = dim / 8;
+    constexpr int kWRow = kAbsorbCols * 2 + 16;   // 16 bytes more than whole lines: eight rows hit distinct banks
+    unsigned char *ws = absorb_sm, *qs = absorb_sm + dim * kWRow;
+    const __nv_bfloat16 *wh = w + static_cast<int64_t>(h) * dim * kv_rank + n0;
+    for (int i = tid; i < dim * 8; i += 128) cp_async_16(smem_u32(ws + (i >> 3) * kWRow + (i & 7) * 16), wh + static_cast<int64_t>(i >> 3) * kv_rank + (i & 7) * 8, 16);
+    for (int i = tid; i < kAbsorbTokens * pieces; i += 128) {
+        const int t = i / pieces, c = i - t * pieces;
+        cp_async_16(smem_u32(qs + t * q_row + c * 16), qh + static_cast<int64_t>(min(t, n - 1)) * H * hs + c * 8, 16);
+    }
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncthreads();
+    float acc[2][2][4] = {};
+    for (int k = 0; k < dim; k += 16) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, smem_u32(ws + (k + (lane & 7) + ((lane >> 3) & 1) * 8) * kWRow + (warp * 16 + (lane >> 4) * 8) * 2));
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            uint32_t a[4];
+            ldmatrix_x4(a, smem_u32(qs + (mt * 16 + (lane & 15)) * q_row + (k + (lane >> 4) * 8) * 2));
+            Mma16816<__nv_bfloat16>::run(acc[mt][0], a, b[0], b[1]);
+            Mma16816<__nv_bfloat16>::run(acc[mt][1], a, b[2], b[3]);
+        }
+    }
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int t = mt * 16 + (lane >> 2) + 8 * e;
+            if (t >= n) continue;
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+                *reinterpret_cast<float2 *>(oh + static_cast<int64_t>(t) * H * row + n0 + warp * 16 + nt * 8 + 2 * (lane & 3)) = make_float2(acc[mt][nt][2 * e], acc[mt][nt][2 * e + 1]);
+        }
+}
+
 }  // namespace
 
 #define HYB_DISPATCH(dtype, CALL) ((dtype) == ATOMA_DTYPE_BF16 ? CALL(__nv_bfloat16) : CALL(float))
@@ -810,6 +878,17 @@ bool hyb_latent_query_absorb_rope(const void *q, const void *w_uk, const float *
         return false;
     }
     const int64_t hs = dim + rot_dim, row = kv_rank + rot_dim;
+    // decoded tokens, whose rows are whole pieces of 16 bytes (a result row: of 8): one launch; more tokens fill the SMs in tiles of 64
+    auto al = [](const void *p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; };
+    const size_t smem = static_cast<size_t>(dim) * (kAbsorbCols * 2 + 16) + kAbsorbTokens * (static_cast<size_t>(dim) * 2 + 16);
+    if (dtype == ATOMA_DTYPE_BF16 && !(g_hybrid_debug & 1) && T <= 64 && dim % 16 == 0 && hs % 8 == 0 && row % 2 == 0 && kv_rank % kAbsorbCols == 0 && smem <= 48 * 1024 &&
+        H <= 65535 && al(q, 16) && al(w_uk, 16) && al(q_lat, 8)) {
+        const dim3 grid(static_cast<unsigned>(kv_rank / kAbsorbCols + (rot_dim > 0 ? 1 : 0)), static_cast<unsigned>((T + kAbsorbTokens - 1) / kAbsorbTokens), static_cast<unsigned>(H));
+        return hybrid::launched(launch_ex(latent_absorb_few_kernel, grid, dim3(128), smem, stream, static_cast<const __nv_bfloat16 *>(q), static_cast<const __nv_bfloat16 *>(w_uk), freq,
+                                          freq_lo, amplitude, static_cast<int>(pairs), interleaved, positions, q_lat, static_cast<int>(T), static_cast<int>(H), static_cast<int>(dim),
+                                          static_cast<int>(rot_dim), static_cast<int>(kv_rank)),
+                                "latent_absorb_few_kernel");
+    }
     if (!hyb_head_project_ld(q, H * hs, hs, w_uk, q_lat, H * row, row, T, H, dim, kv_rank, 1, dtype, stream)) return false;
     if (rot_dim == 0) return true;
 #define CALL(TT) launch_ex(latent_query_rope_kernel<TT>, dim3(static_cast<unsigned>(T)), dim3(256), 0, stream, static_cast<const TT *>(q), freq, freq_lo, amplitude, \

@@ -113,3 +113,18 @@ def test_values_of_a_few_tokens(T, H, n, R, row, gated):
     want = torch.einsum("thr,hnr->thn", x, wd).reshape(T, -1) * s
     mag = torch.einsum("thr,hnr->thn", x.abs(), wd.abs()).reshape(T, -1)
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -8 + 4e-6) * mag * 1.01).all())
+
+
+@pytest.mark.parametrize("T,H,dim,rot,pairs,interleaved,rank", [(1, 3, 128, 64, 32, False, 512), (31, 2, 64, 32, 7, True, 64), (33, 5, 48, 8, 4, False, 192), (64, 4, 128, 0, 0, False, 128), (64, 1, 256, 16, 0, True, 64)])
+def test_absorbed_queries_of_few_tokens(T, H, dim, rot, pairs, interleaved, rank):
+    """One launch for up to 64 tokens: the bits of the product in 64-token tiles and the rotation behind it, which a step of one token more takes."""
+    q = randn_t((65, H * (dim + rot)), 1, torch.bfloat16, DEV)
+    w = randn_t((H * dim, rank), 2, torch.bfloat16, DEV)
+    freq = (10000.0 ** (-torch.arange(pairs, dtype=torch.float32) / max(pairs, 1))).to(DEV) if pairs else None
+    low = (torch.arange(pairs, dtype=torch.float32) * 1e-9).to(DEV) if pairs else None
+    pos = torch.arange(65, device=DEV) * 97
+    run = lambda n: ops.latent_query_absorb_rope(q[:n], w, freq, interleaved, pos[:n], H, dim, rot, rank, freq_lo=low, amplitude=1.25)
+    got, want = run(T), run(65)
+    assert torch.equal(got, want[:T])
+    exact = torch.einsum("thd,hdr->thr", q[:T].double().view(T, H, -1)[..., :dim], w.double().view(H, dim, rank))
+    assert (got[..., :rank].double() - exact).norm() <= 1e-5 * exact.norm()
