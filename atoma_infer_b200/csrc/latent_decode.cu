@@ -169,17 +169,18 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent
             const int64_t token = a.query_start[b];
             // ---- queries -> bfloat16 rows in the products' layout (the products of the sequence before are complete) ----
             const float *q = a.q_lat + token * H * R;
-            for (int i0 = tid; i0 < NH * pieces; i0 += 6 * 128) {   // twelve loads in flight: one at a time took 8 us
-                float4 v[6][2];
+            constexpr int kBatch = 9;   // 32 heads of 576 in two rounds of eighteen loads; three rounds of twelve 55.3 us for 54.1 (32 sequences), one load at a time 8 us a sequence
+            for (int i0 = tid; i0 < NH * pieces; i0 += kBatch * 128) {
+                float4 v[kBatch][2];
 #pragma unroll
-                for (int k = 0; k < 6; ++k) {
+                for (int k = 0; k < kBatch; ++k) {
                     const int i = min(i0 + k * 128, NH * pieces - 1), r = i / pieces, c = i - r * pieces;
                     const float4 *src = reinterpret_cast<const float4 *>(q + static_cast<int64_t>(min(r, H - 1)) * R + c * 8);
                     v[k][0] = src[0];
                     v[k][1] = src[1];
                 }
 #pragma unroll
-                for (int k = 0; k < 6; ++k) {
+                for (int k = 0; k < kBatch; ++k) {
                     const int i = i0 + k * 128, r = i / pieces, c = i - r * pieces;
                     uint4 w = make_uint4(0, 0, 0, 0);
                     if (r < H)
@@ -455,6 +456,8 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent
 
 // The runs of a sequence that several CTAs shared, in CTA order: M = max m, out = sum acc 2^(m - M) / sum l 2^(m - M).  A CTA takes 32 columns of
 // one sequence, a warp four of its heads at a time (16 bytes of a run's [column][heads] row), a lane a column.
+// Bound: latency; the runs' maxima and denominators come a lane each, beside the first eight runs' sums (one after the other: one sequence of 1024 keys, attention and
+// merge, 24.6 us for 20.5, eight of 4096 40 for 34).
 template <int NH>
 __global__ void __launch_bounds__(NH * 8) latent_decode_merge_kernel(const atoma_latent_attn_args a, const float *__restrict__ partial,
                                                                      const float *__restrict__ partial_ml, const int *__restrict__ prefix, int grid) {
@@ -466,27 +469,52 @@ __global__ void __launch_bounds__(NH * 8) latent_decode_merge_kernel(const atoma
     if (last < first) return;
     const int c0 = ld_owner(units, first, ncta), c1 = ld_owner(units, last, ncta);
     if (c0 == c1) return;
+    // Lane j holds run c + j's maxima and denominators of the warp's four heads; the sums' first pieces are under way meanwhile.
+    const int lane = threadIdx.x & 31, runs = c1 - c0 + 1;
+    constexpr int kAhead = 8;
+    const float *sums = partial + (static_cast<int64_t>(b + c0) * Rv + col) * NH + h0;
+    const int64_t pitch = static_cast<int64_t>(Rv) * NH;
+    float4 v[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+        if (k < runs) v[k] = *reinterpret_cast<const float4 *>(sums + k * pitch);
+    auto of_run = [&](int r) -> const float * { return partial_ml + (static_cast<int64_t>(b + c0 + min(r, runs - 1)) * NH + h0) * 2; };
     float M[4], den[4], num[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) M[i] = -INFINITY, den[i] = num[i] = 0.f;
-    for (int c = c0; c <= c1; ++c) {
-        const float *ml = partial_ml + (static_cast<int64_t>(b + c) * NH + h0) * 2;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (h0 + i < H) M[i] = fmaxf(M[i], ml[2 * i]);
+    for (int r = lane; r - lane < runs; r += 32) {
+        const float4 x = *reinterpret_cast<const float4 *>(of_run(r)), y = *reinterpret_cast<const float4 *>(of_run(r) + 4);
+        M[0] = fmaxf(M[0], x.x), M[1] = fmaxf(M[1], x.z), M[2] = fmaxf(M[2], y.x), M[3] = fmaxf(M[3], y.z);
     }
-#pragma unroll 4
-    for (int c = c0; c <= c1; ++c) {
-        const float4 v = *reinterpret_cast<const float4 *>(partial + (static_cast<int64_t>(b + c) * Rv + col) * NH + h0);
-        const float *ml = partial_ml + (static_cast<int64_t>(b + c) * NH + h0) * 2;
-        const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (h0 + i < H) {
-                const float f = exp2f(ml[2 * i] - (M[i] == -INFINITY ? 0.f : M[i]));
-                den[i] = fmaf(ml[2 * i + 1], f, den[i]);
-                num[i] = fmaf(x[i], f, num[i]);
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) M[i] = fmaxf(M[i], __shfl_xor_sync(0xffffffffu, M[i], o));
+    for (int r0 = 0; r0 < runs; r0 += 32) {
+        const float4 x = *reinterpret_cast<const float4 *>(of_run(r0 + lane)), y = *reinterpret_cast<const float4 *>(of_run(r0 + lane) + 4);
+        const float m[4] = {x.x, x.z, y.x, y.z}, l[4] = {x.y, x.w, y.y, y.w};
+        float f[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[i] = exp2f(m[i] - (M[i] == -INFINITY ? 0.f : M[i]));
+        for (int k0 = 0; k0 < 32 && r0 + k0 < runs; k0 += kAhead) {
+            float4 next[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k)
+                if (r0 + k0 + kAhead + k < runs) next[k] = *reinterpret_cast<const float4 *>(sums + (r0 + k0 + kAhead + k) * pitch);
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                const float xs[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float fr = __shfl_sync(0xffffffffu, f[i], k0 + k), lr = __shfl_sync(0xffffffffu, l[i], k0 + k);
+                    if (r0 + k0 + k < runs && h0 + i < H) {
+                        den[i] = fmaf(lr, fr, den[i]);
+                        num[i] = fmaf(xs[i], fr, num[i]);
+                    }
+                }
+                v[k] = next[k];
             }
+        }
     }
     float *out = a.out + (static_cast<int64_t>(a.query_start[b]) * H + h0) * R + col;
 #pragma unroll
