@@ -113,6 +113,20 @@ struct StateTile {
     static __device__ __forceinline__ int at(int row, int col) { return row / R * kPart + row % R * kCols + col; }
 };
 
+// Whether the compute warps hand a token's sums over to the staging warps, which add the lanes' parts and write the outputs: nine instructions of a token's 178 fewer where
+// one warp a scheduler is bound by what it issues.  Only where it was measured to be faster (us, shuffles in the compute warps / handed over): delta rule of 32 heads of
+// 128 x 128, 4000 and 1000 tokens 715 / 681, 184 / 176, three portions 457 / 445; state space of 64 heads of 128 x 64, 4000 tokens 508 / 473.  Eight rows a lane lose
+// (16 heads 568 / 573, state space of 32 heads 355 / 392), heads of 256 and 512 too (987 / 1161, 966 / 981), and gated linear attention, whose staging warps have the decays
+// to form (420 / 643).
+template <int KIND, int R, int PW, bool SHORT>
+constexpr bool kHandOver = !SHORT && KIND != 0 && R == 16 && PW == 8;
+// Read-outs of a token on their way to the staging warps: the lanes' sums, a part's columns together and the parts apart by what lets half a warp's stores hit
+// distinct banks, then what is added to the scaled sum of each column.
+template <int PW, int NW>
+struct ReadOut {
+    static constexpr int kCols = 64 * NW / PW, kPart = kCols + 64 / PW, kAdd = PW * kPart, kFloats = kAdd + kCols;
+};
+
 __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -124,9 +138,10 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
 // by PW-lane shuffles, and the write is one product and one FMA per entry:
 //   q, k as projected; lengths enter as scalars: S^T khat = fk (S^T k)
 //   u = beta (v - g fk S^T k);  o = g fq S^T q + (qhat . khat) u;  S <- g S + k (fk u)
-// What bounds it: the chain of a token (row sum, PW-lane shuffles of 29 cycles each, write: 225 of the 340 cycles a token of the delta rule
-// takes at 16 x 8) beside 64 packed FMAs of two cycles and the staged row's reads, which deliver 128 bytes a cycle to all warps of an SM.
-// Rows kept as bfloat16 in shared memory and converted per warp beat float32 rows (718 us against 729 for 4096 tokens of 32 heads of 128 x 128),
+// What bounds it: what one warp a scheduler issues for a token, some 170 instructions, 64 of them packed FMAs of two cycles, in 330 cycles; the chain alone (row sum,
+// PW-lane shuffles of 29 cycles each, write) is 215.  Delta rule, 4096 tokens of 32 heads of 128 x 128, 733 us: without the shuffles 643, the sums of S^T q 666, the
+// conversions 678; two warps of half the rows a scheduler 811.  Shared memory delivers 128 bytes a cycle to all warps of an SM.
+// Rows kept as bfloat16 in shared memory and converted per warp beat float32 rows (718 us against 729, before sums were handed over, for 4096 tokens of 32 heads of 128 x 128),
 // one column a lane loses to two (924 to 1330 us).  Against one column a lane, 32 rows, rows converted and normed by the staging warps: delta
 // rule 1064 -> 729 us (that case), 504 -> 289 (16 heads, 2000 tokens); state space 794 -> 365 (32 heads of 128 x 64, 4000 tokens); gated linear
 // attention 752 -> 421 (32 heads of 64 x 128, 4000 tokens).
@@ -147,6 +162,10 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
     const int q0 = a.query_start[b], n = a.query_start[b + 1] - q0;
     if (n <= 0) return;
     const int jb = blockIdx.x * COLS, chunk_bytes = chunk * L::kBytes;
+    using RO = ReadOut<PW, NW>;
+    constexpr bool HAND = kHandOver<KIND, R, PW, SHORT>;
+    [[maybe_unused]] float *read_outs = reinterpret_cast<float *>(sm + buffers * chunk_bytes);   // of two chunks
+    __shared__ float2 out_scale[HAND ? 4 : 1][HAND ? 32 : 1];                          // a token's factors of its sum and of what was written: of the chunk before, in hand and next
     if (D < L::kRow || jb + COLS > V) {                          // what lies beyond dim and vdim stays zero
         for (int i = threadIdx.x * 16; i < buffers * chunk_bytes; i += blockDim.x * 16) *reinterpret_cast<uint4 *>(sm + i) = make_uint4(0, 0, 0, 0);
         __syncthreads();
@@ -295,18 +314,42 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
             }
             if (sub == 0 && tok < left) {
                 float4 *s = reinterpret_cast<float4 *>(row + L::kScalars);
+                float2 *scale = HAND ? &out_scale[t0 / chunk & 3][w * mine + tok] : nullptr;
                 if (KIND == 0) {
                     s[0] = make_float4(a.q_scale, dot * a.q_scale, 0.f, 0.f);
                 } else if (KIND == 2) {
                     const float step = softplusf_(to_f(a_now) + dtb);
                     const float g = expf(neg_rate * step);
+                    if (HAND) *scale = make_float2(g * a.q_scale, 1.f);   // what is added comes whole
                     s[0] = make_float4(g, step, g * a.q_scale, dot * a.q_scale);
                 } else {
                     const float fq = a.q_scale / sqrtf(sq + a.unit_eps), fk = 1.0f / sqrtf(sk + a.unit_eps);   // unit length per head, the query scaled
                     const float g = expf(neg_rate * softplusf_(to_f(a_now) + dtb));
                     s[0] = make_float4(g, g * fk, sigmoidf_(to_f(b_now)), fk);
+                    if (HAND) *scale = make_float2(g * fq, dot * fq * fk);
                     s[1] = make_float4(g * fq, dot * fq * fk, 0.f, 0.f);
                 }
+            }
+        };
+        // the read-outs of this warp's tokens of chunk t0: the parts by a binary tree, as lanes add them by xor-shuffles
+        [[maybe_unused]] auto read_out = [&](int t0) {
+            const int left = min(mine, n - t0 - w * mine), c = t0 / chunk;
+            const float *from = read_outs + ((c & 1) * chunk + w * mine) * RO::kFloats;
+            const int64_t out_ld = static_cast<int64_t>(H) * V;
+            float *out = a.out + (static_cast<int64_t>(q0) + t0 + w * mine) * out_ld + h * V + jb;
+#pragma unroll 2
+            for (int i = lane; i < left * COLS; i += 32) {
+                const int t = i / COLS, col = i % COLS;
+                const float *r = from + t * RO::kFloats + col;
+                float o[PW];
+#pragma unroll
+                for (int p = 0; p < PW; ++p) o[p] = r[p * RO::kPart];
+#pragma unroll
+                for (int x = 1; x < PW; x <<= 1)
+#pragma unroll
+                    for (int p = 0; p < PW; p += 2 * x) o[p] += o[p + x];
+                const float2 f = out_scale[c & 3][w * mine + t];
+                if (jb + col < V) out[t * out_ld + col] = fmaf(f.x, o[0], f.y * r[RO::kAdd]);
             }
         };
         issue(0, sm);
@@ -324,9 +367,12 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncwarp();
             if (t0 + chunk < n) scalars(t0 + chunk, sm + nxt * chunk_bytes);
+            if constexpr (HAND)
+                if (t0 > 0) read_out(t0 - chunk);
             cur = nxt;
             __syncthreads();
         }
+        if constexpr (HAND) read_out((n - 1) / chunk * chunk);
         return;
     }
     // ---- compute: rows part * R + r of columns j and j + 1 ----
@@ -392,13 +438,16 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
     const int64_t out_ld = static_cast<int64_t>(H) * V;
     float *out = a.out + static_cast<int64_t>(q0 - 1) * out_ld + h * V + jo;   // of the token before the one in hand
     const bool writes = part < 2 && jo < V;
-    // The read-out of a token: its sums over the lanes are shuffled beside the next token's, so that their latencies are one.  Each of two
+    // The read-out of a token: a lane's sums go to the staging warps (HAND), or its
+    // sums over the lanes are shuffled beside the next token's, so that their latencies are one.  Each of two
     // neighbouring parts takes one column: o_mine + the neighbour's o_give, over the lanes, times o_scale, plus o_add.
     float o_mine = 0.f, o_give = 0.f, o_scale = 0.f, o_add = 0.f;
     __syncthreads();
     int cur = 0;
     for (int t0 = 0; t0 < n; t0 += chunk) {
         const unsigned char *buf = sm + cur * chunk_bytes;
+        [[maybe_unused]] float *ro_t = nullptr;
+        if constexpr (HAND) ro_t = read_outs + (t0 / chunk & 1) * chunk * RO::kFloats + part * RO::kPart + jl;
         const int nt = min(chunk, n - t0);
         struct {
             uint4 k[NP], q[NP];
@@ -419,11 +468,11 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
                 for (int p = 0; p < R / 4; ++p) tk.d[p] = *reinterpret_cast<const ulonglong2 *>(row + L::kDecay + part * R * 4 + p * 16);
             }
             tk.s0 = *reinterpret_cast<const float4 *>(row + L::kScalars);
-            if (KIND == 1) tk.s1 = *reinterpret_cast<const float2 *>(row + L::kScalars + 16);
+            if (KIND == 1 && !HAND) tk.s1 = *reinterpret_cast<const float2 *>(row + L::kScalars + 16);
             fetch_pair(reinterpret_cast<const T *>(row + L::kV) + jl, tk.va, tk.vb);
         };
         if (!SHORT) fetch(0);
-        constexpr int kUnroll = SHORT ? 1 : 4;
+        constexpr int kUnroll = SHORT ? 1 : HAND ? (KIND == 1 ? 6 : 8) : 4;   // delta rule, handed over, 4, 5, 6, 7, 8: 725, 716, 701, 728, 711 us (16: 1148, the instruction cache)
 #pragma unroll kUnroll
         for (int i = 0; i < nt; ++i) {
             if (SHORT) fetch(i);   // registers for more warps instead of a token ahead
@@ -446,12 +495,12 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
             uint64_t g2 = 0;
             if (KIND == 1) {
                 float ka = row_sum<R>(Sa, k2), kb = row_sum<R>(Sb, k2);
-                o += __shfl_xor_sync(0xffffffffu, o_give, CW);
+                if (!HAND) o += __shfl_xor_sync(0xffffffffu, o_give, CW);
 #pragma unroll
                 for (int x = CW; x < 32; x <<= 1) {
                     ka += __shfl_xor_sync(0xffffffffu, ka, x);
                     kb += __shfl_xor_sync(0xffffffffu, kb, x);
-                    if (x > CW) o += __shfl_xor_sync(0xffffffffu, o, x);
+                    if (!HAND && x > CW) o += __shfl_xor_sync(0xffffffffu, o, x);
                 }
                 ua = s0.z * fmaf(-s0.y, ka, va);                   // the decayed state's answer to k
                 ub = s0.z * fmaf(-s0.y, kb, vb);
@@ -459,9 +508,11 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
                 wb = s0.w * ub;
                 g2 = pk2(s0.x, s0.x);
             } else {
-                o += __shfl_xor_sync(0xffffffffu, o_give, CW);
+                if (!HAND) {
+                    o += __shfl_xor_sync(0xffffffffu, o_give, CW);
 #pragma unroll
-                for (int x = 2 * CW; x < 32; x <<= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
+                    for (int x = 2 * CW; x < 32; x <<= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
+                }
                 wa = ua = KIND == 2 ? s0.y * va : va;
                 wb = ub = KIND == 2 ? s0.y * vb : vb;
                 if (KIND == 2) g2 = pk2(s0.x, s0.x);
@@ -470,14 +521,22 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
                     for (int p = 0; p < R / 2; ++p) q2[p] = mul2(q2[p], d2[p]);
                 }
             }
-            if (writes && t0 + i > 0) *out = fmaf(o_scale, o, o_add);
-            out += out_ld;
+            if (!HAND) {
+                if (writes && t0 + i > 0) *out = fmaf(o_scale, o, o_add);
+                out += out_ld;
+            }
             const float qa = row_sum<R>(Sa, q2), qb = row_sum<R>(Sb, q2);
-            o_mine = (part & 1) ? qb : qa;
-            o_give = (part & 1) ? qa : qb;
-            o_scale = KIND == 1 ? s1.x : (KIND == 2 ? s0.z : s0.x);
-            o_add = (KIND == 1 ? s1.y : (KIND == 2 ? s0.w : s0.y)) * ((part & 1) ? ub : ua);
-            if (KIND == 2) o_add = fmaf(skip, (part & 1) ? vb : va, o_add);
+            if constexpr (HAND) {
+                *reinterpret_cast<float2 *>(ro_t + i * RO::kFloats) = make_float2(qa, qb);
+                const float add_a = KIND == 2 ? fmaf(skip, va, s0.w * ua) : ua, add_b = KIND == 2 ? fmaf(skip, vb, s0.w * ub) : ub;
+                if (part == 0) *reinterpret_cast<float2 *>(ro_t + i * RO::kFloats + RO::kAdd) = make_float2(add_a, add_b);
+            } else {
+                o_mine = (part & 1) ? qb : qa;
+                o_give = (part & 1) ? qa : qb;
+                o_scale = KIND == 1 ? s1.x : (KIND == 2 ? s0.z : s0.x);
+                o_add = (KIND == 1 ? s1.y : (KIND == 2 ? s0.w : s0.y)) * ((part & 1) ? ub : ua);
+                if (KIND == 2) o_add = fmaf(skip, (part & 1) ? vb : va, o_add);
+            }
             const uint64_t wa2 = pk2(wa, wa), wb2 = pk2(wb, wb);
 #pragma unroll
             for (int p = 0; p < R / 2; ++p) {
@@ -488,10 +547,12 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
         cur = cur + 1 == kScanBuffers ? 0 : cur + 1;
         __syncthreads();
     }
-    o_mine += __shfl_xor_sync(0xffffffffu, o_give, CW);
+    if (!HAND) {
+        o_mine += __shfl_xor_sync(0xffffffffu, o_give, CW);
 #pragma unroll
-    for (int x = 2 * CW; x < 32; x <<= 1) o_mine += __shfl_xor_sync(0xffffffffu, o_mine, x);
-    if (writes) *out = fmaf(o_scale, o_mine, o_add);
+        for (int x = 2 * CW; x < 32; x <<= 1) o_mine += __shfl_xor_sync(0xffffffffu, o_mine, x);
+        if (writes) *out = fmaf(o_scale, o_mine, o_add);
+    }
 #pragma unroll
     for (int i = 0; i < R / 2; ++i) {
         float2 x[2];
@@ -526,10 +587,11 @@ template <typename T, int KIND, int R, int PW, int NW, int NB, bool SHORT = fals
 cudaError_t launch_scan(const atoma_state_scan_args &a, cudaStream_t stream) {
     using L = Staged<T, KIND, R, PW, NW>;
     // staged tokens per buffer: at most 32, no more than the longest portion can have, and NB CTAs' buffers fit one SM
-    const int64_t fit = 200 * 1024 / NB / (kScanBuffers * L::kBytes);
+    constexpr int kOutBytes = kHandOver<KIND, R, PW, SHORT> ? 2 * ReadOut<PW, NW>::kFloats * 4 : 0;
+    const int64_t fit = 200 * 1024 / NB / (kScanBuffers * L::kBytes + kOutBytes);
     const int chunk = SHORT ? 4 : static_cast<int>(std::max<int64_t>(4, std::min<int64_t>({32, (longest_portion(a) + 3) / 4 * 4, fit / 4 * 4})));
     const int buffers = a.T <= chunk ? 1 : kScanBuffers;   // a step of one chunk fills the first only (whatever share of it is whose: a sequence may have no token)
-    const size_t smem = static_cast<size_t>(buffers) * chunk * L::kBytes + (SHORT ? StateTile<R, PW, NW>::kBytes : 0);
+    const size_t smem = static_cast<size_t>(buffers) * chunk * L::kBytes + (SHORT ? StateTile<R, PW, NW>::kBytes : chunk * kOutBytes);
     if (smem > 48 * 1024) cudaFuncSetAttribute(state_scan_kernel<T, KIND, R, PW, NW, NB, SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
     // copies in pieces of 16 bytes where every row and size allows it, else of 4, else value by value
     const int64_t size = sizeof(T);
