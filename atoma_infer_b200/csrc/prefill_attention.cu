@@ -45,6 +45,7 @@
 #include "common.cuh"
 #include "mha_params.h"
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -185,7 +186,7 @@ __device__ __forceinline__ PfSeq pf_seq(const MhaParams &p, int bidb) {
     const int k_first = (p.cu_k && p.k_cumulative) ? p.cu_k[bidb] : -1, k_start = p.k_batched ? -1 : k_first;
     const int len_k_cache = p.cu_k ? (p.k_cumulative ? p.cu_k[bidb + 1] - k_first : p.cu_k[bidb]) : p.seqlen_k;
     s.len_k = p.seqused_k ? p.seqused_k[bidb] : len_k_cache;
-    if (p.k_batched) s.len_k = min(s.len_k, p.seqlen_k);   // the rows that there are
+    if (p.k_batched) s.len_k = min(s.len_k, p.k_batched);   // the rows that there are
     s.q_off = s.q_start < 0 ? bidb * p.q_bs : static_cast<int64_t>(s.q_start) * p.q_rs;
     s.o_off = s.q_start < 0 ? bidb * p.o_bs : static_cast<int64_t>(s.q_start) * p.o_rs;
     s.k_off = k_start < 0 ? bidb * p.k_bs : static_cast<int64_t>(k_start) * p.k_rs;
@@ -815,8 +816,9 @@ bool launch_prefill(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensor
 constexpr int64_t kPfGatherBytes = 256ll << 20;   // of scratch at most; longer steps stay with the pages
 constexpr int kPfGatherQ = 256, kPfGatherK = 2048;
 int try_launch_gathered(const MhaParams &p, bool is_bf16, const CUtensorMap &mq, cudaStream_t stream) {
-    const int64_t row = static_cast<int64_t>(p.h_k) * p.d, bytes = static_cast<int64_t>(p.b) * p.seqlen_k * row * 2;
-    if (p.d != 128 || p.seqlen_q < kPfGatherQ || p.seqlen_k < kPfGatherK || 2 * bytes > kPfGatherBytes) return 0;
+    // rows for whatever a block table can name: a sequence may be longer than the caller's bound, as it may on the pages
+    const int64_t row = static_cast<int64_t>(p.h_k) * p.d, pitch = std::max<int64_t>(p.seqlen_k, p.bt_bs * p.page), bytes = static_cast<int64_t>(p.b) * pitch * row * 2;
+    if (p.d != 128 || p.seqlen_q < kPfGatherQ || p.seqlen_k < kPfGatherK || pitch > (1 << 24) || 2 * bytes > kPfGatherBytes) return 0;
     // The copy and the kernel that reads it are enqueued together: another thread may use this stream and its scratch.
     static std::mutex together;
     std::lock_guard<std::mutex> lock(together);
@@ -825,13 +827,13 @@ int try_launch_gathered(const MhaParams &p, bool is_bf16, const CUtensorMap &mq,
     MhaParams pp = p;
     pp.block_table = nullptr;
     pp.k = space, pp.v = space + bytes;
-    pp.k_hs = pp.v_hs = p.d, pp.k_rs = pp.v_rs = row, pp.k_bs = pp.v_bs = p.seqlen_k * row;
-    pp.k_batched = 1;
+    pp.k_hs = pp.v_hs = p.d, pp.k_rs = pp.v_rs = row, pp.k_bs = pp.v_bs = pitch * row;
+    pp.k_batched = static_cast<int>(pitch);
     CUtensorMap mk, mv;
-    if (!make_attn_map(&mk, pp.k, p.d, p.h_k, p.seqlen_k, p.b, pp.k_hs, pp.k_rs, pp.k_bs, is_bf16)) return -1;
-    if (!make_attn_map(&mv, pp.v, p.d, p.h_k, p.seqlen_k, p.b, pp.v_hs, pp.v_rs, pp.v_bs, is_bf16)) return -1;
-    const dim3 grid(static_cast<unsigned>((p.seqlen_k + kPfGatherWarps - 1) / kPfGatherWarps), static_cast<unsigned>(p.b));
-    const cudaError_t e = launch_ex(paged_rows_kernel, grid, dim3(32 * kPfGatherWarps), 0, stream, p, reinterpret_cast<uint4 *>(space), reinterpret_cast<uint4 *>(space + bytes), p.seqlen_k);
+    if (!make_attn_map(&mk, pp.k, p.d, p.h_k, pitch, p.b, pp.k_hs, pp.k_rs, pp.k_bs, is_bf16)) return -1;
+    if (!make_attn_map(&mv, pp.v, p.d, p.h_k, pitch, p.b, pp.v_hs, pp.v_rs, pp.v_bs, is_bf16)) return -1;
+    const dim3 grid(static_cast<unsigned>((pitch + kPfGatherWarps - 1) / kPfGatherWarps), static_cast<unsigned>(p.b));
+    const cudaError_t e = launch_ex(paged_rows_kernel, grid, dim3(32 * kPfGatherWarps), 0, stream, p, reinterpret_cast<uint4 *>(space), reinterpret_cast<uint4 *>(space + bytes), static_cast<int>(pitch));
     note_launch();
     if (e != cudaSuccess) {
         set_status(static_cast<int>(e), "paged_rows_kernel: %s", cudaGetErrorString(e));

@@ -75,7 +75,7 @@ def test_gathered_steps_give_the_bits_of_pages(dtype, H, G, page, news, contexts
     run = lambda longest: ops.flash_attn_varlen_with_block_table(q, kc, vc, None, starts(news), starts(lens), max(news), longest, D ** -0.5, None, 0, table.to(DEV))
     got = run(max(lens))
     assert ops.last_mha_path() == "prefill_tc"
-    assert torch.equal(got, run(1 << 22))
+    assert torch.equal(got, run(1 << 22)) and torch.equal(got, run(2048))      # 2048: a bound that some sequences exceed
     _check(got, q, k, v, news, contexts)
     assert hybrid_ops.prefill_timeouts() == 0
 
