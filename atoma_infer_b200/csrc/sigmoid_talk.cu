@@ -466,12 +466,13 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
         return NT % pieces == 0 ? Piece{tid / pieces, NT / pieces, e * 8, g * kS3Keys * (n + 8) + e * 8 - g * n} : Piece{0, 0, 0, 0};
     };
     const Piece k_piece = TMA ? Piece{} : piece_of(D), v_piece = TMA ? Piece{} : piece_of(DV);
-    auto stage = [&](const __nv_bfloat16 *cache, __nv_bfloat16 *dst, int n, const Piece &pc, const int32_t *at) {
+    // Keys or values of tile j.  The map and the barrier come with the call: one cache may serve as both.
+    auto stage = [&](const CUtensorMap *map, uint64_t *full, const __nv_bfloat16 *cache, __nv_bfloat16 *dst, int n, const Piece &pc, int j) {
+        const int32_t *at = slot_s[j & 3];
         if constexpr (TMA) {
             if (tid == 0) {
-                uint64_t *bar = cache == kc ? &k_full[dst != Ks] : &v_full[dst != Vs];
-                mbar_arrive_expect_tx(bar, G * kS3Keys * 128);
-                s3_load(dst, cache == kc ? &map_k : &map_v, bar, max(at[0], 0));
+                mbar_arrive_expect_tx(&full[j & 1], G * kS3Keys * 128);
+                s3_load(dst, map, &full[j & 1], max(at[0], 0));
             }
         } else if (pc.step) {
             for (int jj = pc.key; jj < kS3Keys; jj += pc.step) {
@@ -487,8 +488,8 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
         }
     };
     const int tiles = (j_end - j_begin + kS3Keys - 1) / kS3Keys;
-    stage(kc, Ks, D, k_piece, slot_s[0]);
-    if (tiles > 1) stage(kc, Ks + k_tile, D, k_piece, slot_s[1]);
+    stage(&map_k, k_full, kc, Ks, D, k_piece, 0);
+    if (tiles > 1) stage(&map_k, k_full, kc, Ks + k_tile, D, k_piece, 1);
     cp_async_commit();
     // ---- the talk matrix in three pieces, rows of heads h: [t0 | t1], then [t2 | -] ----
     for (int i = tid; i < H * H; i += NT) {
@@ -663,8 +664,8 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
         // its own pace, so that one's exponentials run beside another's products.
         cp_async_wait_all();
         __syncthreads();
-        stage(vc, Vs + (j & 1) * v_tile, DV, v_piece, slot_s[j & 3]);
-        if (j + 2 < tiles) stage(kc, Ks + (j & 1) * k_tile, D, k_piece, slot_s[(j + 2) & 3]);
+        stage(&map_v, v_full, vc, Vs + (j & 1) * v_tile, DV, v_piece, j);
+        if (j + 2 < tiles) stage(&map_k, k_full, kc, Ks + (j & 1) * k_tile, D, k_piece, j + 2);
         cp_async_commit();
         int next_slot = 0;
         if (tid < kS3Keys) next_slot = look_up(j_begin + (j + 3) * kS3Keys + tid);

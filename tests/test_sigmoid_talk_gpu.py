@@ -5,6 +5,7 @@ rounded to bfloat16 (8 bits: 2^-8 of it at most) before it meets the value, the 
 import pytest
 import torch
 
+from atoma_infer_b200 import _lib
 from atoma_infer_b200 import hybrid_ops as ops
 from helpers import randn_t
 
@@ -138,6 +139,22 @@ def test_same_bits_whatever_the_pages(G):
             used, row = used + each[b], row + n
         outs.append(ops.sigmoid_attention_paged(q, kc, vc, pos, tseq, table.to(DEV), None, hb, talk, H, G, D, D, bs, D ** -0.5, 8.0, 49))
     assert torch.isfinite(outs[0]).all() and all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
+@pytest.mark.parametrize("H,G,bs", [(32, 8, 16), (32, 2, 24), (16, 4, 16)])
+def test_one_cache_as_keys_and_values(H, G, bs):
+    """A cache that serves as both gives the bits of two caches with the same rows: by TMA (pages of whole 16-key tiles), by pieces, and for 16 heads."""
+    D, seqs = 64, ((0, 49), (300, 2))
+    each = [-(-(c + n) // bs) for c, n in seqs]
+    table = torch.zeros((2, max(each)), dtype=torch.int32)
+    table[0, :each[0]], table[1, :each[1]] = torch.arange(each[0]), torch.arange(each[0], sum(each))
+    kc, q = randn_t((sum(each) * bs, G, D), 1, torch.bfloat16, DEV), randn_t((51, H * D), 3, torch.bfloat16, DEV)
+    hb, talk = randn_t((H,), 4, torch.float32, DEV), torch.eye(H, device=DEV) + randn_t((H, H), 5, torch.float32, DEV, scale=0.3)
+    pos = torch.cat([torch.arange(c, c + n) for c, n in seqs]).to(DEV)
+    tseq = torch.tensor([0] * 49 + [1] * 2, dtype=torch.int32, device=DEV)
+    run = lambda vc: ops.sigmoid_attention_paged(q, kc, vc, pos, tseq, table.to(DEV), None, hb, talk, H, G, D, D, bs, D ** -0.5, 8.0, 49)
+    given_up = _lib.lib().atoma_kernel_timeouts()
+    assert torch.equal(run(kc), run(kc.clone())) and _lib.lib().atoma_kernel_timeouts() == given_up
 
 
 def test_capture_on_a_stream_without_scratch():
