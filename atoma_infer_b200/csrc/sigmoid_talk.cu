@@ -11,15 +11,16 @@
 // 2^-25 of a term).
 // One CTA holds all heads (64 accumulator registers per thread for two heads), so there is no cluster exchange, and the keys are cut into segments,
 // whose float32 sums simply add (no softmax): 128 row blocks of one prompt over 74 CTA pairs left the SMs idle half of the time.  A
-// segment is 256 or 512 keys (by the heads) from a multiple of that on whatever the step looks like, so a position's sums depend on its keys alone.  A CTA takes one
-// segment, two neighbours in steps of many, or, in steps whose row blocks fill the SMs without, all of its rows' segments one after the other; the sums between take
+// segment is 512 keys (sigmoid_talk32_kernel: 256) from a multiple of that on whatever the step looks like, so a position's sums depend on its keys alone.  A CTA takes one
+// segment (of the shorter ones two neighbours in steps of many), or, in steps whose row blocks fill the SMs without, all of its rows' segments one after the other; the sums between take
 // at most 256 MiB (kStScratch), and longer steps go in runs of tokens.  Keys of the next tile are copied under the mix, values under the scores.
-// A tile of 2048 tokens, 32 heads of 64 on 8, takes 14000 cycles here (sigmoid_talk32_kernel serves 32 heads where its tiles fit): scores and weights 6000 (four results of the special-function unit per weight are 4100 of them),
+// 32 heads of 64 in pages of whole runs of eight keys go by sigmoid_talk32_kernel, all others by sigmoid_talk_kernel, whose figures these are.  A tile of 2048 tokens, 32 heads
+// of 64 on 8, takes 14000 cycles: scores and weights 6000 (four results of the special-function unit per weight are 4100 of them),
 // the mix 5000 (3100 of the tensor pipe), values 2000.  With 27000: every copy waited for its own block-table entry (5000), a branch per weight kept
 // their chains from overlapping, quotients and exponentials took denormal numbers into account, and registers spilled.
-// 2048 tokens, 32 heads of 64 on 8: 1218 us on the CUDA-core mix (hybrid_attention.cu), 507 with those, 283 here; 2000 tokens of 16 heads 328 and 169.  Prompts of up to
+// 2048 tokens, 32 heads of 64 on 8: 1218 us on the CUDA-core mix (hybrid_attention.cu), 507 with those, 283 now; 2000 tokens of 16 heads 328 and 169.  Prompts of up to
 // some 40 tokens are slower than on CUDA cores, since all heads wait for each other in one CTA (33 tokens of 16 and 32 heads 15.9 and 24.2 us, there 14.3 and 19.1;
-// 64 tokens 16.4 and 26.6, there 22.6 and 32.8); they stay here, so that a position's bits do not follow the step.
+// 64 tokens 16.4 and 26.6, there 22.6 and 32.8); they stay, so that a position's bits do not follow the step.
 #include "common.cuh"
 #include "hybrid_common.cuh"
 
@@ -34,9 +35,10 @@ namespace {
 using namespace hybrid;
 
 constexpr int kStRows = 16, kStKeys = 32, kStPieces = 3;
-// Keys of a segment.  Shorter ones put short prompts on more SMs (32 heads, 600 and 1000 tokens, 512 / 256: 117 / 66, 119 / 68 us; 128 lose from 1000 tokens on) and
-// cost long ones more sums (16 heads, 2000 tokens: 166 / 171).
-constexpr int st_seg_keys(int heads) { return heads == 32 ? 256 : 512; }
+// Keys of a segment, of sigmoid_talk_kernel and of sigmoid_talk32_kernel.  Shorter ones put short prompts on more SMs and cost long ones more sums.  The first, 512 / 256: 16 heads,
+// 2000 tokens 166 / 171 us; 32 heads of 32 and 48 on 16, 1000 and 4000 tokens 153 / 89, 1015 / 1143.  The second: 600 and 1000 tokens 117 / 66, 119 / 68, long ones faster than on the
+// first all the same; 128 lose from 1000 tokens on.
+constexpr int kStSegKeys = 512, kS3SegKeys = 256;
 constexpr int64_t kStScratch = 256ll << 20;
 
 // sigmoid(cap tanh(s / cap) - slope dist + bias), tanh(y) = 1 - 2 / (1 + e^2y).  The unit's estimates of 2^x and of the reciprocal are within 2 and 1 units of the last
@@ -79,22 +81,21 @@ __device__ __forceinline__ void st_split(float x, float (&piece)[kStPieces]) {
 // (blockIdx.z: which segment this CTA takes; sigmoid_talk_sum_kernel adds them), or 1: this CTA takes them all and keeps the running sum there.  Both add the
 // segments in order, so they give the same bits.  No scratch: one chain over all keys.
 template <int HT>
-__global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_sigmoid_attn_args a, int lo, int hi, int slots, int per, float *__restrict__ partial) {
+__global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_sigmoid_attn_args a, int lo, int hi, int slots, float *__restrict__ partial) {
     using L = StLayout<HT>;
-    constexpr int kStSegKeys = st_seg_keys(L::H), H = L::H, NW = 8 * HT, NT = 256 * HT;
+    constexpr int H = L::H, NW = 8 * HT, NT = 256 * HT;
     extern __shared__ __align__(16) unsigned char sm[];
     pdl_launch_dependents();
     pdl_wait();
     const int G = static_cast<int>(a.G), D = static_cast<int>(a.dim), DV = static_cast<int>(a.vdim), bs = static_cast<int>(a.block_size);
-    const int b = blockIdx.y;
-    int seg = blockIdx.z * per;   // the segment in hand
+    const int b = blockIdx.y, seg = blockIdx.z;
     const int t_begin = a.query_start[b], n_q = a.query_start[b + 1] - t_begin;
     const int first = max(0, lo - t_begin + kStRows - 1) / kStRows, last = (min(n_q, hi - t_begin) + kStRows - 1) / kStRows - 1;   // this run's row blocks
     const int blk = last - static_cast<int>(blockIdx.x);   // the rows with the most keys first
     if (n_q <= 0 || blk < first) return;
     const int r0 = blk * kStRows, rows = min(kStRows, n_q - r0), tok0 = t_begin + r0;
     const int ctx = static_cast<int>(a.positions[t_begin]), p0 = ctx + r0, total = ctx + n_q;
-    const int all_end = p0 + rows, j_begin = seg * kStSegKeys, j_end = seg + per >= slots ? all_end : min(all_end, j_begin + per * kStSegKeys);
+    const int all_end = p0 + rows, j_begin = seg * kStSegKeys, j_end = seg == slots - 1 ? all_end : min(all_end, j_begin + kStSegKeys);
     if (j_begin >= all_end) return;
     const int32_t *bt = a.block_tables + static_cast<int64_t>(b) * a.max_blocks;
     unsigned char *weights = sm + L::w_off, *mix = sm + L::m_off, *talk = sm + L::t_off;
@@ -348,10 +349,9 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
                     }
             }
         }
-        if (partial && j0 + kStKeys < j_end && (j0 + kStKeys) % kStSegKeys == 0 && (slots == 1 || seg + 1 < slots)) {   // a segment ends here
+        if (slots == 1 && partial && j0 + kStKeys < j_end && (j0 + kStKeys) % kStSegKeys == 0) {   // a segment ends here
             put(false);
-            if (slots == 1) more = true;
-            else ++seg;
+            more = true;
             fresh = true;
             clear();
         } else if constexpr (HT == 2) {
@@ -384,11 +384,12 @@ constexpr int kS3Keys = 16, kS3Tries = 1 << 18;
 struct S3Layout {
     static constexpr int kPair = 4 * 32 + 16, kRow = kS3Keys * kPair + 16, kW = kStRows * kRow;      // bytes: a pair's weights, a query row's, a tile's
     static constexpr int kMixRow = 2 * kS3Keys + 16, kMixHead = kStRows * kMixRow + 16, kMix = 32 * kMixHead;
-    static constexpr int t_off = 0, kv_off = 8192;   // t, and keys and values by TMA: rows of 128 swizzled bytes
-    __host__ __device__ static constexpr int k_tile(int G, int D, bool tma) { return G * kS3Keys * (tma ? 64 : D + 8); }   // elements
-    __host__ __device__ static size_t total(int G, int D, int DV, bool tma) { return 1024 + kv_off + 2 * kW + 2 * kMix + 4 * (static_cast<size_t>(k_tile(G, D, tma)) + k_tile(G, DV, tma)); }
+    static constexpr int t_off = 0, kv_off = 8192;   // t, and keys and values: rows of 128 swizzled bytes
+    __host__ __device__ static constexpr int tile(int G) { return G * kS3Keys * 64; }   // elements: eight keys of every head, then the other eight
+    __host__ __device__ static constexpr int total(int G) { return 1024 + kv_off + 2 * kW + 2 * kMix + 4 * 2 * tile(G); }
 };
-constexpr int kS3Smem = 226 * 1024;
+constexpr int kS3Groups = 8, kS3Smem = S3Layout::total(kS3Groups);   // key heads at most; the next number that divides 32 does not fit
+static_assert(kS3Smem <= 226 * 1024, "shared memory of a CTA");
 constexpr int kS3Block = 112, kS3D = 48, kS3D12 = 80, kS3Q = 224;   // tensor-memory columns of 128 pairs: pieces, D0, D12; behind both blocks': the queries
 
 __device__ __forceinline__ void s3_st8(uint32_t taddr, const uint32_t (&r)[8]) {
@@ -397,23 +398,24 @@ __device__ __forceinline__ void s3_st8(uint32_t taddr, const uint32_t (&r)[8]) {
                  : "memory");
 }
 
-__device__ __forceinline__ void s3_load(void *dst, const CUtensorMap *map, uint64_t *bar, int row) {   // 16 rows of all heads
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(0), "r"(row), "r"(0)
+__device__ __forceinline__ void s3_load(void *dst, const CUtensorMap *map, uint64_t *bar, int row) {   // 8 or 16 rows (the map's box) of all heads, from a multiple of 8 on
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %3, %3, %4}], [%2];" ::"r"(smem_u32(dst)),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(0), "r"(row >> 3)
                  : "memory");
 }
 
-// TMA: heads of 64 whose pages are whole tiles: a tile's keys are neighbours in the cache and go by one copy each of keys and values.  The cp.async pieces of other
-// shapes cost a tile 1100 to 1700 cycles of issue.
-template <bool TMA>
+// For heads of 64 whose pages are whole runs of eight keys: a tile goes by one TMA copy each of keys and values, by two where its halves may lie in different pages.  With
+// cp.async pieces instead (1100 to 1700 cycles of issue a tile) this kernel loses on long prompts to the one above: 4000 tokens of 32 heads of 64 on 8 in pages of 8 or 4 keys 975 us
+// there, 1107 here by pieces, 862 (pages of 8) here by TMA; of 48 and 32 on 8 912 and 975; of 32 and 48 on 16 1015 and 1143.
 __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const atoma_sigmoid_attn_args a, int lo, int hi, int slots, int per, float *__restrict__ partial, unsigned int *late_out) {
     using L = S3Layout;
-    constexpr int H = 32, NT = 512, kStSegKeys = st_seg_keys(32);
+    constexpr int H = 32, NT = 512;
     extern __shared__ unsigned char sm_raw[];
     unsigned char *sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
     pdl_launch_dependents();
     pdl_wait();
-    const int G = static_cast<int>(a.G), D = TMA ? 64 : static_cast<int>(a.dim), DV = TMA ? 64 : static_cast<int>(a.vdim), bs = static_cast<int>(a.block_size);
+    constexpr int D = 64, DV = 64;
+    const int G = static_cast<int>(a.G), bs = static_cast<int>(a.block_size);
     const int b = blockIdx.y;
     int seg = blockIdx.z * per;   // the segment in hand
     const int t_begin = a.query_start[b], n_q = a.query_start[b + 1] - t_begin;
@@ -422,16 +424,15 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
     if (n_q <= 0 || blk < first) return;
     const int r0 = blk * kStRows, rows = min(kStRows, n_q - r0), tok0 = t_begin + r0;
     const int ctx = static_cast<int>(a.positions[t_begin]), p0 = ctx + r0, total = ctx + n_q;
-    const int all_end = p0 + rows, j_begin = seg * kStSegKeys, j_end = seg + per >= slots ? all_end : min(all_end, j_begin + per * kStSegKeys);
+    const int all_end = p0 + rows, j_begin = seg * kS3SegKeys, j_end = seg + per >= slots ? all_end : min(all_end, j_begin + per * kS3SegKeys);
     if (j_begin >= all_end) return;
     const int32_t *bt = a.block_tables + static_cast<int64_t>(b) * a.max_blocks;
     unsigned char *talk = sm + L::t_off;
-    const int k_tile = L::k_tile(G, D, TMA), v_tile = L::k_tile(G, DV, TMA);
-    __nv_bfloat16 *Ks = reinterpret_cast<__nv_bfloat16 *>(sm + L::kv_off), *Vs = Ks + 2 * k_tile;
-    unsigned char *weights = reinterpret_cast<unsigned char *>(Vs + 2 * v_tile), *mix = weights + 2 * L::kW;
+    const int tile = L::tile(G);
+    __nv_bfloat16 *Ks = reinterpret_cast<__nv_bfloat16 *>(sm + L::kv_off), *Vs = Ks + 2 * tile;
+    unsigned char *weights = reinterpret_cast<unsigned char *>(Vs + 2 * tile), *mix = weights + 2 * L::kW;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t4 = lane & 3, rq = lane >> 2;
-    const __nv_bfloat16 *kc = static_cast<const __nv_bfloat16 *>(a.k_cache), *vc = static_cast<const __nv_bfloat16 *>(a.v_cache);
-    __shared__ int32_t slot_s[4][kS3Keys];   // cache rows of a tile's keys (-1: behind the sequence's end), looked up three tiles ahead
+    __shared__ int32_t slot_s[4][2];   // cache rows of a tile's first and ninth key (-1: behind the sequence's end), looked up three tiles ahead
     __shared__ __align__(8) uint64_t split[2], mixed[2], k_full[2], v_full[2];   // split, mixed: of 128 pairs each
     __shared__ uint32_t tmem_base_s;
     __shared__ int late_s;
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
         const int pg = bs_shift >= 0 ? j >> bs_shift : j / bs;
         return j < total ? bt[pg] * bs + (j - pg * bs) : -1;
     };
-    if (tid < 3 * kS3Keys) slot_s[tid / kS3Keys][tid % kS3Keys] = look_up(j_begin + tid);
+    if (tid < 6) slot_s[tid / 2][tid % 2] = look_up(j_begin + tid * 8);
     if (tid == 0) {
         late_s = 0;
         for (int i = 0; i < 2; ++i) {
@@ -457,40 +458,19 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_s;
-    // A thread's piece of a row is the same for all its keys where the CTA takes whole rows at a time; what it takes to find it is worked out once.
-    struct Piece {
-        int key, step, src, dst;   // first key, keys apart; elements into a key's row of the cache, into the tile
-    };
-    auto piece_of = [&](int n) {
-        const int pieces = G * n / 8, e = tid % pieces, g = e * 8 / n;
-        return NT % pieces == 0 ? Piece{tid / pieces, NT / pieces, e * 8, g * kS3Keys * (n + 8) + e * 8 - g * n} : Piece{0, 0, 0, 0};
-    };
-    const Piece k_piece = TMA ? Piece{} : piece_of(D), v_piece = TMA ? Piece{} : piece_of(DV);
-    // Keys or values of tile j.  The map and the barrier come with the call: one cache may serve as both.
-    auto stage = [&](const CUtensorMap *map, uint64_t *full, const __nv_bfloat16 *cache, __nv_bfloat16 *dst, int n, const Piece &pc, int j) {
-        const int32_t *at = slot_s[j & 3];
-        if constexpr (TMA) {
-            if (tid == 0) {
-                mbar_arrive_expect_tx(&full[j & 1], G * kS3Keys * 128);
-                s3_load(dst, map, &full[j & 1], max(at[0], 0));
-            }
-        } else if (pc.step) {
-            for (int jj = pc.key; jj < kS3Keys; jj += pc.step) {
-                const int slot = at[jj];
-                cp_async_16(smem_u32(dst + pc.dst + jj * (n + 8)), cache + static_cast<int64_t>(max(slot, 0)) * (G * n) + pc.src, slot >= 0 ? 16 : 0);
-            }
-        } else {
-            const int pieces = G * n / 8;
-            for (int i = tid; i < kS3Keys * pieces; i += NT) {
-                const int jj = i / pieces, e = i - jj * pieces, g = e * 8 / n, slot = at[jj];
-                cp_async_16(smem_u32(dst + (g * kS3Keys + jj) * (n + 8) + e * 8 - g * n), cache + static_cast<int64_t>(max(slot, 0)) * (G * n) + e * 8, slot >= 0 ? 16 : 0);
-            }
-        }
+    // Keys or values of tile j, from one thread.  The map and the barrier come with the call: one cache may serve as both.
+    const bool whole = bs % kS3Keys == 0;   // a tile lies in one page
+    auto stage = [&](const CUtensorMap *map, uint64_t *full, __nv_bfloat16 *buffers, int j) {
+        __nv_bfloat16 *dst = buffers + (j & 1) * tile;
+        mbar_arrive_expect_tx(&full[j & 1], G * kS3Keys * 128);
+        s3_load(dst, map, &full[j & 1], max(slot_s[j & 3][0], 0));
+        if (!whole) s3_load(dst + tile / 2, map, &full[j & 1], max(slot_s[j & 3][1], 0));
     };
     const int tiles = (j_end - j_begin + kS3Keys - 1) / kS3Keys;
-    stage(&map_k, k_full, kc, Ks, D, k_piece, 0);
-    if (tiles > 1) stage(&map_k, k_full, kc, Ks + k_tile, D, k_piece, 1);
-    cp_async_commit();
+    if (tid == 0) {
+        stage(&map_k, k_full, Ks, 0);
+        if (tiles > 1) stage(&map_k, k_full, Ks, 1);
+    }
     // ---- the talk matrix in three pieces, rows of heads h: [t0 | t1], then [t2 | -] ----
     for (int i = tid; i < H * H; i += NT) {
         const int h = i / H, g = i % H;
@@ -540,7 +520,7 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
     bool more = false;   // a running sum waits in this token's place
     // the sums of a segment, out of the accumulators: into its place, onto the running sum, or, where no other segment follows or precedes, out
     auto put = [&](bool end) {
-        const bool out = end && (slots == 1 || all_end <= kStSegKeys);
+        const bool out = end && (slots == 1 || all_end <= kS3SegKeys);
 #pragma unroll
         for (int x = 0; x < 2; ++x)
 #pragma unroll
@@ -572,7 +552,7 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
     // ---- scores and weights of this warp's two heads for tile j ----
     auto form_weights_as = [&](auto all_seen, int j) {
         const int j0 = j_begin + j * kS3Keys;
-        const __nv_bfloat16 *kt = Ks + (j & 1) * k_tile;
+        const __nv_bfloat16 *kt = Ks + (j & 1) * tile;
         unsigned char *wt = weights + (j & 1) * L::kW;
         const float base = static_cast<float>(p0 + rq - j0 - 2 * t4);
         float w0[2][4];
@@ -581,20 +561,19 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
             float s[2][4];
 #pragma unroll
             for (int i = 0; i < 2; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
-            const int key = kv_head[x] * kS3Keys + (lane >> 4) * 8 + (lane & 7), odd = (lane >> 3) & 1;
-            const uint32_t kb = smem_u32(kt + key * (TMA ? 64 : D + 8));
+            const int key = ((lane >> 4) * G + kv_head[x]) * 8 + (lane & 7), odd = (lane >> 3) & 1;
+            const uint32_t kb = smem_u32(kt + key * 64);
             uint32_t qf[16];
             tmem_ld_32x32b_x16(tmem_q + x * 16, qf);
             tmem_ld_wait();
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-                if (kk * 16 < D) {
-                    uint32_t r[4];
-                    const uint32_t(&qk)[4] = *reinterpret_cast<const uint32_t(*)[4]>(qf + kk * 4);
-                    ldmatrix_x4(r, kb + (TMA ? ((2 * kk + odd) ^ (lane & 7)) << 4 : kk * 32 + odd * 16));
-                    Mma16816<__nv_bfloat16>::run(s[0], qk, r[0], r[1]);
-                    Mma16816<__nv_bfloat16>::run(s[1], qk, r[2], r[3]);
-                }
+            for (int kk = 0; kk < 4; ++kk) {
+                uint32_t r[4];
+                const uint32_t(&qk)[4] = *reinterpret_cast<const uint32_t(*)[4]>(qf + kk * 4);
+                ldmatrix_x4(r, kb + (((2 * kk + odd) ^ (lane & 7)) << 4));
+                Mma16816<__nv_bfloat16>::run(s[0], qk, r[0], r[1]);
+                Mma16816<__nv_bfloat16>::run(s[1], qk, r[2], r[3]);
+            }
             // weights of hidden pairs are formed too and dropped: without a branch per weight their chains of exponentials and quotients overlap
             auto weigh = [&](auto with_cap) {
 #pragma unroll
@@ -617,42 +596,40 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
         }
     };
     auto form_weights = [&](int j) {
-        if (TMA) wait(&k_full[j & 1], (j >> 1) & 1);
+        wait(&k_full[j & 1], (j >> 1) & 1);
         if (rows == kStRows && j_begin + (j + 1) * kS3Keys - 1 <= p0) form_weights_as(std::true_type{}, j);
         else form_weights_as(std::false_type{}, j);
     };
     // this thread's pair: block of 128 pairs (8 query rows x 16 keys), and which 16 of its heads
     const int block = warp >> 3, half = (warp >> 2) & 1, pair = (warp & 3) * 32 + lane, prow = 8 * block + pair / kS3Keys, pkey = pair % kS3Keys;
     const uint32_t tmem_block = tmem_base + block * kS3Block, tmem_lane = tmem_block + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    cp_async_wait_all();
     __syncthreads();
     form_weights(0);
-    // The sequence ends inside tile j (its last one): what follows in the page is not multiplied in.  Every warp zeroes what it reads.
+    // The sequence ends inside tile j (its last one): what follows in the page (or, in a second copy, of another) is not multiplied in.  Every warp zeroes what it reads.
     auto hide_rows = [&](int j) {
         for (int x = 0; x < 2; ++x)
             for (int i = lane; i < kS3Keys * 8; i += 32)
-                if (j_begin + j * kS3Keys + i / 8 >= total) *reinterpret_cast<uint4 *>(Vs + (j & 1) * v_tile + (kv_head[x] * kS3Keys + i / 8) * 64 + i % 8 * 8) = make_uint4(0, 0, 0, 0);
+                if (j_begin + j * kS3Keys + i / 8 >= total) *reinterpret_cast<uint4 *>(Vs + (j & 1) * tile + ((i / 64 * G + kv_head[x]) * 8 + i / 8 % 8) * 64 + i % 8 * 8) = make_uint4(0, 0, 0, 0);
         __syncwarp();
     };
     // ---- values of tile j: what the mix of all heads has given this warp's two ----
     auto add_values = [&](int j) {
-        if (TMA) wait(&v_full[j & 1], (j >> 1) & 1);
-        if (TMA && j_begin + (j + 1) * kS3Keys > total) hide_rows(j);
+        wait(&v_full[j & 1], (j >> 1) & 1);
+        if (j_begin + (j + 1) * kS3Keys > total) hide_rows(j);
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
-            const uint32_t vb = smem_u32(Vs + (j & 1) * v_tile + (kv_head[x] * kS3Keys + ((lane >> 3) & 1) * 8 + (lane & 7)) * (TMA ? 64 : DV + 8));
+            const uint32_t vb = smem_u32(Vs + (j & 1) * tile + ((((lane >> 3) & 1) * G + kv_head[x]) * 8 + (lane & 7)) * 64);
             uint32_t af[4];
             ldmatrix_x4(af, smem_u32(mix + (j & 1) * L::kMix + (h0 + x) * L::kMixHead + (lane & 15) * L::kMixRow + (lane >> 4) * 16));
 #pragma unroll
-            for (int n2 = 0; n2 < 4; ++n2)
-                if (n2 * 16 < DV) {
-                    uint32_t r[4];
-                    ldmatrix_x4_trans(r, vb + (TMA ? ((2 * n2 + (lane >> 4)) ^ (lane & 7)) << 4 : n2 * 32 + (lane >> 4) * 16));
-                    Mma16816<__nv_bfloat16>::run(o[x][2 * n2], af, r[0], r[1]);
-                    Mma16816<__nv_bfloat16>::run(o[x][2 * n2 + 1], af, r[2], r[3]);
-                }
+            for (int n2 = 0; n2 < 4; ++n2) {
+                uint32_t r[4];
+                ldmatrix_x4_trans(r, vb + (((2 * n2 + (lane >> 4)) ^ (lane & 7)) << 4));
+                Mma16816<__nv_bfloat16>::run(o[x][2 * n2], af, r[0], r[1]);
+                Mma16816<__nv_bfloat16>::run(o[x][2 * n2 + 1], af, r[2], r[3]);
+            }
         }
-        if (partial && j + 1 < tiles && (j_begin + (j + 1) * kS3Keys) % kStSegKeys == 0 && (slots == 1 || seg + 1 < slots)) {   // a segment ends here
+        if (partial && j + 1 < tiles && (j_begin + (j + 1) * kS3Keys) % kS3SegKeys == 0 && (slots == 1 || seg + 1 < slots)) {   // a segment ends here
             put(false);
             if (slots == 1) more = true;
             else ++seg;
@@ -662,13 +639,13 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
     for (int j = 0; j < tiles; ++j) {
         // The one barrier of a tile: its weights, the mixed weights of the tile before, its values and the next tile's keys are there.  What follows, a warp does at
         // its own pace, so that one's exponentials run beside another's products.
-        cp_async_wait_all();
         __syncthreads();
-        stage(&map_v, v_full, vc, Vs + (j & 1) * v_tile, DV, v_piece, j);
-        if (j + 2 < tiles) stage(&map_k, k_full, kc, Ks + (j & 1) * k_tile, D, k_piece, j + 2);
-        cp_async_commit();
+        if (tid == 0) {
+            stage(&map_v, v_full, Vs, j);
+            if (j + 2 < tiles) stage(&map_k, k_full, Ks, j + 2);
+        }
         int next_slot = 0;
-        if (tid < kS3Keys) next_slot = look_up(j_begin + (j + 3) * kS3Keys + tid);
+        if (tid < 2) next_slot = look_up(j_begin + (j + 3) * kS3Keys + tid * 8);
         // ---- split ----
         {
             const float4 *w = reinterpret_cast<const float4 *>(weights + (j & 1) * L::kW + prow * L::kRow + pkey * L::kPair + half * 64);
@@ -741,13 +718,12 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
             }
         }
         tc_fence_before_sync();
-        if (tid < kS3Keys) slot_s[(j + 3) & 3][tid] = next_slot;
+        if (tid < 2) slot_s[(j + 3) & 3][tid] = next_slot;
     }
-    cp_async_wait_all();
     __syncthreads();
     add_values(tiles - 1);
     put(true);
-    if (TMA && tid == 0) {   // whatever happened to the waits, the copies have landed before the CTA leaves
+    if (tid == 0) {   // whatever happened to the waits, the copies have landed before the CTA leaves
         auto landed = [&](uint64_t *bar, int uses) {
             for (int i = 0; uses > 0 && i < kS3Tries && !mbar_try_wait(bar, (uses - 1) & 1); ++i) {
             }
@@ -796,13 +772,13 @@ bool hyb_sigmoid_talk_ok(const atoma_sigmoid_attn_args &a) {
 }
 
 namespace {
-// A cache of rows of G heads of 64: 16 rows of all heads a copy, head by head.
-bool s3_map(CUtensorMap *out, const void *cache, int G) {
+// A cache of rows of G heads of 64 as runs of eight: one or two runs a copy, in each all heads' keys, head by head.
+bool s3_map(CUtensorMap *out, const void *cache, int G, int runs) {
     EncodeTiledFn enc = get_encode_tiled();
     if (!enc) return false;
-    const cuuint64_t dims[3] = {64, 1ull << 31, static_cast<cuuint64_t>(G)}, strides[2] = {static_cast<cuuint64_t>(G) * 128, 128};
-    const cuuint32_t box[3] = {64, kS3Keys, static_cast<cuuint32_t>(G)}, estr[3] = {1, 1, 1};
-    const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(cache), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+    const cuuint64_t g = static_cast<cuuint64_t>(G), dims[4] = {64, 8, g, 1ull << 28}, strides[3] = {g * 128, 128, g * 1024};
+    const cuuint32_t box[4] = {64, 8, static_cast<cuuint32_t>(G), static_cast<cuuint32_t>(runs)}, estr[4] = {1, 1, 1, 1};
+    const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(cache), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r == CUDA_SUCCESS) return true;
     set_status(kErrDriver, "sigmoid_talk: cuTensorMapEncodeTiled failed (CUresult %d)", static_cast<int>(r));
@@ -812,7 +788,10 @@ bool s3_map(CUtensorMap *out, const void *cache, int G) {
 
 bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
     const int64_t longest = a.max_seq_len > 0 ? a.max_seq_len : a.max_blocks * a.block_size;
-    const int64_t seg_keys = st_seg_keys(static_cast<int>(a.H)), segs = std::min<int64_t>(65535, (longest + seg_keys - 1) / seg_keys), blocks = (a.T + kStRows - 1) / kStRows;
+    const int G = static_cast<int>(a.G), D = static_cast<int>(a.dim), DV = static_cast<int>(a.vdim);
+    // by the sizes of the model and its pages alone: a position's bits do not follow the step
+    const bool on_tcgen05 = a.H == 32 && D == 64 && DV == 64 && G <= kS3Groups && a.block_size % 8 == 0;
+    const int64_t seg_keys = on_tcgen05 ? kS3SegKeys : kStSegKeys, segs = std::min<int64_t>(65535, (longest + seg_keys - 1) / seg_keys), blocks = (a.T + kStRows - 1) / kStRows;
     const int64_t place = a.H * a.vdim * 4;   // bytes of a token's sums
     int64_t slots = 1, run = a.T;
     float *partial = nullptr;
@@ -826,16 +805,13 @@ bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
         if (!partial) slots = 1, run = a.T;   // no scratch: one chain needs none
     }
     // two segments a CTA where the row blocks have many: a CTA's start and end cost some four tiles
-    const int per = seg_keys < 512 && slots > 1 && blocks * slots >= 4 * current_device_info().sm_count ? 2 : 1;
-    const int G = static_cast<int>(a.G), D = static_cast<int>(a.dim), DV = static_cast<int>(a.vdim);
-    const bool tma = D == 64 && DV == 64 && a.block_size % kS3Keys == 0;
-    const bool on_tcgen05 = a.H == 32 && S3Layout::total(G, D, DV, tma) <= kS3Smem;   // by the model's sizes alone: a position's bits do not follow the step
-    auto kernel32 = tma ? sigmoid_talk32_kernel<true> : sigmoid_talk32_kernel<false>;
+    const int per = on_tcgen05 && slots > 1 && blocks * slots >= 4 * current_device_info().sm_count ? 2 : 1;
+    const int runs = a.block_size % kS3Keys == 0 ? 2 : 1;
     CUtensorMap map_k{}, map_v{};
-    if (on_tcgen05 && tma && (!s3_map(&map_k, a.k_cache, G) || !s3_map(&map_v, a.v_cache, G))) return false;
+    if (on_tcgen05 && (!s3_map(&map_k, a.k_cache, G, runs) || !s3_map(&map_v, a.v_cache, G, runs))) return false;
     auto kernel = a.H == 16 ? sigmoid_talk_kernel<1> : sigmoid_talk_kernel<2>;
-    const size_t smem = a.H == 16 ? StLayout<1>::total(G, D, DV) : on_tcgen05 ? S3Layout::total(G, D, DV, tma) : StLayout<2>::total(G, D, DV);
-    const cudaError_t attr = on_tcgen05 ? cudaFuncSetAttribute(kernel32, cudaFuncAttributeMaxDynamicSharedMemorySize, kS3Smem)
+    const size_t smem = a.H == 16 ? StLayout<1>::total(G, D, DV) : on_tcgen05 ? S3Layout::total(G) : StLayout<2>::total(G, D, DV);
+    const cudaError_t attr = on_tcgen05 ? cudaFuncSetAttribute(sigmoid_talk32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kS3Smem)
                                         : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
     if (attr != cudaSuccess) return hybrid::launched(attr, "sigmoid_talk_kernel");
     for (int64_t lo = 0; lo < a.T; lo += run) {
@@ -843,8 +819,8 @@ bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
         const dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>(a.B), static_cast<unsigned>((slots + per - 1) / per));
         const dim3 block(16 * static_cast<unsigned>(a.H));
         const int from = static_cast<int>(lo), to = static_cast<int>(hi), places = static_cast<int>(slots);
-        if (!hybrid::launched(on_tcgen05 ? launch_ex(kernel32, grid, block, smem, stream, map_k, map_v, a, from, to, places, per, partial, late_word())
-                                         : launch_ex(kernel, grid, block, smem, stream, a, from, to, places, per, partial),
+        if (!hybrid::launched(on_tcgen05 ? launch_ex(sigmoid_talk32_kernel, grid, block, smem, stream, map_k, map_v, a, from, to, places, per, partial, late_word())
+                                         : launch_ex(kernel, grid, block, smem, stream, a, from, to, places, partial),
                               "sigmoid_talk_kernel"))
             return false;
         if (slots > 1 && !hybrid::launched(launch_ex(sigmoid_talk_sum_kernel, dim3(static_cast<unsigned>(std::min(a.T, hi + kStRows) - lo)), dim3(256), 0, stream, a,

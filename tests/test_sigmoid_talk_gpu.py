@@ -19,6 +19,8 @@ F64 = torch.float64
     (16, 2, 48, 32, 16, ((1500, 20), (511, 2), (0, 16)), 0.0, False, 0.0),      # three segments, one that ends at a row block's last key; no cap, no slopes
     (32, 32, 16, 64, 8, ((600, 5),), 5.0, True, -10.0),                         # one head per key head; weights near 5e-5
     (16, 16, 64, 16, 16, ((0, 700),), 8.0, True, 0.0),                          # a prompt whose later rows take two segments
+    (32, 8, 64, 64, 4, ((0, 33), (1000, 17)), 30.0, True, -1.0),                # pages that hold no run of eight keys: the kernel of other head sizes
+    (32, 8, 48, 32, 16, ((0, 700), (1500, 20)), 8.0, True, -1.0),               # ... whose later rows take two segments, then three
 ])
 def test_against_float64(H, G, D, V, bs, seqs, cap, slopes, bias):
     def edit(talk):
