@@ -407,7 +407,9 @@ __device__ __forceinline__ void s3_load(void *dst, const CUtensorMap *map, uint6
 // For heads of 64 whose pages are whole runs of eight keys: a tile goes by one TMA copy each of keys and values, by two where its halves may lie in different pages.  With
 // cp.async pieces instead (1100 to 1700 cycles of issue a tile) this kernel loses on long prompts to the one above: 4000 tokens of 32 heads of 64 on 8 in pages of 8 or 4 keys 975 us
 // there, 1107 here by pieces, 862 (pages of 8) here by TMA; of 48 and 32 on 8 912 and 975; of 32 and 48 on 16 1015 and 1143.
-__global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const atoma_sigmoid_attn_args a, int lo, int hi, int slots, int per, float *__restrict__ partial, unsigned int *late_out) {
+// Segments add in pairs, the pairs in order: (s0 + s1) + (s2 + s3) + ..  per: segments a CTA takes, 1 (each has a place of its own in `partial`), 2 (a place a pair), or 0: all of its
+// rows', with a place for the first of a pair behind one for the running sum.  All give the same bits.  places: of a token.  No scratch: one chain over all keys.
+__global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const atoma_sigmoid_attn_args a, int lo, int hi, int per, int places, float *__restrict__ partial, unsigned int *late_out) {
     using L = S3Layout;
     constexpr int H = 32, NT = 512;
     extern __shared__ unsigned char sm_raw[];
@@ -424,7 +426,7 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
     if (n_q <= 0 || blk < first) return;
     const int r0 = blk * kStRows, rows = min(kStRows, n_q - r0), tok0 = t_begin + r0;
     const int ctx = static_cast<int>(a.positions[t_begin]), p0 = ctx + r0, total = ctx + n_q;
-    const int all_end = p0 + rows, j_begin = seg * kS3SegKeys, j_end = seg + per >= slots ? all_end : min(all_end, j_begin + per * kS3SegKeys);
+    const int all_end = p0 + rows, j_begin = seg * kS3SegKeys, j_end = blockIdx.z + 1 == gridDim.z ? all_end : min(all_end, j_begin + per * kS3SegKeys);
     if (j_begin >= all_end) return;
     const int32_t *bt = a.block_tables + static_cast<int64_t>(b) * a.max_blocks;
     unsigned char *talk = sm + L::t_off;
@@ -517,26 +519,36 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
     };
     clear();
     const float in = a.softcap > 0.f ? a.scale * 2.8853900817779268f / a.softcap : 0.f;   // e^(2 s / cap) = 2^(in dot)
-    bool more = false;   // a running sum waits in this token's place
-    // the sums of a segment, out of the accumulators: into its place, onto the running sum, or, where no other segment follows or precedes, out
+    // the sums of a segment, out of the accumulators: onto the first of its pair, onto the running sum, and into a place or, where no other segment follows or precedes, out
     auto put = [&](bool end) {
-        const bool out = end && (slots == 1 || all_end <= kS3SegKeys);
+        const bool second = per != 1 && (seg & 1), onto = per == 0 && seg >= 2 && (end || second), out = end && (per == 0 || all_end <= per * kS3SegKeys);
+        const int64_t row_len = static_cast<int64_t>(places) * H * DV;
+        float *mine = partial + (tok0 - lo) * row_len + (per == 0 ? (second ? 0 : H * DV) : (per == 2 ? seg >> 1 : seg) * H * DV);
+        auto each = [&](auto f) {
 #pragma unroll
-        for (int x = 0; x < 2; ++x)
+            for (int x = 0; x < 2; ++x)
 #pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                if (nt * 8 >= DV) continue;
+                for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int row = rq + 8 * e, col = (h0 + x) * DV + nt * 8 + 2 * t4;
-                    if (row >= rows) continue;
-                    float2 s = make_float2(o[x][nt][2 * e], o[x][nt][2 * e + 1]);
-                    float2 *place = reinterpret_cast<float2 *>(partial + (static_cast<int64_t>(tok0 + row - lo) * slots + seg) * H * DV + col);
-                    if (more) s = make_float2(place->x + s.x, place->y + s.y);
-                    if (out) *reinterpret_cast<uint32_t *>(static_cast<__nv_bfloat16 *>(a.out) + static_cast<int64_t>(tok0 + row) * H * DV + col) = pack2<__nv_bfloat16>(s.x, s.y);
-                    else *place = s;
-                }
-            }
+                    for (int e = 0; e < 2; ++e) {
+                        const int row = rq + 8 * e;
+                        if (row < rows) f(o[x][nt][2 * e], o[x][nt][2 * e + 1], row, (h0 + x) * DV + nt * 8 + 2 * t4);
+                    }
+        };
+        auto add = [&](const float *from) {   // all loads before the first store
+            each([&](float &u, float &v, int row, int col) {
+                const float2 f = *reinterpret_cast<const float2 *>(from + row * row_len + col);
+                u = f.x + u, v = f.y + v;
+            });
+        };
+        if (second) add(per == 0 ? mine + H * DV : mine);
+        if (onto) add(second ? mine : mine - H * DV);
+        if (out)
+            each([&](float u, float v, int row, int col) {
+                *reinterpret_cast<uint32_t *>(static_cast<__nv_bfloat16 *>(a.out) + static_cast<int64_t>(tok0 + row) * H * DV + col) = pack2<__nv_bfloat16>(u, v);
+            });
+        else
+            each([&](float u, float v, int row, int col) { *reinterpret_cast<float2 *>(mine + row * row_len + col) = make_float2(u, v); });
     };
     auto wait = [&](uint64_t *bar, uint32_t parity) {   // bounded, for a whole warp
 #pragma unroll 1
@@ -629,10 +641,9 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
                 Mma16816<__nv_bfloat16>::run(o[x][2 * n2 + 1], af, r[2], r[3]);
             }
         }
-        if (partial && j + 1 < tiles && (j_begin + (j + 1) * kS3Keys) % kS3SegKeys == 0 && (slots == 1 || seg + 1 < slots)) {   // a segment ends here
+        if (partial && j + 1 < tiles && (j_begin + (j + 1) * kS3Keys) % kS3SegKeys == 0 && (per == 0 || (per == 2 && !(seg & 1)))) {   // a segment ends here
             put(false);
-            if (slots == 1) more = true;
-            else ++seg;
+            ++seg;
             clear();
         }
     };
@@ -739,8 +750,11 @@ __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_con
     if (tid == 0 && *late && late_out) *reinterpret_cast<volatile unsigned int *>(late_out) = 1;
 }
 
-// A token's segments, in order; tokens of one segment are out already.
-__global__ void __launch_bounds__(256) sigmoid_talk_sum_kernel(const atoma_sigmoid_attn_args a, const float *__restrict__ partial, int lo, int hi, int segs, int seg_keys) {
+// A token's places of seg_keys keys each, in order, or in pairs (sigmoid_talk32_kernel); tokens of one place are out already.  AHEAD: places that a thread asks for at a time.
+// Steps of many tokens hide the latency by their CTAs; few tokens of many places are bound by it (33 tokens behind 30000 keys, 118 places of 32 heads of 64, four / sixteen at a
+// time: 51 / 16 us; 2048 tokens of eight places, the whole call 239 / 268).
+template <int AHEAD>
+__global__ void __launch_bounds__(256) sigmoid_talk_sum_kernel(const atoma_sigmoid_attn_args a, const float *__restrict__ partial, int lo, int hi, int segs, int seg_keys, int pairs) {
     pdl_launch_dependents();
     pdl_wait();
     const int64_t t = lo + static_cast<int64_t>(blockIdx.x);
@@ -749,11 +763,22 @@ __global__ void __launch_bounds__(256) sigmoid_talk_sum_kernel(const atoma_sigmo
     const int n = min(segs, (end + seg_keys - 1) / seg_keys), row = static_cast<int>(a.H * a.vdim);
     if (n < 2 || t_begin + r0 < lo || t_begin + r0 >= hi) return;
     const float *p = partial + (t - lo) * segs * row;
-    for (int i = threadIdx.x * 4; i < row; i += 1024) {
-        float4 s = *reinterpret_cast<const float4 *>(p + i);
-        for (int k = 1; k < n; ++k) {
-            const float4 v = *reinterpret_cast<const float4 *>(p + k * row + i);
-            s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
+    auto plus = [](float4 u, float4 v) { return make_float4(u.x + v.x, u.y + v.y, u.z + v.z, u.w + v.w); };
+    for (int i = (blockIdx.y * 256 + threadIdx.x) * 4; i < row; i += gridDim.y * 1024) {
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k0 = 0; k0 < n; k0 += AHEAD) {
+            float4 v[AHEAD];
+#pragma unroll
+            for (int j = 0; j < AHEAD; ++j)
+                if (k0 + j < n) v[j] = *reinterpret_cast<const float4 *>(p + static_cast<int64_t>(k0 + j) * row + i);
+#pragma unroll
+            for (int j = 0; j < AHEAD; j += 2) {
+                if (k0 + j >= n) break;
+                const bool two = k0 + j + 1 < n;
+                if (pairs && two) v[j] = plus(v[j], v[j + 1]);
+                s = k0 + j > 0 ? plus(s, v[j]) : v[j];
+                if (!pairs && two) s = plus(s, v[j + 1]);
+            }
         }
         *reinterpret_cast<uint2 *>(static_cast<__nv_bfloat16 *>(a.out) + t * row + i) = make_uint2(pack2<__nv_bfloat16>(s.x, s.y), pack2<__nv_bfloat16>(s.z, s.w));
     }
@@ -793,19 +818,32 @@ bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
     const bool on_tcgen05 = a.H == 32 && D == 64 && DV == 64 && G <= kS3Groups && a.block_size % 8 == 0;
     const int64_t seg_keys = on_tcgen05 ? kS3SegKeys : kStSegKeys, segs = std::min<int64_t>(65535, (longest + seg_keys - 1) / seg_keys), blocks = (a.T + kStRows - 1) / kStRows;
     const int64_t place = a.H * a.vdim * 4;   // bytes of a token's sums
-    int64_t slots = 1, run = a.T;
+    int64_t slots = 1, run = a.T;   // places a token; tokens a launch
+    int per = on_tcgen05 ? 0 : 1;   // sigmoid_talk32_kernel: segments a CTA
     float *partial = nullptr;
     if (segs > 1) {
         // a segment per CTA unless the row blocks are four per SM and more, or two and the segments' sums do not fit at once
         auto fits = [&](int64_t n) { return std::max<int64_t>(kStRows, kStScratch / (n * place) / kStRows * kStRows); };
-        const int64_t sms = current_device_info().sm_count;
-        slots = blocks >= 4 * sms || (blocks >= 2 * sms && fits(segs) < a.T) ? 1 : segs;
+        const int64_t sms = current_device_info().sm_count, pairs = (segs + 1) / 2, most = on_tcgen05 ? pairs : segs;
+        const bool chains = blocks >= 4 * sms || (blocks >= 2 * sms && fits(most) < a.T);
+        if (on_tcgen05) {
+            // Two of the shorter segments a CTA, and one place for both, where the row blocks have many (a CTA's start and end cost some four tiles), or where single ones do not
+            // fit at once: a bound of 16384 keys (one that the caller does not know, in a wide table), 600 and 2048 tokens, us, on single places 234 and 478, on
+            // pairs 122 and 357; of 131072 keys 801 and 3368, 435 and 1742.
+            per = chains ? 0 : (fits(segs) < a.T || blocks * segs >= 4 * sms ? 2 : 1);
+            slots = chains ? 2 : (per == 2 ? pairs : segs);
+        } else {
+            slots = chains ? 1 : segs;
+        }
         run = std::min(a.T, fits(slots));
+        if (on_tcgen05 && run < a.T) {   // runs of one length
+            const int64_t n = (a.T + run - 1) / run;
+            run = ((a.T + n - 1) / n + kStRows - 1) / kStRows * kStRows;
+        }
         partial = static_cast<float *>(try_workspace(stream, static_cast<size_t>((run + kStRows) * slots * place), kWorkspaceHybridAttn));   // a run's last row block may end behind it
-        if (!partial) slots = 1, run = a.T;   // no scratch: one chain needs none
+        if (!partial) slots = 1, run = a.T, per = on_tcgen05 ? 0 : 1;   // no scratch: one chain needs none
     }
-    // two segments a CTA where the row blocks have many: a CTA's start and end cost some four tiles
-    const int per = on_tcgen05 && slots > 1 && blocks * slots >= 4 * current_device_info().sm_count ? 2 : 1;
+    const int64_t shares = on_tcgen05 ? (per == 0 ? 1 : (segs + per - 1) / per) : slots;   // CTAs of a row block
     const int runs = a.block_size % kS3Keys == 0 ? 2 : 1;
     CUtensorMap map_k{}, map_v{};
     if (on_tcgen05 && (!s3_map(&map_k, a.k_cache, G, runs) || !s3_map(&map_v, a.v_cache, G, runs))) return false;
@@ -816,17 +854,22 @@ bool hyb_sigmoid_talk(const atoma_sigmoid_attn_args &a, cudaStream_t stream) {
     if (attr != cudaSuccess) return hybrid::launched(attr, "sigmoid_talk_kernel");
     for (int64_t lo = 0; lo < a.T; lo += run) {
         const int64_t hi = std::min(a.T, lo + run), rows = (std::min<int64_t>(hi - lo, a.max_query_len) + kStRows - 1) / kStRows + 1;
-        const dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>(a.B), static_cast<unsigned>((slots + per - 1) / per));
+        const dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>(a.B), static_cast<unsigned>(shares));
         const dim3 block(16 * static_cast<unsigned>(a.H));
         const int from = static_cast<int>(lo), to = static_cast<int>(hi), places = static_cast<int>(slots);
-        if (!hybrid::launched(on_tcgen05 ? launch_ex(sigmoid_talk32_kernel, grid, block, smem, stream, map_k, map_v, a, from, to, places, per, partial, late_word())
+        if (!hybrid::launched(on_tcgen05 ? launch_ex(sigmoid_talk32_kernel, grid, block, smem, stream, map_k, map_v, a, from, to, per, places, partial, late_word())
                                          : launch_ex(kernel, grid, block, smem, stream, a, from, to, places, partial),
                               "sigmoid_talk_kernel"))
             return false;
-        if (slots > 1 && !hybrid::launched(launch_ex(sigmoid_talk_sum_kernel, dim3(static_cast<unsigned>(std::min(a.T, hi + kStRows) - lo)), dim3(256), 0, stream, a,
-                                                    static_cast<const float *>(partial), static_cast<int>(lo), static_cast<int>(hi), static_cast<int>(slots), static_cast<int>(seg_keys)),
-                                          "sigmoid_talk_sum_kernel"))
-            return false;
+        if (shares > 1) {
+            const unsigned tokens = static_cast<unsigned>(std::min(a.T, hi + kStRows) - lo);
+            const bool few = slots >= 24 && static_cast<int>(tokens) <= 2 * current_device_info().sm_count;
+            const dim3 sums(tokens, few ? static_cast<unsigned>((place + 4095) / 4096) : 1);
+            if (!hybrid::launched(launch_ex(few ? sigmoid_talk_sum_kernel<16> : sigmoid_talk_sum_kernel<4>, sums, dim3(256), 0, stream, a, static_cast<const float *>(partial), from, to,
+                                            places, static_cast<int>(per == 2 ? 2 * seg_keys : seg_keys), on_tcgen05 && per == 1 ? 1 : 0),
+                                  "sigmoid_talk_sum_kernel"))
+                return false;
+        }
     }
     return true;
 }

@@ -106,7 +106,8 @@ void atoma_qk_norm_cache(const void *qkv, const float *bias, const float *q_weig
  *   a_g = sigmoid(s + head_bias[g]);   a'_h = sum_g talk[h, g] a_g  (talk NULL = identity)
  *   out[t, h, :] = sum_j a'_h(j) v_j[kv head of h, :]
  * Scores, weights and the sums are float32; keys are visited in position order whatever the batch looks like.  A position of a step that holds a
- * portion of two tokens or more: where its keys' sums are cut (bfloat16 heads that talk: every 512 keys) depends on its keys alone, not on what
+ * portion of two tokens or more: where its keys' sums are cut (bfloat16 heads that talk: every 256 or 512 keys, by the
+ * sizes of the heads and pages) depends on its keys alone, not on what
  * else is in the step or how its sequence was cut into steps.  A step of decoded tokens alone: the cuts follow B and max_seq_len.
  */
 typedef struct atoma_sigmoid_attn_args {

@@ -91,6 +91,8 @@ def _compare(H, G, D, V, bs, seqs, cap, slopes, bias, edit, floor):
     (32, 64, ((4000, 3),)),                        # a longer sequence beside it
     (16, 16, ((0, 4000), (0, 3000), (0, 3000))),   # a step of many tokens, whose CTAs take all segments of their rows
     (32, 64, ((20000, 900),)),                     # sums that take more than one run of tokens
+    (32, 64, ((0, 9600),)),                        # ... whose CTAs take all segments, of the shorter ones
+    (32, 48, ((0, 9600), (20000, 40))),            # the kernel of other head sizes
 ])
 def test_a_position_does_not_depend_on_the_step(H, D, others):
     """The same bits for a sequence alone, beside others, and read in two portions that end anywhere."""
@@ -105,12 +107,14 @@ def test_a_position_does_not_depend_on_the_step(H, D, others):
     q = randn_t((sum(m for _, m in seqs), H * D), 3, torch.bfloat16, DEV)
     hb, talk = randn_t((H,), 4, torch.float32, DEV), torch.eye(H, device=DEV) + randn_t((H, H), 5, torch.float32, DEV, scale=0.3)
 
-    def run(rows, seqs, table):
+    def run(rows, seqs, table, longest=None):
         pos = torch.cat([torch.arange(c, c + m) for c, m in seqs]).to(DEV)
         tseq = torch.arange(len(seqs), dtype=torch.int32).repeat_interleave(torch.tensor([m for _, m in seqs])).to(DEV)
-        return ops.sigmoid_attention_paged(rows, kc, vc, pos, tseq, table.to(DEV), None, hb, talk, H, G, D, D, bs, D ** -0.5, 8.0, max(m for _, m in seqs))
+        return ops.sigmoid_attention_paged(rows, kc, vc, pos, tseq, table.to(DEV), None, hb, talk, H, G, D, D, bs, D ** -0.5, 8.0, max(m for _, m in seqs), None, longest)
 
     alone = run(q[:n], seqs[:1], table[:1])
+    wide = torch.cat([table[:1], torch.zeros((1, 1100), dtype=torch.int32)], 1)   # ... or in a wide table, its length unknown: single segments' sums do not fit at once
+    assert torch.equal(run(q[:n], seqs[:1], wide, 0), alone)
     assert torch.equal(run(q, seqs, table)[:n], alone)
     assert torch.equal(run(q[:701], [(0, 701)], table[:1]), alone[:701])
     assert torch.equal(run(q[701:n], [(701, 600)], table[:1]), alone[701:])
@@ -159,9 +163,10 @@ def test_one_cache_as_keys_and_values(H, G, bs):
     assert torch.equal(run(kc), run(kc.clone())) and _lib.lib().atoma_kernel_timeouts() == given_up
 
 
-def test_capture_on_a_stream_without_scratch():
+@pytest.mark.parametrize("H,D", [(16, 32), (32, 64)])
+def test_capture_on_a_stream_without_scratch(H, D):
     """A long prompt captured on a stream that has run nothing: segments need scratch that cannot be had there, whole rows need none."""
-    H, G, D, bs, n = 16, 2, 32, 16, 1100
+    G, bs, n = 2, 16, 1100
     kc, vc, q = (randn_t((1104, *s), i, torch.bfloat16, DEV) for i, s in enumerate([(G, D), (G, D), (H * D,)]))
     table, pos, tseq = torch.arange(69, dtype=torch.int32, device=DEV)[None], torch.arange(n, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
     talk, hb = randn_t((H, H), 5, torch.float32, DEV), torch.zeros(H, device=DEV)
