@@ -117,9 +117,10 @@ struct StateTile {
 // one warp a scheduler is bound by what it issues.  Only where it was measured to be faster (us, shuffles in the compute warps / handed over): delta rule of 32 heads of
 // 128 x 128, 4000 and 1000 tokens 715 / 681, 184 / 176, three portions 457 / 445; state space of 64 heads of 128 x 64, 4000 tokens 508 / 473.  Eight rows a lane lose
 // (16 heads 568 / 573, state space of 32 heads 355 / 392), heads of 256 and 512 too (987 / 1161, 966 / 981), and gated linear attention, whose staging warps have the decays
-// to form (420 / 643).
-template <int KIND, int R, int PW, bool SHORT>
-constexpr bool kHandOver = !SHORT && KIND != 0 && R == 16 && PW == 8;
+// to form (420 / 643).  Float32 rows: the delta rule loses in CTAs of four warps (32 heads of 128 x 128, 4000 tokens 742 / 785, two portions of 500 199 / 209) and gains in
+// those of eight (32 portions of 40 tokens 245 / 233); the state space gains in both (64 heads of 128 x 64, 4000 tokens 606 / 488).
+template <typename T, int KIND, int R, int PW, int NW, bool SHORT>
+constexpr bool kHandOver = !SHORT && (KIND == 2 || (KIND == 1 && (sizeof(T) == 2 || NW == 8))) && R == 16 && PW == 8;
 // Read-outs of a token on their way to the staging warps: the lanes' sums, a part's columns together and the parts apart by what lets half a warp's stores hit
 // distinct banks, then what is added to the scaled sum of each column.
 template <int PW, int NW>
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
     if (n <= 0) return;
     const int jb = blockIdx.x * COLS, chunk_bytes = chunk * L::kBytes;
     using RO = ReadOut<PW, NW>;
-    constexpr bool HAND = kHandOver<KIND, R, PW, SHORT>;
+    constexpr bool HAND = kHandOver<T, KIND, R, PW, NW, SHORT>;
     [[maybe_unused]] float *read_outs = reinterpret_cast<float *>(sm + buffers * chunk_bytes);   // of two chunks
     __shared__ float2 out_scale[HAND ? 4 : 1][HAND ? 32 : 1];                          // a token's factors of its sum and of what was written: of the chunk before, in hand and next
     if (D < L::kRow || jb + COLS > V) {                          // what lies beyond dim and vdim stays zero
@@ -587,7 +588,7 @@ template <typename T, int KIND, int R, int PW, int NW, int NB, bool SHORT = fals
 cudaError_t launch_scan(const atoma_state_scan_args &a, cudaStream_t stream) {
     using L = Staged<T, KIND, R, PW, NW>;
     // staged tokens per buffer: at most 32, no more than the longest portion can have, and NB CTAs' buffers fit one SM
-    constexpr int kOutBytes = kHandOver<KIND, R, PW, SHORT> ? 2 * ReadOut<PW, NW>::kFloats * 4 : 0;
+    constexpr int kOutBytes = kHandOver<T, KIND, R, PW, NW, SHORT> ? 2 * ReadOut<PW, NW>::kFloats * 4 : 0;
     const int64_t fit = 200 * 1024 / NB / (kScanBuffers * L::kBytes + kOutBytes);
     const int chunk = SHORT ? 4 : static_cast<int>(std::max<int64_t>(4, std::min<int64_t>({32, (longest_portion(a) + 3) / 4 * 4, fit / 4 * 4})));
     const int buffers = a.T <= chunk ? 1 : kScanBuffers;   // a step of one chunk fills the first only (whatever share of it is whose: a sequence may have no token)
