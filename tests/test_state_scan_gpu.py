@@ -48,9 +48,12 @@ def test_splits_and_copies_give_the_same_bits(rule, D, V, dtype):
     assert torch.isfinite(out).all() and torch.isfinite(state).all()
     sixteen = run(rows, [0, n], 16)
     assert torch.equal(sixteen[0], out) and torch.equal(sixteen[1], state)
-    short = [torch.cat([t] + [t[:1]] * (B - 1)) for t in rows]           # the portions of the others have one token
-    wide = run(short, [0] + list(range(n, n + B)))
+    many = [torch.cat([t] + [t[:6]] * (B - 1)) for t in rows]            # six tokens each: no step of short portions, so the first one's chunks go through the CTAs of eight warps
+    wide = run(many, [0] + [n + 6 * b for b in range(B)])
     assert torch.equal(wide[0][:n], out) and torch.equal(wide[1][0], state[0])
+    short = [torch.cat([t] + [t[:1]] * (B - 1)) for t in rows]           # the portions of the others have one token: the mean is below four, short CTAs
+    few = run(short, [0] + list(range(n, n + B)))
+    assert torch.equal(few[0][:n], out) and torch.equal(few[1][0], state[0])
     for shift in (1, 2):
         padded = []
         for t in rows:
