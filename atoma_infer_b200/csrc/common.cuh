@@ -57,6 +57,7 @@ unsigned int *late_word();
 // the older pages before its grid dependency resolves).
 enum : int { kLaunchPdl = 1, kLaunchConstWeights = 2, kLaunchStableCache = 4 };
 int launch_flags();
+void set_next_mha_rows(int64_t rows);   // query rows of the call that follows on this thread, which the ABI does not carry (one-shot; 0: unknown)
 void set_next_decode_stable_cache(int v);   // per-call form of kLaunchStableCache (thread-local, one-shot)
 int take_next_decode_stable_cache();
 // "What the NEXT kernel of the stream will stream first" (the decode-step executor knows: the next GEMM's

@@ -48,7 +48,9 @@ int launch_flags() { return g_launch_flags.load(std::memory_order_relaxed); }
 // step executor, run_mha_stream_flags), consumed by the next paged-decode launch on this thread.
 namespace {
 thread_local int t_next_stable_cache = 0;
+thread_local int64_t t_next_mha_rows = 0;
 }
+void set_next_mha_rows(int64_t rows) { t_next_mha_rows = rows; }
 namespace {
 std::mutex g_trace_mu;
 unsigned long long *g_step_trace = nullptr;
@@ -246,6 +248,8 @@ void run_mha_impl(void *q_ptr, void *k_ptr, void *v_ptr, void *o_ptr, void *soft
                   float softcap, cudaStream_t stream) {
     clear_status();
     set_mha_path("none");
+    const int64_t rows_q = t_next_mha_rows;
+    t_next_mha_rows = 0;
     if (b == 0 || h == 0 || seqlen_q == 0) return;
     // The reference compiles sliding windows and soft-capping OUT (FLASHATTENTION_DISABLE_LOCAL / _SOFTCAP,
     // static_switch.h:7-11) and silently computes full attention for them.
@@ -286,6 +290,7 @@ void run_mha_impl(void *q_ptr, void *k_ptr, void *v_ptr, void *o_ptr, void *soft
     p.alibi = static_cast<const float *>(alibi_slopes_ptr);
     p.cu_q = cu_seqlens_q_ptr; p.cu_k = cu_seqlens_k_ptr; p.seqused_k = seqused_k;
     p.block_table = block_table;
+    p.rows_q = cu_seqlens_q_ptr ? rows_q : 0;
     p.q_bs = q_batch_stride; p.k_bs = k_batch_stride; p.v_bs = v_batch_stride; p.o_bs = o_batch_stride;
     p.q_rs = q_row_stride; p.k_rs = k_row_stride; p.v_rs = v_row_stride; p.o_rs = o_row_stride;
     p.q_hs = q_head_stride; p.k_hs = k_head_stride; p.v_hs = v_head_stride; p.o_hs = o_head_stride;

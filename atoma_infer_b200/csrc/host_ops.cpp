@@ -16,6 +16,10 @@
 #include <string>
 #include <vector>
 
+namespace atoma {
+void set_next_mha_rows(int64_t rows);   // flash_api.cu
+}
+
 namespace {
 
 thread_local char t_msg[1024];
@@ -550,6 +554,7 @@ extern "C" const char *atoma_mha_execute(const atoma_mha_plan *plan, void *out, 
                                          int use_legacy_stream, atoma_stream_t stream) {
     if (!out) return fail("atoma_mha_execute: output buffer is required");
     const atoma_mha_args &a = plan->args;
+    atoma::set_next_mha_rows(plan->out_rank == 3 && !plan->seqlenq_ngroups_swapped ? plan->out_shape[0] : 0);
     if (use_legacy_stream) {
         run_mha(a.q_ptr, a.k_ptr, a.v_ptr, out, softmax_lse, a.alibi_slopes_ptr, a.cu_seqlens_q_ptr,
                 a.cu_seqlens_k_ptr, a.is_seqlens_k_cumulative, a.q_batch_stride, a.k_batch_stride,

@@ -46,6 +46,7 @@
 #include "mha_params.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -388,16 +389,17 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 if (nt[t] > 0)
                     load_tile(QkPieces(), d_k, sq + t * C::kQkBytes, &map_q, &q_full[t], qg, p.q_rs, m0[t], len_q, si.q_row0 + m0[t],
                               head, si.q_batch, kL2EvictFirst);
+            const int there = EXACT ? 1 << 30 : len_k;   // gathered rows are whole tiles
             int k_issued = 0, v_issued = 0;
             if constexpr (PAGED) paged_loads(2);
             for (int j = n_lo; !PAGED && j < n_max; ++j) {
                 const int jj = j - n_lo, ks = jj % kKStages, vs = jj % kVStages;
                 if (!pf_wait_all(&k_empty[ks], ((jj / kKStages) & 1) ^ 1, late)) break;
-                load_tile(QkPieces(), d_k, sk + ks * C::kQkBytes, &map_k, &k_full[ks], kg, p.k_rs, j * kPfN, len_k,
+                load_tile(QkPieces(), d_k, sk + ks * C::kQkBytes, &map_k, &k_full[ks], kg, p.k_rs, j * kPfN, there,
                           si.k_row0 + j * kPfN, kvh, si.k_batch, kL2EvictLast);
                 ++k_issued;
                 if (!pf_wait_all(&v_empty[vs], ((jj / kVStages) & 1) ^ 1, late)) break;
-                load_tile(VPieces(), D, sv + vs * C::kVBytes, &map_v, &v_full[vs], vg, p.v_rs, j * kPfN, len_k,
+                load_tile(VPieces(), D, sv + vs * C::kVBytes, &map_v, &v_full[vs], vg, p.v_rs, j * kPfN, there,
                           si.k_row0 + j * kPfN, vh, si.k_batch, kL2EvictLast);
                 ++v_issued;
             }
@@ -716,15 +718,22 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
 }
 
-// Keys and values of a paged step into rows of their own: sequence b's from b * pitch on, all heads of a row together.  One warp per key; bound by the bytes (16-byte pieces).
+// Keys and values of a paged step into rows of their own: sequence b's from b * pitch on, all heads of a row together, and zeros up to a whole tile.  One warp per key; bound by
+// the bytes (16-byte pieces).
 constexpr int kPfGatherWarps = 8;
 __global__ void __launch_bounds__(32 * kPfGatherWarps) paged_rows_kernel(const MhaParams p, uint4 *__restrict__ k_out, uint4 *__restrict__ v_out, int pitch) {
     pdl_launch_dependents();
     pdl_wait();
     const int b = blockIdx.y, key = blockIdx.x * kPfGatherWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const PfSeq si = pf_seq(p, b);
-    if (key >= min(si.len_k, pitch) || si.len_q <= 0) return;
-    const int pg = key / p.page, per = p.d / 8, pieces = p.h_k * per;
+    const int keys = min(si.len_k, pitch), per = p.d / 8, pieces = p.h_k * per;
+    if (key >= (keys + kPfN - 1) / kPfN * kPfN || si.len_q <= 0) return;
+    if (key >= keys) {
+        const int64_t row = (static_cast<int64_t>(b) * pitch + key) * pieces;
+        for (int c = lane; c < pieces; c += 32) k_out[row + c] = v_out[row + c] = make_uint4(0, 0, 0, 0);
+        return;
+    }
+    const int pg = key / p.page;
     const int64_t page = p.block_table[static_cast<int64_t>(b) * p.bt_bs + pg], in = key - pg * p.page, row = (static_cast<int64_t>(b) * pitch + key) * pieces;
     const uint16_t *k = static_cast<const uint16_t *>(p.k) + page * p.k_bs + in * p.k_rs, *v = static_cast<const uint16_t *>(p.v) + page * p.v_bs + in * p.v_rs;
 #pragma unroll 4
@@ -809,16 +818,48 @@ bool launch_prefill(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensor
 }
 
 // A paged step whose keys and values are gathered first, so that the kernel for contiguous ones serves it, with the same bits: 1 = launched, 0 = not taken, -1 = error.
-// A tile of keys that TMA copies and one thread a row works on takes 4700 cycles, one that three warps copy and two threads a row work on 5100; the gather reads and
-// writes every key once (8 us for 5100 keys of 8 heads).  32 query heads of 128 on 8, pages / rows, us: 2048, 1500 and 531 tokens behind 0, 1003 and 37 155 / 146, 3000
-// tokens 124 / 119, 1024 behind 8000 203 / 194, 512 behind 4000 108 / 104, 256 behind 3000 80 / 78; 1024 tokens 32.8 / 33.8, 129 behind 1000 34.8 / 39.9: what is
-// short pays for the second launch.  Heads of 64 gain nothing (123 / 123, 99 / 102).
+// A tile of keys that TMA copies and one thread a row works on is faster than one that three warps copy and two threads a row work on; the gather reads and writes every key
+// of every sequence once.  So it is taken where what the tiles save is sure to pay for it (gather_pays).  Heads of 64 gain nothing (123 / 123, 99 / 102).
 constexpr int64_t kPfGatherBytes = 256ll << 20;   // of scratch at most; longer steps stay with the pages
 constexpr int kPfGatherQ = 256, kPfGatherK = 2048;
+
+// Whether the gather pays for itself however the step's rows lie on its sequences: the host knows their number, their sum (rows, or, unknown, 0: one portion is sure) and the longest
+// portion and sequence.  Saved, us, fitted to 200 steps: 0.38 a tile of keys and wave of CTAs where they fill the SMs, 0.30 a tile of the longest CTA; the gather 4 and its bytes at
+// 8 TB/s.  The least that m portions of a mean length can save: they are new prompts, or all lie behind as many keys as there can be, and the other sequences' keys are gathered for
+// one row each.
+// Pages / rows, us, of steps taken: 32 heads on 8: 2048, 1500 and 531 tokens behind 0, 1003 and 37 160.8 / 154.6, 2048, 2030 and 1 behind 0, 0 and 2502 168 / 163, 4096 205 / 190, 8192 681 / 615,
+// 1024 behind 8000 211 / 206, 256 behind 3000 88 / 85; 8 on 1: 512 behind 4000 111 / 103, 3000 78 / 78; 16 on 16: 8192 357 / 339.
+// Of steps left: 300 tokens beside seven decoded behind up to 4000 keys 168 / 179 and (8 on 1) 84 / 87, four portions of 256 behind 4000 117 / 128, 256 beside fifteen decoded behind 4095
+// 317 / 339; 16 on 16: 1024 behind 1100 62 / 67, eight of 256 behind 2000 74 / 114.
+bool gather_pays(const MhaParams &p, int sms) {
+    const double longest_q = p.seqlen_q, longest_k = std::max(p.seqlen_k, p.seqlen_q), rows = p.rows_q > 0 ? static_cast<double>(p.rows_q) : longest_q;
+    auto pays = [&](double m, double q, double c, double keys) {
+        const double blocks = std::max(1.0, q / (kQTiles * kPfM));
+        const double saved = std::max(0.30 * (q + c) / kPfN, 0.38 * m * p.h * (blocks * (blocks + 1.0) + blocks * c / kPfN) / sms);
+        return saved >= 4.0 + keys * p.h_k * p.d * 8.0 / 8e6;
+    };
+    if (p.b == 1) return pays(1.0, longest_q, longest_k - longest_q, longest_k);
+    const int most = p.rows_q > 0 ? p.b : 1;
+    for (int m = std::max(1, static_cast<int>(std::min<double>(p.b, std::ceil(rows / longest_q)))); m <= most; ++m) {
+        const double q = std::min(longest_q, rows / m), behind = std::max(0.0, longest_k - q);
+        for (const double c : {0.0, behind})
+            if (!pays(m, q, c, rows + m * c + (p.b - m) * longest_k)) return false;
+    }
+    return true;
+}
+
 int try_launch_gathered(const MhaParams &p, bool is_bf16, const CUtensorMap &mq, cudaStream_t stream) {
-    // rows for whatever a block table can name: a sequence may be longer than the caller's bound, as it may on the pages
-    const int64_t row = static_cast<int64_t>(p.h_k) * p.d, pitch = std::max<int64_t>(p.seqlen_k, p.bt_bs * p.page), bytes = static_cast<int64_t>(p.b) * pitch * row * 2;
-    if (p.d != 128 || p.seqlen_q < kPfGatherQ || p.seqlen_k < kPfGatherK || pitch > (1 << 24) || 2 * bytes > kPfGatherBytes) return 0;
+    // whole tiles of rows for whatever a block table can name: a sequence may be longer than the caller's bound, as it may on the pages
+    const int64_t row = static_cast<int64_t>(p.h_k) * p.d, named = std::max<int64_t>(p.seqlen_k, p.bt_bs * p.page), pitch = (named + kPfN - 1) / kPfN * kPfN;
+    const int64_t bytes = static_cast<int64_t>(p.b) * pitch * row * 2;
+    if (p.d != 128 || p.seqlen_q < kPfGatherQ || p.seqlen_k < kPfGatherK || named > (1 << 24) || 2 * bytes > kPfGatherBytes || !gather_pays(p, current_device_info().sm_count)) return 0;
+    // A graph may be replayed on any stream, where the scratch of the stream that it was captured on is not its own.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (capturing != cudaStreamCaptureStatusNone) return 0;
     // The copy and the kernel that reads it are enqueued together: another thread may use this stream and its scratch.
     static std::mutex together;
     std::lock_guard<std::mutex> lock(together);

@@ -51,13 +51,17 @@ def test_same_bits_whatever_the_pages(D, dtype, H, G, page, news, contexts):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("H,G,page,news,contexts", [
-    (4, 2, 16, (256,), (1792,)),                        # the shortest step that is gathered
-    (3, 1, 48, (300, 1, 33), (2100, 0, 1991)),          # pages that straddle tiles, a decoded token, a sequence shorter than a tile
-    (2, 2, 256, (1000, 640), (1100, 1408)),
+@pytest.mark.parametrize("H,G,page,news,contexts,gathered", [
+    (4, 2, 16, (256,), (1792,), True),                           # the shortest step that is gathered
+    (3, 1, 48, (300, 1, 33), (2100, 0, 1991), False),            # what so few rows save is not sure to pay for three sequences' keys
+    (2, 2, 256, (1000, 640), (1100, 1408), False),
+    (2, 1, 48, (4000, 3900, 1), (0, 100, 2500), True),           # pages that straddle tiles, a decoded token, a sequence that ends inside a tile
+    (2, 1, 16, (3000, 2950), (72, 122), True),                   # both end with a whole tile
+    (32, 32, 16, (256,), (1792,), False),                        # many key heads: the copy is the larger part
 ])
-def test_gathered_steps_give_the_bits_of_pages(dtype, H, G, page, news, contexts):
-    """A bound on the longest sequence that would take too much scratch leaves the step on its pages; rows behind a sequence's end and unused pages hold NaN."""
+def test_gathered_steps_give_the_bits_of_pages(dtype, H, G, page, news, contexts, gathered):
+    """A bound on the longest sequence that would take too much scratch leaves the step on its pages, as does a capture, whose graph may be replayed beside other work on the
+    capture's stream; rows behind a sequence's end and unused pages hold NaN."""
     D, lens = 128, [n + c for n, c in zip(news, contexts)]
     q = randn_t((sum(news), H, D), 1, dtype, DEV)
     each = [-(-n // page) for n in lens]
@@ -72,10 +76,23 @@ def test_gathered_steps_give_the_bits_of_pages(dtype, H, G, page, news, contexts
         kc.view(-1, G, D)[slot], vc.view(-1, G, D)[slot] = k[row:row + n], v[row:row + n]
         used, row = used + each[b], row + n
     starts = lambda x: torch.tensor([sum(x[:i]) for i in range(len(x) + 1)], dtype=torch.int32, device=DEV)
-    run = lambda longest: ops.flash_attn_varlen_with_block_table(q, kc, vc, None, starts(news), starts(lens), max(news), longest, D ** -0.5, None, 0, table.to(DEV))
+    args = q, kc, vc, None, starts(news), starts(lens), max(news)
+    table = table.to(DEV)
+
+    def run(longest):
+        ops.reset_launch_count()
+        return ops.flash_attn_varlen_with_block_table(*args, longest, D ** -0.5, None, 0, table)
+
     got = run(max(lens))
-    assert ops.last_mha_path() == "prefill_tc"
-    assert torch.equal(got, run(1 << 22)) and torch.equal(got, run(2048))      # 2048: a bound that some sequences exceed
+    assert ops.last_mha_path() == "prefill_tc" and ops.launch_count() == (2 if gathered else 1)      # a copy, then the products
+    assert torch.equal(got, run(1 << 22)) and ops.launch_count() == 1
+    assert torch.equal(got, run(2048))                                         # a bound that some sequences exceed
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        again = run(max(lens))
+    assert ops.launch_count() == 1
+    graph.replay()
+    assert torch.equal(got, again)
     _check(got, q, k, v, news, contexts)
     assert hybrid_ops.prefill_timeouts() == 0
 
