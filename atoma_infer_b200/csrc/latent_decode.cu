@@ -456,8 +456,9 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const atoma_latent
 
 // The runs of a sequence that several CTAs shared, in CTA order: M = max m, out = sum acc 2^(m - M) / sum l 2^(m - M).  A CTA takes 32 columns of
 // one sequence, a warp four of its heads at a time (16 bytes of a run's [column][heads] row), a lane a column.
-// Bound: latency; the runs' maxima and denominators come a lane each, beside the first eight runs' sums (one after the other: one sequence of 1024 keys, attention and
-// merge, 24.6 us for 20.5, eight of 4096 40 for 34).
+// Bound: latency.  Many runs: their maxima and denominators come a lane each, beside the first eight runs' sums (one after the other: one sequence of 1024 keys, attention and
+// merge, 24.6 us for 20.5, eight of 4096 40 for 34).  Few, as where sequences outnumber the SMs: every lane reads all of it at once, without shuffles (32 heads, 128 sequences of
+// 200 keys, attention and merge, one after the other / a lane each / so 44.9 / 52.8 / 44.2 us, 96 of 4000 122 / 128 / 120).
 template <int NH>
 __global__ void __launch_bounds__(NH * 8) latent_decode_merge_kernel(const atoma_latent_attn_args a, const float *__restrict__ partial,
                                                                      const float *__restrict__ partial_ml, const int *__restrict__ prefix, int grid) {
@@ -468,51 +469,74 @@ __global__ void __launch_bounds__(NH * 8) latent_decode_merge_kernel(const atoma
     const int units = prefix[B], ncta = min(grid, units), first = prefix[b], last = prefix[b + 1] - 1;
     if (last < first) return;
     const int c0 = ld_owner(units, first, ncta), c1 = ld_owner(units, last, ncta);
-    if (c0 == c1) return;
-    // Lane j holds run c + j's maxima and denominators of the warp's four heads; the sums' first pieces are under way meanwhile.
+    if (c0 == c1 || h0 >= H) return;   // whole warps
     const int lane = threadIdx.x & 31, runs = c1 - c0 + 1;
-    constexpr int kAhead = 8;
     const float *sums = partial + (static_cast<int64_t>(b + c0) * Rv + col) * NH + h0;
     const int64_t pitch = static_cast<int64_t>(Rv) * NH;
-    float4 v[kAhead];
-#pragma unroll
-    for (int k = 0; k < kAhead; ++k)
-        if (k < runs) v[k] = *reinterpret_cast<const float4 *>(sums + k * pitch);
     auto of_run = [&](int r) -> const float * { return partial_ml + (static_cast<int64_t>(b + c0 + min(r, runs - 1)) * NH + h0) * 2; };
     float M[4], den[4], num[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) M[i] = -INFINITY, den[i] = num[i] = 0.f;
-    for (int r = lane; r - lane < runs; r += 32) {
-        const float4 x = *reinterpret_cast<const float4 *>(of_run(r)), y = *reinterpret_cast<const float4 *>(of_run(r) + 4);
-        M[0] = fmaxf(M[0], x.x), M[1] = fmaxf(M[1], x.z), M[2] = fmaxf(M[2], y.x), M[3] = fmaxf(M[3], y.z);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) M[i] = fmaxf(M[i], __shfl_xor_sync(0xffffffffu, M[i], o));
-    for (int r0 = 0; r0 < runs; r0 += 32) {
-        const float4 x = *reinterpret_cast<const float4 *>(of_run(r0 + lane)), y = *reinterpret_cast<const float4 *>(of_run(r0 + lane) + 4);
-        const float m[4] = {x.x, x.z, y.x, y.z}, l[4] = {x.y, x.w, y.y, y.w};
-        float f[4];
+    auto highest = [&](const float4 &x, const float4 &y) { M[0] = fmaxf(M[0], x.x), M[1] = fmaxf(M[1], x.z), M[2] = fmaxf(M[2], y.x), M[3] = fmaxf(M[3], y.z); };
+    auto factors = [&](const float4 &x, const float4 &y, float (&f)[4], float (&l)[4]) {
+        const float m[4] = {x.x, x.z, y.x, y.z};
+        l[0] = x.y, l[1] = x.w, l[2] = y.y, l[3] = y.w;
 #pragma unroll
         for (int i = 0; i < 4; ++i) f[i] = exp2f(m[i] - (M[i] == -INFINITY ? 0.f : M[i]));
-        for (int k0 = 0; k0 < 32 && r0 + k0 < runs; k0 += kAhead) {
-            float4 next[kAhead];
+    };
+    constexpr int kFew = 4, kAhead = 8;
+    if (runs <= kFew) {   // every lane reads all of it at once
+        float4 v[kFew], x[kFew], y[kFew];
 #pragma unroll
-            for (int k = 0; k < kAhead; ++k)
-                if (r0 + k0 + kAhead + k < runs) next[k] = *reinterpret_cast<const float4 *>(sums + (r0 + k0 + kAhead + k) * pitch);
+        for (int k = 0; k < kFew; ++k)
+            if (k < runs) {
+                x[k] = *reinterpret_cast<const float4 *>(of_run(k)), y[k] = *reinterpret_cast<const float4 *>(of_run(k) + 4);
+                v[k] = *reinterpret_cast<const float4 *>(sums + k * pitch);
+            }
 #pragma unroll
-            for (int k = 0; k < kAhead; ++k) {
+        for (int k = 0; k < kFew; ++k)
+            if (k < runs) highest(x[k], y[k]);
+#pragma unroll
+        for (int k = 0; k < kFew; ++k)
+            if (k < runs) {
                 const float xs[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+                float f[4], l[4];
+                factors(x[k], y[k], f, l);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float fr = __shfl_sync(0xffffffffu, f[i], k0 + k), lr = __shfl_sync(0xffffffffu, l[i], k0 + k);
-                    if (r0 + k0 + k < runs && h0 + i < H) {
-                        den[i] = fmaf(lr, fr, den[i]);
-                        num[i] = fmaf(xs[i], fr, num[i]);
+                for (int i = 0; i < 4; ++i) den[i] = fmaf(l[i], f[i], den[i]), num[i] = fmaf(xs[i], f[i], num[i]);
+            }
+    } else {
+        // Lane j holds run c + j's maxima and denominators of the warp's four heads; the sums' first pieces are under way meanwhile.
+        float4 v[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (k < runs) v[k] = *reinterpret_cast<const float4 *>(sums + k * pitch);
+        for (int r = lane; r - lane < runs; r += 32) highest(*reinterpret_cast<const float4 *>(of_run(r)), *reinterpret_cast<const float4 *>(of_run(r) + 4));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) M[i] = fmaxf(M[i], __shfl_xor_sync(0xffffffffu, M[i], o));
+        for (int r0 = 0; r0 < runs; r0 += 32) {
+            float f[4], l[4];
+            factors(*reinterpret_cast<const float4 *>(of_run(r0 + lane)), *reinterpret_cast<const float4 *>(of_run(r0 + lane) + 4), f, l);
+            for (int k0 = 0; k0 < 32 && r0 + k0 < runs; k0 += kAhead) {
+                float4 next[kAhead];
+#pragma unroll
+                for (int k = 0; k < kAhead; ++k)
+                    if (r0 + k0 + kAhead + k < runs) next[k] = *reinterpret_cast<const float4 *>(sums + (r0 + k0 + kAhead + k) * pitch);
+#pragma unroll
+                for (int k = 0; k < kAhead; ++k) {
+                    const float xs[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float fr = __shfl_sync(0xffffffffu, f[i], k0 + k), lr = __shfl_sync(0xffffffffu, l[i], k0 + k);
+                        if (r0 + k0 + k < runs) {
+                            den[i] = fmaf(lr, fr, den[i]);
+                            num[i] = fmaf(xs[i], fr, num[i]);
+                        }
                     }
+                    v[k] = next[k];
                 }
-                v[k] = next[k];
             }
         }
     }
