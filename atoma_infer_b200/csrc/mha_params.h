@@ -55,7 +55,7 @@ struct MhaParams {
     // a paged step that both prompt kernels serve: attn_tile_kernel the sequences with short_for_prefill(), prefill_attn_kernel the others
     int split_short;
     int64_t rows_q;       // query rows of all sequences (0: unknown)
-    int k_batched;        // tcgen05 prefill kernel only: sequence b's keys start at b k_bs also where cu_k holds offsets; so many rows there are (0: as cu_k says)
+    int k_batched;        // tcgen05 prefill kernel on gathered keys only: sequence b's start at b k_bs also where cu_k holds offsets; so many rows there are
     unsigned int *late;   // set by the prefill kernel's launcher: where it says that a wait ran out (late_word())
 };
 

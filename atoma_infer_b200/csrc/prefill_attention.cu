@@ -179,15 +179,16 @@ struct PfSeq {
     int q_start;             // cu_q[b] or -1
 };
 
+template <bool ROWS>   // gathered keys: sequence b's start at b k_bs, and there are k_batched of them
 __device__ __forceinline__ PfSeq pf_seq(const MhaParams &p, int bidb) {
     PfSeq s;
     // reference block_info.h:14-36
     s.q_start = p.cu_q ? p.cu_q[bidb] : -1;
     s.len_q = p.cu_q ? p.cu_q[bidb + 1] - s.q_start : p.seqlen_q;
-    const int k_first = (p.cu_k && p.k_cumulative) ? p.cu_k[bidb] : -1, k_start = p.k_batched ? -1 : k_first;
+    const int k_first = (p.cu_k && p.k_cumulative) ? p.cu_k[bidb] : -1, k_start = ROWS ? -1 : k_first;
     const int len_k_cache = p.cu_k ? (p.k_cumulative ? p.cu_k[bidb + 1] - k_first : p.cu_k[bidb]) : p.seqlen_k;
     s.len_k = p.seqused_k ? p.seqused_k[bidb] : len_k_cache;
-    if (p.k_batched) s.len_k = min(s.len_k, p.k_batched);   // the rows that there are
+    if (ROWS) s.len_k = min(s.len_k, p.k_batched);   // the rows that there are
     s.q_off = s.q_start < 0 ? bidb * p.q_bs : static_cast<int64_t>(s.q_start) * p.q_rs;
     s.o_off = s.q_start < 0 ? bidb * p.o_bs : static_cast<int64_t>(s.q_start) * p.o_rs;
     s.k_off = k_start < 0 ? bidb * p.k_bs : static_cast<int64_t>(k_start) * p.k_rs;
@@ -238,7 +239,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // 154 and 242 us head by head, 105, 145 and 206 so).  Tiles behind a sequence's end leave at once.
     const int m_block = gridDim.z - 1 - blockIdx.z, head = blockIdx.x, bidb = blockIdx.y;
     pdl_wait();
-    const PfSeq si = pf_seq(p, bidb);
+    const PfSeq si = pf_seq<EXACT>(p, bidb);
     if (m_block * kQTiles * kPfM >= si.len_q || (PAGED && p.split_short && short_for_prefill(D, si.len_q, si.len_k))) return;
 
     if (tid == 0) {
@@ -725,7 +726,7 @@ __global__ void __launch_bounds__(32 * kPfGatherWarps) paged_rows_kernel(const M
     pdl_launch_dependents();
     pdl_wait();
     const int b = blockIdx.y, key = blockIdx.x * kPfGatherWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const PfSeq si = pf_seq(p, b);
+    const PfSeq si = pf_seq<false>(p, b);
     const int keys = min(si.len_k, pitch), per = p.d / 8, pieces = p.h_k * per;
     if (key >= (keys + kPfN - 1) / kPfN * kPfN || si.len_q <= 0) return;
     if (key >= keys) {
