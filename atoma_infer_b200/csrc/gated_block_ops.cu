@@ -159,7 +159,9 @@ __global__ void __launch_bounds__(kRowThreads) gated_residual_norm_kernel(const 
 
 // out[t, :] = the sum of token t's expert rows in the order k = 0 .. top - 1, in float32.  Bound: bytes (every row read once, every sum written once).  A thread takes
 // four columns (a warp's load of a row is then 256 or 512 bytes, its store 512) and asks for four rows' pieces before it adds the first, two CTAs of columns
-// a token and more.  A layer of 4000 tokens, six rows of 4096 in bfloat16 (262 MB): 988 us with a filled output that the residual kernel then adds to, 974 so; 32 tokens 289, 282.
+// a token and more.  For callers that hold no residual (hybrid_ops.moe_experts); the engine's layers sum in gated_residual_norm_kernel.  A whole layer with a filled output that the
+// residual kernel then adds to / so, us: 4000 tokens, six rows of 4096 in bfloat16, 915 / 892, four of 2048 263 / 253, two of 1024 99 / 89; one token 81 / 75, 54 / 48, 42 / 40 (L2
+// flushed; 50 layers of 1 to 4000 tokens take 0.88 to 1.03 of the time, where a layer's own spread is 2 to 5 %).
 constexpr int kSumThreads = 256;
 template <typename T>
 __global__ void __launch_bounds__(kSumThreads) expert_rows_sum_kernel(const T *__restrict__ rows, const int32_t *__restrict__ pair_row, float *__restrict__ out, int top, int width, int vec) {

@@ -6,7 +6,7 @@
 // gated activation in the epilogue, then down.  bfloat16 rows of whole 16-byte pieces: dense segments in chunks of up to 256 rows on the
 // tcgen05 CTA pairs (gemm_pair.cu); other shapes and float32: segments padded to 64-row tiles.  A row's arithmetic does not depend on which tile or segment position it lands in,
 // so a token's result is independent of the batch around it.  The token's rows are summed, in the order of k,
-// by the residual kernel (atoma_gated_residual_norm).
+// by the residual kernel (atoma_gated_residual_norm), or, for a caller without a residual, by atoma_expert_rows_sum.
 #include "common.cuh"
 #include "gemm_pair.h"
 #include "hybrid_common.cuh"

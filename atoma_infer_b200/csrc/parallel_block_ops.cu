@@ -652,7 +652,9 @@ __global__ void __launch_bounds__(256) latent_query_rope_kernel(const T *__restr
 
 // Queries of a few tokens into the latent space, their rotated part beside them: q_lat[t, h, :kv_rank] = q[t, h, :dim] . w_uk[h] and the rotation of what follows, by one
 // launch.  Bound: latency (32 tokens of 32 heads move 9 MB).  A CTA takes 32 tokens x 64 columns of one head with all of its operands in flight at once, or, the last
-// of a head, that head's rotations.  32 tokens of 32 heads of 128 + 64 on 512: a product in 64-token tiles and a rotation behind it 16.3 us a call, this 12.9.
+// of a head, that head's rotations.  32 tokens of 32 heads of 128 + 64 on 512: a product in 64-token tiles and a rotation behind it 16.3 us a call, this 12.9; with the L2 cache
+// flushed, 1, 33 and 64 tokens 19.5 / 10.3, 19.6 / 14.4, 19.5 / 14.4, of 128 heads 37.9 / 13.3, 42.0 / 20.6, 43.8 / 22.5.  4 to 128 heads of 128 or 192 + 64 and of 128 alone on 512, of 64 +
+// 32 on 256: 1 to 64 tokens take 0.3 to 0.95 of the time.
 constexpr int kAbsorbTokens = 32, kAbsorbCols = 64;
 __global__ void __launch_bounds__(128) latent_absorb_few_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat16 *__restrict__ w, const float *__restrict__ freq,
                                                                 const float *__restrict__ freq_lo, float amplitude, int pairs, int interleaved,

@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(256 * HT, 1) sigmoid_talk_kernel(const atoma_s
 //   weights  of the next tile, and values of the last one, while the mix runs; one barrier of the CTA a tile of 16 keys
 // Queries lie in tensor memory, the sums in registers; keys are copied two tiles ahead, values one.
 // Bound: latencies.  A tile takes 5500 cycles: weights 2400 (2050 of the special-function unit), values 1000, the split 700, mixed weights 600, the rest waits; 42 % of
-// the issue slots.  2048 tokens, 32 heads of 64 on 8: 283 us with the mix on mma.sync in tiles of 32 keys, 242 so.  Tried: an exponential of each weight as a polynomial 258;
+// the issue slots.  2048 tokens, 32 heads of 64 on 8: 283 us with the mix on mma.sync in tiles of 32 keys, 240 so.  Tried: an exponential of each weight as a polynomial 258;
 // sums in tensor memory and queries in registers 248; queries in shared memory and three barriers a tile 275.
 constexpr int kS3Keys = 16, kS3Tries = 1 << 18;
 struct S3Layout {
@@ -406,7 +406,7 @@ __device__ __forceinline__ void s3_load(void *dst, const CUtensorMap *map, uint6
 
 // For heads of 64 whose pages are whole runs of eight keys: a tile goes by one TMA copy each of keys and values, by two where its halves may lie in different pages.  With
 // cp.async pieces instead (1100 to 1700 cycles of issue a tile) this kernel loses on long prompts to the one above: 4000 tokens of 32 heads of 64 on 8 in pages of 8 or 4 keys 975 us
-// there, 1107 here by pieces, 862 (pages of 8) here by TMA; of 48 and 32 on 8 912 and 975; of 32 and 48 on 16 1015 and 1143.
+// there, 1107 here by pieces, 835 (pages of 8) here by TMA; of 48 and 32 on 8 912 and 975; of 32 and 48 on 16 1015 and 1143.
 // Segments add in pairs, the pairs in order: (s0 + s1) + (s2 + s3) + ..  per: segments a CTA takes, 1 (each has a place of its own in `partial`), 2 (a place a pair), or 0: all of its
 // rows', with a place for the first of a pair behind one for the running sum.  All give the same bits.  places: of a token.  No scratch: one chain over all keys.
 __global__ void __launch_bounds__(512, 1) sigmoid_talk32_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const atoma_sigmoid_attn_args a, int lo, int hi, int per, int places, float *__restrict__ partial, unsigned int *late_out) {

@@ -140,11 +140,11 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src) {
 //   q, k as projected; lengths enter as scalars: S^T khat = fk (S^T k)
 //   u = beta (v - g fk S^T k);  o = g fq S^T q + (qhat . khat) u;  S <- g S + k (fk u)
 // What bounds it: what one warp a scheduler issues for a token, some 170 instructions, 64 of them packed FMAs of two cycles, in 330 cycles; the chain alone (row sum,
-// PW-lane shuffles of 29 cycles each, write) is 215.  Delta rule, 4096 tokens of 32 heads of 128 x 128, 733 us: without the shuffles 643, the sums of S^T q 666, the
-// conversions 678; two warps of half the rows a scheduler 811.  Shared memory delivers 128 bytes a cycle to all warps of an SM.
+// PW-lane shuffles of 29 cycles each, write) is 215.  Delta rule, 4096 tokens of 32 heads of 128 x 128, 699 us; before sums were handed over 733, and of that without the
+// shuffles 643, the sums of S^T q 666, the conversions 678; two warps of half the rows a scheduler 811.  Shared memory delivers 128 bytes a cycle to all warps of an SM.
 // Rows kept as bfloat16 in shared memory and converted per warp beat float32 rows (718 us against 729, before sums were handed over, for 4096 tokens of 32 heads of 128 x 128),
 // one column a lane loses to two (924 to 1330 us).  Against one column a lane, 32 rows, rows converted and normed by the staging warps: delta
-// rule 1064 -> 729 us (that case), 504 -> 289 (16 heads, 2000 tokens); state space 794 -> 365 (32 heads of 128 x 64, 4000 tokens); gated linear
+// rule 1064 -> 729 us (that case, before sums were handed over), 504 -> 289 (16 heads, 2000 tokens); state space 794 -> 365 (32 heads of 128 x 64, 4000 tokens); gated linear
 // attention 752 -> 421 (32 heads of 64 x 128, 4000 tokens).
 // SHORT: steps of a few tokens a sequence are bound by the states, read and written once.  What counts there is bytes on their way: four CTAs an SM (no token ahead
 // in registers), and the state through shared memory in pieces of 16 bytes, since the 8 to 32 bytes of a row that a warp's columns are touch as many
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(32 * (NW + kStagers), NB) state_scan_kernel(co
             fetch_pair(reinterpret_cast<const T *>(row + L::kV) + jl, tk.va, tk.vb);
         };
         if (!SHORT) fetch(0);
-        constexpr int kUnroll = SHORT ? 1 : HAND ? (KIND == 1 ? 6 : 8) : 4;   // delta rule, handed over, 4, 5, 6, 7, 8: 725, 716, 701, 728, 711 us (16: 1148, the instruction cache)
+        constexpr int kUnroll = SHORT ? 1 : HAND ? (KIND == 1 ? 6 : 8) : 4;   // delta rule, handed over, 4, 5, 6, 7, 8: 725, 716, 701, 728, 711 us (16: 1148, the instruction cache, whose edge an edit of the loop moves: time these again then)
 #pragma unroll kUnroll
         for (int i = 0; i < nt; ++i) {
             if (SHORT) fetch(i);   // registers for more warps instead of a token ahead
