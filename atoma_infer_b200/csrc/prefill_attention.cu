@@ -833,7 +833,8 @@ constexpr int kPfGatherQ = 256, kPfGatherK = 2048;
 // Of steps left: 300 tokens beside seven decoded behind up to 4000 keys 168 / 179 and (8 on 1) 84 / 87, four portions of 256 behind 4000 117 / 128, 256 beside fifteen decoded behind 4095
 // 317 / 339; 16 on 16: 1024 behind 1100 62 / 67, eight of 256 behind 2000 74 / 114.
 bool gather_pays(const MhaParams &p, int sms) {
-    const double longest_q = p.seqlen_q, longest_k = std::max(p.seqlen_k, p.seqlen_q), rows = p.rows_q > 0 ? static_cast<double>(p.rows_q) : longest_q;
+    const double longest_q = p.rows_q > 0 ? static_cast<double>(std::min<int64_t>(p.rows_q, p.seqlen_q)) : p.seqlen_q;
+    const double longest_k = std::max<double>(p.seqlen_k, longest_q), rows = p.rows_q > 0 ? static_cast<double>(p.rows_q) : longest_q;
     auto pays = [&](double m, double q, double c, double keys) {
         const double blocks = std::max(1.0, q / (kQTiles * kPfM));
         const double saved = std::max(0.30 * (q + c) / kPfN, 0.38 * m * p.h * (blocks * (blocks + 1.0) + blocks * c / kPfN) / sms);

@@ -76,16 +76,18 @@ def test_gathered_steps_give_the_bits_of_pages(dtype, H, G, page, news, contexts
         kc.view(-1, G, D)[slot], vc.view(-1, G, D)[slot] = k[row:row + n], v[row:row + n]
         used, row = used + each[b], row + n
     starts = lambda x: torch.tensor([sum(x[:i]) for i in range(len(x) + 1)], dtype=torch.int32, device=DEV)
-    args = q, kc, vc, None, starts(news), starts(lens), max(news)
+    args = q, kc, vc, None, starts(news), starts(lens)
     table = table.to(DEV)
 
-    def run(longest):
+    def run(longest, longest_q=max(news)):
         ops.reset_launch_count()
-        return ops.flash_attn_varlen_with_block_table(*args, longest, D ** -0.5, None, 0, table)
+        return ops.flash_attn_varlen_with_block_table(*args, longest_q, longest, D ** -0.5, None, 0, table)
 
     got = run(max(lens))
     assert ops.last_mha_path() == "prefill_tc" and ops.launch_count() == (2 if gathered else 1)      # a copy, then the products
     assert torch.equal(got, run(1 << 22)) and ops.launch_count() == 1
+    if len(news) == 1:                                                         # a loose bound on the portion saves nothing
+        assert torch.equal(got, run(max(lens), max(news) + 8192)) and ops.launch_count() == (2 if gathered else 1)
     assert torch.equal(got, run(2048))                                         # a bound that some sequences exceed
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
